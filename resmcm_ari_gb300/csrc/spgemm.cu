@@ -77,9 +77,35 @@ __device__ __forceinline__ void add_shared_chk(uint32_t *p, uint32_t v, bool &ov
     const uint32_t old = atomicAdd(p, v);
     ovf |= old > 0xffffffffu - v;
 }
+// Adds to shared-memory counters.  A 64-bit shared-memory add is a
+// compare-and-swap loop; two 32-bit adds do the same work natively: the low
+// half's old value tells its carry (each wrap of the half is seen by exactly
+// one add), and the high half is touched only when there is something to
+// add to it.  Between barriers a counter's halves may disagree; it is read
+// only after one.
+// Bound by latency and occupancy around the adds, so the gain is small:
+// twelve-matrix uint64 chain of 50,000-vertex types 17.5 -> 16.9 ms, a fused
+// batch of 64 walks 14.8 -> 14.0 ms.
+__device__ __forceinline__ void add_shared(uint32_t *p, uint32_t v) { atomicAdd(p, v); }
+__device__ __forceinline__ void add_shared(uint64_t *p, uint64_t v) {
+    uint32_t *h = (uint32_t *)p;   // little endian: the low half first
+    const uint32_t lo = (uint32_t)v;
+    const uint32_t old = atomicAdd(h, lo);
+    const uint32_t hi = (uint32_t)(v >> 32) + (old > 0xffffffffu - lo ? 1u : 0u);
+    if (hi) atomicAdd(h + 1, hi);
+}
+// The high half's sum of added parts and carries wraps exactly when the
+// counter does (an added part plus carry that wraps by itself included).
 __device__ __forceinline__ void add_shared_chk(uint64_t *p, uint64_t v, bool &ovf) {
-    const unsigned long long old = atomicAdd((unsigned long long *)p, (unsigned long long)v);
-    ovf |= old > ~0ull - v;
+    uint32_t *h = (uint32_t *)p;
+    const uint32_t lo = (uint32_t)v, vh = (uint32_t)(v >> 32);
+    const uint32_t old = atomicAdd(h, lo);
+    const uint32_t hi = vh + (old > 0xffffffffu - lo ? 1u : 0u);
+    ovf |= hi < vh;
+    if (hi) {
+        const uint32_t oh = atomicAdd(h + 1, hi);
+        ovf |= oh > 0xffffffffu - hi;
+    }
 }
 
 template <typename T>
@@ -736,7 +762,6 @@ template <typename V, bool NUMERIC>
 __global__ void __launch_bounds__(kWarpWarps * 32) k_warp(DevCsr A, DevCsr B, DevCsr C, const int32_t *rows,
                                                           int32_t nrows, int64_t *cnt, int *st,
                                                           const uint8_t *bin_of) {
-    using AtomV = typename std::conditional<sizeof(V) == 4, unsigned int, unsigned long long>::type;
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ int32_t s_pre[kWarpWarps][33];
     __shared__ int64_t s_bs[kWarpWarps][32];
@@ -774,7 +799,7 @@ __global__ void __launch_bounds__(kWarpWarps * 32) k_warp(DevCsr A, DevCsr B, De
             warp_row_products<V, true, false>(A, B, a0, a1, s_pre[warp], s_bs[warp], s_va[warp], ovf,
                                               [&](int32_t c, V p) {
                                                   mark(c);
-                                                  atomicAdd((AtomV *)(acc + c), (AtomV)p);
+                                                  add_shared(acc + c, p);
                                               });
         }
         glo = __reduce_or_sync(kFull, glo);
@@ -1063,9 +1088,6 @@ __device__ __forceinline__ void stream_long(ChunkStage<V> &sg, int cnt, const De
 __device__ __forceinline__ void red_shared_add(uint32_t addr, uint32_t v) {
     asm volatile("red.shared.add.u32 [%0], %1;" ::"r"(addr), "r"(v));
 }
-__device__ __forceinline__ void red_shared_add(uint32_t addr, uint64_t v) {
-    asm volatile("red.shared.add.u64 [%0], %1;" ::"r"(addr), "l"(v));
-}
 
 // stream_long for rows that need neither overflow checks nor presence bytes:
 // add(col, product) only.  Each lane keeps one pointer pair into the B
@@ -1160,7 +1182,7 @@ __device__ __forceinline__ uint32_t hash_slot(int32_t c) {
 template <typename V, bool NUMERIC, int S>
 __device__ __forceinline__ void hash_add(V *slot, V p, bool checked, bool &ovf) {
     if (checked) add_shared_chk(slot, p, ovf);
-    else atomicAdd((typename std::conditional<sizeof(V) == 4, unsigned int, unsigned long long>::type *)slot, p);
+    else add_shared(slot, p);
 }
 
 template <typename V, bool NUMERIC, int S>
@@ -1475,7 +1497,6 @@ __global__ void __launch_bounds__(kDenseThreads) k_dense(DevCsr A, DevCsr B, Dev
     static_assert(kChunk == NT, "the dense kernel stages one A entry per thread");
     constexpr int IPT = kChunk / NT;
     constexpr int NW = NT / 32;
-    using AtomV = typename std::conditional<sizeof(V) == 4, unsigned int, unsigned long long>::type;
     extern __shared__ __align__(16) unsigned char smem[];
     // PRES = false: no presence bytes (every row's counters mark presence;
     // launched only when every value is >= 1 and no row can overflow)
@@ -1521,7 +1542,7 @@ __global__ void __launch_bounds__(kDenseThreads) k_dense(DevCsr A, DevCsr B, Dev
             if (track) present[lc] = 1;
             if (NUMERIC) {
                 if (checked) add_shared_chk(acc + lc, p, ovf);
-                else atomicAdd((AtomV *)(acc + lc), (AtomV)p);
+                else add_shared(acc + lc, p);
             }
         };
         if constexpr (NUMERIC) {
@@ -1830,7 +1851,6 @@ __global__ void __launch_bounds__(kSplitThreads) k_dense_split(DevCsr A, DevCsr 
     constexpr int NT = kSplitThreads;
     constexpr int kPull = 4;   // register accumulators per thread: rows of up to 4 * NT columns
     static_assert(kChunk == NT, "one staged A entry per thread");
-    using AtomV = typename std::conditional<sizeof(V) == 4, unsigned int, unsigned long long>::type;
     const V *Aval = (const V *)A.val;
     const V *Bval = (const V *)B.val;
     extern __shared__ __align__(16) unsigned char smem[];
@@ -1911,7 +1931,7 @@ __global__ void __launch_bounds__(kSplitThreads) k_dense_split(DevCsr A, DevCsr 
                 stream_chunk<NT, V, true>(sg, n, B, checked, ovf, [&](int32_t c, V p) {
                     if (PRES) present[c] = 1;
                     if (checked) add_shared_chk(acc + c, p, ovf);
-                    else atomicAdd((AtomV *)(acc + c), (AtomV)p);
+                    else add_shared(acc + c, p);
                 });
             } else if (checked) {
                 auto vis = [&](int32_t c, V p) {
@@ -1936,7 +1956,7 @@ __global__ void __launch_bounds__(kSplitThreads) k_dense_split(DevCsr A, DevCsr 
                 if (!done) {
                     auto vis = [&](int32_t c, V p) {
                         if (PRES) present[c] = 1;
-                        atomicAdd((AtomV *)(acc + c), (AtomV)p);
+                        add_shared(acc + c, p);
                     };
                     if (tl) stream_long_fast<V, true, false>(sg, tl, B, ovf, vis);
                     stream_chunk<NT, V, true>(sg, n, B, false, ovf, vis);
