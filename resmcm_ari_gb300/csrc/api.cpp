@@ -118,7 +118,7 @@ int32_t mat_alloc(rmcm_handle *h, int64_t rows, int64_t cols, int64_t nnz, int32
 
 void mat_release(rmcm_handle *h, rmcm_mat *m) {
     if (!m) return;
-    if (m->rowsum) dev_free(h, m->rowsum, 8 * (m->d.rows + 1) + 8 * m->d.rows);
+    if (m->rowinfo) dev_free(h, m->rowinfo, rowinfo_bytes(m));
     if (m->est_long) dev_free(h, m->est_long, 4 * (int64_t)m->n_est_long);
     if (m->xfer_done) cudaEventDestroy(m->xfer_done);
     dev_free(h, m->d.rowptr, 8 * (m->d.rows + 1));
@@ -815,9 +815,9 @@ int32_t chain_exec(rmcm_handle *h, rmcm_mat *const *mats, int32_t len, const int
                 rmcm_mat *view = new rmcm_mat(*A);
                 view->d.rowptr = A->d.rowptr + r0;
                 view->d.rows = r1 - r0;
-                view->d.rowsum = nullptr;
                 view->d.info = nullptr;
-                view->rowsum = nullptr;
+                view->d.vmax = nullptr;
+                view->rowinfo = nullptr;
                 view->est_long = nullptr;
                 view->n_est_long = -1;
                 view->xfer_done = nullptr;
@@ -830,7 +830,7 @@ int32_t chain_exec(rmcm_handle *h, rmcm_mat *const *mats, int32_t len, const int
                 rc = spgemm(h, view, B, &Cb, &fl, nullptr);
                 h->abort_on_certain_overflow = false;
                 cudaEventRecord(ev[4], s);
-                if (view->rowsum) dev_free(h, view->rowsum, 8 * (view->d.rows + 1) + 8 * view->d.rows);
+                if (view->rowinfo) dev_free(h, view->rowinfo, rowinfo_bytes(view));
                 delete view;
                 if (rc == RMCM_EOVERFLOW && widen && cur == RMCM_VAL_U32 && !Cb) {
                     rc = RMCM_OK;

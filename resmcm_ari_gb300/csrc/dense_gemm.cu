@@ -827,8 +827,8 @@ int32_t dense_part_build64(rmcm_handle *h, const DevCsr &A, const DevCsr &B, Den
     RMCM_TRY(select_heavy(h, A, B, true, hs));
     // B's largest value (row sums' last slot; 1 for a matrix of ones)
     uint64_t bmax = 1;
-    if (B.rowsum) {
-        RMCM_CUDA(h, cudaMemcpyAsync(h->h_pinned + 24, B.rowsum + B.rows, 8, cudaMemcpyDeviceToHost, h->stream));
+    if (B.vmax) {
+        RMCM_CUDA(h, cudaMemcpyAsync(h->h_pinned + 24, B.vmax, 8, cudaMemcpyDeviceToHost, h->stream));
         RMCM_CUDA(h, cudaStreamSynchronize(h->stream));
         bmax = (uint64_t)h->h_pinned[24];
     }

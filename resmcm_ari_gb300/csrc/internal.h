@@ -29,10 +29,13 @@ struct DevCsr {
     int64_t *rowptr = nullptr;
     int32_t *col = nullptr;
     void *val = nullptr;
-    const uint64_t *rowsum = nullptr;   // per-row sum of values (saturating); null when every value is 1
-    // with rowsum: per row {length, row sum saturated to 0xffffffff}, one
-    // 8-byte gather where the analysis of a uint32 product needs both
-    const uint2 *info = nullptr;
+    // per row {length, sum of its values, largest addition it can make to one
+    // column}, what the analysis of a product gathers per entry of its left
+    // operand in one sector: uint32 matrices 16 bytes, 32 bits each (sums
+    // saturated to 0xffffffff), uint64 ones 32 bytes, 64 bits each
+    // (saturated); null when every value is 1
+    const void *info = nullptr;
+    const uint64_t *vmax = nullptr;     // with info: the matrix's largest value
 };
 
 // Device-side status words, one int each (set with atomicOr, never cleared by kernels).
@@ -111,8 +114,8 @@ struct rmcm_mat {
     bool ones = false;                  // every value is 1 (leaves): row sums are row lengths
     bool positive = false;              // every value is >= 1 (a counter > 0 then marks presence)
     bool distinct = false;              // no column repeats within a row
-    uint64_t *rowsum = nullptr;         // lazily computed row sums (device, rows + 1: the largest value last), owned
-                                        // followed by `rows` uint2 {length, sum saturated to 32 bits}
+    char *rowinfo = nullptr;            // lazily computed row records (device, rowinfo_bytes), owned: see DevCsr::info;
+                                        // the largest value follows them
     int64_t max_row = -1;               // longest row (entries); -1 when unknown
     // rows longer than kEstLongRow entries, ascending (device), when known:
     // the estimator gives each a whole CTA
@@ -208,6 +211,9 @@ bool copy_out_launch(const void *const *src, void *const *dst_host, const int64_
 int32_t check_status(rmcm_handle *h);
 
 inline int64_t val_bytes(int32_t valtype) { return valtype == RMCM_VAL_U64 ? 8 : 4; }
+// Row records of a matrix and its largest value (rmcm_mat::rowinfo).
+inline int64_t rowinfo_records(const rmcm_mat *m) { return (m->valtype == RMCM_VAL_U64 ? 32 : 16) * m->d.rows; }
+inline int64_t rowinfo_bytes(const rmcm_mat *m) { return rowinfo_records(m) + 8; }
 
 // ---- kernels (host launchers) --------------------------------------------
 // spgemm.cu

@@ -47,17 +47,20 @@ namespace rmcm {
 namespace {
 
 constexpr unsigned kFull = 0xffffffffu;
-constexpr int kEmptyBin = 0x7f;   // bin code of rows with no products
-constexpr int kRiskyBit = 0x80;   // bin_of flag: the row's total count may exceed the value type
+constexpr int kBinMask = 0x0f;    // bin_of: the row's bin, and two flags
+constexpr int kEmptyBin = 0x0f;   // bin code of rows with no products
+constexpr int kNarrowBit = 0x40;  // flag (uint64 products): no count of the row exceeds 32 bits
+constexpr int kRiskyBit = 0x80;   // flag: a count of the row may exceed the value type
 
 // Shared-memory windows of the dense bin (columns per window).
 constexpr int32_t kDenseWinU32 = 40960;       // 160 KB counters + 40 KB presence bytes
 constexpr int32_t kDenseWinU64 = 22528;       // 176 KB counters + 22 KB presence bytes
 constexpr int32_t kDenseWinSym = 196608;      // presence bytes only: 192 KB
 constexpr int kDenseThreads = 512;
-// B is packed for the dense bin when the product has at least this many
-// multiply-adds per entry of B.
-constexpr int64_t kPackReuse = 64;
+// B is packed for the warp and dense bins when the product has at least this
+// many multiply-adds per entry of B (packing reads 8 or 12 bytes an entry and
+// writes 4; each use then reads 4).
+constexpr int64_t kPackReuse = 4;
 
 __device__ __forceinline__ void raise_status(int *st, int word) { atomicOr(st + word, 1); }
 
@@ -164,13 +167,6 @@ __device__ __forceinline__ unsigned long long sat_add(unsigned long long a, unsi
     return a > ~0ull - b ? ~0ull : a + b;
 }
 
-// Warp per row of A: flops and bin; per-bin row counts and the longest
-// A row of the dense bin (it sizes the cursor scratch).  It also bounds the
-// row's total count S = sum_k A[r][k] * rowsum(B[k]) (saturating): no entry
-// of the row can exceed S, so a row with S within the value type is marked
-// safe (its kernels skip the overflow checks), and a row with S greater than
-// (its possible distinct columns) x (largest value) is certain to overflow,
-// which raises *certain.
 // Per-product totals of the analysis, accumulated per CTA in shared memory
 // and added to the global words once per CTA.
 struct AnalyzeOut {
@@ -230,21 +226,23 @@ __device__ __forceinline__ void analyze_shared_flush(AnalyzeShared &sh, const An
     }
 }
 
-// Bin, overflow flags and totals of row r from its products f and its
-// saturating count bound srow.
+// Bin, overflow flags and totals of row r from its products f, its total
+// count srow and its count bound mrow (both saturating).
 template <typename V>
-__device__ __forceinline__ void analyze_row(int64_t r, int64_t f, unsigned long long srow, int64_t alen,
+__device__ __forceinline__ void analyze_row(int64_t r, int64_t f, unsigned long long srow,
+                                            unsigned long long mrow, int64_t alen,
                                             int64_t ncols, const BinParams &bp, const AnalyzeOut &o,
                                             AnalyzeShared &sh) {
     const int b = classify(f, ncols, bp);
     const unsigned long long vmax = sizeof(V) == 4 ? 0xffffffffull : ~0ull;
-    const bool risky = sizeof(V) == 4 ? srow > vmax : srow == ~0ull;
+    const bool risky = sizeof(V) == 4 ? mrow > vmax : mrow == ~0ull;
+    const bool total_over = sizeof(V) == 4 && srow > vmax;
     o.flops[r] = f;
-    o.bin_of[r] = (uint8_t)(b | (risky ? kRiskyBit : 0));
+    o.bin_of[r] = (uint8_t)(b | (risky ? kRiskyBit : 0) | (sizeof(V) == 8 && mrow <= 0xffffffffull ? kNarrowBit : 0));
     if (f) atomicAdd(&sh.flops, (unsigned long long)f);
     if (risky && b != kEmptyBin) atomicAdd(&sh.risky, 1);
-    if (sizeof(V) == 4 && risky) atomicMax(&sh.max_total, srow);
-    if (sizeof(V) == 4 && risky) {
+    if (total_over) atomicMax(&sh.max_total, srow);
+    if (total_over) {
         const unsigned long long distinct = (unsigned long long)min(f, ncols);
         if (srow == ~0ull || srow / vmax > distinct) sh.certain = 1;
     }
@@ -262,91 +260,92 @@ __device__ __forceinline__ void analyze_row(int64_t r, int64_t f, unsigned long 
     }
 }
 
-// Products and count bound of A entries [k0, k1) (strided by `step` from k0).
+// Length, value sum and largest column addition of row a of B, as the
+// analysis needs them: a uint32 matrix's saturated fields are read as 2^32
+// (upper bounds stay upper bounds, and a sum that large is past every limit
+// the total is compared with).
+struct RowRec {
+    int64_t len;
+    unsigned long long sum, top;
+};
+
 template <typename V>
-__device__ __forceinline__ void analyze_entries(const DevCsr &A, const DevCsr &B, int64_t k0, int64_t k1, int step,
-                                                int64_t &f, unsigned long long &srow) {
+__device__ __forceinline__ RowRec row_rec(const DevCsr &B, int32_t a, bool b_distinct) {
+    RowRec x;
+    if (B.info) {
+        if (sizeof(V) == 4) {
+            const uint4 q = __ldg((const uint4 *)B.info + a);
+            x.len = q.x;
+            x.sum = q.y == 0xffffffffu ? (1ull << 32) : q.y;
+            x.top = q.z == 0xffffffffu ? (1ull << 32) : q.z;
+        } else {
+            const ulonglong2 q = __ldg((const ulonglong2 *)B.info + 2 * (int64_t)a);
+            x.len = (int64_t)q.x;
+            x.sum = q.y;
+            x.top = __ldg((const unsigned long long *)B.info + 4 * (int64_t)a + 2);
+        }
+    } else {
+        // ones: a column is hit once per row unless columns repeat
+        x.len = B.rowptr[a + 1] - B.rowptr[a];
+        x.sum = (unsigned long long)x.len;
+        x.top = b_distinct ? (x.len > 0 ? 1ull : 0ull) : x.sum;
+    }
+    return x;
+}
+
+__device__ __forceinline__ unsigned long long sat_mul(unsigned long long a, unsigned long long b) {
+    return __umul64hi(a, b) ? ~0ull : a * b;
+}
+
+// Products, total count and count bound of A entries [k0, k1) (strided by
+// `step` from k0): srow = sum_k A[k] * rowsum(B[k]), the row's total count,
+// mrow = sum_k A[k] * (largest entry of B[k]), which no single count exceeds.
+// Four entries per step: their gathers are independent and overlap.
+template <typename V>
+__device__ __forceinline__ void analyze_entries(const DevCsr &A, const DevCsr &B, bool a_ones, bool b_distinct,
+                                                int64_t k0, int64_t k1, int step, int64_t &f,
+                                                unsigned long long &srow, unsigned long long &mrow) {
     const V *Aval = (const V *)A.val;
     int64_t k = k0;
-    if (sizeof(V) == 4 && B.info) {
-        // uint32: one 8-byte gather per entry (length, row sum saturated to
-        // 32 bits, read as 2^32 when saturated: the bound stays an upper
-        // bound and the exact total stays a lower one)
-        auto bsum_of = [](uint32_t s) -> unsigned long long { return s == 0xffffffffu ? (1ull << 32) : s; };
-        for (; k + 3 * (int64_t)step < k1; k += 4 * (int64_t)step) {
-            int32_t a[4];
-            unsigned long long av[4];
-#pragma unroll
-            for (int u = 0; u < 4; u++) {
-                a[u] = A.col[k + u * step];
-                av[u] = Aval[k + u * step];
-            }
-            uint2 in[4];
-#pragma unroll
-            for (int u = 0; u < 4; u++) in[u] = B.info[a[u]];
-#pragma unroll
-            for (int u = 0; u < 4; u++) {
-                f += in[u].x;
-                const unsigned long long bs = bsum_of(in[u].y);
-                const unsigned long long prod = __umul64hi(av[u], bs) ? ~0ull : av[u] * bs;
-                srow = sat_add(srow, prod);
-            }
-        }
-        for (; k < k1; k += step) {
-            const uint2 in = B.info[A.col[k]];
-            f += in.x;
-            const unsigned long long av = Aval[k], bs = bsum_of(in.y);
-            const unsigned long long prod = __umul64hi(av, bs) ? ~0ull : av * bs;
-            srow = sat_add(srow, prod);
-        }
-        return;
-    }
-    // four entries per step: their gathers are independent and overlap
     for (; k + 3 * (int64_t)step < k1; k += 4 * (int64_t)step) {
         int32_t a[4];
         unsigned long long av[4];
+        RowRec x[4];
 #pragma unroll
         for (int u = 0; u < 4; u++) {
             a[u] = A.col[k + u * step];
-            av[u] = Aval[k + u * step];
+            av[u] = a_ones ? 1ull : (unsigned long long)Aval[k + u * step];
         }
-        int64_t lo[4], hi[4];
+#pragma unroll
+        for (int u = 0; u < 4; u++) x[u] = row_rec<V>(B, a[u], b_distinct);
 #pragma unroll
         for (int u = 0; u < 4; u++) {
-            lo[u] = B.rowptr[a[u]];
-            hi[u] = B.rowptr[a[u] + 1];
-        }
-        unsigned long long bsum[4];
-#pragma unroll
-        for (int u = 0; u < 4; u++) bsum[u] = B.rowsum ? B.rowsum[a[u]] : (unsigned long long)(hi[u] - lo[u]);
-#pragma unroll
-        for (int u = 0; u < 4; u++) {
-            f += hi[u] - lo[u];
-            const unsigned long long prod = __umul64hi(av[u], bsum[u]) ? ~0ull : av[u] * bsum[u];
-            srow = sat_add(srow, prod);
+            f += x[u].len;
+            srow = sat_add(srow, sat_mul(av[u], x[u].sum));
+            mrow = sat_add(mrow, sat_mul(av[u], x[u].top));
         }
     }
     for (; k < k1; k += step) {
-        const int32_t a = A.col[k];
-        const int64_t len = B.rowptr[a + 1] - B.rowptr[a];
-        f += len;
-        const unsigned long long bsum = B.rowsum ? B.rowsum[a] : (unsigned long long)len;
-        const unsigned long long av = Aval[k];
-        const unsigned long long prod = __umul64hi(av, bsum) ? ~0ull : av * bsum;
-        srow = sat_add(srow, prod);
+        const unsigned long long av = a_ones ? 1ull : (unsigned long long)Aval[k];
+        const RowRec x = row_rec<V>(B, A.col[k], b_distinct);
+        f += x.len;
+        srow = sat_add(srow, sat_mul(av, x.sum));
+        mrow = sat_add(mrow, sat_mul(av, x.top));
     }
 }
 
 // Warp per row of A: flops and bin; per-bin row counts and the longest
-// A row of the dense bin (it sizes the cursor scratch).  It also bounds the
-// row's total count S = sum_k A[r][k] * rowsum(B[k]) (saturating): no entry
-// of the row can exceed S, so a row with S within the value type is marked
-// safe (its kernels skip the overflow checks), and a row with S greater than
-// (its possible distinct columns) x (largest value) is certain to overflow,
-// which raises *certain.  Rows with more than long_min entries are left to
-// k_analyze_long (appended to long_list) so no warp walks a huge row alone.
+// A row of the dense bin (it sizes the cursor scratch).  A row whose count
+// bound (analyze_entries) is within the value type is safe: its kernels skip
+// the overflow checks; the bound takes the largest entry of each B row, not
+// its sum, so a row is risky only when a single count may really get there.
+// A row whose total count is greater than (its possible distinct columns) x
+// (largest value) is certain to overflow, which raises *certain.  Rows with
+// more than long_min entries are left to k_analyze_long (appended to
+// long_list) so no warp walks a huge row alone.
 template <typename V>
-__global__ void __launch_bounds__(256) k_analyze(DevCsr A, DevCsr B, BinParams bp, AnalyzeOut o, int64_t long_min,
+__global__ void __launch_bounds__(256) k_analyze(DevCsr A, DevCsr B, bool a_ones, bool b_distinct, BinParams bp,
+                                                 AnalyzeOut o, int64_t long_min,
                                                  int32_t *long_list, int32_t *nlong) {
     __shared__ AnalyzeShared sh;
     analyze_shared_init(sh);
@@ -360,24 +359,34 @@ __global__ void __launch_bounds__(256) k_analyze(DevCsr A, DevCsr B, BinParams b
             continue;
         }
         int64_t f = 0;
-        unsigned long long srow = 0;
-        analyze_entries<V>(A, B, a0 + lane, a1, 32, f, srow);
+        unsigned long long srow = 0, mrow = 0;
+        analyze_entries<V>(A, B, a_ones, b_distinct, a0 + lane, a1, 32, f, srow, mrow);
         f = warp_sum(f);
 #pragma unroll
-        for (int d = 16; d > 0; d >>= 1) srow = sat_add(srow, __shfl_xor_sync(kFull, srow, d));
-        if (lane == 0) analyze_row<V>(r, f, srow, a1 - a0, B.cols, bp, o, sh);
+        for (int d = 16; d > 0; d >>= 1) {
+            srow = sat_add(srow, __shfl_xor_sync(kFull, srow, d));
+            mrow = sat_add(mrow, __shfl_xor_sync(kFull, mrow, d));
+        }
+        if (lane == 0) analyze_row<V>(r, f, srow, mrow, a1 - a0, B.cols, bp, o, sh);
     }
     __syncthreads();
     analyze_shared_flush(sh, o);
 }
 
 // Long rows: the whole grid walks each long row, CTA b taking the b-th slice
-// of its entries; partial products (int64) and count bounds (uint64, with a
-// saturation flag) meet in per-row accumulators.
+// of its entries; partial products (int64), totals and count bounds (uint64,
+// with saturation flags) meet in per-row accumulators.
+__device__ __forceinline__ void sat_accumulate(unsigned long long *acc, unsigned long long v, int32_t *sat, int flag) {
+    if (!v) return;
+    const unsigned long long old = atomicAdd(acc, v);
+    if (v == ~0ull || old > ~0ull - v) atomicOr(sat, flag);
+}
+
 template <typename V>
-__global__ void __launch_bounds__(256) k_analyze_long(DevCsr A, DevCsr B, const int32_t *long_list,
-                                                      const int32_t *nlong, unsigned long long *acc_f,
-                                                      unsigned long long *acc_s, int32_t *sat) {
+__global__ void __launch_bounds__(256) k_analyze_long(DevCsr A, DevCsr B, bool a_ones, bool b_distinct,
+                                                      const int32_t *long_list, const int32_t *nlong,
+                                                      unsigned long long *acc_f, unsigned long long *acc_s,
+                                                      unsigned long long *acc_m, int32_t *sat) {
     const int nl = *nlong;
     const int lane = threadIdx.x & 31;
     for (int j = 0; j < nl; j++) {
@@ -385,17 +394,18 @@ __global__ void __launch_bounds__(256) k_analyze_long(DevCsr A, DevCsr B, const 
         const int64_t a0 = A.rowptr[r], alen = A.rowptr[r + 1] - a0;
         const int64_t k0 = a0 + alen * blockIdx.x / gridDim.x, k1 = a0 + alen * (blockIdx.x + 1) / gridDim.x;
         int64_t f = 0;
-        unsigned long long srow = 0;
-        analyze_entries<V>(A, B, k0 + threadIdx.x, k1, blockDim.x, f, srow);
+        unsigned long long srow = 0, mrow = 0;
+        analyze_entries<V>(A, B, a_ones, b_distinct, k0 + threadIdx.x, k1, blockDim.x, f, srow, mrow);
         f = warp_sum(f);
 #pragma unroll
-        for (int d = 16; d > 0; d >>= 1) srow = sat_add(srow, __shfl_xor_sync(kFull, srow, d));
+        for (int d = 16; d > 0; d >>= 1) {
+            srow = sat_add(srow, __shfl_xor_sync(kFull, srow, d));
+            mrow = sat_add(mrow, __shfl_xor_sync(kFull, mrow, d));
+        }
         if (lane == 0) {
             if (f) atomicAdd(acc_f + j, (unsigned long long)f);
-            if (srow) {
-                const unsigned long long old = atomicAdd(acc_s + j, srow);
-                if (srow == ~0ull || old > ~0ull - srow) atomicOr(sat + j, 1);
-            }
+            sat_accumulate(acc_s + j, srow, sat + j, 1);
+            sat_accumulate(acc_m + j, mrow, sat + j, 2);
         }
     }
 }
@@ -404,170 +414,133 @@ template <typename V>
 __global__ void __launch_bounds__(256) k_analyze_long_finish(DevCsr A, DevCsr B, BinParams bp, AnalyzeOut o,
                                                              const int32_t *long_list, const int32_t *nlong,
                                                              const unsigned long long *acc_f,
-                                                             const unsigned long long *acc_s, const int32_t *sat) {
+                                                             const unsigned long long *acc_s,
+                                                             const unsigned long long *acc_m, const int32_t *sat) {
     __shared__ AnalyzeShared sh;
     analyze_shared_init(sh);
     __syncthreads();
     const int nl = *nlong;
     for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < nl; j += gridDim.x * blockDim.x) {
         const int32_t r = long_list[j];
-        const unsigned long long srow = sat[j] ? ~0ull : acc_s[j];
-        analyze_row<V>(r, (int64_t)acc_f[j], srow, A.rowptr[r + 1] - A.rowptr[r], B.cols, bp, o, sh);
+        const unsigned long long srow = (sat[j] & 1) ? ~0ull : acc_s[j], mrow = (sat[j] & 2) ? ~0ull : acc_m[j];
+        analyze_row<V>(r, (int64_t)acc_f[j], srow, mrow, A.rowptr[r + 1] - A.rowptr[r], B.cols, bp, o, sh);
     }
     __syncthreads();
     analyze_shared_flush(sh, o);
 }
 
-// Saturating row sums of a matrix's values (warp per row); out[M.rows]
-// (zeroed by the caller) receives the largest value, info[r] the row's
-// {length, sum saturated to 0xffffffff}.
+// Row records of a matrix (DevCsr::info; warp per row) and its largest value
+// (*vmax, zeroed by the caller).  The largest addition a row makes to one
+// column is its largest value, or its sum when columns may repeat in a row.
 template <typename V>
-__global__ void k_rowsum(DevCsr M, uint64_t *out, uint2 *info) {
+__global__ void k_rowinfo(DevCsr M, bool distinct, void *info, unsigned long long *vmax) {
     const int lane = threadIdx.x & 31;
     const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
     const V *v = (const V *)M.val;
-    unsigned long long vmax = 0;
+    unsigned long long all = 0;
     for (int64_t r = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; r < M.rows; r += nwarps) {
-        unsigned long long sum = 0;
-        for (int64_t q = M.rowptr[r] + lane; q < M.rowptr[r + 1]; q += 32) {
+        const int64_t q0 = M.rowptr[r], q1 = M.rowptr[r + 1];
+        unsigned long long sum = 0, top = 0;
+        for (int64_t q = q0 + lane; q < q1; q += 32) {
             const unsigned long long x = (unsigned long long)v[q];
             sum = sat_add(sum, x);
-            vmax = x > vmax ? x : vmax;
+            top = x > top ? x : top;
         }
 #pragma unroll
-        for (int d = 16; d > 0; d >>= 1) sum = sat_add(sum, __shfl_xor_sync(kFull, sum, d));
+        for (int d = 16; d > 0; d >>= 1) {
+            sum = sat_add(sum, __shfl_xor_sync(kFull, sum, d));
+            const unsigned long long o = __shfl_xor_sync(kFull, top, d);
+            top = o > top ? o : top;
+        }
+        all = top > all ? top : all;
+        if (!distinct) top = sum;
         if (lane == 0) {
-            out[r] = sum;
-            info[r] = make_uint2((uint32_t)min(M.rowptr[r + 1] - M.rowptr[r], (int64_t)0xffffffff),
-                                 sum > 0xffffffffull ? 0xffffffffu : (uint32_t)sum);
+            if (sizeof(V) == 4) {
+                ((uint4 *)info)[r] = make_uint4((uint32_t)min(q1 - q0, (int64_t)0xffffffff),
+                                                (uint32_t)min(sum, 0xffffffffull), (uint32_t)min(top, 0xffffffffull), 0);
+            } else {
+                ((ulonglong2 *)info)[2 * r] = make_ulonglong2((unsigned long long)(q1 - q0), sum);
+                ((ulonglong2 *)info)[2 * r + 1] = make_ulonglong2(top, 0);
+            }
         }
     }
-#pragma unroll
-    for (int d = 16; d > 0; d >>= 1) {
-        const unsigned long long o = __shfl_xor_sync(kFull, vmax, d);
-        vmax = o > vmax ? o : vmax;
-    }
-    if (lane == 0 && vmax) atomicMax((unsigned long long *)out + M.rows, vmax);
+    if (lane == 0 && all) atomicMax(vmax, all);
 }
 
-// Packed copy of B for the dense bin's plain path: entry q becomes
-// (value << cbits) | column at a position of its own row such that the r-th
-// entry of every shared-memory bank (column mod 32) lands in group r, groups
-// in order and banks ascending within a group.  Any 32 consecutive positions
-// then touch each bank at most twice (once per group they straddle), where
-// the sorted order puts several columns of a sparse row on one bank.  Ranks
-// within a bank follow the sorted order, so the layout is deterministic.
-// An entry's position is start[rank] + (banks below its own in group rank),
-// from per-rank tables (group masks and starts) when no bank holds more than
-// kPackRanks entries of the row, else from the bank totals directly.
-constexpr int kPackWarps = 4;
-constexpr int kPackRanks = 1024;
-
-__global__ void __launch_bounds__(kPackWarps * 32) k_pack_banked(DevCsr B, int32_t cbits, uint32_t *pk, int *st) {
-    __shared__ int32_t s_cnt[kPackWarps][32];
-    __shared__ uint32_t s_mask[kPackWarps][kPackRanks];   // banks with more than r entries
-    __shared__ int32_t s_start[kPackWarps][kPackRanks];   // first position of group r
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    int32_t *cnt = s_cnt[warp];
-    uint32_t *gmask = s_mask[warp];
-    int32_t *gstart = s_start[warp];
-    const uint32_t *bv = (const uint32_t *)B.val;
-    const unsigned lt_mask = (1u << lane) - 1u;
-    const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
-    for (int64_t r = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; r < B.rows; r += nwarps) {
-        const int64_t q0 = B.rowptr[r], q1 = B.rowptr[r + 1];
-        if (q0 == q1) continue;
-        cnt[lane] = 0;
-        __syncwarp();
-        for (int64_t q = q0 + lane; q < q1; q += 32) atomicAdd(&cnt[B.col[q] & 31], 1);
-        __syncwarp();
-        const int32_t total = cnt[lane];   // entries of bank `lane`
-        __syncwarp();
-        cnt[lane] = 0;                     // running rank per bank
-        const int32_t max_total = __reduce_max_sync(kFull, total);
-        const bool tab = max_total <= kPackRanks;
-        if (tab) {
-            int32_t run = 0;
-            for (int32_t g = 0; g < max_total; g++) {
-                const uint32_t m = __ballot_sync(kFull, total > g);
-                if (lane == 0) {
-                    gmask[g] = m;
-                    gstart[g] = run;
-                }
-                run += __popc(m);
-            }
+// Packed copy of B for the row kernels: entry q becomes
+// (value << cbits) | column, one word to load per position instead of two.
+template <typename V>
+__global__ void __launch_bounds__(256) k_pack(DevCsr B, int32_t cbits, uint32_t *pk, int *st) {
+    const V *bv = (const V *)B.val;
+    const int64_t step = (int64_t)gridDim.x * blockDim.x;
+    bool wide = false;
+    for (int64_t q0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; q0 < B.nnz; q0 += 4 * step) {
+        uint32_t c[4];
+        V x[4];
+#pragma unroll
+        for (int u = 0; u < 4; u++) {
+            const int64_t q = q0 + u * step;
+            c[u] = q < B.nnz ? (uint32_t)B.col[q] : 0u;
+            x[u] = q < B.nnz ? bv[q] : (V)0;
         }
-        __syncwarp();
-        for (int64_t base = q0; base < q1; base += 32) {
-            const int64_t q = base + lane;
-            const bool ok = q < q1;
-            const int32_t c = ok ? B.col[q] : 0;
-            const int32_t bank = ok ? (c & 31) : 32 + lane;
-            const unsigned peers = __match_any_sync(kFull, bank);
-            const int32_t rank = ok ? cnt[bank] + __popc(peers & lt_mask) : 0;
-            __syncwarp();
-            if (ok && lane == 31 - __clz(peers)) cnt[bank] += __popc(peers);
-            __syncwarp();
-            int32_t pos = 0;
-            if (tab) {
-                if (ok) pos = gstart[rank] + __popc(gmask[rank] & ((1u << bank) - 1u));
-            } else {
-                // entries before (rank, bank): min(total_b, rank) of every
-                // bank, plus one of each lower bank that reaches this rank
-#pragma unroll 8
-                for (int b = 0; b < 32; b++) {
-                    const int32_t t = __shfl_sync(kFull, total, b);
-                    pos += min(t, rank) + ((b < bank && t > rank) ? 1 : 0);
-                }
-            }
-            if (ok) {
-                const uint32_t x = bv[q];
-                // the host checked the largest value; a replay on other values would not fit
-                if (x >> (32 - cbits)) raise_status(st, kInvariant);
-                pk[q0 + pos] = (x << cbits) | (uint32_t)c;
-            }
+#pragma unroll
+        for (int u = 0; u < 4; u++) {
+            const int64_t q = q0 + u * step;
+            // the host checked the largest value; a replay on other values would not fit
+            wide |= (x[u] >> (32 - cbits)) != 0;
+            if (q < B.nnz) pk[q] = ((uint32_t)x[u] << cbits) | c[u];
         }
-        __syncwarp();
     }
+    if (wide) raise_status(st, kInvariant);
 }
 
 // Row ids into per-bin lists laid out back to back (offsets from bin_count).
-__global__ void __launch_bounds__(256) k_scatter(int64_t m, const uint8_t *bin_of, const int32_t *bin_count,
-                                                 int32_t *bin_cursor, int32_t *lists, int64_t *cnt) {
+// Rows of the dense and rank bins within a factor of eight of the bin's
+// heaviest come first in their lists: a CTA that took one of them last would
+// work on alone while the others are done.
+__global__ void __launch_bounds__(256) k_scatter(int64_t m, const uint8_t *bin_of, const int64_t *flops,
+                                                 const int32_t *bin_count, const unsigned long long *dense_max,
+                                                 const unsigned long long *rank_max, int32_t *front, int32_t *back,
+                                                 int32_t *lists, int64_t *cnt) {
     // slots are handed out per tile of 256 rows: lanes of a warp with the
     // same bin take consecutive ranks (one shared add per warp and bin), the
     // tile one global add per bin, so a million rows do not queue on a few
     // global counters
-    __shared__ int32_t off[kNumBins], s_cnt[kNumBins], s_base[kNumBins];
+    constexpr int K = 2 * kNumBins;   // per bin: heavy rows from the front, the others from the back
+    __shared__ int32_t off[kNumBins + 1], s_cnt[K], s_base[K];
     const int tid = threadIdx.x, lane = tid & 31;
     if (tid == 0) {
         int32_t s = 0;
         for (int b = 0; b < kNumBins; b++) { off[b] = s; s += bin_count[b]; }
+        off[kNumBins] = s;
     }
+    const int64_t heavy_dense = (int64_t)(*dense_max >> 3), heavy_rank = (int64_t)(*rank_max >> 3);
     for (int64_t r0 = (int64_t)blockIdx.x * 256; r0 < m; r0 += (int64_t)gridDim.x * 256) {
-        if (tid < kNumBins) s_cnt[tid] = 0;
+        if (tid < K) s_cnt[tid] = 0;
         __syncthreads();
         const int64_t r = r0 + tid;
-        int b = kEmptyBin;
+        int b = kEmptyBin, key = K;
         if (r < m) {
-            b = bin_of[r] & ~kRiskyBit;
+            b = bin_of[r] & kBinMask;
             if (b == kEmptyBin) cnt[r] = 0;   // rows without products have no entries
+            else key = 2 * b + ((b == kBinDense && flops[r] > heavy_dense) || (b == kBinRank && flops[r] > heavy_rank) ? 0 : 1);
         }
-        const unsigned peers = __match_any_sync(kFull, b);
+        const unsigned peers = __match_any_sync(kFull, key);
         const int leader = __ffs(peers) - 1;
         int32_t wbase = 0;
-        if (lane == leader && b != kEmptyBin) wbase = atomicAdd(&s_cnt[b], __popc(peers));
+        if (lane == leader && key != K) wbase = atomicAdd(&s_cnt[key], __popc(peers));
         wbase = __shfl_sync(kFull, wbase, leader);
         const int32_t rank = wbase + __popc(peers & ((1u << lane) - 1u));
         __syncthreads();
-        if (tid < kNumBins && s_cnt[tid]) s_base[tid] = atomicAdd(bin_cursor + tid, s_cnt[tid]);
+        if (tid < K && s_cnt[tid]) s_base[tid] = atomicAdd((tid & 1 ? back : front) + (tid >> 1), s_cnt[tid]);
         __syncthreads();
-        if (b != kEmptyBin) lists[off[b] + s_base[b] + rank] = (int32_t)r;
+        if (key != K) {
+            const int32_t p = s_base[key] + rank;
+            lists[key & 1 ? off[b + 1] - 1 - p : off[b] + p] = (int32_t)r;
+        }
         __syncthreads();
     }
 }
-
-
 
 // ------------------------------------------------------------------------
 // tiny bin: one warp per row, <= 32 products held one per lane
@@ -761,7 +734,7 @@ __device__ __forceinline__ void warp_row_products(const DevCsr A, const DevCsr B
 template <typename V, bool NUMERIC>
 __global__ void __launch_bounds__(kWarpWarps * 32) k_warp(DevCsr A, DevCsr B, DevCsr C, const int32_t *rows,
                                                           int32_t nrows, int64_t *cnt, int *st,
-                                                          const uint8_t *bin_of) {
+                                                          const uint8_t *bin_of, bool risky_only) {
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ int32_t s_pre[kWarpWarps][33];
     __shared__ int64_t s_bs[kWarpWarps][32];
@@ -778,6 +751,7 @@ __global__ void __launch_bounds__(kWarpWarps * 32) k_warp(DevCsr A, DevCsr B, De
     for (int64_t wi = (int64_t)blockIdx.x * kWarpWarps + warp; wi < nrows; wi += (int64_t)gridDim.x * kWarpWarps) {
         const int32_t r = rows[wi];
         const int64_t a0 = A.rowptr[r], a1 = A.rowptr[r + 1];
+        if (risky_only && !(bin_of[r] & kRiskyBit)) continue;   // k_row_warp has taken it
         const bool checked = NUMERIC && (bin_of[r] & kRiskyBit) != 0;
         uint32_t glo = 0, ghi = 0;   // 32-column groups this lane touched
         auto mark = [&](int32_t c) {
@@ -1136,7 +1110,7 @@ __device__ __forceinline__ void stream_long_plain(ChunkStage<V> &sg, int cnt, co
     }
 }
 
-// stream_long_plain over the packed copy of B (k_pack_banked): one load per
+// stream_long_plain over the packed copy of B (k_pack): one load per
 // position, column and value split from the word.
 template <typename Add>
 __device__ __forceinline__ void stream_long_packed(ChunkStage<uint32_t> &sg, int cnt, const uint32_t *pk,
@@ -1454,6 +1428,8 @@ __global__ void __launch_bounds__(NT) k_hash(DevCsr A, DevCsr B, DevCsr C, const
     if (__syncthreads_or(ovf) && tid == 0) raise_status(st, kOverflow);
 }
 
+#include "row_kernels.cuh"
+
 // ------------------------------------------------------------------------
 // dense bin: one CTA per row, windowed presence bytes + counters in shared memory
 // ------------------------------------------------------------------------
@@ -1473,35 +1449,33 @@ __global__ void __launch_bounds__(NT) k_hash(DevCsr A, DevCsr B, DevCsr C, const
 // stride `tstride` entries) and its length goes to cnt[r]; the symbolic pass
 // is skipped for these rows and k_copy_rows compacts the slots into C.
 // Per-product extras of the dense bin (single-window rows only): the packed
-// copy of B (k_pack_banked) and the tensor-core part of the product (S: the
-// dense part's counts in the product's value type, one row of gld per row of
-// A; skip[u] flags the inner indices it covers, whose A entries the kernel
-// leaves out).
+// copy of B (k_pack) and, for k_row_window, the tensor-core part of
+// the product (S: the dense part's counts in the product's value type, one
+// row of gld per row of A; row r's other entries of A are lcnt[r] from
+// rowptr[r]).
 struct DenseExtra {
     const uint32_t *pk = nullptr;
     int32_t cbits = 0;
     const void *S = nullptr;
     int64_t gld = 0;
-    const uint8_t *skip = nullptr;
-    const int32_t *lcnt = nullptr;   // with S: row r has lcnt[r] entries (A's light ones) from rowptr[r]
+    const int32_t *lcnt = nullptr;
 };
 
-template <typename V, bool NUMERIC, bool TEMP, bool PRES = true>
+template <typename V, bool NUMERIC, bool TEMP>
 __global__ void __launch_bounds__(kDenseThreads) k_dense(DevCsr A, DevCsr B, DevCsr C, const int32_t *rows,
                                                          int32_t nrows, int64_t *cnt, int32_t *cursors,
                                                          int64_t cur_stride, int32_t W, int *st, int64_t tstride,
                                                          const uint8_t *bin_of, bool positive, bool b_distinct,
-                                                         bool abort_mode, DenseExtra ex) {
+                                                         bool abort_mode, bool risky_only, bool by_row,
+                                                         DenseExtra ex) {
     constexpr int NT = kDenseThreads;
     constexpr int kPull = 4;   // register accumulators per thread: windows of up to 4 * NT columns
     static_assert(kChunk == NT, "the dense kernel stages one A entry per thread");
     constexpr int IPT = kChunk / NT;
     constexpr int NW = NT / 32;
     extern __shared__ __align__(16) unsigned char smem[];
-    // PRES = false: no presence bytes (every row's counters mark presence;
-    // launched only when every value is >= 1 and no row can overflow)
     uint8_t *present = smem;
-    V *acc = (V *)(PRES ? smem + (((size_t)W + 15) & ~(size_t)15) : smem);
+    V *acc = (V *)(smem + (((size_t)W + 15) & ~(size_t)15));
     __shared__ ChunkStage<V> sg;
     __shared__ int64_t s_warp[NW];
     __shared__ int32_t s_next;
@@ -1510,8 +1484,7 @@ __global__ void __launch_bounds__(kDenseThreads) k_dense(DevCsr A, DevCsr B, Dev
     const unsigned lt_mask = (1u << lane) - 1u;
     const V *Aval = (const V *)A.val;
     const V *Bval = (const V *)B.val;
-    if (PRES)
-        for (int i = tid; i < W / 16; i += NT) ((uint4 *)present)[i] = make_uint4(0, 0, 0, 0);
+    for (int i = tid; i < W / 16; i += NT) ((uint4 *)present)[i] = make_uint4(0, 0, 0, 0);
     if (NUMERIC)
         for (int i = tid; i < W; i += NT) acc[i] = 0;
     const bool multi = B.cols > W;
@@ -1526,12 +1499,13 @@ __global__ void __launch_bounds__(kDenseThreads) k_dense(DevCsr A, DevCsr B, Dev
             if (s_abort) break;
         }
         const int32_t r = rows[ri];
-        const int64_t a0 = A.rowptr[r], a1 = ex.lcnt ? a0 + ex.lcnt[r] : A.rowptr[r + 1];
+        if (risky_only && !(bin_of[r] & kRiskyBit)) continue;   // k_row_window has taken it
+        const int64_t a0 = A.rowptr[r], a1 = A.rowptr[r + 1];
         // A row that cannot overflow needs no checks, and when every input
         // value is >= 1 its counters alone mark presence (no count is 0).
         const bool checked = NUMERIC && (bin_of[r] & kRiskyBit) != 0;
-        const bool track = PRES && (!NUMERIC || checked || !positive);
-        const int64_t row_base = TEMP ? (int64_t)ri * tstride : (NUMERIC ? C.rowptr[r] : 0);
+        const bool track = !NUMERIC || checked || !positive;
+        const int64_t row_base = TEMP ? (int64_t)(by_row ? r : ri) * tstride : (NUMERIC ? C.rowptr[r] : 0);
         const int64_t row_end = TEMP ? row_base + tstride : (NUMERIC ? C.rowptr[r + 1] : 0);
         int64_t out = row_base;
         int64_t total = 0;
@@ -1545,14 +1519,6 @@ __global__ void __launch_bounds__(kDenseThreads) k_dense(DevCsr A, DevCsr B, Dev
                 else add_shared(acc + lc, p);
             }
         };
-        if constexpr (NUMERIC) {
-            if (ex.S) {
-                // the row's tensor-core part seeds the counters (one window)
-                const V *g = (const V *)ex.S + (int64_t)r * ex.gld;
-                for (int c = tid; c < (int)B.cols; c += NT) acc[c] = g[c];
-                __syncthreads();
-            }
-        }
         while (true) {
             const int64_t w1 = min(w0 + (int64_t)W, B.cols);
             if (tid == 0) s_next = INT_MAX;
@@ -1579,8 +1545,7 @@ __global__ void __launch_bounds__(kDenseThreads) k_dense(DevCsr A, DevCsr B, Dev
                         const int64_t k = k0 + t;
                         const int32_t a = A.col[k];
                         const int64_t bs = B.rowptr[a];
-                        // inner indices of the tensor-core part contribute through G
-                        const int64_t be = (ex.skip && ex.skip[a]) ? bs : B.rowptr[a + 1];
+                        const int64_t be = B.rowptr[a + 1];
                         int64_t lo = bs, hi = be;
                         if (multi) {
                             if (!first) lo = bs + cur[k - a0];
@@ -1892,18 +1857,23 @@ __global__ void __launch_bounds__(kSplitThreads) k_dense_split(DevCsr A, DevCsr 
         bool pulled = false;
         for (int64_t k0 = ka; k0 < kb; k0 += kChunk) {
             const int n = (int)(kb - k0 < (int64_t)kChunk ? kb - k0 : (int64_t)kChunk);
-            int64_t len1[1] = {0};
             bool full = false, lng = false;
+            int64_t own_lo = 0, own_hi = 0;   // this thread's short entry
+            V own_a = 0;
             if (tid < n) {
                 const int32_t a = A.col[k0 + tid];
                 const int64_t b0 = B.rowptr[a];
                 const int64_t len = B.rowptr[a + 1] - b0;
                 full = pull_ok && len == wc;
-                lng = sizeof(V) == 4 && !full && len >= kLongRow;   // uint64: flattened stream only
+                lng = !full && len >= kLongRow;
                 sg.bs[tid] = b0;
                 sg.len[tid] = (int32_t)len;
                 sg.va[tid] = Aval[k0 + tid];
-                len1[0] = (full || lng) ? 0 : len;
+                if (!full && !lng) {
+                    own_lo = b0;
+                    own_hi = b0 + len;
+                    own_a = sg.va[tid];
+                }
             }
             // lists of full entries (register path) and long ones (a warp each)
             const unsigned fb = __ballot_sync(kFull, full), lb = __ballot_sync(kFull, lng);
@@ -1912,7 +1882,7 @@ __global__ void __launch_bounds__(kSplitThreads) k_dense_split(DevCsr A, DevCsr 
                 sg.wl[warp] = __popc(lb);
             }
             if (tid == 0) sg.ctr = 0;
-            stage_scan<NT>(len1, sg.pre, sg.warp_tot);
+            __syncthreads();
             int pf = 0, tf = 0, pl = 0, tl = 0;
             for (int w = 0; w < NT / 32; w++) {
                 if (w < warp) {
@@ -1925,42 +1895,43 @@ __global__ void __launch_bounds__(kSplitThreads) k_dense_split(DevCsr A, DevCsr 
             if (full) sg.flist[pf + __popc(fb & lt_mask)] = tid;
             if (lng) sg.llist[pl + __popc(lb & lt_mask)] = tid;
             __syncthreads();
-            // the row's overflow test is chosen here, not per product (uint64
-            // keeps the single flattened stream: the split costs it spills)
-            if constexpr (sizeof(V) == 8) {
-                stream_chunk<NT, V, true>(sg, n, B, checked, ovf, [&](int32_t c, V p) {
-                    if (PRES) present[c] = 1;
-                    if (checked) add_shared_chk(acc + c, p, ovf);
-                    else add_shared(acc + c, p);
-                });
-            } else if (checked) {
+            // the row's overflow test is chosen here, not per product; short
+            // entries are added by the thread that staged them
+            if (checked) {
                 auto vis = [&](int32_t c, V p) {
                     if (PRES) present[c] = 1;
                     add_shared_chk(acc + c, p, ovf);
                 };
                 if (tl) stream_long_fast<V, true, true>(sg, tl, B, ovf, vis);
-                stream_chunk<NT, V, true>(sg, n, B, true, ovf, vis);
+                for (int64_t q = own_lo; q < own_hi; q++) vis(__ldg(B.col + q), mul_chk(own_a, __ldg(Bval + q), ovf));
             } else {
-                bool done = false;
-                if constexpr (sizeof(V) == 4 && !PRES) {
-                    // uint32 counters alone: 32-bit shared addresses, packed B when given
-                    const uint32_t acc_s = (uint32_t)__cvta_generic_to_shared(acc);
-                    auto add = [&](int32_t c, V p) { red_shared_add(acc_s + (uint32_t)c * 4u, p); };
-                    if (tl) {
-                        if (pk) stream_long_packed(sg, tl, pk, cbits, add);
-                        else stream_long_fast<V, true, false>(sg, tl, B, ovf, add);
+                auto vis = [&](int32_t c, V p) {
+                    if (PRES) present[c] = 1;
+                    add_shared(acc + c, p);
+                };
+                if (tl) {
+                    bool done = false;
+                    if constexpr (sizeof(V) == 4 && !PRES) {
+                        if (pk) {
+                            stream_long_packed(sg, tl, pk, cbits, vis);
+                            done = true;
+                        }
                     }
-                    stream_chunk<NT, V, true>(sg, n, B, false, ovf, add);
-                    done = true;
+                    if (!done) stream_long_fast<V, true, false>(sg, tl, B, ovf, vis);
                 }
-                if (!done) {
-                    auto vis = [&](int32_t c, V p) {
-                        if (PRES) present[c] = 1;
-                        add_shared(acc + c, p);
-                    };
-                    if (tl) stream_long_fast<V, true, false>(sg, tl, B, ovf, vis);
-                    stream_chunk<NT, V, true>(sg, n, B, false, ovf, vis);
+                int64_t q = own_lo;
+                for (; q + 3 < own_hi; q += 4) {
+                    int32_t c[4];
+                    V v[4];
+#pragma unroll
+                    for (int u = 0; u < 4; u++) {
+                        c[u] = __ldg(B.col + q + u);
+                        v[u] = __ldg(Bval + q + u);
+                    }
+#pragma unroll
+                    for (int u = 0; u < 4; u++) vis(c[u], (V)(own_a * v[u]));
                 }
+                for (; q < own_hi; q++) vis(__ldg(B.col + q), (V)(own_a * __ldg(Bval + q)));
             }
             for (int i0 = 0; i0 < tf; i0 += 4) {
                 pulled = true;
@@ -2444,7 +2415,7 @@ __global__ void __launch_bounds__(kRankThreads) k_rank_split_val(DevCsr A, DevCs
 __global__ void k_short_cap(int64_t m, const uint8_t *bin_of, const int64_t *flops, int64_t cols, uint32_t mask,
                             int64_t *cap) {
     for (int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r < m; r += (int64_t)gridDim.x * blockDim.x) {
-        const int b = bin_of[r] & ~kRiskyBit;
+        const int b = bin_of[r] & kBinMask;
         cap[r] = (b != kEmptyBin && ((mask >> b) & 1u)) ? (flops[r] < cols ? flops[r] : cols) : 0;
     }
 }
@@ -2459,7 +2430,7 @@ __global__ void __launch_bounds__(256) k_copy_short(int64_t m, const uint8_t *bi
     const int lane = threadIdx.x & 31;
     const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
     for (int64_t r = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; r < m; r += nw) {
-        const int b = bin_of[r] & ~kRiskyBit;
+        const int b = bin_of[r] & kBinMask;
         if (b == kEmptyBin || !((mask >> b) & 1u)) continue;
         const int64_t d0 = C.rowptr[r], len = C.rowptr[r + 1] - d0, s0 = trow[r];
         for (int64_t i0 = lane; i0 < len; i0 += 128) {
@@ -2485,20 +2456,16 @@ __global__ void __launch_bounds__(256) k_copy_short(int64_t m, const uint8_t *bi
     }
 }
 
-__global__ void k_iota(int32_t *v, int32_t n) {
-    for (int32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) v[i] = i;
-}
-
 // Compacts TEMP-mode slots into C: row rows[ri] has cnt = rowptr[r+1]-rowptr[r]
-// entries at slot ri of the temporary.
+// entries at slot ri of the temporary (its own number with by_row).
 template <typename V>
 __global__ void __launch_bounds__(256) k_copy_rows(const int32_t *rows, int32_t nrows, DevCsr C, const int32_t *tcol,
-                                                   const V *tval, int64_t tstride) {
+                                                   const V *tval, int64_t tstride, bool by_row) {
     for (int32_t ri = blockIdx.x; ri < nrows; ri += gridDim.x) {
         const int32_t r = rows[ri];
         const int64_t b = C.rowptr[r], n = C.rowptr[r + 1] - b;
-        const int32_t *sc = tcol + (int64_t)ri * tstride;
-        const V *sv = tval + (int64_t)ri * tstride;
+        const int32_t *sc = tcol + (int64_t)(by_row ? r : ri) * tstride;
+        const V *sv = tval + (int64_t)(by_row ? r : ri) * tstride;
         for (int64_t i = threadIdx.x; i < n; i += blockDim.x) {
             C.col[b + i] = sc[i];
             ((V *)C.val)[b + i] = sv[i];
@@ -2692,7 +2659,9 @@ struct DenseTemp {
     int64_t stride = 0;
     int64_t bytes = 0, vbytes = 0;   // the two allocations (columns, counts)
     bool no_risky = false;            // no row can overflow: with positive inputs, no presence bytes
-    // packed copy of B (k_pack_banked) for the plain path of single-window rows
+    int32_t *next_row = nullptr;      // device counter of k_row_window, zero
+    bool by_row = false;              // slots are numbered by row, not by place in the list
+    // packed copy of B (k_pack) for the plain path of single-window rows
     const uint32_t *pk = nullptr;
     int32_t cbits = 0;
     void *pk_mem = nullptr;
@@ -2731,7 +2700,7 @@ struct RankSplit {
 };
 
 // Rows with fewer products than this are never split.
-constexpr int64_t kSplitMinFlops = 1 << 20;
+constexpr int64_t kSplitMinFlops = 1 << 17;
 constexpr int64_t kSplitMinLight = 1 << 18;   // light products of rows beside a tensor-core part
 
 // A rows with more entries than this are analysed by the whole grid.
@@ -2752,11 +2721,45 @@ DenseExtra dense_extra(const DenseTemp *t, bool single_pass) {
     return e;
 }
 
+// Operands of the row kernels (row_kernels.cuh), for the products they take.
+template <typename V>
+struct LeanArgs {
+    const V *aval;     // null: A holds ones
+    RowB<V> B;
+};
+
+// Dense-bin rows, one window wide, into the row-padded temporary T
+// (k_row_window).  As many threads per CTA as fill an SM with the CTAs its
+// shared memory holds: narrow windows run many small CTAs (a row of a few
+// dozen entries cannot feed 16 warps), a window that leaves room for one CTA
+// runs 1024 threads.
+template <typename V>
+int32_t launch_row_window(rmcm_handle *h, const DevCsr &A, const V *aval, const RowB<V> &B, const DevCsr &T,
+                          const int32_t *rows, int32_t n, int64_t tstride, int64_t ncols, int64_t *cnt,
+                          const uint8_t *bin_of, const DenseExtra &ex, int32_t *next_row, bool by_row) {
+    const int32_t W = (int32_t)((ncols + 127) / 128 * 128);
+    const int64_t sm = (int64_t)W * sizeof(V);
+    auto go = [&](auto kern, int nt) -> int32_t {
+        RMCM_TRY(set_smem(h, kern, sm));
+        const int per_sm = std::max(1, occupancy(h, kern, nt, sm));
+        const int grid = (int)std::min<int64_t>((int64_t)n, (int64_t)h->sm_count * per_sm);
+        kern<<<grid, nt, sm, h->stream>>>(A, aval, B, T, rows, n, tstride, W, (int32_t)ncols, cnt, bin_of,
+                                          (const V *)ex.S, ex.gld, ex.lcnt, next_row, by_row);
+        return RMCM_OK;
+    };
+    const int64_t per_sm = (n + h->sm_count - 1) / h->sm_count;   // rows an SM gets
+    const bool pk = B.words != nullptr;
+    if (sm <= 16 * 1024 && per_sm >= 8) return go(pk ? k_row_window<V, 128, true> : k_row_window<V, 128, false>, 128);
+    if (sm <= 40 * 1024 && per_sm >= 4) return go(pk ? k_row_window<V, 256, true> : k_row_window<V, 256, false>, 256);
+    if (sm <= 88 * 1024 && per_sm >= 2) return go(pk ? k_row_window<V, 512, true> : k_row_window<V, 512, false>, 512);
+    return go(pk ? k_row_window<V, 1024, true> : k_row_window<V, 1024, false>, 1024);
+}
+
 template <typename V, bool NUMERIC>
 int32_t launch_bins(rmcm_handle *h, const DevCsr &A, const DevCsr &B, const DevCsr &C, const int32_t *lists,
                     const int32_t *counts, int32_t dense_max_alen, int64_t *cnt, int32_t *cursor_base,
                     int64_t cursor_cap, const DenseTemp *temp, const uint8_t *bin_of, bool positive,
-                    bool b_distinct, const RankSplit *rs, uint32_t bin_mask = ~0u) {
+                    bool b_distinct, const RankSplit *rs, const LeanArgs<V> *lean, uint32_t bin_mask = ~0u) {
     cudaStream_t s = h->stream;
     int *st = h->d_status;
     int32_t off = 0;
@@ -2769,12 +2772,23 @@ int32_t launch_bins(rmcm_handle *h, const DevCsr &A, const DevCsr &B, const DevC
         if (n == 0 || !((bin_mask >> b) & 1u)) continue;
         switch (b) {
             case kBinWarp: {
+                if (NUMERIC && lean) {
+                    const int32_t W = (int32_t)((ncols + 127) / 128 * 128);
+                    const int64_t sm = (int64_t)kWarpWarps * W * sizeof(V);
+                    auto kern = lean->B.words ? k_row_warp<V, true> : k_row_warp<V, false>;
+                    RMCM_TRY(set_smem(h, kern, sm));
+                    const int per_sm = std::max(1, occupancy(h, kern, kWarpWarps * 32, sm));
+                    const int grid = grid_for(h, (int64_t)n * 32, kWarpWarps * 32, per_sm);
+                    kern<<<grid, kWarpWarps * 32, sm, s>>>(A, lean->aval, lean->B, C, list, n, W, cnt, bin_of, st);
+                    if (temp->no_risky) break;
+                    h->launches++;
+                }
                 const int64_t sm = (int64_t)kWarpWarps * (kWarpCols + (NUMERIC ? (int64_t)kWarpCols * sizeof(V) : 0));
                 auto kern = k_warp<V, NUMERIC>;
                 RMCM_TRY(set_smem(h, kern, sm));
                 const int per_sm = std::max(1, occupancy(h, kern, kWarpWarps * 32, sm));
                 const int grid = grid_for(h, (int64_t)n * 32, kWarpWarps * 32, per_sm);
-                kern<<<grid, kWarpWarps * 32, sm, s>>>(A, B, C, list, n, cnt, st, bin_of);
+                kern<<<grid, kWarpWarps * 32, sm, s>>>(A, B, C, list, n, cnt, st, bin_of, NUMERIC && lean != nullptr);
                 break;
             }
             case kBinTiny: {
@@ -2866,21 +2880,8 @@ int32_t launch_bins(rmcm_handle *h, const DevCsr &A, const DevCsr &B, const DevC
                     if (!NUMERIC) {
                         // one pass: columns + counts into the padded slots, lengths to cnt
                         const int64_t W = (ncols + 31) / 32 * 32;
-                        // every value >= 1 and no row able to overflow: the
-                        // counters alone mark presence, so the window holds only
-                        // them (a smaller CTA, more of them per SM)
-                        const int64_t sm_full = ((W + 15) & ~15LL) + W * (int64_t)sizeof(V);
-                        const int64_t sm_lite = W * (int64_t)sizeof(V);
-                        bool lite = false;
-                        if (positive && temp->no_risky) {
-                            RMCM_TRY(set_smem(h, k_dense<V, true, true>, sm_full));
-                            RMCM_TRY(set_smem(h, k_dense<V, true, true, false>, sm_lite));
-                            // only where dropping the bytes fits more CTAs per SM
-                            lite = occupancy(h, k_dense<V, true, true, false>, kDenseThreads, sm_lite) >
-                                   occupancy(h, k_dense<V, true, true>, kDenseThreads, sm_full);
-                        }
-                        const int64_t sm = lite ? sm_lite : sm_full;
-                        auto kern = lite ? k_dense<V, true, true, false> : k_dense<V, true, true>;
+                        const int64_t sm_lite = W * (int64_t)sizeof(V), sm = ((W + 15) & ~15LL) + sm_lite;
+                        auto kern = k_dense<V, true, true>;
                         RMCM_TRY(set_smem(h, kern, sm));
                         const int per_sm = (int)std::max<int64_t>(1, std::min<int64_t>(4, (200 * 1024) / std::max<int64_t>(sm, 1)));
                         const int grid = (int)std::min<int64_t>((int64_t)n, (int64_t)h->sm_count * per_sm);
@@ -2896,7 +2897,7 @@ int32_t launch_bins(rmcm_handle *h, const DevCsr &A, const DevCsr &B, const DevC
                         if (temp->split) {
                             // the split rows run on the second stream, beside the dense bin
                             const bool slite = positive && temp->no_risky;
-                            const int64_t ssm = slite ? sm_lite : sm_full;
+                            const int64_t ssm = slite ? sm_lite : sm;
                             auto ks = slite ? k_dense_split<V, false> : k_dense_split<V, true>;
                             RMCM_TRY(set_smem(h, ks, ssm));
                             RMCM_CUDA(h, cudaEventRecord(h->ev_fork, s));
@@ -2917,10 +2918,17 @@ int32_t launch_bins(rmcm_handle *h, const DevCsr &A, const DevCsr &B, const DevC
                         // kernel takes its front
                         const int32_t *dl = temp->split ? temp->perm : list;
                         const int32_t dn = temp->split ? temp->n_front : n;
-                        if (dn > 0)
+                        if (dn > 0 && lean)
+                            RMCM_TRY(launch_row_window<V>(h, Al, temp->dpart.S ? (const V *)Al.val : lean->aval,
+                                                          lean->B, T, dl, dn, temp->stride, ncols, cnt, bin_of,
+                                                          dense_extra(temp, true), temp->next_row, temp->by_row));
+                        if (dn > 0 && (!lean || !temp->no_risky)) {
                             kern<<<std::max(1, std::min(grid, dn)), kDenseThreads, sm, s>>>(
                                 Al, B, T, dl, dn, cnt, nullptr, 0, (int32_t)W, st, temp->stride, bin_of, positive,
-                                b_distinct, h->abort_on_certain_overflow, dense_extra(temp, true));
+                                b_distinct, h->abort_on_certain_overflow, lean != nullptr, temp->by_row,
+                                dense_extra(temp, true));
+                            if (lean) h->launches++;
+                        }
                         if (temp->split) {
                             RMCM_CUDA(h, cudaEventRecord(h->ev_join, h->aux));
                             RMCM_CUDA(h, cudaStreamWaitEvent(s, h->ev_join, 0));
@@ -2928,7 +2936,7 @@ int32_t launch_bins(rmcm_handle *h, const DevCsr &A, const DevCsr &B, const DevC
                     } else {
                         const int grid = (int)std::min<int64_t>((int64_t)n, (int64_t)h->sm_count * 8);
                         k_copy_rows<V><<<grid, 256, 0, s>>>(temp->split ? temp->perm : list, n, C, temp->col,
-                                                             (const V *)temp->val, temp->stride);
+                                                             (const V *)temp->val, temp->stride, temp->by_row);
                     }
                     break;
                 }
@@ -2946,7 +2954,7 @@ int32_t launch_bins(rmcm_handle *h, const DevCsr &A, const DevCsr &B, const DevC
                     grid = (int)std::max<int64_t>(1, cursor_cap / stride);
                 }
                 kern<<<grid, kDenseThreads, sm, s>>>(A, B, C, list, n, cnt, cursor_base, stride, (int32_t)W, st, 0, bin_of,
-                                                     positive, b_distinct, h->abort_on_certain_overflow,
+                                                     positive, b_distinct, h->abort_on_certain_overflow, false, false,
                                                      NUMERIC && !multi ? dense_extra(temp, false) : DenseExtra{});
                 break;
             }
@@ -2985,20 +2993,20 @@ int32_t spgemm_t(rmcm_handle *h, const rmcm_mat *Am, const rmcm_mat *Bm, rmcm_ma
     cudaStream_t s = h->stream;
     const bool replay = plan && plan->mode == 2;
     const bool record = plan && plan->mode == 1;
-    // row sums of B bound the counts of every output row (computed once per matrix)
-    if (!Bm->ones && !Bm->rowsum && Bm->d.rows > 0) {
+    // row records of B bound the counts of every output row (computed once per matrix)
+    if (!Bm->ones && !Bm->rowinfo && Bm->d.rows > 0) {
         rmcm_mat *Bw = const_cast<rmcm_mat *>(Bm);
-        RMCM_TRY(dev_alloc(h, (void **)&Bw->rowsum, 8 * (Bm->d.rows + 1) + 8 * Bm->d.rows));
-        RMCM_CUDA(h, cudaMemsetAsync(Bw->rowsum + Bm->d.rows, 0, 8, s));
-        k_rowsum<V><<<grid_for(h, Bm->d.rows * 32, 256, 8), 256, 0, s>>>(Bm->d, Bw->rowsum,
-                                                                          (uint2 *)(Bw->rowsum + Bm->d.rows + 1));
+        RMCM_TRY(dev_alloc(h, (void **)&Bw->rowinfo, rowinfo_bytes(Bm)));
+        unsigned long long *vm = (unsigned long long *)(Bw->rowinfo + rowinfo_records(Bm));
+        RMCM_CUDA(h, cudaMemsetAsync(vm, 0, 8, s));
+        k_rowinfo<V><<<grid_for(h, Bm->d.rows * 32, 256, 8), 256, 0, s>>>(Bm->d, Bm->distinct, Bw->rowinfo, vm);
         h->launches++;
         RMCM_CUDA(h, cudaGetLastError());
     }
     const DevCsr A = Am->d;
     DevCsr B = Bm->d;
-    B.rowsum = Bm->ones ? nullptr : Bm->rowsum;
-    B.info = B.rowsum ? (const uint2 *)(Bm->rowsum + Bm->d.rows + 1) : nullptr;
+    B.info = Bm->ones ? nullptr : Bm->rowinfo;
+    B.vmax = B.info ? (const uint64_t *)(Bm->rowinfo + rowinfo_records(Bm)) : nullptr;
     const bool positive = Am->positive && Bm->positive;
     const int64_t m = A.rows;
     // scratch layout: flops[m] i64 | cnt[m] i64 | tile sums | bin_of[m] u8 | lists[m] i32 | small counters | cursors
@@ -3022,22 +3030,25 @@ int32_t spgemm_t(rmcm_handle *h, const rmcm_mat *Am, const rmcm_mat *Bm, rmcm_ma
     int64_t *tiles = (int64_t *)(sc + o_tiles);
     uint8_t *bin_of = (uint8_t *)(sc + o_bin);
     int32_t *lists = (int32_t *)(sc + o_lists);
-    // small: [0..6] bin counts, [8..14] bin cursors, [16] longest dense A row,
+    // small: [0..7] bin counts, [8..15] and [22..29] bin cursors (front, back),
+    // [16] longest dense A row,
     // [32..33] total flops (u64), [36..37] largest dense-row flops (u64),
     // [40] overflow certain, [42] dense split slots, [43] long A rows,
     // [44..45] longest C row (u64), [46] unsplit dense rows, [48..51]
     // profiling sums, [52] rank split slots, [53] unsplit rank rows,
     // [54..55] largest rank-row flops (u64), [56] rows that may overflow,
-    // [58..59] largest value of B (u64, when B may be packed), [60..61]
-    // largest total bound S of a row that may overflow (uint32), [18..19]
+    // [58..59] largest value of B (u64, when B may be packed), [62] row counter
+    // of k_row_window, [60..61] largest total of a row whose total may exceed
+    // the value type (uint32), [18..19]
     // and [20..21] slots of the single-pass temporary for the short-row bins'
     // and the rank bin's rows (u64)
     int32_t *small = (int32_t *)(sc + o_small);
     RMCM_CUDA(h, cudaMemsetAsync(small, 0, 256, s));
-    // B may be packed for the dense bin (uint32, positive, one window)
-    const bool pack_cand = sizeof(V) == 4 && positive && B.cols >= 2 && B.cols <= kDenseWinU32 && B.nnz > 0;
-    if (pack_cand && !Bm->ones && !replay)
-        RMCM_CUDA(h, cudaMemcpyAsync(small + 58, Bm->rowsum + Bm->d.rows, 8, cudaMemcpyDeviceToDevice, s));
+    // B may be packed for the warp and dense bins (positive, one window)
+    const bool pack_cand = positive && !Bm->ones && B.cols >= 2 &&
+                           B.cols <= (sizeof(V) == 4 ? kDenseWinU32 : kDenseWinU64) && B.nnz > 0;
+    if (pack_cand && !replay)
+        RMCM_CUDA(h, cudaMemcpyAsync(small + 58, B.vmax, 8, cudaMemcpyDeviceToDevice, s));
 
     ProdRecord *rec = nullptr;
     size_t rec_idx = 0;
@@ -3078,24 +3089,28 @@ int32_t spgemm_t(rmcm_handle *h, const rmcm_mat *Am, const rmcm_mat *Bm, rmcm_ma
         const bool long_rows = Am->max_row > kLongAnalyze;
         const int64_t max_long = A.nnz / kLongAnalyze + 1;
         if (long_rows) {
-            long_bytes = 24 * max_long + 256;
+            long_bytes = 32 * max_long + 256;
             RMCM_TRY(dev_alloc(h, (void **)&long_mem, long_bytes));
             RMCM_CUDA(h, cudaMemsetAsync(long_mem, 0, long_bytes, s));
         }
         int32_t *nlong = small + 43;
         unsigned long long *acc_f = long_rows ? (unsigned long long *)long_mem : nullptr;
         unsigned long long *acc_s = long_rows ? acc_f + max_long : nullptr;
-        int32_t *lsat = long_rows ? (int32_t *)(acc_s + max_long) : nullptr;
+        unsigned long long *acc_m = long_rows ? acc_s + max_long : nullptr;
+        int32_t *lsat = long_rows ? (int32_t *)(acc_m + max_long) : nullptr;
         int32_t *llist = long_rows ? lsat + max_long : nullptr;
-        k_analyze<V><<<grid_for(h, m * 32, 256, 8), 256, 0, s>>>(A, B, bp, ao, long_rows ? kLongAnalyze : INT64_MAX,
-                                                                  llist, nlong);
+        k_analyze<V><<<grid_for(h, m * 32, 256, 8), 256, 0, s>>>(
+            A, B, Am->ones, Bm->distinct, bp, ao, long_rows ? kLongAnalyze : INT64_MAX, llist, nlong);
         h->launches++;
         if (long_rows) {
-            k_analyze_long<V><<<h->sm_count * 4, 256, 0, s>>>(A, B, llist, nlong, acc_f, acc_s, lsat);
-            k_analyze_long_finish<V><<<4, 256, 0, s>>>(A, B, bp, ao, llist, nlong, acc_f, acc_s, lsat);
+            k_analyze_long<V><<<h->sm_count * 4, 256, 0, s>>>(A, B, Am->ones, Bm->distinct, llist, nlong, acc_f, acc_s,
+                                                                 acc_m, lsat);
+            k_analyze_long_finish<V><<<4, 256, 0, s>>>(A, B, bp, ao, llist, nlong, acc_f, acc_s, acc_m, lsat);
             h->launches += 2;
         }
-        k_scatter<<<grid_for(h, m, 256, 8), 256, 0, s>>>(m, bin_of, small, small + 8, lists, cnt);
+        k_scatter<<<grid_for(h, m, 256, 8), 256, 0, s>>>(
+            m, bin_of, flops, small, (const unsigned long long *)(small + 36), (const unsigned long long *)(small + 54),
+            small + 8, small + 22, lists, cnt);
         h->launches += 1;
         if (long_mem) {
             dev_free(h, long_mem, long_bytes);
@@ -3115,6 +3130,7 @@ int32_t spgemm_t(rmcm_handle *h, const rmcm_mat *Am, const rmcm_mat *Bm, rmcm_ma
     int32_t dense_max_alen = 0;
     int64_t flops_total = 0;
     int64_t cap_short = 0, cap_rank = 0;
+    uint64_t bmax = 1;   // B's largest value (when it may be packed; ones otherwise)
     bool certain = false;
     if (replay) {
         memcpy(counts, plan->counts, sizeof(counts));
@@ -3128,6 +3144,7 @@ int32_t spgemm_t(rmcm_handle *h, const rmcm_mat *Am, const rmcm_mat *Bm, rmcm_ma
         memcpy(&flops_total, (int32_t *)h->h_pinned + 32, sizeof(int64_t));
         memcpy(&cap_short, (int32_t *)h->h_pinned + 18, sizeof(int64_t));
         memcpy(&cap_rank, (int32_t *)h->h_pinned + 20, sizeof(int64_t));
+        if (pack_cand) memcpy(&bmax, (int32_t *)h->h_pinned + 58, sizeof(uint64_t));
         certain = ((int32_t *)h->h_pinned)[40] != 0;
         if (sizeof(V) == 4 && h->abort_on_certain_overflow && !certain) {
             // a row whose total exceeds 16 x 2^32 averages more than 2^32/128
@@ -3203,6 +3220,7 @@ int32_t spgemm_t(rmcm_handle *h, const rmcm_mat *Am, const rmcm_mat *Bm, rmcm_ma
         else risky_rows = ((int32_t *)h->h_pinned)[56];
         if (record) plan->risky_rows = risky_rows;
         dtemp.no_risky = risky_rows == 0;
+        dtemp.next_row = small + 62;
     }
     {
         // Tensor-core part (dense_gemm.cu): every row with products in the
@@ -3227,8 +3245,6 @@ int32_t spgemm_t(rmcm_handle *h, const rmcm_mat *Am, const rmcm_mat *Bm, rmcm_ma
             cudaEvent_t e0 = rec ? h->prof[rec_idx].ev[6] : nullptr, e1 = rec ? h->prof[rec_idx].ev[7] : nullptr;
             int32_t drc = RMCM_OK;
             if (sizeof(V) == 4) {
-                uint64_t bmax = 1;
-                if (!Bm->ones) memcpy(&bmax, (int32_t *)h->h_pinned + 58, sizeof(uint64_t));
                 drc = dense_part_build(h, A, B, bmax, dtemp.dpart, e0, e1, skewed);
             } else {
                 drc = dense_part_build64(h, A, B, dtemp.dpart, e0, e1);
@@ -3250,10 +3266,9 @@ int32_t spgemm_t(rmcm_handle *h, const rmcm_mat *Am, const rmcm_mat *Bm, rmcm_ma
         int32_t cbits = 0;
         if (replay) {
             cbits = plan->pack_cbits;
-        } else if (pack_cand && counts[kBinDense] > 0 && flops_total >= kPackReuse * B.nnz && !dtemp.dpart.S) {
-            // (with a tensor-core part the light rows left are short: no packing)
-            uint64_t bmax = 1;
-            if (!Bm->ones) memcpy(&bmax, (int32_t *)h->h_pinned + 58, sizeof(uint64_t));
+        } else if (pack_cand && counts[kBinDense] + counts[kBinWarp] > 0 &&
+                   flops_total >= (dtemp.dpart.S ? 16 : 1) * kPackReuse * B.nnz) {
+            // (beside a tensor-core part only the light rows use it)
             const int32_t cb = 32 - __builtin_clz((uint32_t)(B.cols - 1));
             if (cb < 32 && bmax < (1ull << (32 - cb))) cbits = cb;
         }
@@ -3264,8 +3279,7 @@ int32_t spgemm_t(rmcm_handle *h, const rmcm_mat *Am, const rmcm_mat *Bm, rmcm_ma
                 dtemp.cbits = cbits;
                 dtemp.pk_mem = p;
                 dtemp.pk_bytes = 4 * B.nnz;
-                k_pack_banked<<<grid_for(h, B.rows * 32, kPackWarps * 32, 6), kPackWarps * 32, 0, s>>>(
-                    B, cbits, (uint32_t *)p, h->d_status);
+                k_pack<V><<<grid_for(h, (B.nnz + 3) / 4, 256, 8), 256, 0, s>>>(B, cbits, (uint32_t *)p, h->d_status);
                 h->launches++;
                 RMCM_CUDA(h, cudaGetLastError());
             } else if (replay) {
@@ -3510,6 +3524,17 @@ int32_t spgemm_t(rmcm_handle *h, const rmcm_mat *Am, const rmcm_mat *Bm, rmcm_ma
     }
     const uint32_t other_bins = stemp.active ? ~short_mask : ~0u;
 
+    // every input >= 1: the row kernels without presence bytes and checks take
+    // the rows that cannot overflow
+    LeanArgs<V> lean_args{Am->ones ? nullptr : (const V *)A.val,
+                          {B.rowptr, B.col, (const V *)B.val, dtemp.pk, dtemp.cbits, 0}};
+    if (Bm->ones) {
+        lean_args.B.words = (const uint32_t *)B.col;
+        lean_args.B.cbits = 31;
+        lean_args.B.addend = 1;
+    }
+    const LeanArgs<V> *lean = positive ? &lean_args : nullptr;
+
     // symbolic
     rmcm_mat *C = nullptr;
     int32_t rc = mat_alloc(h, m, B.cols, -1, Am->valtype, &C);
@@ -3523,11 +3548,7 @@ int32_t spgemm_t(rmcm_handle *h, const rmcm_mat *Am, const rmcm_mat *Bm, rmcm_ma
     // every row single-pass dense (no split): slot i of the temporary is row i,
     // so a product whose rows all come out full can keep it as C
     const bool all_dense = dtemp.active && !dtemp.split && counts[kBinDense] == m;
-    if (all_dense) {
-        k_iota<<<grid_for(h, m, 256, 8), 256, 0, s>>>(lists, (int32_t)m);
-        h->launches++;
-        if (cudaGetLastError() != cudaSuccess) rc = set_error(h, RMCM_ECUDA, "row list launch");
-    }
+    dtemp.by_row = all_dense;
     if (rc == RMCM_OK && stemp.active) {
         // the short-row bins, once, into the temporary (lengths to cnt)
         DevCsr T = C->d;
@@ -3536,11 +3557,11 @@ int32_t spgemm_t(rmcm_handle *h, const rmcm_mat *Am, const rmcm_mat *Bm, rmcm_ma
         T.val = stemp.val;
         T.nnz = stemp.total;
         rc = launch_bins<V, true>(h, A, B, T, lists, counts, dense_max_alen, cnt, cursors, cursor_cap, &dtemp, bin_of,
-                                  positive, Bm->distinct, &rsplit, short_mask);
+                                  positive, Bm->distinct, &rsplit, lean, short_mask);
     }
     if (rc == RMCM_OK)
         rc = launch_bins<V, false>(h, A, B, C->d, lists, counts, dense_max_alen, cnt, cursors, cursor_cap, &dtemp,
-                                   bin_of, positive, Bm->distinct, &rsplit, other_bins);
+                                   bin_of, positive, Bm->distinct, &rsplit, lean, other_bins);
     if (rc == RMCM_OK)
         rc = scan_rowptr(h, cnt, m, C->d.rowptr, tiles, (unsigned long long *)(small + 44), replay ? plan->nnz : -1);
     if (rec) cudaEventRecord(h->prof[rec_idx].ev[3], s);
@@ -3598,7 +3619,7 @@ int32_t spgemm_t(rmcm_handle *h, const rmcm_mat *Am, const rmcm_mat *Bm, rmcm_ma
     }
     if (rc == RMCM_OK && !adopt)
         rc = launch_bins<V, true>(h, A, B, C->d, lists, counts, dense_max_alen, nullptr, cursors, cursor_cap, &dtemp,
-                                  bin_of, positive, Bm->distinct, &rsplit, other_bins);
+                                  bin_of, positive, Bm->distinct, &rsplit, lean, other_bins);
     drop_short();
     const int32_t gemm_limbs = dtemp.dpart.S ? dtemp.dpart.limbs * dtemp.dpart.alimbs : 0;
     const int64_t gemm_inner = dtemp.dpart.S ? dtemp.dpart.heavy : 0;

@@ -71,3 +71,81 @@ def test_uint64_overflow_is_seen_at_its_exact_limit(native, engine, n, over):
     if not over:
         rp, col, val = C.download()
         assert col[-1] == n - 1 and int(val[-1]) == 2 ** 64 - 1
+
+
+# B row lengths around the points where a row kernel changes how an entry's
+# products are spread (4 | 5, 64 | 65), around whole blocks of 128, and empty
+SPREAD = np.array([0, 1, 3, 4, 5, 7, 8, 9, 15, 16, 17, 31, 33, 63, 64, 65, 127, 128, 129, 255, 257, 300])
+
+
+@pytest.mark.parametrize("vt", ["VAL_U32", "VAL_U64"])
+@pytest.mark.parametrize("n", [127, 128, 129, 2047, 2048, 2049, 4100, 10300, 22528, 22529, 40960])
+def test_row_kernels_at_their_widths(native, engine, n, vt):
+    """Every width at which another kernel, CTA size or window takes the rows;
+    rows from one entry to more than a CTA lists at a time; some rows of a
+    uint64 product stay below 2^32, some do not."""
+    rng = np.random.default_rng(n)
+    k = 1500
+    B = random_csr(rng, k, n, rng.choice(SPREAD, k), hi=6)
+    m = 260
+    a_len = np.concatenate([rng.integers(1, 60, m - 4), [k, 1030, 513, 511]])
+    A = random_csr(rng, m, k, a_len, hi=6)
+    if vt == "VAL_U64":
+        A.data[A.indptr[5]:A.indptr[40]] *= np.uint64(2 ** 34)
+    check_product(native, engine, A, B, getattr(native, vt))
+
+
+@pytest.mark.parametrize("n", [900, 5000])
+def test_safe_and_risky_rows_in_one_product(native, engine, n):
+    """uint32 rows whose bound passes 2^32 (none overflows: their large values
+    meet different columns) beside rows that cannot."""
+    rng = np.random.default_rng(n)
+    k = 300
+    B = random_csr(rng, k, n, rng.integers(20, 200, k), hi=3)
+    A = random_csr(rng, 200, k, rng.integers(2, 60, 200), hi=4)
+    A = A.tolil()
+    for r in range(0, 200, 7):           # two entries of 2^30 and B rows of ones that do not meet
+        A[r, k - 1] = 2 ** 31
+        A[r, k - 2] = 2 ** 31
+    A = A.tocsr().astype(np.uint64)
+    B = B.tolil()
+    B[k - 1, :] = 0
+    B[k - 2, :] = 0
+    B[k - 1, 0:n // 3:2] = 1
+    B[k - 2, 1:n // 3:2] = 1
+    B = B.tocsr().astype(np.uint64)
+    B.eliminate_zeros()
+    check_product(native, engine, A, B, native.VAL_U32)
+
+
+@pytest.mark.parametrize("n", [600, 3000])
+def test_ones_and_repeated_columns(native, engine, n):
+    """Leaves are matrices of ones, and may hold a column twice in a row."""
+    rng = np.random.default_rng(n)
+    k, m = 400, 300
+    lens = rng.choice(SPREAD, k)
+    col = [np.sort(rng.integers(0, n, x)) for x in lens]          # with repeats
+    rp = np.concatenate([[0], np.cumsum(lens)]).astype(np.int64)
+    bc = np.concatenate(col).astype(np.int32)
+    A = random_csr(rng, m, k, rng.integers(1, 80, m), hi=2)
+    B = sp.csr_matrix((np.ones(bc.size, np.uint64), bc, rp), shape=(k, n))
+    ref = (A.astype(np.uint64) @ B).tocsr()
+    ref.sum_duplicates()
+    ref.sort_indices()
+    for vt in (native.VAL_U32, native.VAL_U64):
+        Am = engine.upload(A.indptr, A.indices, cols=k, valtype=vt)
+        Bm = engine.upload(rp, bc, cols=n, valtype=vt)
+        rp2, col2, val2 = engine.spgemm(Am, Bm).download()
+        assert np.array_equal(rp2, ref.indptr) and np.array_equal(col2, ref.indices)
+        assert np.array_equal(val2.astype(np.uint64), ref.data)
+
+
+def test_heavy_rows_are_split_below_the_general_threshold(native, engine):
+    """Rows of 2^17 products and more in a small product go to several CTAs."""
+    rng = np.random.default_rng(3)
+    k, n = 4000, 6000
+    B = random_csr(rng, k, n, rng.choice(SPREAD, k), hi=4)
+    lens = np.concatenate([rng.integers(1, 40, 120), [k, k, 3000]])
+    A = random_csr(rng, lens.size, k, lens, hi=4)
+    for vt in (native.VAL_U32, native.VAL_U64):
+        check_product(native, engine, A, B, vt)
