@@ -816,6 +816,7 @@ int32_t chain_exec(rmcm_handle *h, rmcm_mat *const *mats, int32_t len, const int
                 view->d.rowptr = A->d.rowptr + r0;
                 view->d.rows = r1 - r0;
                 view->d.info = nullptr;
+                view->d.top = nullptr;
                 view->d.vmax = nullptr;
                 view->rowinfo = nullptr;
                 view->est_long = nullptr;

@@ -29,12 +29,12 @@ struct DevCsr {
     int64_t *rowptr = nullptr;
     int32_t *col = nullptr;
     void *val = nullptr;
-    // per row {length, sum of its values, largest addition it can make to one
-    // column}, what the analysis of a product gathers per entry of its left
-    // operand in one sector: uint32 matrices 16 bytes, 32 bits each (sums
-    // saturated to 0xffffffff), uint64 ones 32 bytes, 64 bits each
-    // (saturated); null when every value is 1
+    // per row {length, sum of its values}, what the analysis of a product
+    // gathers per entry of its left operand: uint32 matrices 32 bits each (sums
+    // saturated to 0xffffffff), uint64 ones 64 bits each (saturated); null when
+    // every value is 1
     const void *info = nullptr;
+    const void *top = nullptr;          // with info: per row the largest addition it can make to one column (value type)
     const uint64_t *vmax = nullptr;     // with info: the matrix's largest value
 };
 
@@ -114,8 +114,8 @@ struct rmcm_mat {
     bool ones = false;                  // every value is 1 (leaves): row sums are row lengths
     bool positive = false;              // every value is >= 1 (a counter > 0 then marks presence)
     bool distinct = false;              // no column repeats within a row
-    char *rowinfo = nullptr;            // lazily computed row records (device, rowinfo_bytes), owned: see DevCsr::info;
-                                        // the largest value follows them
+    char *rowinfo = nullptr;            // lazily computed row records (device, rowinfo_bytes), owned: DevCsr::info,
+                                        // the largest value, then DevCsr::top
     int64_t max_row = -1;               // longest row (entries); -1 when unknown
     // rows longer than kEstLongRow entries, ascending (device), when known:
     // the estimator gives each a whole CTA
@@ -211,9 +211,9 @@ bool copy_out_launch(const void *const *src, void *const *dst_host, const int64_
 int32_t check_status(rmcm_handle *h);
 
 inline int64_t val_bytes(int32_t valtype) { return valtype == RMCM_VAL_U64 ? 8 : 4; }
-// Row records of a matrix and its largest value (rmcm_mat::rowinfo).
-inline int64_t rowinfo_records(const rmcm_mat *m) { return (m->valtype == RMCM_VAL_U64 ? 32 : 16) * m->d.rows; }
-inline int64_t rowinfo_bytes(const rmcm_mat *m) { return rowinfo_records(m) + 8; }
+// Row records of a matrix, its largest value and its rows' (rmcm_mat::rowinfo).
+inline int64_t rowinfo_records(const rmcm_mat *m) { return 2 * val_bytes(m->valtype) * m->d.rows; }
+inline int64_t rowinfo_bytes(const rmcm_mat *m) { return rowinfo_records(m) + 8 + val_bytes(m->valtype) * m->d.rows; }
 
 // ---- kernels (host launchers) --------------------------------------------
 // spgemm.cu

@@ -32,12 +32,6 @@
 constexpr int kOwnLen = 4;
 constexpr int kMidLen = 64;
 
-// The value of entry q; a matrix of ones is passed without values.
-template <typename V>
-__device__ __forceinline__ V value_at(const V *v, int64_t q) {
-    return v ? __ldg(v + q) : (V)1;
-}
-
 // Right operand of a row kernel: columns and values, or (PK) one 32-bit word
 // per entry: column in the low cbits, value - addend above them (a matrix of
 // ones is its column array with cbits 31 and addend 1).
@@ -100,26 +94,30 @@ struct Window {
 };
 
 // A thread's E entries of A from k (stride `step`, below a1): B row starts and
-// lengths and A values, the loads of all entries in flight together.
+// lengths and A values.  Loads past the end go to the row's first entry and
+// count for nothing: a branch around the dependent loads would keep them from
+// being in flight together.
 template <int E, typename V>
-__device__ __forceinline__ void load_entries(const DevCsr &A, const V *aval, const RowB<V> &B, int64_t k, int step,
-                                             int64_t a1, int64_t (&bs)[E], int32_t (&len)[E], V (&va)[E]) {
+__device__ __forceinline__ void load_entries(const DevCsr &A, const V *aval, const RowB<V> &B, int64_t a0, int64_t k,
+                                             int step, int64_t a1, int64_t (&bs)[E], int32_t (&len)[E], V (&va)[E]) {
     int32_t a[E];
+    int64_t be[E];
 #pragma unroll
-    for (int u = 0; u < E; u++) {
-        const bool ok = k + u * step < a1;
-        a[u] = ok ? __ldg(A.col + k + u * step) : -1;
-        va[u] = ok ? value_at(aval, k + u * step) : (V)0;
+    for (int u = 0; u < E; u++) a[u] = __ldg(A.col + (k + u * step < a1 ? k + u * step : a0));
+    if (aval) {
+#pragma unroll
+        for (int u = 0; u < E; u++) va[u] = __ldg(aval + (k + u * step < a1 ? k + u * step : a0));
+    } else {
+#pragma unroll
+        for (int u = 0; u < E; u++) va[u] = 1;
     }
 #pragma unroll
     for (int u = 0; u < E; u++) {
-        bs[u] = 0;
-        len[u] = 0;
-        if (a[u] >= 0) {
-            bs[u] = __ldg(B.rowptr + a[u]);
-            len[u] = (int32_t)(__ldg(B.rowptr + a[u] + 1) - bs[u]);
-        }
+        bs[u] = __ldg(B.rowptr + a[u]);
+        be[u] = __ldg(B.rowptr + a[u] + 1);
     }
+#pragma unroll
+    for (int u = 0; u < E; u++) len[u] = k + u * step < a1 ? (int32_t)(be[u] - bs[u]) : 0;
 }
 
 // The short ones (up to kOwnLen positions) among a thread's E entries, a
@@ -231,7 +229,7 @@ __device__ __forceinline__ void row_warp_products(const DevCsr &A, const V *aval
         int64_t bs[E];
         int32_t len[E];
         V va[E];
-        load_entries<E>(A, aval, B, k0 + lane, 32, a1, bs, len, va);
+        load_entries<E>(A, aval, B, a0, k0 + lane, 32, a1, bs, len, va);
         // listed: mid entries from the front, long ones from the back
         int nm = 0, nl = 0;
 #pragma unroll
@@ -339,7 +337,7 @@ __device__ __forceinline__ void row_window_products(const DevCsr &A, const V *av
         int64_t bs[E];
         int32_t len[E];
         V va[E];
-        load_entries<E>(A, aval, B, k0 + tid, NT, a1, bs, len, va);
+        load_entries<E>(A, aval, B, a0, k0 + tid, NT, a1, bs, len, va);
 #pragma unroll
         for (int u = 0; u < E; u++) {
             const unsigned mid = __ballot_sync(kFull, len[u] > kOwnLen && len[u] <= kMidLen);

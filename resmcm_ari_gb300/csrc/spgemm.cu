@@ -59,8 +59,9 @@ constexpr int32_t kDenseWinSym = 196608;      // presence bytes only: 192 KB
 constexpr int kDenseThreads = 512;
 // B is packed for the warp and dense bins when the product has at least this
 // many multiply-adds per entry of B (packing reads 8 or 12 bytes an entry and
-// writes 4; each use then reads 4).
+// writes 4; each use then reads 4) and enough of them to repay the launch.
 constexpr int64_t kPackReuse = 4;
+constexpr int64_t kPackMinFlops = 1 << 20;
 
 __device__ __forceinline__ void raise_status(int *st, int word) { atomicOr(st + word, 1); }
 
@@ -184,256 +185,395 @@ struct AnalyzeOut {
     unsigned long long *rank_cap;         // the same over the rank bin's rows
 };
 
+// A thread's part of them: kept in registers over all its rows (a shared
+// 64-bit atomic per row would queue every warp of the CTA on one address).
+struct AnalyzeAcc {
+    unsigned long long flops = 0, max_total = 0, short_cap = 0, rank_cap = 0;
+    long long max_dense = 0, max_rank = 0;
+    int32_t max_alen = 0, risky = 0, certain = 0;
+};
+
+constexpr int kAnalyzeThreads = 256;
+
 struct AnalyzeShared {
-    int32_t cnt[kNumBins];
-    int32_t max_alen;
-    int32_t certain;
-    int32_t risky;
-    unsigned long long flops;
-    unsigned long long max_flops;
-    unsigned long long max_rank_flops;
-    unsigned long long max_total;
-    unsigned long long short_cap, rank_cap;
+    int32_t cnt[kAnalyzeThreads / 32][kNumBins];   // rows per bin, a set per warp
+    unsigned long long part[kAnalyzeThreads / 32][6];
+    int32_t small[kAnalyzeThreads / 32][3];
 };
 
 __device__ __forceinline__ void analyze_shared_init(AnalyzeShared &sh) {
-    if (threadIdx.x < kNumBins) sh.cnt[threadIdx.x] = 0;
-    if (threadIdx.x == 0) {
-        sh.max_alen = 0;
-        sh.certain = 0;
-        sh.risky = 0;
-        sh.flops = 0;
-        sh.max_flops = 0;
-        sh.max_rank_flops = 0;
-        sh.max_total = 0;
-        sh.short_cap = 0;
-        sh.rank_cap = 0;
-    }
+    for (int i = threadIdx.x; i < kAnalyzeThreads / 32 * kNumBins; i += kAnalyzeThreads) (&sh.cnt[0][0])[i] = 0;
+    __syncthreads();
 }
 
-__device__ __forceinline__ void analyze_shared_flush(AnalyzeShared &sh, const AnalyzeOut &o) {
-    if (threadIdx.x < kNumBins && sh.cnt[threadIdx.x]) atomicAdd(o.bin_count + threadIdx.x, sh.cnt[threadIdx.x]);
-    if (threadIdx.x == 0) {
-        if (sh.flops) atomicAdd(o.flops_total, sh.flops);
-        if (sh.max_alen) atomicMax(o.dense_max_alen, sh.max_alen);
-        if (sh.max_flops) atomicMax(o.dense_max_flops, sh.max_flops);
-        if (sh.max_rank_flops) atomicMax(o.rank_max_flops, sh.max_rank_flops);
-        if (sh.certain) atomicOr(o.certain, 1);
-        if (sh.risky) atomicAdd(o.risky_rows, sh.risky);
-        if (sh.max_total) atomicMax(o.max_total, sh.max_total);
-        if (sh.short_cap) atomicAdd(o.short_cap, sh.short_cap);
-        if (sh.rank_cap) atomicAdd(o.rank_cap, sh.rank_cap);
+__device__ __forceinline__ unsigned long long warp_max_u64(unsigned long long v) {
+#pragma unroll
+    for (int d = 16; d > 0; d >>= 1) {
+        const unsigned long long o = __shfl_xor_sync(kFull, v, d);
+        v = o > v ? o : v;
     }
+    return v;
 }
 
-// Bin, overflow flags and totals of row r from its products f, its total
-// count srow and its count bound mrow (both saturating).
-template <typename V>
-__device__ __forceinline__ void analyze_row(int64_t r, int64_t f, unsigned long long srow,
-                                            unsigned long long mrow, int64_t alen,
-                                            int64_t ncols, const BinParams &bp, const AnalyzeOut &o,
-                                            AnalyzeShared &sh) {
-    const int b = classify(f, ncols, bp);
-    const unsigned long long vmax = sizeof(V) == 4 ? 0xffffffffull : ~0ull;
-    const bool risky = sizeof(V) == 4 ? mrow > vmax : mrow == ~0ull;
-    const bool total_over = sizeof(V) == 4 && srow > vmax;
-    o.flops[r] = f;
-    o.bin_of[r] = (uint8_t)(b | (risky ? kRiskyBit : 0) | (sizeof(V) == 8 && mrow <= 0xffffffffull ? kNarrowBit : 0));
-    if (f) atomicAdd(&sh.flops, (unsigned long long)f);
-    if (risky && b != kEmptyBin) atomicAdd(&sh.risky, 1);
-    if (total_over) atomicMax(&sh.max_total, srow);
-    if (total_over) {
-        const unsigned long long distinct = (unsigned long long)min(f, ncols);
-        if (srow == ~0ull || srow / vmax > distinct) sh.certain = 1;
+// Every thread of the CTA calls it: totals to the global words, one atomic
+// per word and CTA.
+__device__ __forceinline__ void analyze_flush(AnalyzeShared &sh, const AnalyzeAcc &acc, const AnalyzeOut &o) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    unsigned long long v[6] = {acc.flops, acc.short_cap, acc.rank_cap, acc.max_total, (unsigned long long)acc.max_dense,
+                               (unsigned long long)acc.max_rank};
+#pragma unroll
+    for (int i = 0; i < 6; i++) v[i] = i < 3 ? warp_sum(v[i]) : warp_max_u64(v[i]);
+    const int32_t alen = __reduce_max_sync(kFull, acc.max_alen), risky = __reduce_add_sync(kFull, acc.risky);
+    const int32_t certain = (int32_t)__reduce_or_sync(kFull, (unsigned)acc.certain);
+    if (lane == 0) {
+#pragma unroll
+        for (int i = 0; i < 6; i++) sh.part[warp][i] = v[i];
+        sh.small[warp][0] = alen;
+        sh.small[warp][1] = risky;
+        sh.small[warp][2] = certain;
     }
-    if (b != kEmptyBin) {
-        atomicAdd(&sh.cnt[b], 1);
-        // slots of the single-pass temporary, should the row take it
-        const unsigned long long cap = (unsigned long long)(f < ncols ? f : ncols);
-        if (b == kBinRank) atomicAdd(&sh.rank_cap, cap);
-        else if (b != kBinDense) atomicAdd(&sh.short_cap, cap);
-        if (b == kBinDense) {
-            atomicMax(&sh.max_alen, (int32_t)(alen < (int64_t)INT_MAX ? alen : (int64_t)INT_MAX));
-            atomicMax(&sh.max_flops, (unsigned long long)f);
+    __syncthreads();
+    constexpr int NW = kAnalyzeThreads / 32;
+    const int t = threadIdx.x;
+    if (t < kNumBins) {
+        int32_t n = 0;
+        for (int w = 0; w < NW; w++) n += sh.cnt[w][t];
+        if (n) atomicAdd(o.bin_count + t, n);
+    } else if (t >= 32 && t < 38) {
+        const int i = t - 32;
+        unsigned long long x = 0;
+        for (int w = 0; w < NW; w++) x = i < 3 ? x + sh.part[w][i] : max(x, sh.part[w][i]);
+        unsigned long long *dst[6] = {o.flops_total, o.short_cap, o.rank_cap, o.max_total, o.dense_max_flops,
+                                      o.rank_max_flops};
+        if (x) {
+            if (i < 3) atomicAdd(dst[i], x);
+            else atomicMax(dst[i], x);
         }
-        if (b == kBinRank) atomicMax(&sh.max_rank_flops, (unsigned long long)f);
+    } else if (t == 64) {
+        int32_t al = 0, ri = 0, ce = 0;
+        for (int w = 0; w < NW; w++) {
+            al = max(al, sh.small[w][0]);
+            ri += sh.small[w][1];
+            ce |= sh.small[w][2];
+        }
+        if (al) atomicMax(o.dense_max_alen, al);
+        if (ri) atomicAdd(o.risky_rows, ri);
+        if (ce) atomicOr(o.certain, 1);
     }
 }
 
-// Length, value sum and largest column addition of row a of B, as the
-// analysis needs them: a uint32 matrix's saturated fields are read as 2^32
-// (upper bounds stay upper bounds, and a sum that large is past every limit
-// the total is compared with).
-struct RowRec {
-    int64_t len;
-    unsigned long long sum, top;
+// What the analysis gathers over a row's entries: products, total count and
+// the largest count any column can reach (an upper bound), the last two
+// modulo 2^64 with a flag for a sum that went past it.
+struct RowSums {
+    int64_t f = 0;
+    unsigned long long total = 0, bound = 0;
+    uint32_t over = 0;   // 1: total, 2: bound
 };
 
+// Bin, overflow flags and totals of row r.
 template <typename V>
-__device__ __forceinline__ RowRec row_rec(const DevCsr &B, int32_t a, bool b_distinct) {
-    RowRec x;
-    if (B.info) {
-        if (sizeof(V) == 4) {
-            const uint4 q = __ldg((const uint4 *)B.info + a);
-            x.len = q.x;
-            x.sum = q.y == 0xffffffffu ? (1ull << 32) : q.y;
-            x.top = q.z == 0xffffffffu ? (1ull << 32) : q.z;
-        } else {
-            const ulonglong2 q = __ldg((const ulonglong2 *)B.info + 2 * (int64_t)a);
-            x.len = (int64_t)q.x;
-            x.sum = q.y;
-            x.top = __ldg((const unsigned long long *)B.info + 4 * (int64_t)a + 2);
-        }
+__device__ __forceinline__ void analyze_row(int64_t r, const RowSums &x, int64_t alen, int64_t ncols,
+                                            const BinParams &bp, const AnalyzeOut &o, int32_t *cnt, AnalyzeAcc &acc) {
+    const int64_t f = x.f;
+    const int b = classify(f, ncols, bp);
+    const unsigned long long vmax = sizeof(V) == 4 ? 0xffffffffull : ~0ull;
+    const unsigned long long srow = (x.over & 1u) ? ~0ull : x.total, mrow = (x.over & 2u) ? ~0ull : x.bound;
+    const bool risky = sizeof(V) == 4 ? mrow > vmax : mrow == ~0ull;
+    o.flops[r] = f;
+    o.bin_of[r] = (uint8_t)(b | (risky ? kRiskyBit : 0) | (sizeof(V) == 8 && mrow <= 0xffffffffull ? kNarrowBit : 0));
+    if (b == kEmptyBin) return;
+    acc.flops += (unsigned long long)f;
+    acc.risky += risky;
+    if (sizeof(V) == 4 && srow > vmax) {
+        acc.max_total = max(acc.max_total, srow);
+        const unsigned long long distinct = (unsigned long long)min(f, ncols);
+        if (srow == ~0ull || srow / vmax > distinct) acc.certain = 1;
+    }
+    atomicAdd(cnt + b, 1);
+    // slots of the single-pass temporary, should the row take it
+    const unsigned long long cap = (unsigned long long)(f < ncols ? f : ncols);
+    if (b == kBinRank) {
+        acc.rank_cap += cap;
+        acc.max_rank = max(acc.max_rank, (long long)f);
+    } else if (b == kBinDense) {
+        acc.max_alen = max(acc.max_alen, (int32_t)(alen < (int64_t)INT_MAX ? alen : (int64_t)INT_MAX));
+        acc.max_dense = max(acc.max_dense, (long long)f);
     } else {
-        // ones: a column is hit once per row unless columns repeat
-        x.len = B.rowptr[a + 1] - B.rowptr[a];
-        x.sum = (unsigned long long)x.len;
-        x.top = b_distinct ? (x.len > 0 ? 1ull : 0ull) : x.sum;
+        acc.short_cap += cap;
     }
-    return x;
 }
 
-__device__ __forceinline__ unsigned long long sat_mul(unsigned long long a, unsigned long long b) {
-    return __umul64hi(a, b) ? ~0ull : a * b;
+__device__ __forceinline__ void add_over(unsigned long long &s, unsigned long long v, uint32_t &over, uint32_t flag) {
+    s += v;
+    over |= s < v ? flag : 0u;
 }
 
-// Products, total count and count bound of A entries [k0, k1) (strided by
-// `step` from k0): srow = sum_k A[k] * rowsum(B[k]), the row's total count,
-// mrow = sum_k A[k] * (largest entry of B[k]), which no single count exceeds.
-// Four entries per step: their gathers are independent and overlap.
-template <typename V>
-__device__ __forceinline__ void analyze_entries(const DevCsr &A, const DevCsr &B, bool a_ones, bool b_distinct,
-                                                int64_t k0, int64_t k1, int step, int64_t &f,
-                                                unsigned long long &srow, unsigned long long &mrow) {
+// Entries [k, k1) of a row, strided by `step`, into x; four entries per step,
+// so that their gathers overlap.  A1 / B1: the matrix holds ones (its values
+// are not read; the row lengths of a B of ones come from its row pointers).
+// SUMS adds products and totals, BOUND the count bound.
+template <typename V, bool A1, bool B1, bool SUMS, bool BOUND, int E>
+__device__ __forceinline__ void analyze_step(const DevCsr &A, const DevCsr &B, bool b_distinct, int64_t k, int step,
+                                             RowSums &x) {
     const V *Aval = (const V *)A.val;
-    int64_t k = k0;
-    for (; k + 3 * (int64_t)step < k1; k += 4 * (int64_t)step) {
-        int32_t a[4];
-        unsigned long long av[4];
-        RowRec x[4];
+    int32_t a[E];
+    unsigned long long av[E], sum[E], top[E];
+    int64_t len[E];
 #pragma unroll
-        for (int u = 0; u < 4; u++) {
-            a[u] = A.col[k + u * step];
-            av[u] = a_ones ? 1ull : (unsigned long long)Aval[k + u * step];
-        }
-#pragma unroll
-        for (int u = 0; u < 4; u++) x[u] = row_rec<V>(B, a[u], b_distinct);
-#pragma unroll
-        for (int u = 0; u < 4; u++) {
-            f += x[u].len;
-            srow = sat_add(srow, sat_mul(av[u], x[u].sum));
-            mrow = sat_add(mrow, sat_mul(av[u], x[u].top));
-        }
+    for (int u = 0; u < E; u++) {
+        a[u] = __ldg(A.col + k + u * step);
+        av[u] = A1 ? 1ull : (unsigned long long)__ldg(Aval + k + u * step);
     }
-    for (; k < k1; k += step) {
-        const unsigned long long av = a_ones ? 1ull : (unsigned long long)Aval[k];
-        const RowRec x = row_rec<V>(B, A.col[k], b_distinct);
-        f += x.len;
-        srow = sat_add(srow, sat_mul(av, x.sum));
-        mrow = sat_add(mrow, sat_mul(av, x.top));
-    }
-}
-
-// Warp per row of A: flops and bin; per-bin row counts and the longest
-// A row of the dense bin (it sizes the cursor scratch).  A row whose count
-// bound (analyze_entries) is within the value type is safe: its kernels skip
-// the overflow checks; the bound takes the largest entry of each B row, not
-// its sum, so a row is risky only when a single count may really get there.
-// A row whose total count is greater than (its possible distinct columns) x
-// (largest value) is certain to overflow, which raises *certain.  Rows with
-// more than long_min entries are left to k_analyze_long (appended to
-// long_list) so no warp walks a huge row alone.
-template <typename V>
-__global__ void __launch_bounds__(256) k_analyze(DevCsr A, DevCsr B, bool a_ones, bool b_distinct, BinParams bp,
-                                                 AnalyzeOut o, int64_t long_min,
-                                                 int32_t *long_list, int32_t *nlong) {
-    __shared__ AnalyzeShared sh;
-    analyze_shared_init(sh);
-    __syncthreads();
-    const int lane = threadIdx.x & 31;
-    const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
-    for (int64_t r = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; r < A.rows; r += nwarps) {
-        const int64_t a0 = A.rowptr[r], a1 = A.rowptr[r + 1];
-        if (a1 - a0 > long_min) {
-            if (lane == 0) long_list[atomicAdd(nlong, 1)] = (int32_t)r;
+#pragma unroll
+    for (int u = 0; u < E; u++) {
+        if (B1) {
+            len[u] = __ldg(B.rowptr + a[u] + 1) - __ldg(B.rowptr + a[u]);
+            sum[u] = (unsigned long long)len[u];
+            top[u] = b_distinct ? (len[u] > 0 ? 1ull : 0ull) : sum[u];
             continue;
         }
-        int64_t f = 0;
-        unsigned long long srow = 0, mrow = 0;
-        analyze_entries<V>(A, B, a_ones, b_distinct, a0 + lane, a1, 32, f, srow, mrow);
-        f = warp_sum(f);
-#pragma unroll
-        for (int d = 16; d > 0; d >>= 1) {
-            srow = sat_add(srow, __shfl_xor_sync(kFull, srow, d));
-            mrow = sat_add(mrow, __shfl_xor_sync(kFull, mrow, d));
+        if (SUMS && sizeof(V) == 4) {
+            const uint2 q = __ldg((const uint2 *)B.info + a[u]);
+            len[u] = q.x;
+            // a saturated sum is read as 2^32: past every limit the total is
+            // compared with
+            sum[u] = q.y == 0xffffffffu ? (1ull << 32) : q.y;
+        } else if (SUMS) {
+            const ulonglong2 q = __ldg((const ulonglong2 *)B.info + a[u]);
+            len[u] = (int64_t)q.x;
+            sum[u] = q.y;
         }
-        if (lane == 0) analyze_row<V>(r, f, srow, mrow, a1 - a0, B.cols, bp, o, sh);
+        if (BOUND) {
+            const V t = __ldg((const V *)B.top + a[u]);
+            top[u] = sizeof(V) == 4 && t == (V)0xffffffffu ? (1ull << 32) : (unsigned long long)t;
+        }
     }
-    __syncthreads();
-    analyze_shared_flush(sh, o);
+#pragma unroll
+    for (int u = 0; u < E; u++) {
+        if (SUMS) {
+            x.f += len[u];
+            if (!A1 && sizeof(V) == 8) x.over |= __umul64hi(av[u], sum[u]) ? 1u : 0u;
+            add_over(x.total, A1 ? sum[u] : av[u] * sum[u], x.over, 1u);   // uint32: (2^32 - 1) * 2^32 fits
+        }
+        if (BOUND) {
+            if (!A1 && sizeof(V) == 8) x.over |= __umul64hi(av[u], top[u]) ? 2u : 0u;
+            add_over(x.bound, A1 ? top[u] : av[u] * top[u], x.over, 2u);
+        }
+    }
 }
 
-// Long rows: the whole grid walks each long row, CTA b taking the b-th slice
-// of its entries; partial products (int64), totals and count bounds (uint64,
-// with saturation flags) meet in per-row accumulators.
+template <typename V, bool A1, bool B1, bool SUMS, bool BOUND>
+__device__ __forceinline__ void analyze_entries(const DevCsr &A, const DevCsr &B, bool b_distinct, int64_t k,
+                                                int64_t k1, int step, RowSums &x) {
+    for (; k + 3 * (int64_t)step < k1; k += 4 * (int64_t)step)
+        analyze_step<V, A1, B1, SUMS, BOUND, 4>(A, B, b_distinct, k, step, x);
+    for (; k < k1; k += step) analyze_step<V, A1, B1, SUMS, BOUND, 1>(A, B, b_distinct, k, step, x);
+}
+
+// x of the G aligned lanes of a group, in all of them.
+template <bool SUMS, bool BOUND>
+__device__ __forceinline__ void group_sums(RowSums &x, int G) {
+    for (int d = G >> 1; d > 0; d >>= 1) {
+        x.over |= __shfl_xor_sync(kFull, x.over, d);
+        if (SUMS) {
+            x.f += __shfl_xor_sync(kFull, x.f, d);
+            const unsigned long long t = __shfl_xor_sync(kFull, x.total, d);
+            add_over(x.total, t, x.over, 1u);
+        }
+        if (BOUND) {
+            const unsigned long long b = __shfl_xor_sync(kFull, x.bound, d);
+            add_over(x.bound, b, x.over, 2u);
+        }
+    }
+    // (a lane's own overflow in the last step)
+    for (int d = G >> 1; d > 0; d >>= 1) x.over |= __shfl_xor_sync(kFull, x.over, d);
+}
+
+// The count bound matters only for a row whose total, a weaker bound, does not
+// already show that every count fits 32 bits.
+__device__ __forceinline__ bool needs_bound(const RowSums &x) { return (x.over & 1u) || x.total > 0xffffffffull; }
+
+// Products, bin and flags of every row of A; per-bin row counts and the
+// longest A row of the dense bin (it sizes the cursor scratch).  A row whose
+// count bound is within the value type is safe: its kernels skip the overflow
+// checks; the bound takes the largest entry of each B row, not its sum, so a
+// row is risky only when a single count may really get there.  A row whose
+// total count is greater than (its possible distinct columns) x (largest
+// value) is certain to overflow, which raises *certain.
+//
+// G lanes per row, by the average row length (analyze_lanes): bound by
+// instruction issue, above all the reductions over a row's lanes, which serve
+// 32 / G rows at a time, and on large products by the gathers of B's records
+// (8 bytes, so that the popular ones stay in the L1; the bound's own gathers
+// only follow for rows whose total leaves it open).  Rows longer than 64 G are
+// taken by the whole warp after their group, rows with more than long_min
+// entries by the whole grid (k_analyze_long, through long_list).
+// Before (a warp per row, one shared 64-bit atomic per row and total, slices
+// of every long row for every CTA): one million rows of 20 entries on a leaf
+// 508 us, now 230; 2,000 rows of 4,500 entries 298 us, now 118; 20,000 rows of
+// 7,900 entries 589 us, now 577 (the gathers).
+template <typename V, bool A1, bool B1>
+__global__ void __launch_bounds__(kAnalyzeThreads, 4) k_analyze(DevCsr A, DevCsr B, bool b_distinct, BinParams bp,
+                                                             AnalyzeOut o, int G, int64_t long_min,
+                                                             int32_t *long_list, int32_t *nlong) {
+    __shared__ AnalyzeShared sh;
+    analyze_shared_init(sh);
+    AnalyzeAcc acc;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int sub = lane & (G - 1), rows = 32 / G;
+    const int64_t step = ((int64_t)gridDim.x * kAnalyzeThreads >> 5) * rows;
+    for (int64_t r0 = (((int64_t)blockIdx.x * kAnalyzeThreads + threadIdx.x) >> 5) * rows; r0 < A.rows; r0 += step) {
+        const int64_t r = r0 + lane / G;
+        const bool row = r < A.rows;
+        int64_t a0 = 0, a1 = 0;
+        if (row) {
+            a0 = A.rowptr[r];
+            a1 = A.rowptr[r + 1];
+        }
+        const bool grid_row = a1 - a0 > long_min;
+        const bool warp_row = !grid_row && G < 32 && a1 - a0 > 64 * (int64_t)G;
+        if (grid_row && sub == 0) long_list[atomicAdd(nlong, 1)] = (int32_t)r;
+        RowSums x;
+        const int64_t e1 = grid_row || warp_row ? a0 : a1;   // entries for the group
+        analyze_entries<V, A1, B1, true, B1>(A, B, b_distinct, a0 + sub, e1, G, x);
+        group_sums<true, B1>(x, G);
+        if (!B1) {
+            const bool more = needs_bound(x);
+            if (__any_sync(kFull, more)) {
+                analyze_entries<V, A1, B1, false, true>(A, B, b_distinct, a0 + sub, more ? e1 : a0, G, x);
+                group_sums<false, true>(x, G);
+            }
+            if (!more) x.bound = x.total;
+        }
+        unsigned wide = __ballot_sync(kFull, warp_row && sub == 0);
+        while (wide) {
+            const int src = __ffs(wide) - 1;
+            wide &= wide - 1;
+            const int64_t b0 = __shfl_sync(kFull, a0, src), b1 = __shfl_sync(kFull, a1, src);
+            RowSums y;
+            analyze_entries<V, A1, B1, true, B1>(A, B, b_distinct, b0 + lane, b1, 32, y);
+            group_sums<true, B1>(y, 32);
+            if (!B1) {
+                if (needs_bound(y)) {   // (the same in every lane)
+                    analyze_entries<V, A1, B1, false, true>(A, B, b_distinct, b0 + lane, b1, 32, y);
+                    group_sums<false, true>(y, 32);
+                } else {
+                    y.bound = y.total;
+                }
+            }
+            if (lane == src) x = y;
+        }
+        if (row && sub == 0 && !grid_row) analyze_row<V>(r, x, a1 - a0, B.cols, bp, o, sh.cnt[warp], acc);
+    }
+    analyze_flush(sh, acc, o);
+}
+
+// Long rows: their pieces of kLongPiece entries are dealt to the CTAs in turn;
+// partial products (int64), totals and count bounds (uint64, with saturation
+// flags) meet in per-row accumulators.
+constexpr int kLongPiece = 2048;
+
 __device__ __forceinline__ void sat_accumulate(unsigned long long *acc, unsigned long long v, int32_t *sat, int flag) {
     if (!v) return;
     const unsigned long long old = atomicAdd(acc, v);
-    if (v == ~0ull || old > ~0ull - v) atomicOr(sat, flag);
+    if (old > ~0ull - v) atomicOr(sat, flag);
 }
 
-template <typename V>
-__global__ void __launch_bounds__(256) k_analyze_long(DevCsr A, DevCsr B, bool a_ones, bool b_distinct,
-                                                      const int32_t *long_list, const int32_t *nlong,
-                                                      unsigned long long *acc_f, unsigned long long *acc_s,
-                                                      unsigned long long *acc_m, int32_t *sat) {
+template <typename V, bool A1, bool B1>
+__global__ void __launch_bounds__(kAnalyzeThreads) k_analyze_long(DevCsr A, DevCsr B, bool b_distinct,
+                                                                  const int32_t *long_list, const int32_t *nlong,
+                                                                  unsigned long long *acc_f,
+                                                                  unsigned long long *acc_s,
+                                                                  unsigned long long *acc_m, int32_t *sat) {
+    __shared__ int32_t s_first[kAnalyzeThreads + 1];   // first piece of each row of the batch
+    __shared__ int32_t s_warp[kAnalyzeThreads / 32];
     const int nl = *nlong;
-    const int lane = threadIdx.x & 31;
-    for (int j = 0; j < nl; j++) {
-        const int32_t r = long_list[j];
-        const int64_t a0 = A.rowptr[r], alen = A.rowptr[r + 1] - a0;
-        const int64_t k0 = a0 + alen * blockIdx.x / gridDim.x, k1 = a0 + alen * (blockIdx.x + 1) / gridDim.x;
-        int64_t f = 0;
-        unsigned long long srow = 0, mrow = 0;
-        analyze_entries<V>(A, B, a_ones, b_distinct, k0 + threadIdx.x, k1, blockDim.x, f, srow, mrow);
-        f = warp_sum(f);
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    int64_t done = 0;                                  // pieces of the batches before
+    for (int j0 = 0; j0 < nl; j0 += kAnalyzeThreads) {
+        // pieces of up to 256 rows, scanned
+        int32_t np = 0;
+        if (j0 + tid < nl) {
+            const int32_t r = long_list[j0 + tid];
+            np = (int32_t)((A.rowptr[r + 1] - A.rowptr[r] + kLongPiece - 1) / kLongPiece);
+        }
+        int32_t incl = np;
 #pragma unroll
-        for (int d = 16; d > 0; d >>= 1) {
-            srow = sat_add(srow, __shfl_xor_sync(kFull, srow, d));
-            mrow = sat_add(mrow, __shfl_xor_sync(kFull, mrow, d));
+        for (int d = 1; d < 32; d <<= 1) {
+            const int32_t o = __shfl_up_sync(kFull, incl, d);
+            if (lane >= d) incl += o;
         }
-        if (lane == 0) {
-            if (f) atomicAdd(acc_f + j, (unsigned long long)f);
-            sat_accumulate(acc_s + j, srow, sat + j, 1);
-            sat_accumulate(acc_m + j, mrow, sat + j, 2);
+        if (lane == 31) s_warp[warp] = incl;
+        __syncthreads();
+        int32_t base = 0;
+        for (int w = 0; w < warp; w++) base += s_warp[w];
+        s_first[tid + 1] = base + incl;
+        if (tid == 0) s_first[0] = 0;
+        __syncthreads();
+        const int32_t total = s_first[kAnalyzeThreads];
+        // this CTA's pieces of the batch: those with (done + piece) mod grid == block
+        int32_t p = (int32_t)(((int64_t)blockIdx.x - done % gridDim.x + gridDim.x) % gridDim.x);
+        for (; p < total; p += gridDim.x) {
+            int lo = 0, hi = kAnalyzeThreads - 1;      // last row with s_first <= p
+            while (lo < hi) {
+                const int mid = (lo + hi + 1) >> 1;
+                if (s_first[mid] <= p) lo = mid;
+                else hi = mid - 1;
+            }
+            const int j = j0 + lo;
+            const int32_t r = long_list[j];
+            const int64_t k0 = A.rowptr[r] + (int64_t)(p - s_first[lo]) * kLongPiece;
+            const int64_t k1 = min(k0 + kLongPiece, A.rowptr[r + 1]);
+            RowSums x;
+            analyze_entries<V, A1, B1, true, true>(A, B, b_distinct, k0 + tid, k1, kAnalyzeThreads, x);
+            group_sums<true, true>(x, 32);
+            if (lane == 0) {
+                if (x.f) atomicAdd(acc_f + j, (unsigned long long)x.f);
+                if (x.over) atomicOr(sat + j, (int32_t)x.over);
+                sat_accumulate(acc_s + j, x.total, sat + j, 1);
+                sat_accumulate(acc_m + j, x.bound, sat + j, 2);
+            }
         }
+        done += total;
+        __syncthreads();   // the table is free
     }
 }
 
 template <typename V>
-__global__ void __launch_bounds__(256) k_analyze_long_finish(DevCsr A, DevCsr B, BinParams bp, AnalyzeOut o,
-                                                             const int32_t *long_list, const int32_t *nlong,
-                                                             const unsigned long long *acc_f,
-                                                             const unsigned long long *acc_s,
-                                                             const unsigned long long *acc_m, const int32_t *sat) {
+__global__ void __launch_bounds__(kAnalyzeThreads) k_analyze_long_finish(
+    DevCsr A, DevCsr B, BinParams bp, AnalyzeOut o, const int32_t *long_list, const int32_t *nlong,
+    const unsigned long long *acc_f, const unsigned long long *acc_s, const unsigned long long *acc_m,
+    const int32_t *sat) {
     __shared__ AnalyzeShared sh;
     analyze_shared_init(sh);
-    __syncthreads();
+    AnalyzeAcc acc;
     const int nl = *nlong;
     for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < nl; j += gridDim.x * blockDim.x) {
         const int32_t r = long_list[j];
-        const unsigned long long srow = (sat[j] & 1) ? ~0ull : acc_s[j], mrow = (sat[j] & 2) ? ~0ull : acc_m[j];
-        analyze_row<V>(r, (int64_t)acc_f[j], srow, mrow, A.rowptr[r + 1] - A.rowptr[r], B.cols, bp, o, sh);
+        RowSums x;
+        x.f = (int64_t)acc_f[j];
+        x.total = acc_s[j];
+        x.bound = acc_m[j];
+        x.over = (uint32_t)sat[j];
+        analyze_row<V>(r, x, A.rowptr[r + 1] - A.rowptr[r], B.cols, bp, o, sh.cnt[threadIdx.x >> 5], acc);
     }
-    __syncthreads();
-    analyze_shared_flush(sh, o);
+    analyze_flush(sh, acc, o);
 }
 
-// Row records of a matrix (DevCsr::info; warp per row) and its largest value
-// (*vmax, zeroed by the caller).  The largest addition a row makes to one
+// Lanes per row of k_analyze: about a quarter of the average row, so that
+// most lanes hold a step of four entries.
+inline int analyze_lanes(int64_t rows, int64_t nnz) {
+    int g = 2;
+    while (g < 32 && rows * 4 * g < nnz) g <<= 1;
+    return g;
+}
+
+// Row records of a matrix (DevCsr::info and top; warp per row) and its largest
+// value (*vmax, zeroed by the caller).  The largest addition a row makes to one
 // column is its largest value, or its sum when columns may repeat in a row.
 template <typename V>
-__global__ void k_rowinfo(DevCsr M, bool distinct, void *info, unsigned long long *vmax) {
+__global__ void k_rowinfo(DevCsr M, bool distinct, V *info, V *top_out, unsigned long long *vmax) {
     const int lane = threadIdx.x & 31;
     const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
     const V *v = (const V *)M.val;
@@ -454,14 +594,11 @@ __global__ void k_rowinfo(DevCsr M, bool distinct, void *info, unsigned long lon
         }
         all = top > all ? top : all;
         if (!distinct) top = sum;
+        const unsigned long long vm = sizeof(V) == 4 ? 0xffffffffull : ~0ull;
         if (lane == 0) {
-            if (sizeof(V) == 4) {
-                ((uint4 *)info)[r] = make_uint4((uint32_t)min(q1 - q0, (int64_t)0xffffffff),
-                                                (uint32_t)min(sum, 0xffffffffull), (uint32_t)min(top, 0xffffffffull), 0);
-            } else {
-                ((ulonglong2 *)info)[2 * r] = make_ulonglong2((unsigned long long)(q1 - q0), sum);
-                ((ulonglong2 *)info)[2 * r + 1] = make_ulonglong2(top, 0);
-            }
+            info[2 * r] = (V)min((unsigned long long)(q1 - q0), vm);
+            info[2 * r + 1] = (V)min(sum, vm);
+            top_out[r] = (V)min(top, vm);
         }
     }
     if (lane == 0 && all) atomicMax(vmax, all);
@@ -2703,8 +2840,11 @@ struct RankSplit {
 constexpr int64_t kSplitMinFlops = 1 << 17;
 constexpr int64_t kSplitMinLight = 1 << 18;   // light products of rows beside a tensor-core part
 
-// A rows with more entries than this are analysed by the whole grid.
-constexpr int64_t kLongAnalyze = 16384;
+// A rows with more entries than this are analysed by the whole grid: twice the
+// average row, between a piece of it and what one warp walks in about 100 us.
+inline int64_t long_analyze(int64_t rows, int64_t nnz) {
+    return std::min<int64_t>(16384, std::max<int64_t>(kLongPiece, rows > 0 ? 2 * nnz / rows : 0));
+}
 
 // Extras of a dense-bin launch: the packed copy of B, and (single-pass rows
 // only) the tensor-core part.
@@ -2999,7 +3139,8 @@ int32_t spgemm_t(rmcm_handle *h, const rmcm_mat *Am, const rmcm_mat *Bm, rmcm_ma
         RMCM_TRY(dev_alloc(h, (void **)&Bw->rowinfo, rowinfo_bytes(Bm)));
         unsigned long long *vm = (unsigned long long *)(Bw->rowinfo + rowinfo_records(Bm));
         RMCM_CUDA(h, cudaMemsetAsync(vm, 0, 8, s));
-        k_rowinfo<V><<<grid_for(h, Bm->d.rows * 32, 256, 8), 256, 0, s>>>(Bm->d, Bm->distinct, Bw->rowinfo, vm);
+        k_rowinfo<V><<<grid_for(h, Bm->d.rows * 32, 256, 8), 256, 0, s>>>(
+            Bm->d, Bm->distinct, (V *)Bw->rowinfo, (V *)(vm + 1), vm);
         h->launches++;
         RMCM_CUDA(h, cudaGetLastError());
     }
@@ -3007,6 +3148,7 @@ int32_t spgemm_t(rmcm_handle *h, const rmcm_mat *Am, const rmcm_mat *Bm, rmcm_ma
     DevCsr B = Bm->d;
     B.info = Bm->ones ? nullptr : Bm->rowinfo;
     B.vmax = B.info ? (const uint64_t *)(Bm->rowinfo + rowinfo_records(Bm)) : nullptr;
+    B.top = B.info ? (const void *)(B.vmax + 1) : nullptr;
     const bool positive = Am->positive && Bm->positive;
     const int64_t m = A.rows;
     // scratch layout: flops[m] i64 | cnt[m] i64 | tile sums | bin_of[m] u8 | lists[m] i32 | small counters | cursors
@@ -3085,9 +3227,10 @@ int32_t spgemm_t(rmcm_handle *h, const rmcm_mat *Am, const rmcm_mat *Bm, rmcm_ma
                       (unsigned long long *)(small + 60),
                       (unsigned long long *)(small + 18),
                       (unsigned long long *)(small + 20)};
-        // rows longer than kLongAnalyze entries: walked by the whole grid
-        const bool long_rows = Am->max_row > kLongAnalyze;
-        const int64_t max_long = A.nnz / kLongAnalyze + 1;
+        // rows longer than long_min entries: walked by the whole grid
+        const int64_t long_min = long_analyze(m, A.nnz);
+        const bool long_rows = Am->max_row > long_min;
+        const int64_t max_long = A.nnz / long_min + 1;
         if (long_rows) {
             long_bytes = 32 * max_long + 256;
             RMCM_TRY(dev_alloc(h, (void **)&long_mem, long_bytes));
@@ -3099,13 +3242,25 @@ int32_t spgemm_t(rmcm_handle *h, const rmcm_mat *Am, const rmcm_mat *Bm, rmcm_ma
         unsigned long long *acc_m = long_rows ? acc_s + max_long : nullptr;
         int32_t *lsat = long_rows ? (int32_t *)(acc_m + max_long) : nullptr;
         int32_t *llist = long_rows ? lsat + max_long : nullptr;
-        k_analyze<V><<<grid_for(h, m * 32, 256, 8), 256, 0, s>>>(
-            A, B, Am->ones, Bm->distinct, bp, ao, long_rows ? kLongAnalyze : INT64_MAX, llist, nlong);
+        auto analyze = [&](auto a1, auto b1) {
+            constexpr bool A1 = decltype(a1)::value, B1 = decltype(b1)::value;
+            const int G = analyze_lanes(m, A.nnz);
+            k_analyze<V, A1, B1><<<grid_for(h, m * G, kAnalyzeThreads, 8), kAnalyzeThreads, 0, s>>>(
+                A, B, Bm->distinct, bp, ao, G, long_rows ? long_min : INT64_MAX, llist, nlong);
+            if (long_rows)
+                k_analyze_long<V, A1, B1><<<h->sm_count * 4, kAnalyzeThreads, 0, s>>>(A, B, Bm->distinct, llist, nlong, acc_f,
+                                                                         acc_s, acc_m, lsat);
+        };
+        const std::true_type yes;
+        const std::false_type no;
+        if (Am->ones && Bm->ones) analyze(yes, yes);
+        else if (Am->ones) analyze(yes, no);
+        else if (Bm->ones) analyze(no, yes);
+        else analyze(no, no);
         h->launches++;
         if (long_rows) {
-            k_analyze_long<V><<<h->sm_count * 4, 256, 0, s>>>(A, B, Am->ones, Bm->distinct, llist, nlong, acc_f, acc_s,
-                                                                 acc_m, lsat);
-            k_analyze_long_finish<V><<<4, 256, 0, s>>>(A, B, bp, ao, llist, nlong, acc_f, acc_s, acc_m, lsat);
+            k_analyze_long_finish<V><<<4, kAnalyzeThreads, 0, s>>>(A, B, bp, ao, llist, nlong, acc_f, acc_s, acc_m,
+                                                                   lsat);
             h->launches += 2;
         }
         k_scatter<<<grid_for(h, m, 256, 8), 256, 0, s>>>(
@@ -3266,7 +3421,7 @@ int32_t spgemm_t(rmcm_handle *h, const rmcm_mat *Am, const rmcm_mat *Bm, rmcm_ma
         int32_t cbits = 0;
         if (replay) {
             cbits = plan->pack_cbits;
-        } else if (pack_cand && counts[kBinDense] + counts[kBinWarp] > 0 &&
+        } else if (pack_cand && counts[kBinDense] + counts[kBinWarp] > 0 && flops_total >= kPackMinFlops &&
                    flops_total >= (dtemp.dpart.S ? 16 : 1) * kPackReuse * B.nnz) {
             // (beside a tensor-core part only the light rows use it)
             const int32_t cb = 32 - __builtin_clz((uint32_t)(B.cols - 1));

@@ -149,3 +149,43 @@ def test_heavy_rows_are_split_below_the_general_threshold(native, engine):
     A = random_csr(rng, lens.size, k, lens, hi=4)
     for vt in (native.VAL_U32, native.VAL_U64):
         check_product(native, engine, A, B, vt)
+
+
+@pytest.mark.parametrize("avg", [1, 3, 9, 40, 200])
+@pytest.mark.parametrize("vt", ["VAL_U32", "VAL_U64"])
+def test_analysis_at_every_row_length(native, engine, avg, vt):
+    """The average row sets the lanes per row; rows past 64 times that many
+    entries, past a piece of the grid's and past two pieces go other ways."""
+    rng = np.random.default_rng(avg)
+    k, n = 6000, 700
+    lens = np.concatenate([rng.integers(0, 2 * avg + 1, 900), [130, 257, 600, 2047, 2048, 2049, 4096, 4097, 6000]])
+    A = random_csr(rng, lens.size, k, rng.permutation(lens), hi=5)
+    B = random_csr(rng, k, n, rng.integers(0, 6, k), hi=5)
+    check_product(native, engine, A, B, getattr(native, vt))
+    ones = sp.csr_matrix((np.ones(A.nnz, np.uint64), A.indices, A.indptr), shape=A.shape)
+    check_product(native, engine, ones, B, getattr(native, vt))
+
+
+@pytest.mark.parametrize("n", [40, 5000, 60000])
+@pytest.mark.parametrize("over", [0, 1])
+def test_uint32_overflow_is_seen_at_its_exact_limit(native, engine, n, over):
+    """A count of 2^32 - 1 is no overflow, 2^32 is one, beside columns whose
+    totals alone pass 2^32."""
+    k = 70
+    vals = np.array([2 ** 31, 2 ** 30, 2 ** 30 - (k - 3)] + [1] * (k - 3), np.uint64)     # sums to 2^32
+    if not over:
+        vals[-1] = 0
+    cols = np.stack([np.full(k, n - 1), np.arange(k) % (n - 1)], 1)
+    other = np.where(np.arange(k) < n - 1, 2 ** 31, 1).astype(np.uint64)[: k]
+    other[n - 1:] = 1
+    B = sp.csr_matrix((np.stack([vals, other], 1).reshape(-1), (np.repeat(np.arange(k), 2), cols.reshape(-1))),
+                      shape=(k, n))
+    A = sp.csr_matrix(np.ones((1, k), np.uint64))
+    h = ctypes.c_void_p()
+    Am, Bm = upload(native, engine, A, native.VAL_U32), upload(native, engine, B, native.VAL_U32)
+    rc = native.lib().rmcm_spgemm(engine._h, Am._h, Bm._h, ctypes.byref(h))
+    C = native.Matrix(engine, h.value)
+    assert rc == (native.EOVERFLOW if over else native.OK)
+    if not over:
+        rp, col, val = C.download()
+        assert col[-1] == n - 1 and int(val[-1]) == 2 ** 32 - 1
