@@ -1566,6 +1566,7 @@ __global__ void __launch_bounds__(NT) k_hash(DevCsr A, DevCsr B, DevCsr C, const
 }
 
 #include "row_kernels.cuh"
+#include "sort_rows.cuh"
 
 // ------------------------------------------------------------------------
 // dense bin: one CTA per row, windowed presence bytes + counters in shared memory
@@ -2861,6 +2862,25 @@ DenseExtra dense_extra(const DenseTemp *t, bool single_pass) {
     return e;
 }
 
+// The bins of the 512- and 2048-slot hash tables hold rows of at most 2^bits
+// (256 and 1024) products at the default load of 0.5 and below; k_sort takes
+// them when the columns leave that many bits of a 32-bit key.
+inline bool sort_takes(const rmcm_handle *h, int64_t ncols, int bits) {
+    return h->tune.hash_load <= 0.5 && ncols <= (1LL << (32 - bits));
+}
+
+template <typename V, int BITS>
+int32_t launch_sort(rmcm_handle *h, const DevCsr &A, const DevCsr &B, bool a_ones, bool b_ones, const DevCsr &C,
+                    const int32_t *rows, int32_t n, int64_t *cnt, const uint8_t *bin_of) {
+    const int64_t sm = kSortWarps * (int64_t)sizeof(SortStage<V, BITS>);
+    auto kern = k_sort<V, BITS>;
+    RMCM_TRY(set_smem(h, kern, sm));
+    const int per_sm = std::max(1, occupancy(h, kern, kSortWarps * 32, sm));
+    kern<<<grid_for(h, (int64_t)n * 32, kSortWarps * 32, per_sm), kSortWarps * 32, sm, h->stream>>>(
+        A, B, a_ones, b_ones, C, rows, n, cnt, h->d_status, bin_of);
+    return RMCM_OK;
+}
+
 // Operands of the row kernels (row_kernels.cuh), for the products they take.
 template <typename V>
 struct LeanArgs {
@@ -2899,7 +2919,8 @@ template <typename V, bool NUMERIC>
 int32_t launch_bins(rmcm_handle *h, const DevCsr &A, const DevCsr &B, const DevCsr &C, const int32_t *lists,
                     const int32_t *counts, int32_t dense_max_alen, int64_t *cnt, int32_t *cursor_base,
                     int64_t cursor_cap, const DenseTemp *temp, const uint8_t *bin_of, bool positive,
-                    bool b_distinct, const RankSplit *rs, const LeanArgs<V> *lean, uint32_t bin_mask = ~0u) {
+                    bool b_distinct, const RankSplit *rs, const LeanArgs<V> *lean, bool a_ones, bool b_ones,
+                    uint32_t bin_mask = ~0u) {
     cudaStream_t s = h->stream;
     int *st = h->d_status;
     int32_t off = 0;
@@ -2948,6 +2969,10 @@ int32_t launch_bins(rmcm_handle *h, const DevCsr &A, const DevCsr &B, const DevC
                 break;
             }
             case kBinHash512: {
+                if (NUMERIC && sort_takes(h, ncols, 8)) {
+                    RMCM_TRY((launch_sort<V, 8>(h, A, B, a_ones, b_ones, C, list, n, cnt, bin_of)));
+                    break;
+                }
                 constexpr int S = 512, NT = 128;
                 const int64_t sm = S * 4 + (NUMERIC ? S * sizeof(V) : 0);
                 auto kern = k_hash<V, NUMERIC, S, NT>;
@@ -2956,6 +2981,10 @@ int32_t launch_bins(rmcm_handle *h, const DevCsr &A, const DevCsr &B, const DevC
                 break;
             }
             case kBinHash2k: {
+                if (NUMERIC && sort_takes(h, ncols, 10)) {
+                    RMCM_TRY((launch_sort<V, 10>(h, A, B, a_ones, b_ones, C, list, n, cnt, bin_of)));
+                    break;
+                }
                 constexpr int S = 2048, NT = 256;
                 const int64_t sm = S * 4 + (NUMERIC ? S * sizeof(V) : 0);
                 auto kern = k_hash<V, NUMERIC, S, NT>;
@@ -3712,11 +3741,11 @@ int32_t spgemm_t(rmcm_handle *h, const rmcm_mat *Am, const rmcm_mat *Bm, rmcm_ma
         T.val = stemp.val;
         T.nnz = stemp.total;
         rc = launch_bins<V, true>(h, A, B, T, lists, counts, dense_max_alen, cnt, cursors, cursor_cap, &dtemp, bin_of,
-                                  positive, Bm->distinct, &rsplit, lean, short_mask);
+                                  positive, Bm->distinct, &rsplit, lean, Am->ones, Bm->ones, short_mask);
     }
     if (rc == RMCM_OK)
         rc = launch_bins<V, false>(h, A, B, C->d, lists, counts, dense_max_alen, cnt, cursors, cursor_cap, &dtemp,
-                                   bin_of, positive, Bm->distinct, &rsplit, lean, other_bins);
+                                   bin_of, positive, Bm->distinct, &rsplit, lean, Am->ones, Bm->ones, other_bins);
     if (rc == RMCM_OK)
         rc = scan_rowptr(h, cnt, m, C->d.rowptr, tiles, (unsigned long long *)(small + 44), replay ? plan->nnz : -1);
     if (rec) cudaEventRecord(h->prof[rec_idx].ev[3], s);
@@ -3774,7 +3803,7 @@ int32_t spgemm_t(rmcm_handle *h, const rmcm_mat *Am, const rmcm_mat *Bm, rmcm_ma
     }
     if (rc == RMCM_OK && !adopt)
         rc = launch_bins<V, true>(h, A, B, C->d, lists, counts, dense_max_alen, nullptr, cursors, cursor_cap, &dtemp,
-                                  bin_of, positive, Bm->distinct, &rsplit, lean, other_bins);
+                                  bin_of, positive, Bm->distinct, &rsplit, lean, Am->ones, Bm->ones, other_bins);
     drop_short();
     const int32_t gemm_limbs = dtemp.dpart.S ? dtemp.dpart.limbs * dtemp.dpart.alimbs : 0;
     const int64_t gemm_inner = dtemp.dpart.S ? dtemp.dpart.heavy : 0;

@@ -189,3 +189,55 @@ def test_uint32_overflow_is_seen_at_its_exact_limit(native, engine, n, over):
     if not over:
         rp, col, val = C.download()
         assert col[-1] == n - 1 and int(val[-1]) == 2 ** 32 - 1
+
+
+@pytest.mark.parametrize("vt", ["VAL_U32", "VAL_U64"])
+@pytest.mark.parametrize("n", [41000, 100003, 2 ** 22, 2 ** 22 + 1, 2 ** 24, 2 ** 24 + 1])
+def test_sorted_rows_at_their_limits(native, engine, n, vt):
+    """Rows of exactly 33, 127..129, 255..257, 511..513 and 1023..1025 products
+    on outputs around the widest whose columns fit a key; few distinct columns,
+    the last one among them; B rows of every length up to one of 1,025."""
+    rng = np.random.default_rng(n % 1000)
+    want = [33, 64, 127, 128, 129, 255, 256, 257, 511, 512, 513, 1023, 1024, 1025]
+    parts = [1, 2, 7, 8, 9, 31, 64, 65, 200]
+    brow, acol, alen = [], [], []
+    for w in want:
+        for style in range(3):
+            left, used = w, 0
+            while left:
+                x = left if style == 0 else min(left, int(rng.choice(parts[: 4 + 5 * (style == 1)])))
+                acol.append(len(brow))
+                brow.append(x)
+                left -= x
+                used += 1
+            alen.append(used)
+    k = len(brow)
+    pool = np.unique(np.concatenate([rng.integers(0, n, 1500), [0, n - 1]]))
+    cols = [np.sort(rng.choice(pool, x, replace=False)) for x in brow]
+    cols[0][-1] = n - 1
+    rp = np.concatenate([[0], np.cumsum(brow)])
+    B = sp.csr_matrix((rng.integers(1, 50, rp[-1], dtype=np.uint64), np.concatenate(cols), rp), shape=(k, n))
+    ap = np.concatenate([[0], np.cumsum(alen)])
+    A = sp.csr_matrix((rng.integers(1, 50, k, dtype=np.uint64), np.array(acol), ap), shape=(len(alen), k))
+    check_product(native, engine, A, B, getattr(native, vt))
+
+
+@pytest.mark.parametrize("terms", [40, 200, 700])
+def test_sorted_rows_report_overflow(native, engine, terms):
+    """Equal columns that only together pass the value type, in one lane's
+    share of the sorted row and across many lanes'."""
+    n = 60000
+    for vt, top in ((native.VAL_U32, 32), (native.VAL_U64, 64)):
+        each = -(-2 ** top // terms)
+        for over in (0, 1):
+            v = np.full(terms, each if over else each - 1, np.uint64)
+            rp = np.arange(terms + 1, dtype=np.int64)
+            col = np.full(terms, 12345, np.int32)
+            Am = engine.upload(np.array([0, terms]), np.arange(terms, dtype=np.int32), cols=terms, valtype=vt)
+            Bm = engine.upload(rp, col, cols=n, val=v, valtype=vt)
+            h = ctypes.c_void_p()
+            rc = native.lib().rmcm_spgemm(engine._h, Am._h, Bm._h, ctypes.byref(h))
+            C = native.Matrix(engine, h.value)
+            assert rc == (native.EOVERFLOW if over else native.OK)
+            if not over:
+                assert int(C.download()[2][0]) == terms * (each - 1)
