@@ -10,18 +10,19 @@
 //
 // One launch per level i computes every j > i at once, so each M_i is read
 // once: a level stores q = 1 - r (r rounded first, then 1 - r rounded, the
-// value the reference's next level forms) row-major as q[v * len + j], so
-// the next level multiplies the gathered q directly and a row's gathers for
-// all j are one contiguous run of doubles.
-// Mapping: a warp per row; the warp is split into G groups of JP lanes
-// (JP = next power of two >= number of j), lane (g, j) multiplies the factors
-// of entries g, g+G, ... for target j, and the G partial products are
+// value the reference's next level forms), the len - i values of a row one
+// after another (its own, then targets i + 1 ..), so the next level multiplies
+// the gathered q directly, a row's gathers for all j are one contiguous run of
+// doubles, and no level's table is wider than its targets.
+// Mapping: lane (row, g, jo) multiplies the factors of entries g, g + G, ...
+// of its row for target i + 1 + jo, and the G partial products of a row are
 // combined with shuffles in a fixed order.  Sums of c_ij are per-warp, then
-// per-block (fixed warp order), then a one-block pass over the block partials
-// (fixed order): the estimate is bit-for-bit reproducible run to run.
+// per-block (fixed warp order), then a pass over the block partials (fixed
+// order): the estimate is bit-for-bit reproducible run to run.
 // Every multiply and add is an explicit round-to-nearest intrinsic, so no
 // fused multiply-add changes the rounding against the reference's
 // `tmp_rho *= (1 - r)` and `nnz += s * dim`.
+#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -48,152 +49,257 @@ struct LevelArgs {
     double dims[kMaxLen];   // dims[j] = cols of M_j
 };
 
-// prod over entries k = k0, k0 + G, ... < k1 of q_next[col_k][j] (= 1 - r).
-// A lane with at least four entries keeps four independent partial products
-// (entries taken in turn) so four gathers and multiply chains are in flight,
-// combined in a fixed order ((p0 p1)(p2 p3)); a shorter run multiplies
-// serially (no combining multiplies).  Reproducible run to run.
-__device__ __forceinline__ double factor_product(const DevCsr &M, const double *q_next, int32_t len, int j,
-                                                 int64_t k0, int64_t k1, int G) {
-    int64_t k = k0;
-    if (k + 3 * (int64_t)G < k1) {
-        double p[4] = {1.0, 1.0, 1.0, 1.0};
-        for (; k + 3 * (int64_t)G < k1; k += 4 * (int64_t)G) {
-            int32_t v[4];
+// prod over entries k = k0, k0 + G, ... < k1 of q_next[col_k * stride] (= 1 - r)
+// for the rows that several warps share: eight independent partial products
+// per lane, the next entries' columns loaded while the factors arrive, so one
+// gather's latency a step of eight; combined in a fixed order.
+__device__ __forceinline__ double factor_product(const DevCsr &M, const double *q_next, int32_t stride, int64_t k0,
+                                                 int64_t k1, int G) {
+    constexpr int U = 8;
+    double p[U];
+    int32_t v[U];
 #pragma unroll
-            for (int u = 0; u < 4; u++) v[u] = M.col[k + u * G];
-            double q[4];
-#pragma unroll
-            for (int u = 0; u < 4; u++) q[u] = q_next[(int64_t)v[u] * len + j];
-#pragma unroll
-            for (int u = 0; u < 4; u++) p[u] = __dmul_rn(p[u], q[u]);
-        }
-        // the last 0..3 entries, into p[0], p[1], p[2] in turn
-#pragma unroll
-        for (int u = 0; u < 3; u++) {
-            if (k < k1) {
-                p[u] = __dmul_rn(p[u], q_next[(int64_t)M.col[k] * len + j]);
-                k += G;
-            }
-        }
-        return __dmul_rn(__dmul_rn(p[0], p[1]), __dmul_rn(p[2], p[3]));
+    for (int u = 0; u < U; u++) {
+        p[u] = 1.0;
+        v[u] = k0 + u * (int64_t)G < k1 ? __ldg(M.col + k0 + u * (int64_t)G) : -1;
     }
-    double p = 1.0;
-    for (; k < k1; k += G) p = __dmul_rn(p, q_next[(int64_t)M.col[k] * len + j]);
-    return p;
+    for (int64_t k = k0; k < k1; k += U * (int64_t)G) {
+        double q[U];
+#pragma unroll
+        for (int u = 0; u < U; u++) q[u] = v[u] >= 0 ? __ldg(q_next + (int64_t)v[u] * stride) : 1.0;
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+            const int64_t kn = k + (U + u) * (int64_t)G;
+            v[u] = kn < k1 ? __ldg(M.col + kn) : -1;
+        }
+#pragma unroll
+        for (int u = 0; u < U; u++) p[u] = __dmul_rn(p[u], q[u]);
+    }
+    return __dmul_rn(__dmul_rn(__dmul_rn(p[0], p[1]), __dmul_rn(p[2], p[3])),
+                     __dmul_rn(__dmul_rn(p[4], p[5]), __dmul_rn(p[6], p[7])));
 }
 
-// Rows per warp step: 32 when every warp of a full grid (blocks_cap CTAs)
-// still gets several steps, fewer for short matrices so that warps stay busy.
+// Rows per warp and chunk: 32 when that leaves a quarter of a full grid's
+// warps (blocks_cap CTAs) with a chunk, fewer for shorter matrices.
 inline int32_t level_tile(int64_t rows, int64_t blocks_cap) {
-    const int64_t warps = blocks_cap * (kEstThreads / 32);
+    const int64_t warps = blocks_cap * (kEstThreads / 32) / 4;
     int32_t t = 32;
-    while (t > 1 && rows < warps * t * 4) t >>= 1;
+    while (t > 1 && rows < warps * t) t >>= 1;
     return t;
 }
 
 // One level of one chain, as CTA `bid` of `nblk` (the same work split and
 // summation order whether the CTA belongs to a one-chain launch or to a
 // launch over many chains).
+//
+// Bound by the FP64 pipe: a warp's multiply holds it for many cycles whatever
+// its active lanes, so lanes are packed.  The warp's rows take 1, 2, 4 ..
+// groups of jp lanes, enough for four entries a lane (32 / jp groups at most),
+// and are laid out group after group, the largest first: every step multiplies
+// 32 / jp groups' entries, three multiplies and one per halving of the largest
+// row in it.  A row of more than kWideLane entries a lane would hold up the
+// warp; the CTA's warps multiply a slice of each such row together afterwards.
+// Against a row per warp step (one to three of 32 lanes busy on most rows of a
+// Zipf leaf) and 4,096 entries as one warp's share: a six-matrix chain over the
+// 1,000,000 x 300,000 leaf with 20M entries 1,626 -> 777 us in all (its two
+// 20M-entry levels 355 -> 200 and 353 -> 220 us, the 2,000-row level 377 -> 43,
+// the last matrix, a row per thread now, 54 -> 9, the nine rows of up to
+// 53,000 entries 183 -> 37).
+constexpr int kWideLane = 64;
+
 __device__ __forceinline__ void res_level_body(const DevCsr &M, const double *q_next, double *q_cur,
                                                const LevelArgs &la, double *partial, bool skip_long, int64_t bid,
                                                int64_t nblk) {
-    __shared__ double s_tp[kEstThreads / 32][32 * kMaxLen];   // tile products: [t * jp + jo]
+    constexpr int NW = kEstThreads / 32;
+    if (la.nj == 0) {
+        // the chain's last matrix: its own densities only, a row per thread
+        for (int64_t u = bid * kEstThreads + threadIdx.x; u < M.rows; u += nblk * kEstThreads) {
+            const double r = __ddiv_rn((double)(M.rowptr[u + 1] - M.rowptr[u]), la.dim_leaf);
+            q_cur[u] = __dsub_rn(1.0, r > 1.0 ? 1.0 : r);
+        }
+        return;
+    }
+    __shared__ double s_tp[NW][32 * kMaxLen];   // tile products: [t * jp + jo]
+    __shared__ double s_wide[NW][kMaxLen];      // slices of a wide row
+    __shared__ uint8_t s_ord[NW][32];           // the warp's rows, most groups first
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int G = 32 / la.jp;
-    const int g = lane / la.jp;
-    const int jo = lane % la.jp;                 // offset of j above i+1
+    const unsigned lt_mask = (1u << lane) - 1u;
+    const int T = la.tile;                      // rows per warp and chunk (1 .. 32)
+    const int jp = la.jp, qs = la.nj + 1;       // values per row of q_cur
+    const int ng = 32 / jp;                     // groups per step
+    const int emax = 31 - __clz(ng);
+    const int64_t wide_min = kWideLane * (int64_t)ng;
+    const int jo = lane & (jp - 1);             // target i + 1 + jo
     const bool active_j = jo < la.nj;
-    const int j = la.i + 1 + jo;
-    const double dimj = active_j ? la.dims[j] : 0.0;
-    double term_sum = 0.0;                       // this lane's rows of target j
-    const int T = la.tile;                       // rows per warp step (1 .. 32)
+    const double dimj = active_j ? la.dims[la.i + 1 + jo] : 0.0;
+    double term_sum = 0.0;                      // this lane's rows of target jo
     double *tp = s_tp[warp];
-    const int64_t nwarps = (nblk * blockDim.x) >> 5;
-    for (int64_t t0 = ((bid * blockDim.x + threadIdx.x) >> 5) * T; t0 < M.rows; t0 += nwarps * T) {
+    for (int64_t c0 = bid * (NW * T); c0 < M.rows; c0 += nblk * (NW * T)) {
+        const int64_t t0 = c0 + (int64_t)warp * T;
+        const int nrow = t0 >= M.rows ? 0 : M.rows - t0 < (int64_t)T ? (int)(M.rows - t0) : T;
         // r_ii of the tile's rows, a lane each (one division for T rows)
         int64_t my_a0 = 0, my_len = 0;
-        if (lane < T && t0 + lane < M.rows) {
+        if (lane < nrow) {
             const int64_t ul = t0 + lane;
             my_a0 = M.rowptr[ul];
             my_len = M.rowptr[ul + 1] - my_a0;
             double r = __ddiv_rn((double)my_len, la.dim_leaf);
             r = r > 1.0 ? 1.0 : r;
-            q_cur[ul * la.len + la.i] = __dsub_rn(1.0, r);
+            q_cur[ul * qs] = __dsub_rn(1.0, r);
         }
-        if (la.nj == 0) continue;
-        const int nrow = M.rows - t0 < (int64_t)T ? (int)(M.rows - t0) : T;
-        uint32_t skipped = 0;
-        for (int t = 0; t < nrow; t++) {
-            const int64_t a0 = __shfl_sync(kFull, my_a0, t), rl = __shfl_sync(kFull, my_len, t);
-            if (skip_long && rl > kEstLongRow) {   // a CTA of k_res_long takes it
-                skipped |= 1u << t;
-                continue;
+        const bool is_long = skip_long && my_len > kEstLongRow;   // a cluster of k_res_long takes it
+        const uint32_t skipped = __ballot_sync(kFull, is_long);
+        const uint32_t wide = __ballot_sync(kFull, !is_long && my_len > wide_min);
+        // the row's groups: 2^e of them, -1 for none (its product is 1, or
+        // another part of the kernel's)
+        int e = -1;
+        if (lane < nrow && my_len > 0 && !(((skipped | wide) >> lane) & 1u)) {
+            e = my_len <= 4 ? 0 : 32 - __clz((int)((my_len + 3) / 4 - 1));
+            e = e < emax ? e : emax;
+        }
+        if (lane < nrow && my_len == 0)
+            for (int x = 0; x < la.nj; x++) tp[lane * jp + x] = 1.0;
+        // class x's rows take groups base[x] .. in order of rank, from place[x]
+        int base[6], place[6], groups = 0, placed = 0;
+#pragma unroll
+        for (int x = 5; x >= 0; x--) {
+            const unsigned of = __ballot_sync(kFull, e == x);
+            base[x] = groups;
+            place[x] = placed;
+            if (e == x) s_ord[warp][placed + __popc(of & lt_mask)] = (uint8_t)lane;
+            groups += __popc(of) << x;
+            placed += __popc(of);
+        }
+        __syncwarp();
+        for (int s0 = 0; s0 < groups; s0 += ng) {
+            // this lane's group, and the class it lies in: the least with
+            // base <= s (bases ascend as classes descend)
+            const bool live = s0 + lane / jp < groups;
+            const int s = live ? s0 + lane / jp : groups - 1;
+            int x = 5, bx = base[5], px = place[5];
+#pragma unroll
+            for (int y = 4; y >= 0; y--) {
+                if (s >= base[y]) {
+                    x = y;
+                    bx = base[y];
+                    px = place[y];
+                }
             }
-            double prod = 1.0;
-            if (active_j) prod = factor_product(M, q_next, la.len, j, a0 + g, a0 + rl, G);
-            // combine the group products (fixed butterfly order); groups past
-            // the row's entries hold exactly 1.0, so those steps are skipped
-            const int ng = rl < (int64_t)G ? (int)rl : G;
-            for (int d = la.jp; d < 32 && d < la.jp * ng; d <<= 1) {
-                const double o = __shfl_xor_sync(kFull, prod, d);
-                prod = __dmul_rn(prod, o);
+            const int t = s_ord[warp][px + ((s - bx) >> x)];
+            const int G = 1 << x, g = (s - bx) & (G - 1);
+            const int64_t a0 = __shfl_sync(kFull, my_a0, t);
+            const int64_t rl = __shfl_sync(kFull, my_len, t);
+            int64_t k = a0 + g;
+            const int64_t k1 = live && active_j ? a0 + rl : a0;
+            double p[4];
+#pragma unroll
+            for (int u = 0; u < 4; u++)
+                p[u] = k + u * G < k1 ? __ldg(q_next + (int64_t)__ldg(M.col + k + u * G) * la.nj + jo) : 1.0;
+            for (k += 4 * G; k < k1; k += 4 * G) {
+                double q[4];
+#pragma unroll
+                for (int u = 0; u < 4; u++)
+                    q[u] = k + u * G < k1 ? __ldg(q_next + (int64_t)__ldg(M.col + k + u * G) * la.nj + jo) : 1.0;
+#pragma unroll
+                for (int u = 0; u < 4; u++) p[u] = __dmul_rn(p[u], q[u]);
             }
-            if (g == 0 && active_j) tp[t * la.jp + jo] = prod;
+            double prod = __dmul_rn(__dmul_rn(p[0], p[1]), __dmul_rn(p[2], p[3]));
+            // a row's groups are consecutive and aligned to their number: combine
+            // them pairwise (fixed order); rows of fewer groups keep theirs
+            const int most = __reduce_max_sync(kFull, live ? x : 0);
+            for (int d = 0; d < most; d++) {
+                const double o = __shfl_xor_sync(kFull, prod, jp << d);
+                if (d < x) prod = __dmul_rn(prod, o);
+            }
+            if (live && g == 0 && active_j) tp[t * jp + jo] = prod;
+        }
+        // wide rows of the CTA's tiles, in row order: every warp a slice
+        if (__syncthreads_or(wide != 0)) {
+            __shared__ uint32_t s_mask[NW];
+            if (lane == 0) s_mask[warp] = wide;
+            __syncthreads();
+            const int G = 32 / jp, wg = lane / jp;
+            for (int w = 0; w < NW; w++) {
+                for (uint32_t m = s_mask[w]; m; m &= m - 1) {
+                    const int t = __ffs(m) - 1;
+                    const int64_t u = c0 + (int64_t)w * T + t;
+                    const int64_t a0 = M.rowptr[u], len = M.rowptr[u + 1] - a0;
+                    const int64_t k0 = a0 + len * warp / NW, k1 = a0 + len * (warp + 1) / NW;
+                    double prod = 1.0;
+                    if (active_j) prod = factor_product(M, q_next + jo, la.nj, k0 + wg, k1, G);
+                    for (int d = jp; d < 32; d <<= 1) prod = __dmul_rn(prod, __shfl_xor_sync(kFull, prod, d));
+                    if (wg == 0 && active_j) s_wide[warp][jo] = prod;
+                    __syncthreads();
+                    if ((int)threadIdx.x < la.nj) {
+                        double p = 1.0;
+                        for (int x = 0; x < NW; x++) p = __dmul_rn(p, s_wide[x][threadIdx.x]);
+                        s_tp[w][t * jp + threadIdx.x] = p;
+                    }
+                    __syncthreads();
+                }
+            }
         }
         __syncwarp();
         // per (row, target): r = 1 - prod, its term r * dim_j, and q = 1 - r
-        // for the next level; lane (g, jo) takes rows g, g + G, ...
+        // for the next level; a lane takes every (32 / jp)-th row
         if (active_j) {
-            for (int t = g; t < nrow; t += G) {
+            for (int t = lane / jp; t < nrow; t += 32 / jp) {
                 if ((skipped >> t) & 1u) continue;
-                const double r = __dsub_rn(1.0, tp[t * la.jp + jo]);
-                q_cur[(t0 + t) * la.len + j] = __dsub_rn(1.0, r);
+                const double r = __dsub_rn(1.0, tp[t * jp + jo]);
+                q_cur[(t0 + t) * qs + 1 + jo] = __dsub_rn(1.0, r);
                 term_sum = __dadd_rn(term_sum, __dmul_rn(r, dimj));
             }
         }
         __syncwarp();
     }
-    // this warp's sums per target, over the groups in a fixed order
-    for (int d = la.jp; d < 32; d <<= 1) term_sum = __dadd_rn(term_sum, __shfl_xor_sync(kFull, term_sum, d));
-    // block partials: partial[block * len + j]
-    __shared__ double s_part[kEstThreads / 32][kMaxLen];
-    if (g == 0 && active_j) s_part[warp][jo] = term_sum;
+    // this warp's sums per target, over its lanes in a fixed order
+    for (int d = jp; d < 32; d <<= 1) term_sum = __dadd_rn(term_sum, __shfl_xor_sync(kFull, term_sum, d));
+    // block partials: partial[block * kMaxLen + jo]
+    __shared__ double s_part[NW][kMaxLen];
+    if (lane < jp && active_j) s_part[warp][jo] = term_sum;
     __syncthreads();
     if (threadIdx.x < la.nj) {
         double acc = 0.0;
-        for (int w = 0; w < kEstThreads / 32; w++) acc = __dadd_rn(acc, s_part[w][threadIdx.x]);
+        for (int w = 0; w < NW; w++) acc = __dadd_rn(acc, s_part[w][threadIdx.x]);
         partial[bid * kMaxLen + threadIdx.x] = acc;
     }
 }
 
-__global__ void __launch_bounds__(kEstThreads) k_res_level(DevCsr M, const double *q_next, double *q_cur,
+__global__ void __launch_bounds__(kEstThreads, 5) k_res_level(DevCsr M, const double *q_next, double *q_cur,
                                                            LevelArgs la, double *partial, bool skip_long) {
     res_level_body(M, q_next, q_cur, la, partial, skip_long, blockIdx.x, gridDim.x);
 }
 
-// A CTA per long row (rows listed ascending): warp w multiplies the factors
-// of the w-th of 32 equal slices of the row, grouped as in k_res_level, and
-// the 32 warp products are combined in warp order.  The row's terms
-// s * dim_j go to partial[block], after the partials of k_res_level, so the
-// reduction still adds them in a fixed order.
-constexpr int kEstLongThreads = 1024;
+// A cluster of CTAs per long row (rows listed ascending): each of the
+// cluster's warps multiplies the factors of one of as many equal slices of the
+// row, the CTA's warp products are combined in warp order and the CTAs' (read
+// through distributed shared memory) in rank order.  One SM's FP64 pipe takes
+// 110 us for a row of 53,000 entries and five targets; eight take it in turn.
+// The row's terms s * dim_j go to the partial of its place in the list, after
+// the partials of k_res_level, so the reduction still adds them in a fixed
+// order.
+constexpr int kEstLongThreads = 256;
+constexpr int kEstLongCluster = 8;
 
 __device__ __forceinline__ void res_long_body(const DevCsr &M, const double *q_next, double *q_cur,
                                               const LevelArgs &la, const int32_t *long_rows, double *partial,
-                                              int64_t bid) {
-    __shared__ double s_prod[kEstLongThreads / 32][kMaxLen];
+                                              int64_t place) {
+    constexpr int NW = kEstLongThreads / 32, NS = NW * kEstLongCluster;
+    __shared__ double s_prod[NW][kMaxLen];
+    __shared__ double s_cta[kMaxLen];
+    cooperative_groups::cluster_group cluster = cooperative_groups::this_cluster();
+    const int rank = (int)cluster.block_rank();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int G = 32 / la.jp;
     const int g = lane / la.jp;
     const int jo = lane % la.jp;
-    const bool active_j = jo < la.nj && g < G;
-    const int j = la.i + 1 + jo;
-    const int64_t u = long_rows[bid];
+    const bool active_j = jo < la.nj;
+    const int64_t u = long_rows[place];
     const int64_t a0 = M.rowptr[u], len = M.rowptr[u + 1] - a0;
-    const int64_t k0 = a0 + len * warp / (kEstLongThreads / 32), k1 = a0 + len * (warp + 1) / (kEstLongThreads / 32);
+    const int slice = rank * NW + warp;
+    const int64_t k0 = a0 + len * slice / NS, k1 = a0 + len * (slice + 1) / NS;
     double prod = 1.0;
-    if (active_j) prod = factor_product(M, q_next, la.len, j, k0 + g, k1, G);
+    if (active_j) prod = factor_product(M, q_next + jo, la.nj, k0 + g, k1, G);
     for (int d = la.jp; d < 32; d <<= 1) {
         const double o = __shfl_xor_sync(kFull, prod, d);
         prod = __dmul_rn(prod, o);
@@ -202,39 +308,57 @@ __device__ __forceinline__ void res_long_body(const DevCsr &M, const double *q_n
     __syncthreads();
     if ((int)threadIdx.x < la.nj) {
         double p = 1.0;
-        for (int w = 0; w < kEstLongThreads / 32; w++) p = __dmul_rn(p, s_prod[w][threadIdx.x]);
-        const int jj = la.i + 1 + threadIdx.x;
+        for (int w = 0; w < NW; w++) p = __dmul_rn(p, s_prod[w][threadIdx.x]);
+        s_cta[threadIdx.x] = p;
+    }
+    cluster.sync();
+    if (rank == 0 && (int)threadIdx.x < la.nj) {
+        double p = s_cta[threadIdx.x];
+        for (int c = 1; c < kEstLongCluster; c++) p = __dmul_rn(p, cluster.map_shared_rank(s_cta, c)[threadIdx.x]);
         const double sv = __dsub_rn(1.0, p);
-        q_cur[u * la.len + jj] = __dsub_rn(1.0, sv);   // q = 1 - r for the next level
-        partial[bid * kMaxLen + threadIdx.x] = __dmul_rn(sv, la.dims[jj]);
+        q_cur[u * (la.nj + 1) + 1 + threadIdx.x] = __dsub_rn(1.0, sv);   // q = 1 - r for the next level
+        partial[place * kMaxLen + threadIdx.x] = __dmul_rn(sv, la.dims[la.i + 1 + threadIdx.x]);
     }
+    cluster.sync();   // the products are read: the CTAs may go
 }
 
-__global__ void __launch_bounds__(kEstLongThreads) k_res_long(DevCsr M, const double *q_next, double *q_cur,
-                                                              LevelArgs la, const int32_t *long_rows,
-                                                              double *partial) {
-    res_long_body(M, q_next, q_cur, la, long_rows, partial, blockIdx.x);
+__global__ void __cluster_dims__(kEstLongCluster, 1, 1) __launch_bounds__(kEstLongThreads)
+    k_res_long(DevCsr M, const double *q_next, double *q_cur, LevelArgs la, const int32_t *long_rows, double *partial) {
+    res_long_body(M, q_next, q_cur, la, long_rows, partial, blockIdx.x / kEstLongCluster);
 }
 
-// One block: c[i*len + j] = sum over blocks (fixed pairwise order).
-__device__ __forceinline__ void res_reduce_body(const double *partial, int32_t nblocks, const LevelArgs &la, double *c) {
+// One block, target jo: c[i*len + j] = sum over blocks (fixed pairwise order).
+__device__ __forceinline__ void res_reduce_body(const double *partial, int32_t nblocks, int32_t len, int32_t i, int jo,
+                                                double *c) {
     __shared__ double s[256];
-    for (int jo = 0; jo < la.nj; jo++) {
-        double acc = 0.0;
-        for (int b = threadIdx.x; b < nblocks; b += blockDim.x) acc = __dadd_rn(acc, partial[(int64_t)b * kMaxLen + jo]);
-        s[threadIdx.x] = acc;
-        __syncthreads();
-        for (int w = blockDim.x / 2; w > 0; w >>= 1) {
-            if ((int)threadIdx.x < w) s[threadIdx.x] = __dadd_rn(s[threadIdx.x], s[threadIdx.x + w]);
-            __syncthreads();
-        }
-        if (threadIdx.x == 0) c[la.i * la.len + la.i + 1 + jo] = s[0];
+    double acc = 0.0;
+    for (int b = threadIdx.x; b < nblocks; b += blockDim.x) acc = __dadd_rn(acc, partial[(int64_t)b * kMaxLen + jo]);
+    s[threadIdx.x] = acc;
+    __syncthreads();
+    for (int w = blockDim.x / 2; w > 0; w >>= 1) {
+        if ((int)threadIdx.x < w) s[threadIdx.x] = __dadd_rn(s[threadIdx.x], s[threadIdx.x + w]);
         __syncthreads();
     }
+    if (threadIdx.x == 0) c[i * len + i + 1 + jo] = s[0];
 }
 
+// A CTA per target of one level.
 __global__ void __launch_bounds__(256) k_res_reduce(const double *partial, int32_t nblocks, LevelArgs la, double *c) {
-    res_reduce_body(partial, nblocks, la, c);
+    res_reduce_body(partial, nblocks, la.len, la.i, blockIdx.x, c);
+}
+
+// Every estimate of a chain in one launch: CTA (j, i) sums level i's partials
+// of target j, or clears an entry on or below the diagonal.
+struct ReduceArgs {
+    int32_t len;
+    int32_t nblocks[kMaxLen];       // partials of each level
+    int32_t first[kMaxLen];         // its first one
+};
+
+__global__ void __launch_bounds__(256) k_res_reduce_all(const double *partial, ReduceArgs ra, double *c) {
+    const int i = blockIdx.y, j = blockIdx.x;
+    if (j > i) res_reduce_body(partial + (int64_t)ra.first[i] * kMaxLen, ra.nblocks[i], ra.len, i, j - i - 1, c);
+    else if (threadIdx.x == 0) c[i * ra.len + j] = 0.0;
 }
 
 // Many chains at once: job j is one level of one chain, exactly the launch
@@ -264,21 +388,23 @@ __device__ __forceinline__ int find_job(const LevelJob *jobs, int njobs, int64_t
     return lo;
 }
 
-__global__ void __launch_bounds__(kEstThreads) k_res_level_multi(const LevelJob *jobs, int32_t njobs) {
+__global__ void __launch_bounds__(kEstThreads, 5) k_res_level_multi(const LevelJob *jobs, int32_t njobs) {
     const LevelJob &jb = jobs[find_job(jobs, njobs, blockIdx.x, false)];
     res_level_body(jb.M, jb.q_next, jb.q_cur, jb.la, jb.partial, jb.nlong > 0, (int64_t)blockIdx.x - jb.first,
                    jb.blocks);
 }
 
-__global__ void __launch_bounds__(kEstLongThreads) k_res_long_multi(const LevelJob *jobs, int32_t njobs) {
-    const LevelJob &jb = jobs[find_job(jobs, njobs, blockIdx.x, true)];
-    res_long_body(jb.M, jb.q_next, jb.q_cur, jb.la, jb.long_rows, jb.partial + jb.blocks * kMaxLen,
-                  (int64_t)blockIdx.x - jb.lfirst);
+__global__ void __cluster_dims__(kEstLongCluster, 1, 1) __launch_bounds__(kEstLongThreads)
+    k_res_long_multi(const LevelJob *jobs, int32_t njobs) {
+    const int64_t place = blockIdx.x / kEstLongCluster;
+    const LevelJob &jb = jobs[find_job(jobs, njobs, place, true)];
+    res_long_body(jb.M, jb.q_next, jb.q_cur, jb.la, jb.long_rows, jb.partial + jb.blocks * kMaxLen, place - jb.lfirst);
 }
 
 __global__ void __launch_bounds__(256) k_res_reduce_multi(const LevelJob *jobs) {
     const LevelJob &jb = jobs[blockIdx.x];
-    if (jb.la.nj > 0) res_reduce_body(jb.partial, (int32_t)(jb.blocks + jb.nlong), jb.la, jb.c);
+    if ((int)blockIdx.y < jb.la.nj)
+        res_reduce_body(jb.partial, (int32_t)(jb.blocks + jb.nlong), jb.la.len, jb.la.i, blockIdx.y, jb.c);
 }
 
 }  // namespace
@@ -295,16 +421,27 @@ int32_t estimate(rmcm_handle *h, rmcm_mat *const *chain, int32_t len, double *c_
     }
     // grid is fixed by the row count only, so the reduction order is stable
     const int64_t blocks_cap = (int64_t)h->sm_count * 8;
-    int64_t long_cap = 0;
-    for (int i = 0; i < len; i++) long_cap = std::max<int64_t>(long_cap, chain[i]->n_est_long);
     auto al = [](int64_t x) { return (x + 255) & ~255LL; };
     const int64_t rbytes = al(8 * max_rows * len);
-    const int64_t pbytes = al(8 * (blocks_cap + long_cap) * kMaxLen);
+    // block partials of every level, one after another, summed by one launch
+    ReduceArgs ra{};
+    ra.len = len;
+    int64_t nparts = 0;
+    for (int i = len - 1; i >= 0; i--) {
+        const int64_t rows = chain[i]->d.rows, tile = level_tile(rows, blocks_cap);
+        const int64_t blocks = std::max<int64_t>(
+            1, std::min((rows + tile * (kEstThreads / 32) - 1) / (tile * (kEstThreads / 32)), blocks_cap));
+        const int32_t nlong = i < len - 1 && chain[i]->n_est_long > 0 ? chain[i]->n_est_long : 0;
+        ra.first[i] = (int32_t)nparts;
+        ra.nblocks[i] = (int32_t)(blocks + nlong);
+        nparts += blocks + nlong;
+    }
+    const int64_t pbytes = al(8 * nparts * kMaxLen);
     double *r_a = nullptr, *r_b = nullptr, *part = nullptr;
     RMCM_TRY(dev_alloc(h, (void **)&r_a, 2 * rbytes + pbytes));
     r_b = (double *)((char *)r_a + rbytes);
     part = (double *)((char *)r_a + 2 * rbytes);
-    cudaError_t e = cudaMemsetAsync(c_dev, 0, sizeof(double) * len * len, s);
+    cudaError_t e = cudaSuccess;
     double *r_cur = r_a, *r_next = r_b;
     for (int i = len - 1; i >= 0 && e == cudaSuccess; i--) {
         const DevCsr &M = chain[i]->d;
@@ -318,24 +455,25 @@ int32_t estimate(rmcm_handle *h, rmcm_mat *const *chain, int32_t len, double *c_
         la.dim_leaf = (double)M.cols;
         for (int j = 0; j < len; j++) la.dims[j] = (double)chain[j]->d.cols;
         la.tile = level_tile(M.rows, blocks_cap);
-        int64_t blocks = (M.rows + (int64_t)la.tile * (kEstThreads / 32) - 1) / ((int64_t)la.tile * (kEstThreads / 32));
-        blocks = std::max<int64_t>(1, std::min(blocks, blocks_cap));
         // rows of more than kEstLongRow entries (known for uploaded matrices)
-        // get a whole CTA each
+        // get a cluster of CTAs each
         const int32_t nlong = la.nj > 0 && chain[i]->n_est_long > 0 ? chain[i]->n_est_long : 0;
-        k_res_level<<<(unsigned)blocks, kEstThreads, 0, s>>>(M, r_next, r_cur, la, part, nlong > 0);
+        const int32_t blocks = ra.nblocks[i] - nlong;
+        double *lp = part + (int64_t)ra.first[i] * kMaxLen;
+        k_res_level<<<(unsigned)blocks, kEstThreads, 0, s>>>(M, r_next, r_cur, la, lp, nlong > 0);
         h->launches++;
         if (nlong > 0) {
-            k_res_long<<<(unsigned)nlong, kEstLongThreads, 0, s>>>(M, r_next, r_cur, la, chain[i]->est_long,
-                                                                   part + blocks * kMaxLen);
-            h->launches++;
-        }
-        if (la.nj > 0) {
-            k_res_reduce<<<1, 256, 0, s>>>(part, (int32_t)(blocks + nlong), la, c_dev);
+            k_res_long<<<(unsigned)(nlong * kEstLongCluster), kEstLongThreads, 0, s>>>(M, r_next, r_cur, la, chain[i]->est_long,
+                                                                   lp + (int64_t)blocks * kMaxLen);
             h->launches++;
         }
         e = cudaGetLastError();
         std::swap(r_cur, r_next);
+    }
+    if (e == cudaSuccess) {
+        k_res_reduce_all<<<dim3((unsigned)len, (unsigned)len), 256, 0, s>>>(part, ra, c_dev);
+        h->launches++;
+        e = cudaGetLastError();
     }
     dev_free(h, r_a, 2 * rbytes + pbytes);
     if (e != cudaSuccess) return cuda_error(h, e, "estimator launch");
@@ -422,11 +560,13 @@ int32_t estimate_multi(rmcm_handle *h, const EstChain *chains, int32_t n, TableA
         k_res_level_multi<<<(unsigned)nb, kEstThreads, 0, s>>>((const LevelJob *)dp, (int32_t)jobs.size());
         h->launches++;
         if (nl > 0) {
-            k_res_long_multi<<<(unsigned)nl, kEstLongThreads, 0, s>>>((const LevelJob *)dp, (int32_t)jobs.size());
+            k_res_long_multi<<<(unsigned)(nl * kEstLongCluster), kEstLongThreads, 0, s>>>((const LevelJob *)dp, (int32_t)jobs.size());
             h->launches++;
         }
-        k_res_reduce_multi<<<(unsigned)jobs.size(), 256, 0, s>>>((const LevelJob *)dp);
-        h->launches++;
+        if (st > 0) {   // (the first step is every chain's last level: no targets)
+            k_res_reduce_multi<<<dim3((unsigned)jobs.size(), (unsigned)st), 256, 0, s>>>((const LevelJob *)dp);
+            h->launches++;
+        }
         e = cudaGetLastError();
     }
     dev_free(h, buf, std::max<int64_t>(off[n], 256));
@@ -538,7 +678,7 @@ extern "C" RMCM_API int32_t rmcm_estimate_noalloc(int32_t len, const int64_t *ro
         int64_t blocks = (M.rows + (int64_t)la.tile * (kEstThreads / 32) - 1) / ((int64_t)la.tile * (kEstThreads / 32));
         blocks = std::max<int64_t>(1, std::min(blocks, blocks_cap));
         k_res_level<<<(unsigned)blocks, kEstThreads, 0, s>>>(M, r_next, r_cur, la, part, false);
-        if (la.nj > 0) k_res_reduce<<<1, 256, 0, s>>>(part, (int32_t)blocks, la, c_dev);
+        if (la.nj > 0) k_res_reduce<<<(unsigned)la.nj, 256, 0, s>>>(part, (int32_t)blocks, la, c_dev);
         e = cudaGetLastError();
         std::swap(r_cur, r_next);
     }

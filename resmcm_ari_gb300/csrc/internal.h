@@ -118,7 +118,7 @@ struct rmcm_mat {
                                         // the largest value, then DevCsr::top
     int64_t max_row = -1;               // longest row (entries); -1 when unknown
     // rows longer than kEstLongRow entries, ascending (device), when known:
-    // the estimator gives each a whole CTA
+    // the estimator gives each a cluster of CTAs
     int32_t *est_long = nullptr;
     int32_t n_est_long = -1;            // -1: not known (the estimator walks every row per warp)
     cudaEvent_t xfer_done = nullptr;    // end of a pending asynchronous download (transfer stream)
@@ -178,7 +178,7 @@ struct rmcm_graph {
 
 namespace rmcm {
 
-// Rows with more entries than this get a whole CTA in the estimator.
+// Rows with more entries than this get a cluster of CTAs in the estimator.
 constexpr int64_t kEstLongRow = 4096;
 
 // ---- error plumbing ------------------------------------------------------

@@ -241,3 +241,54 @@ def test_sorted_rows_report_overflow(native, engine, terms):
             assert rc == (native.EOVERFLOW if over else native.OK)
             if not over:
                 assert int(C.download()[2][0]) == terms * (each - 1)
+
+
+def _estimates(mats, dims):
+    """The estimates in float64 from sums of logarithms."""
+    L = len(mats)
+    c = np.zeros((L, L))
+    after = {}
+    for i in range(L - 1, -1, -1):
+        rp, col = mats[i]
+        lens = np.diff(rp)
+        now = {i: np.minimum(1.0, lens / dims[i + 1])}
+        for j, r in after.items():
+            with np.errstate(divide="ignore"):
+                t = np.concatenate([np.log1p(-r)[col], [0.0]])
+            sums = np.where(lens > 0, np.add.reduceat(t, rp[:-1]), 0.0)
+            now[j] = -np.expm1(sums)
+            c[i, j] = now[j].sum() * dims[j + 1]
+        after = now
+    return c
+
+
+@pytest.mark.parametrize("length", [2, 3, 5, 9, 16])
+@pytest.mark.parametrize("n", [7, 900, 30000])
+def test_estimates_at_every_row_length(native, engine, length, n):
+    """Rows of every class of lanes (1 .. 4, 5 .. 8, ... entries), around the
+    length a CTA shares and the length a cluster takes, empty rows; chains from
+    one target to fifteen (1, 2, 4, 8 and 16 lanes a group).  A row's product of
+    up to 9,000 factors is off by at most 9,000 roundings of a value below 1,
+    1e-12; the densities here are above 1e-4, and their errors average out over
+    the rows: 1e-9 relative, the parity tolerance of the estimates."""
+    rng = np.random.default_rng(n + length)
+    mats, dims = [], [n]
+    special = [0, 1, 2, 3, 4, 5, 8, 9, 16, 17, 32, 33, 64, 65, 127, 128, 129, 130, 255, 257, 2047, 2049, 4095, 4096, 4097,
+               8192, 9000]
+    for i in range(length):
+        cols = int(rng.integers(9001, 12000)) if i < length - 1 else 5000
+        rows = dims[-1]
+        lens = rng.integers(0, 12, rows)
+        at = rng.choice(rows, min(rows, len(special)), replace=False)
+        lens[at] = rng.permutation(special)[: at.size]
+        lens = np.minimum(lens, cols)
+        rp = np.concatenate([[0], np.cumsum(lens)]).astype(np.int64)
+        col = np.concatenate([np.sort(rng.choice(cols, int(k), replace=False)) for k in lens]).astype(np.int32)
+        mats.append((rp, col))
+        dims.append(cols)
+    chain = [engine.upload(rp, col, cols=dims[i + 1]) for i, (rp, col) in enumerate(mats)]
+    got = engine.estimate(chain)
+    again = engine.estimate(chain)
+    assert np.array_equal(got, again)
+    want = _estimates(mats, dims)
+    np.testing.assert_allclose(got, want, rtol=1e-9, atol=0)
