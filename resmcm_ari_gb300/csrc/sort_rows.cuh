@@ -14,51 +14,69 @@ struct SortStage {
     V va[32];
 };
 
-// Ascending bitonic sort of 32 R keys, key i = lane R + r in k[r]: partners
-// less than R apart are registers of one lane, the others R / distance lanes
-// away.
+// Ascending sort of 32 R keys, key i = lane R + r in k[r], by merges of runs
+// of kk / 2: the first step of a merge compares mirror images (i with its
+// complement in the run of kk), which leaves every later step ascending, so
+// that a pair of registers costs a minimum and a maximum and no direction.
+// Partners less than R apart are registers of one lane, the others lie
+// distance / R lanes away.
 template <int R>
-__device__ __forceinline__ void bitonic_sort(uint32_t (&k)[R], int lane) {
+__device__ __forceinline__ void merge_sort(uint32_t (&k)[R], int lane) {
 #pragma unroll
     for (int kk = 2; kk <= 32 * R; kk <<= 1) {
+        if (kk <= R) {
 #pragma unroll
-        for (int j = kk >> 1; j > 0; j >>= 1) {
+            for (int r = 0; r < R; r++) {
+                const int o = r ^ (kk - 1);
+                if (r > o) continue;
+                const uint32_t lo = min(k[r], k[o]), hi = max(k[r], k[o]);
+                k[r] = lo;
+                k[o] = hi;
+            }
+        } else {
+            const bool low = (lane & (kk / (2 * R))) == 0;
+            uint32_t o[R];
+#pragma unroll
+            for (int r = 0; r < R; r++) o[r] = __shfl_xor_sync(kFull, k[R - 1 - r], kk / R - 1);
+#pragma unroll
+            for (int r = 0; r < R; r++) k[r] = low ? min(k[r], o[r]) : max(k[r], o[r]);
+        }
+#pragma unroll
+        for (int j = kk >> 2; j > 0; j >>= 1) {
             if (j >= R) {
-                const int d = j / R;
-                const bool up = kk >= 32 * R || (lane & (kk / R)) == 0;
-                const bool keep_min = ((lane & d) == 0) == up;
+                const bool low = (lane & (j / R)) == 0;
 #pragma unroll
                 for (int r = 0; r < R; r++) {
-                    const uint32_t o = __shfl_xor_sync(kFull, k[r], d);
-                    k[r] = keep_min ? min(k[r], o) : max(k[r], o);
+                    const uint32_t o = __shfl_xor_sync(kFull, k[r], j / R);
+                    k[r] = low ? min(k[r], o) : max(k[r], o);
                 }
             } else {
 #pragma unroll
                 for (int r = 0; r < R; r++) {
                     if (r & j) continue;
-                    // (the run's direction: bit kk of lane R + r)
-                    const bool up = kk >= 32 * R || (kk >= R ? (lane & (kk / R)) == 0 : (r & kk) == 0);
                     const uint32_t lo = min(k[r], k[r | j]), hi = max(k[r], k[r | j]);
-                    k[r] = up ? lo : hi;
-                    k[r | j] = up ? hi : lo;
+                    k[r] = lo;
+                    k[r | j] = hi;
                 }
             }
         }
     }
 }
 
-// Sorts the staged products (n <= 32 R of them) by column, adds equal columns
-// and leaves the row in sg.key / sg.val; returns its length.
+// Sorts n <= 32 R products (key: column << BITS | place of its product in val)
+// by column, adds equal columns and leaves the row in key / val; returns its
+// length.  The first product of a column stores its place in the row, the
+// others add to it: most columns of such a row have one product.
 template <int R, int BITS, typename V>
-__device__ __forceinline__ int sort_merge(SortStage<V, BITS> &sg, int n, int lane, bool &ovf) {
+__device__ __forceinline__ int sort_merge(uint32_t *key, V *val, int n, int lane, bool checked, bool &ovf) {
     uint32_t k[R];
 #pragma unroll
-    for (int r = 0; r < R; r++) k[r] = lane * R + r < n ? sg.key[lane * R + r] : 0xffffffffu;
-    bitonic_sort<R>(k, lane);
+    for (int r = 0; r < R; r++) k[r] = lane * R + r < n ? key[lane * R + r] : 0xffffffffu;
+    merge_sort<R>(k, lane);
     V v[R];
 #pragma unroll
-    for (int r = 0; r < R; r++) v[r] = lane * R + r < n ? sg.val[k[r] & ((1u << BITS) - 1u)] : (V)0;
-    // heads of runs of one column; (n products sort to the front)
+    for (int r = 0; r < R; r++) v[r] = lane * R + r < n ? val[k[r] & ((1u << BITS) - 1u)] : (V)0;
+    // heads of runs of one column (the n products sort to the front)
     const uint32_t before = __shfl_up_sync(kFull, k[R - 1], 1);
     uint32_t heads = 0;
 #pragma unroll
@@ -67,55 +85,26 @@ __device__ __forceinline__ int sort_merge(SortStage<V, BITS> &sg, int n, int lan
         const bool first = r == 0 && lane == 0;
         if (lane * R + r < n && (first || (p >> BITS) != (k[r] >> BITS))) heads |= 1u << r;
     }
-    int incl = __popc(heads);
-#pragma unroll
-    for (int d = 1; d < 32; d <<= 1) {
-        const int o = __shfl_up_sync(kFull, incl, d);
-        if (lane >= d) incl += o;
-    }
-    const int pos0 = incl - __popc(heads);
+    const int incl = warp_incl_scan(__popc(heads));
+    const int last = incl - __popc(heads) - 1;   // place of the run that is open before this lane
     const int total = __shfl_sync(kFull, incl, 31);
-    // the part of this lane before its first head belongs to a run of an
-    // earlier lane: suffix sums over lanes, stopping at lanes with a head
-    auto add = [&](V &s, V x) {
-        s += x;
-        ovf |= s < x;
-    };
-    V lead = 0;
-#pragma unroll
-    for (int r = 0; r < R; r++) {
-        if (!(heads & ((2u << r) - 1u))) add(lead, v[r]);
-    }
-    bool stop = heads != 0;
-    V tail = lead;   // lead of this lane and of the lanes after it up to (including) the first with a head
-#pragma unroll
-    for (int d = 1; d < 32; d <<= 1) {
-        const V o = __shfl_down_sync(kFull, tail, d);
-        const bool os = __shfl_down_sync(kFull, stop, d);
-        if (lane + d < 32 && !stop) {
-            add(tail, o);
-            stop = os;
-        }
-    }
-    V next = __shfl_down_sync(kFull, tail, 1);
-    if (lane == 31) next = 0;
-    __syncwarp();   // keys and products are in registers: the stage takes the row
-    int pos = pos0 - 1;
-    V sum = 0;
+    __syncwarp();   // keys and products are in registers: their memory takes the row
 #pragma unroll
     for (int r = 0; r < R; r++) {
         if ((heads >> r) & 1u) {
-            if (pos >= pos0) sg.val[pos] = sum;
-            pos++;
-            sg.key[pos] = k[r] >> BITS;
-            sum = v[r];
-        } else if (pos >= pos0) {
-            add(sum, v[r]);
+            const int pos = last + __popc(heads & ((2u << r) - 1u));
+            key[pos] = k[r] >> BITS;
+            val[pos] = v[r];
         }
     }
-    if (pos >= pos0) {
-        add(sum, next);
-        sg.val[pos] = sum;
+    __syncwarp();
+#pragma unroll
+    for (int r = 0; r < R; r++) {
+        if (lane * R + r < n && !((heads >> r) & 1u)) {
+            V *sum = val + last + __popc(heads & ((2u << r) - 1u));
+            if (checked) add_shared_chk(sum, v[r], ovf);
+            else add_shared(sum, v[r]);
+        }
     }
     __syncwarp();
     return total;
@@ -124,7 +113,7 @@ __device__ __forceinline__ int sort_merge(SortStage<V, BITS> &sg, int n, int lan
 // Bound by instruction issue: the sort's compare-exchanges.  A key holds the
 // column and the product's number, so the sort moves one register per product
 // whatever the value type; the products wait in shared memory and are added
-// after it.  Against a CTA with a hash table, whose barriers and shared-memory
+// where their columns come out.  Against a CTA with a hash table, whose barriers and shared-memory
 // sort these rows took before: 52,860 rows of 68 products on 131,071 columns
 // 355 -> 71 us, 25,195 uint64 rows of 120 258 -> 57 us; up to 1,024 products
 // 581 -> 440 us (a wave of 64 chains).
@@ -189,8 +178,8 @@ __global__ void __launch_bounds__(kSortWarps * 32) k_sort(DevCsr A, DevCsr B, bo
             if (lane == 0) raise_status(st, kInvariant);
             n = MAX;
         }
-        const int total = n <= MAX / 2 ? sort_merge<MAX / 64, BITS>(sg, n, lane, ovf)
-                                       : sort_merge<MAX / 32, BITS>(sg, n, lane, ovf);
+        const int total = n <= MAX / 2 ? sort_merge<MAX / 64, BITS>(sg.key, sg.val, n, lane, checked, ovf)
+                                       : sort_merge<MAX / 32, BITS>(sg.key, sg.val, n, lane, checked, ovf);
         const int64_t base = C.rowptr[r];
         const int64_t rlen = C.rowptr[r + 1] - base;
         if (lane == 0) {

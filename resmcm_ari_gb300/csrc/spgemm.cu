@@ -47,8 +47,9 @@ namespace rmcm {
 namespace {
 
 constexpr unsigned kFull = 0xffffffffu;
-constexpr int kBinMask = 0x0f;    // bin_of: the row's bin, and two flags
+constexpr int kBinMask = 0x0f;    // bin_of: the row's bin, and flags
 constexpr int kEmptyBin = 0x0f;   // bin code of rows with no products
+constexpr int kDoneBit = 0x20;    // flag: k_bucket has written the row
 constexpr int kNarrowBit = 0x40;  // flag (uint64 products): no count of the row exceeds 32 bits
 constexpr int kRiskyBit = 0x80;   // flag: a count of the row may exceed the value type
 
@@ -1567,6 +1568,7 @@ __global__ void __launch_bounds__(NT) k_hash(DevCsr A, DevCsr B, DevCsr C, const
 
 #include "row_kernels.cuh"
 #include "sort_rows.cuh"
+#include "bucket_rows.cuh"
 
 // ------------------------------------------------------------------------
 // dense bin: one CTA per row, windowed presence bytes + counters in shared memory
@@ -2237,6 +2239,7 @@ __global__ void __launch_bounds__(kRankThreads) k_rank(DevCsr A, DevCsr B, DevCs
     bool ovf = false;
     for (int32_t ri = blockIdx.x; ri < nrows; ri += gridDim.x) {
         const int32_t r = rows[ri];
+        if (NUMERIC && (bin_of[r] & kDoneBit)) continue;
         const int64_t a0 = A.rowptr[r], a1 = A.rowptr[r + 1];
         const bool checked = NUMERIC && (bin_of[r] & kRiskyBit) != 0;
         for (int i = tid; i < nwords / 4; i += NT) ((uint4 *)bits)[i] = make_uint4(0, 0, 0, 0);
@@ -2798,6 +2801,9 @@ struct DenseTemp {
     int64_t bytes = 0, vbytes = 0;   // the two allocations (columns, counts)
     bool no_risky = false;            // no row can overflow: with positive inputs, no presence bytes
     int32_t *next_row = nullptr;      // device counter of k_row_window, zero
+    int32_t *bucket_rows = nullptr;   // two of k_bucket
+    const int64_t *row_flops = nullptr;   // products per row
+    int64_t max_rank_flops = 0;       // the rank bin's largest
     bool by_row = false;              // slots are numbered by row, not by place in the list
     // packed copy of B (k_pack) for the plain path of single-window rows
     const uint32_t *pk = nullptr;
@@ -2878,6 +2884,23 @@ int32_t launch_sort(rmcm_handle *h, const DevCsr &A, const DevCsr &B, bool a_one
     const int per_sm = std::max(1, occupancy(h, kern, kSortWarps * 32, sm));
     kern<<<grid_for(h, (int64_t)n * 32, kSortWarps * 32, per_sm), kSortWarps * 32, sm, h->stream>>>(
         A, B, a_ones, b_ones, C, rows, n, cnt, h->d_status, bin_of);
+    return RMCM_OK;
+}
+
+// Rank-bin rows of min_flops + 1 .. BucketCap<NT>::max_flops products.
+template <typename V, int NT>
+int32_t launch_bucket(rmcm_handle *h, const DevCsr &A, const DevCsr &B, bool a_ones, bool b_ones, const DevCsr &C,
+                      const int32_t *rows, int32_t n, const DenseTemp *temp, int64_t min_flops, int64_t *cnt,
+                      const uint8_t *bin_of, int which) {
+    auto kern = k_bucket<V, NT>;
+    const int64_t sm = (int64_t)sizeof(BucketShared<V, NT>);
+    RMCM_TRY(set_smem(h, kern, sm));
+    const int per_sm = std::max(1, occupancy(h, kern, NT, sm));
+    kern<<<std::min(n, h->sm_count * per_sm), NT, sm, h->stream>>>(A, B, a_ones, b_ones, C, rows, n, temp->row_flops,
+                                                                   min_flops, cnt, h->d_status,
+                                                                   const_cast<uint8_t *>(bin_of),
+                                                                   temp->bucket_rows + which);
+    h->launches++;
     return RMCM_OK;
 }
 
@@ -3036,6 +3059,14 @@ int32_t launch_bins(rmcm_handle *h, const DevCsr &A, const DevCsr &B, const DevC
                 }
                 const int32_t *rl = split ? rs->perm : list;
                 const int32_t rn = split ? rs->n_front : n;
+                if (NUMERIC && rn > 0) {
+                    // k_rank takes the rows these leave: too many products, or too
+                    // many on one range of columns
+                    RMCM_TRY((launch_bucket<V, 128>(h, A, B, a_ones, b_ones, C, rl, rn, temp, 0, cnt, bin_of, 0)));
+                    if (temp->max_rank_flops > BucketCap<128>::max_flops)
+                        RMCM_TRY((launch_bucket<V, 512>(h, A, B, a_ones, b_ones, C, rl, rn, temp,
+                                                        BucketCap<128>::max_flops, cnt, bin_of, 1)));
+                }
                 if (rn > 0)
                     kern<<<std::max(1, std::min(grid, rn)), kRankThreads, sm, s>>>(A, B, C, rl, rn, cnt, st, bin_of);
                 if (split) {
@@ -3209,7 +3240,7 @@ int32_t spgemm_t(rmcm_handle *h, const rmcm_mat *Am, const rmcm_mat *Bm, rmcm_ma
     // profiling sums, [52] rank split slots, [53] unsplit rank rows,
     // [54..55] largest rank-row flops (u64), [56] rows that may overflow,
     // [58..59] largest value of B (u64, when B may be packed), [62] row counter
-    // of k_row_window, [60..61] largest total of a row whose total may exceed
+    // of k_row_window, [30..31] of k_bucket, [60..61] largest total of a row whose total may exceed
     // the value type (uint32), [18..19]
     // and [20..21] slots of the single-pass temporary for the short-row bins'
     // and the rank bin's rows (u64)
@@ -3405,6 +3436,8 @@ int32_t spgemm_t(rmcm_handle *h, const rmcm_mat *Am, const rmcm_mat *Bm, rmcm_ma
         if (record) plan->risky_rows = risky_rows;
         dtemp.no_risky = risky_rows == 0;
         dtemp.next_row = small + 62;
+        dtemp.bucket_rows = small + 30;
+        dtemp.row_flops = flops;
     }
     {
         // Tensor-core part (dense_gemm.cu): every row with products in the
@@ -3555,6 +3588,7 @@ int32_t spgemm_t(rmcm_handle *h, const rmcm_mat *Am, const rmcm_mat *Bm, rmcm_ma
     if (replay) max_rank_f = plan->max_rank_flops;
     else memcpy(&max_rank_f, (int32_t *)h->h_pinned + 54, sizeof(int64_t));
     if (record) plan->max_rank_flops = max_rank_f;
+    dtemp.max_rank_flops = max_rank_f;
     if (counts[kBinRank] > 0) {
         const int64_t fpart = std::max<int64_t>(kSplitMinFlops, flops_total / ((int64_t)h->sm_count * 4));
         if (max_rank_f > fpart) {

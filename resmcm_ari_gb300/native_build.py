@@ -31,7 +31,7 @@ CUDA_HOME = os.environ.get("CUDA_HOME", "/usr/local/cuda")
 NVCC = os.path.join(CUDA_HOME, "bin", "nvcc") if os.path.exists(os.path.join(CUDA_HOME, "bin", "nvcc")) else "nvcc"
 CU_SOURCES = ["spgemm.cu", "estimator.cu", "chain_dp.cu", "dense_gemm.cu", "tc_gemm.cu", "batch_fused.cu"]
 CPP_SOURCES = ["api.cpp", "server.cpp"]
-HEADERS = ["internal.h", "row_kernels.cuh", "sort_rows.cuh"]
+HEADERS = ["internal.h", "row_kernels.cuh", "sort_rows.cuh", "bucket_rows.cuh"]
 NVCC_FLAGS = ARCH + ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC,-fvisibility=hidden",
                      "-I" + INCLUDE, "-I" + CSRC]
 CXX_FLAGS = ["-O2", "-std=c++17", "-fPIC", "-fvisibility=hidden", "-fopenmp", "-I" + INCLUDE, "-I" + CSRC,

@@ -292,3 +292,40 @@ def test_estimates_at_every_row_length(native, engine, length, n):
     assert np.array_equal(got, again)
     want = _estimates(mats, dims)
     np.testing.assert_allclose(got, want, rtol=1e-9, atol=0)
+
+
+@pytest.mark.parametrize("vt", ["VAL_U32", "VAL_U64"])
+def test_bucketed_rows(native, vt):
+    """Rows of an output wider than a window, from the fewest products the rank
+    bin takes to several times what a CTA holds: uniform columns, columns in one
+    narrow range (a bucket too full: the bitmap kernel's rows), one column many
+    times, the first and the last column; B rows of every length."""
+    eng = native.Engine(device=0)
+    rng = np.random.default_rng(11)
+    n = 700_001
+    k = 3000
+    lens = rng.choice([1, 2, 5, 9, 31, 33, 63, 64, 65, 128, 129, 200], k)
+    cols = []
+    for i, x in enumerate(lens):
+        if i < 1500:
+            c = rng.choice(n, x, replace=False)                       # anywhere
+        elif i < 2300:
+            c = 5000 + rng.choice(600, x, replace=False)              # one narrow range
+        else:
+            c = np.concatenate([[0, n - 1, 77][: min(3, x)], 100 + rng.choice(n - 200, max(0, x - 3), replace=False)])
+            c = np.unique(c)
+            while c.size < x:
+                c = np.unique(np.concatenate([c, rng.integers(100, n - 2, x - c.size)]))
+        cols.append(np.sort(c))
+    rp = np.concatenate([[0], np.cumsum(lens)])
+    B = sp.csr_matrix((rng.integers(1, 30, rp[-1], dtype=np.uint64), np.concatenate(cols), rp), shape=(k, n))
+    picks = []
+    for lo, hi in ((0, 1500), (1500, 2300), (2300, 3000), (0, 3000)):
+        for take in (20, 60, 90, 150, 240, 400, 690):
+            picks.append(np.sort(lo + rng.choice(hi - lo, take, replace=False)))
+    ap = np.concatenate([[0], np.cumsum([p.size for p in picks])])
+    A = sp.csr_matrix((rng.integers(1, 30, ap[-1], dtype=np.uint64), np.concatenate(picks), ap), shape=(len(picks), k))
+    f = np.array([lens[p].sum() for p in picks])
+    assert f.min() < 1100 and (f > 8448).sum() > 3 and (f > 33792).sum() > 1
+    check_product(native, eng, A, B, getattr(native, vt))
+    eng.close()
