@@ -2598,7 +2598,8 @@ __global__ void __launch_bounds__(256) k_copy_short(int64_t m, const uint8_t *bi
 }
 
 // Compacts TEMP-mode slots into C: row rows[ri] has cnt = rowptr[r+1]-rowptr[r]
-// entries at slot ri of the temporary (its own number with by_row).
+// entries at slot ri of the temporary (its own number with by_row).  Four
+// entries per thread in flight, the temporary read past the caches.
 template <typename V>
 __global__ void __launch_bounds__(256) k_copy_rows(const int32_t *rows, int32_t nrows, DevCsr C, const int32_t *tcol,
                                                    const V *tval, int64_t tstride, bool by_row) {
@@ -2607,9 +2608,23 @@ __global__ void __launch_bounds__(256) k_copy_rows(const int32_t *rows, int32_t 
         const int64_t b = C.rowptr[r], n = C.rowptr[r + 1] - b;
         const int32_t *sc = tcol + (int64_t)(by_row ? r : ri) * tstride;
         const V *sv = tval + (int64_t)(by_row ? r : ri) * tstride;
-        for (int64_t i = threadIdx.x; i < n; i += blockDim.x) {
-            C.col[b + i] = sc[i];
-            ((V *)C.val)[b + i] = sv[i];
+        for (int64_t i0 = threadIdx.x; i0 < n; i0 += 4 * (int64_t)blockDim.x) {
+            int32_t c[4];
+            V v[4];
+#pragma unroll
+            for (int u = 0; u < 4; u++) {
+                const int64_t i = i0 + u * (int64_t)blockDim.x;
+                c[u] = i < n ? __ldcs(sc + i) : 0;
+                v[u] = i < n ? __ldcs(sv + i) : (V)0;
+            }
+#pragma unroll
+            for (int u = 0; u < 4; u++) {
+                const int64_t i = i0 + u * (int64_t)blockDim.x;
+                if (i < n) {
+                    C.col[b + i] = c[u];
+                    ((V *)C.val)[b + i] = v[u];
+                }
+            }
         }
     }
 }

@@ -329,3 +329,19 @@ def test_bucketed_rows(native, vt):
     assert f.min() < 1100 and (f > 8448).sum() > 3 and (f > 33792).sum() > 1
     check_product(native, eng, A, B, getattr(native, vt))
     eng.close()
+
+
+@pytest.mark.parametrize("vt", ["VAL_U32", "VAL_U64"])
+@pytest.mark.parametrize("k", [248, 256, 257])
+def test_every_index_of_full_matrices_is_heavy(native, vt, k):
+    """Widths that are multiples of the sampling step: a full matrix shows
+    every column to the heavy-index selection, not one in eight."""
+    eng = native.Engine(device=0)
+    eng.set_tuning(gemm_min_mflops=1)
+    rng = np.random.default_rng(k)
+    A = sp.csr_matrix(rng.integers(1, 40, (520, k), dtype=np.uint64))
+    B = sp.csr_matrix(rng.integers(1, 40, (k, 264), dtype=np.uint64))
+    eng.set_profiling(1)
+    check_product(native, eng, A, B, getattr(native, vt))
+    assert eng.product_stats()[-1]["gemm_inner"] == k
+    eng.close()
