@@ -149,6 +149,13 @@ int32_t status_eval(rmcm_handle *h) {
     return set_error(h, RMCM_EOVERFLOW, "a path count overflowed the value type");
 }
 
+int32_t product_status(rmcm_handle *h) {
+    if (!h->status_read) return check_status(h);
+    const int32_t rc = status_eval(h);
+    if (rc != RMCM_OK) h->status_read = false;   // (the device words are cleared)
+    return rc;
+}
+
 int32_t check_status(rmcm_handle *h) {
     RMCM_TRY(status_fetch(h));
     RMCM_CUDA(h, cudaStreamSynchronize(h->stream));
@@ -699,38 +706,29 @@ int32_t chain_exec(rmcm_handle *h, rmcm_mat *const *mats, int32_t len, const int
     }
     // (a) estimator
     double *c_dev = nullptr;
-    char *ord = nullptr;
-    const int64_t ord_bytes = 8 * 256 + 4 * 256 + 4 * 64;
     RMCM_TRY(dev_alloc(h, (void **)&c_dev, 8 * 256));
     rc = estimate(h, mats, len, c_dev);
-    if (rc == RMCM_OK) rc = dev_alloc(h, (void **)&ord, ord_bytes);
-    if (rc != RMCM_OK) {
-        dev_free(h, c_dev, 8 * 256);
-        return rc;
-    }
     cudaEventRecord(ev[1], s);
-    // (b) DP + order
-    int32_t *pairs_dev = (int32_t *)(ord + 8 * 256 + 4 * 256);
-    rc = chain_order_dev(h, c_dev, len, (int32_t *)(ord + 8 * 256), (double *)ord, pairs_dev);
+    // (b) DP + order, its tables straight to pinned memory
+    int32_t *pairs_pin = (int32_t *)(h->h_pinned + kPinnedPairs);
+    if (rc == RMCM_OK)
+        rc = chain_order_dev(h, c_dev, len, (int32_t *)(h->h_pinned + kPinnedSplit),
+                             (double *)(h->h_pinned + kPinnedCost), pairs_pin);
     cudaEventRecord(ev[2], s);
-    if (rc == RMCM_OK) {
-        if (fixed_pairs) {
-            memcpy(pairs, fixed_pairs, sizeof(int32_t) * 2 * (len - 1));
-        } else {
-            cudaError_t e = cudaMemcpyAsync(h->h_pinned, pairs_dev, sizeof(int32_t) * 2 * (len - 1), cudaMemcpyDeviceToHost, s);
-            if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-            if (e != cudaSuccess) rc = cuda_error(h, e, "order download");
-            else memcpy(pairs, h->h_pinned, sizeof(int32_t) * 2 * (len - 1));
-        }
-    }
     if (rc == RMCM_OK && sink) {
         // the whole chain's estimated nnz sizes the result's blocks
-        cudaError_t e = cudaMemcpyAsync(h->h_pinned, c_dev + (len - 1), sizeof(double), cudaMemcpyDeviceToHost, s);
-        if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+        const cudaError_t e =
+            cudaMemcpyAsync(h->h_pinned, c_dev + (len - 1), sizeof(double), cudaMemcpyDeviceToHost, s);
         if (e != cudaSuccess) rc = cuda_error(h, e, "estimate download");
-        else memcpy(&est_result, h->h_pinned, sizeof(double));
     }
-    dev_free(h, ord, ord_bytes);
+    if (rc == RMCM_OK && (sink || !fixed_pairs)) {
+        const cudaError_t e = cudaStreamSynchronize(s);
+        if (e != cudaSuccess) rc = cuda_error(h, e, "order download");
+    }
+    if (rc == RMCM_OK) {
+        memcpy(pairs, fixed_pairs ? fixed_pairs : pairs_pin, sizeof(int32_t) * 2 * (len - 1));
+        if (sink) memcpy(&est_result, h->h_pinned, sizeof(double));
+    }
     dev_free(h, c_dev, 8 * 256);
     if (rc != RMCM_OK) return rc;
     }
@@ -784,6 +782,17 @@ int32_t chain_exec(rmcm_handle *h, rmcm_mat *const *mats, int32_t len, const int
         return RMCM_OK;
     };
     double spgemm_s = 0;
+    // events around each product, read once the chain is done (a product run
+    // again in uint64 takes another pair)
+    int n_ev = 0;
+    auto next_event = [&](cudaEvent_t *out) -> int32_t {
+        if (n_ev >= (int)(sizeof(h->prod_ev) / sizeof(h->prod_ev[0])))
+            return set_error(h, RMCM_EINTERNAL, "chain: product events");
+        cudaEvent_t &e = h->prod_ev[n_ev++];
+        if (!e) RMCM_CUDA(h, cudaEventCreate(&e));
+        *out = e;
+        return RMCM_OK;
+    };
     for (int p = 0; p < len - 1 && rc == RMCM_OK; p++) {
         const int k = pairs[2 * p], l = pairs[2 * p + 1];
         const int sz = (int)stack.size();
@@ -887,7 +896,11 @@ int32_t chain_exec(rmcm_handle *h, rmcm_mat *const *mats, int32_t len, const int
             delivered = true;
             break;
         }
-        cudaEventRecord(ev[3], s);
+        cudaEvent_t ev_a = nullptr, ev_b = nullptr;
+        rc = next_event(&ev_a);
+        if (rc == RMCM_OK) rc = next_event(&ev_b);
+        if (rc != RMCM_OK) break;
+        cudaEventRecord(ev_a, s);
         rmcm_mat *C = nullptr;
         int64_t fl = 0;
         h->abort_on_certain_overflow = widen && cur == RMCM_VAL_U32;
@@ -895,7 +908,8 @@ int32_t chain_exec(rmcm_handle *h, rmcm_mat *const *mats, int32_t len, const int
         plan.mode = log ? 1 : 0;
         rc = spgemm(h, A, B, &C, &fl, log ? &plan : nullptr);
         h->abort_on_certain_overflow = false;
-        cudaEventRecord(ev[4], s);
+        cudaEventRecord(ev_b, s);
+        if (!C) n_ev -= 2;   // nothing was multiplied
         if (rc == RMCM_EOVERFLOW && widen && cur == RMCM_VAL_U32 && !C) {
             // overflow is certain from the row-sum bound: escalate before computing
             rc = RMCM_OK;
@@ -919,24 +933,10 @@ int32_t chain_exec(rmcm_handle *h, rmcm_mat *const *mats, int32_t len, const int
             continue;
         }
         if (rc != RMCM_OK) break;
-        // one wait for the product and, when it may overflow, its status
-        const bool want_status = widen && cur == RMCM_VAL_U32;
-        if (want_status) {
-            rc = status_fetch(h);
-            if (rc == RMCM_OK) {
-                const cudaError_t e = cudaStreamSynchronize(s);
-                if (e != cudaSuccess) rc = cuda_error(h, e, "chain");
-            }
-            if (rc != RMCM_OK) {
-                mat_release(h, C);
-                break;
-            }
-        } else {
-            cudaEventSynchronize(ev[4]);
-        }
-        spgemm_s += elapsed_s(ev[3], ev[4]);
-        if (want_status) {
-            const int32_t st = status_eval(h);
+        // a product that may overflow reports before the next one uses it (most
+        // read their status back with their size)
+        if (widen && cur == RMCM_VAL_U32) {
+            const int32_t st = product_status(h);
             if (st == RMCM_EOVERFLOW) {
                 // escalate: drop C, widen the live intermediates, redo this product
                 mat_release(h, C);
@@ -994,6 +994,7 @@ int32_t chain_exec(rmcm_handle *h, rmcm_mat *const *mats, int32_t len, const int
     }
     cudaEventRecord(ev[5], s);
     RMCM_CUDA(h, cudaEventSynchronize(ev[5]));
+    for (int q = 0; q + 1 < n_ev; q += 2) spgemm_s += elapsed_s(h->prod_ev[q], h->prod_ev[q + 1]);
     // the ablation orders run no estimator, as efficient/l2r.cpp and naive.cpp
     tm.es_s = host_dp_s >= 0 ? 0.0 : elapsed_s(ev[0], ev[1]);
     tm.dp_s = host_dp_s >= 0 ? host_dp_s : elapsed_s(ev[1], ev[2]);
@@ -1012,7 +1013,7 @@ int32_t chain_exec(rmcm_handle *h, rmcm_mat *const *mats, int32_t len, const int
         log->nnz = stack[0]->d.nnz;
         log->valtype = cur;
     }
-    rc = check_status(h);
+    rc = product_status(h);   // (the words gather over the products)
     if (rc == RMCM_EOVERFLOW) stack[0]->positive = false;   // wrapped counts may be 0
     if (t) *t = tm;
     return rc;
@@ -1189,7 +1190,7 @@ RMCM_API int32_t rmcm_create(rmcm_handle **out, const rmcm_opts *opts) {
     if (e == cudaSuccess) e = cudaMalloc((void **)&h->d_status, sizeof(int) * kNumStatus);
     if (e == cudaSuccess) e = cudaMemset(h->d_status, 0, sizeof(int) * kNumStatus);
     if (e == cudaSuccess) e = cudaMallocHost((void **)&h->h_status, sizeof(int) * kNumStatus);
-    if (e == cudaSuccess) e = cudaMallocHost((void **)&h->h_pinned, sizeof(int64_t) * 64);
+    if (e == cudaSuccess) e = cudaMallocHost((void **)&h->h_pinned, sizeof(int64_t) * kPinnedWords);
     size_t free_b = 0, total_b = 0;
     if (e == cudaSuccess) e = cudaMemGetInfo(&free_b, &total_b);
     if (e == cudaSuccess) {
@@ -1235,6 +1236,8 @@ RMCM_API int32_t rmcm_destroy(rmcm_handle *h) {
     if (h->h_status) cudaFreeHost(h->h_status);
     if (h->h_pinned) cudaFreeHost(h->h_pinned);
     for (auto &e : h->ev)
+        if (e) cudaEventDestroy(e);
+    for (auto &e : h->prod_ev)
         if (e) cudaEventDestroy(e);
     if (h->xfer) cudaStreamDestroy(h->xfer);
     if (h->ev_fork) cudaEventDestroy(h->ev_fork);
@@ -1558,43 +1561,26 @@ RMCM_API int32_t rmcm_transfers_wait(rmcm_handle *h) {
 
 RMCM_API int32_t rmcm_estimate(rmcm_handle *h, rmcm_mat *const *chain, int32_t len, double *c_out) {
     if (!h || !chain || !c_out) return RMCM_EINVAL;
-    double *c_dev = nullptr;
-    RMCM_TRY(dev_alloc(h, (void **)&c_dev, 8 * 256));
-    int32_t rc = estimate(h, chain, len, c_dev);
-    if (rc == RMCM_OK) {
-        cudaError_t e = cudaMemcpyAsync(c_out, c_dev, sizeof(double) * len * len, cudaMemcpyDeviceToHost, h->stream);
-        if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
-        if (e != cudaSuccess) rc = cuda_error(h, e, "estimate download");
-    }
-    dev_free(h, c_dev, 8 * 256);
-    return rc;
+    double *c_pin = (double *)(h->h_pinned + kPinnedC);   // the reduction writes pinned memory
+    RMCM_TRY(estimate(h, chain, len, c_pin));
+    RMCM_CUDA(h, cudaStreamSynchronize(h->stream));
+    memcpy(c_out, c_pin, sizeof(double) * len * len);
+    return RMCM_OK;
 }
 
 RMCM_API int32_t rmcm_order(rmcm_handle *h, const double *c, int32_t len, int32_t *split, double *cost,
                             int32_t *pairs) {
     if (!h || !c || len < 1 || len > 16) return set_error(h, RMCM_EINVAL, "order: bad arguments");
-    char *buf = nullptr;
-    const int64_t bytes = 8 * 256 + 4 * 256 + 8 * 256 + 4 * 64;
-    RMCM_TRY(dev_alloc(h, (void **)&buf, bytes));
-    double *c_dev = (double *)buf;
-    int32_t *s_dev = (int32_t *)(buf + 8 * 256);
-    double *m_dev = (double *)(buf + 8 * 256 + 4 * 256);
-    int32_t *p_dev = (int32_t *)(buf + 8 * 256 + 4 * 256 + 8 * 256);
-    cudaStream_t s = h->stream;
-    int32_t rc = RMCM_OK;
-    cudaError_t e = cudaMemcpyAsync(c_dev, c, sizeof(double) * len * len, cudaMemcpyHostToDevice, s);
-    if (e != cudaSuccess) rc = cuda_error(h, e, "order upload");
-    if (rc == RMCM_OK) rc = chain_order_dev(h, c_dev, len, s_dev, m_dev, p_dev);
-    if (rc == RMCM_OK) {
-        e = cudaSuccess;
-        if (split) e = cudaMemcpyAsync(split, s_dev, 4 * len * len, cudaMemcpyDeviceToHost, s);
-        if (e == cudaSuccess && cost) e = cudaMemcpyAsync(cost, m_dev, 8 * len * len, cudaMemcpyDeviceToHost, s);
-        if (e == cudaSuccess && pairs && len > 1) e = cudaMemcpyAsync(pairs, p_dev, 4 * 2 * (len - 1), cudaMemcpyDeviceToHost, s);
-        if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-        if (e != cudaSuccess) rc = cuda_error(h, e, "order download");
-    }
-    dev_free(h, buf, bytes);
-    return rc;
+    // the kernel reads and writes the handle's pinned memory: one launch, one wait
+    double *c_pin = (double *)(h->h_pinned + kPinnedC), *m_pin = (double *)(h->h_pinned + kPinnedCost);
+    int32_t *s_pin = (int32_t *)(h->h_pinned + kPinnedSplit), *p_pin = (int32_t *)(h->h_pinned + kPinnedPairs);
+    memcpy(c_pin, c, sizeof(double) * len * len);
+    RMCM_TRY(chain_order_dev(h, c_pin, len, s_pin, m_pin, p_pin));
+    RMCM_CUDA(h, cudaStreamSynchronize(h->stream));
+    if (split) memcpy(split, s_pin, 4 * len * len);
+    if (cost) memcpy(cost, m_pin, 8 * len * len);
+    if (pairs && len > 1) memcpy(pairs, p_pin, 4 * 2 * (len - 1));
+    return RMCM_OK;
 }
 
 RMCM_API int32_t rmcm_spgemm(rmcm_handle *h, const rmcm_mat *A, const rmcm_mat *B, rmcm_mat **C) {
@@ -1602,7 +1588,7 @@ RMCM_API int32_t rmcm_spgemm(rmcm_handle *h, const rmcm_mat *A, const rmcm_mat *
     *C = nullptr;
     int32_t rc = spgemm(h, A, B, C, nullptr);
     if (rc != RMCM_OK) return rc;
-    rc = check_status(h);
+    rc = product_status(h);
     if (rc == RMCM_EOVERFLOW) (*C)->positive = false;   // wrapped counts may be 0
     if (rc != RMCM_OK && rc != RMCM_EOVERFLOW) {
         mat_release(h, *C);

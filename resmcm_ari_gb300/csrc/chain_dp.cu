@@ -264,37 +264,11 @@ int32_t mat_digest_launch(rmcm_handle *h, const rmcm_mat *m, uint64_t *out_dev, 
 
 int32_t chain_order_dev(rmcm_handle *h, const double *c_dev, int32_t len, int32_t *split_dev, double *cost_dev,
                         int32_t *pairs_dev) {
-    // single-chain form: c_dev is len*len; stage it into the 16x16 batched layout
+    // (the kernel's tables of one chain are compact: len*len)
     if (len < 1 || len > kMaxLen) return set_error(h, RMCM_EINVAL, "order: chain length must be 1..16");
-    cudaStream_t s = h->stream;
-    const int64_t cbytes = sizeof(double) * kMaxLen * kMaxLen;
-    char *buf = nullptr;
-    const int64_t total = cbytes + 256 + 4 * kMaxLen * kMaxLen + cbytes + 4 * 2 * kMaxLen;
-    RMCM_TRY(dev_alloc(h, (void **)&buf, total + 1024));
-    double *c16 = (double *)buf;
-    int32_t *lens = (int32_t *)(buf + cbytes);
-    int32_t *sp16 = (int32_t *)(buf + cbytes + 256);
-    double *cost16 = (double *)(buf + cbytes + 256 + 4 * kMaxLen * kMaxLen);
-    int32_t *pairs16 = (int32_t *)((char *)cost16 + cbytes);
-    cudaError_t e = cudaMemcpyAsync(c16, c_dev, sizeof(double) * len * len, cudaMemcpyDeviceToDevice, s);
-    if (e == cudaSuccess) {
-        int32_t L = len;
-        e = cudaMemcpyAsync(lens, &L, sizeof(int32_t), cudaMemcpyHostToDevice, s);
-    }
-    if (e == cudaSuccess) {
-        k_chain_dp<<<1, 32, 0, s>>>(c16, lens, 1, sp16, cost16, pairs16, 0);
-        h->launches++;
-        e = cudaGetLastError();
-    }
-    if (e == cudaSuccess && split_dev)
-        e = cudaMemcpyAsync(split_dev, sp16, sizeof(int32_t) * len * len, cudaMemcpyDeviceToDevice, s);
-    if (e == cudaSuccess && cost_dev)
-        e = cudaMemcpyAsync(cost_dev, cost16, sizeof(double) * len * len, cudaMemcpyDeviceToDevice, s);
-    if (e == cudaSuccess && pairs_dev && len > 1)
-        e = cudaMemcpyAsync(pairs_dev, pairs16, sizeof(int32_t) * 2 * (len - 1), cudaMemcpyDeviceToDevice, s);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(s);   // host value of L must outlive the copy
-    dev_free(h, buf, total + 1024);
-    if (e != cudaSuccess) return cuda_error(h, e, "chain order");
+    k_chain_dp<<<1, 32, 0, h->stream>>>(c_dev, nullptr, 1, split_dev, cost_dev, pairs_dev, len);
+    h->launches++;
+    RMCM_CUDA(h, cudaGetLastError());
     return RMCM_OK;
 }
 

@@ -38,6 +38,11 @@ struct DevCsr {
     const uint64_t *vmax = nullptr;     // with info: the matrix's largest value
 };
 
+// The pinned area: 64 words for read-backs, then a chain's estimates (256
+// doubles), split (256 int32), cost (256 doubles) and pairs (64 int32).
+constexpr int kPinnedC = 64, kPinnedSplit = kPinnedC + 256, kPinnedCost = kPinnedSplit + 128,
+              kPinnedPairs = kPinnedCost + 256, kPinnedWords = kPinnedPairs + 32;
+
 // Device-side status words, one int each (set with atomicOr, never cleared by kernels).
 enum StatusWord { kOverflow = 0, kInvariant = 1, kArena = 2, kTimeout = 3, kNumStatus = 8 };
 
@@ -138,11 +143,13 @@ struct rmcm_handle {
     std::string last_error;
     int *d_status = nullptr;        // kNumStatus ints
     int *h_status = nullptr;        // pinned mirror
-    int64_t *h_pinned = nullptr;    // small pinned transfer area (64 int64)
+    int64_t *h_pinned = nullptr;    // small pinned transfer area (kPinnedWords int64), which kernels may write
+    bool status_read = false;       // h_status holds the words after the last product's last check
     // scratch (grown on demand, stream-ordered)
     void *scratch = nullptr;
     int64_t scratch_bytes = 0;
     cudaEvent_t ev[8] = {};
+    cudaEvent_t prod_ev[64] = {};   // around each product of a chain, created on first use
     // second stream for work that overlaps the main stream's kernels inside
     // one operation (forked and joined with the two events)
     cudaStream_t aux = nullptr;
@@ -209,6 +216,8 @@ void mat_release(rmcm_handle *h, rmcm_mat *m);
 bool copy_out_launch(const void *const *src, void *const *dst_host, const int64_t *bytes, cudaStream_t s);
 // Read and clear the device status words; maps them to a status code.
 int32_t check_status(rmcm_handle *h);
+// The same for words already read back (rmcm_handle::status_read), else check_status.
+int32_t product_status(rmcm_handle *h);
 
 inline int64_t val_bytes(int32_t valtype) { return valtype == RMCM_VAL_U64 ? 8 : 4; }
 // Row records of a matrix, its largest value and its rows' (rmcm_mat::rowinfo).

@@ -261,9 +261,9 @@ __device__ __forceinline__ void row_warp_products(const DevCsr &A, const V *aval
 }
 
 template <typename V, bool PK>
-__global__ void __launch_bounds__(kWarpWarps * 32, 8) k_row_warp(DevCsr A, const V *aval, RowB<V> B, DevCsr C,
-                                                                 const int32_t *rows, int32_t nrows, int32_t W,
-                                                                 int64_t *cnt, const uint8_t *bin_of, int *st) {
+__device__ __forceinline__ void warp_window_rows(const DevCsr &A, const V *aval, const RowB<V> &B, const DevCsr &C,
+                                                 const int32_t *rows, int32_t nrows, int32_t W, int64_t *cnt,
+                                                 const uint8_t *bin_of, int *st, int64_t first, int64_t nwarps) {
     extern __shared__ __align__(16) unsigned char smem[];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const unsigned lt_mask = (1u << lane) - 1u;
@@ -272,7 +272,7 @@ __global__ void __launch_bounds__(kWarpWarps * 32, 8) k_row_warp(DevCsr A, const
     WarpList<V> &sl = lists[warp];
     for (int i = lane; i < W; i += 32) win.set(i, 0);
     __syncwarp();
-    for (int64_t wi = (int64_t)blockIdx.x * kWarpWarps + warp; wi < nrows; wi += (int64_t)gridDim.x * kWarpWarps) {
+    for (int64_t wi = first; wi < nrows; wi += nwarps) {
         const int32_t r = rows[wi];
         const int64_t a0 = A.rowptr[r], a1 = A.rowptr[r + 1];
         const uint8_t flags = bin_of[r];
@@ -292,6 +292,14 @@ __global__ void __launch_bounds__(kWarpWarps * 32, 8) k_row_warp(DevCsr A, const
         }
         __syncwarp();
     }
+}
+
+template <typename V, bool PK>
+__global__ void __launch_bounds__(kWarpWarps * 32, 8) k_row_warp(DevCsr A, const V *aval, RowB<V> B, DevCsr C,
+                                                                 const int32_t *rows, int32_t nrows, int32_t W,
+                                                                 int64_t *cnt, const uint8_t *bin_of, int *st) {
+    warp_window_rows<V, PK>(A, aval, B, C, rows, nrows, W, cnt, bin_of, st,
+                            (int64_t)blockIdx.x * kWarpWarps + (threadIdx.x >> 5), (int64_t)gridDim.x * kWarpWarps);
 }
 
 // ---- a CTA per row ------------------------------------------------------------

@@ -118,9 +118,9 @@ __device__ __forceinline__ int sort_merge(uint32_t *key, V *val, int n, int lane
 // 355 -> 71 us, 25,195 uint64 rows of 120 258 -> 57 us; up to 1,024 products
 // 581 -> 440 us (a wave of 64 chains).
 template <typename V, int BITS>
-__global__ void __launch_bounds__(kSortWarps * 32) k_sort(DevCsr A, DevCsr B, bool a_ones, bool b_ones, DevCsr C,
-                                                          const int32_t *rows, int32_t nrows, int64_t *cnt, int *st,
-                                                          const uint8_t *bin_of) {
+__device__ __forceinline__ void sort_rows(const DevCsr &A, const DevCsr &B, bool a_ones, bool b_ones, const DevCsr &C,
+                                          const int32_t *rows, int32_t nrows, int64_t *cnt, int *st,
+                                          const uint8_t *bin_of, int64_t first, int64_t nwarps) {
     constexpr int MAX = 1 << BITS;
     extern __shared__ __align__(16) unsigned char smem[];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -128,7 +128,7 @@ __global__ void __launch_bounds__(kSortWarps * 32) k_sort(DevCsr A, DevCsr B, bo
     const V *Aval = (const V *)A.val;
     const V *Bval = (const V *)B.val;
     bool ovf = false;
-    for (int64_t wi = (int64_t)blockIdx.x * kSortWarps + warp; wi < nrows; wi += (int64_t)gridDim.x * kSortWarps) {
+    for (int64_t wi = first; wi < nrows; wi += nwarps) {
         const int32_t r = rows[wi];
         const int64_t a0 = A.rowptr[r], a1 = A.rowptr[r + 1];
         const bool checked = (bin_of[r] & kRiskyBit) != 0;
@@ -195,4 +195,12 @@ __global__ void __launch_bounds__(kSortWarps * 32) k_sort(DevCsr A, DevCsr B, bo
         __syncwarp();
     }
     if (__any_sync(kFull, ovf) && lane == 0) raise_status(st, kOverflow);
+}
+
+template <typename V, int BITS>
+__global__ void __launch_bounds__(kSortWarps * 32) k_sort(DevCsr A, DevCsr B, bool a_ones, bool b_ones, DevCsr C,
+                                                          const int32_t *rows, int32_t nrows, int64_t *cnt, int *st,
+                                                          const uint8_t *bin_of) {
+    sort_rows<V, BITS>(A, B, a_ones, b_ones, C, rows, nrows, cnt, st, bin_of,
+                       (int64_t)blockIdx.x * kSortWarps + (threadIdx.x >> 5), (int64_t)gridDim.x * kSortWarps);
 }

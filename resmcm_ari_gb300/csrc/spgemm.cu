@@ -680,20 +680,104 @@ __global__ void __launch_bounds__(256) k_scatter(int64_t m, const uint8_t *bin_o
     }
 }
 
+// Exclusive scan of v over the CTA; the sum in *total.
+__device__ __forceinline__ int64_t block_scan_i64(int64_t v, int64_t *s_warp, int64_t *total) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    int64_t incl = v;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+        const int64_t o = __shfl_up_sync(kFull, incl, d);
+        if (lane >= d) incl += o;
+    }
+    if (lane == 31) s_warp[warp] = incl;
+    __syncthreads();
+    int64_t base = 0, tot = 0;
+    for (int w = 0; w < (int)(blockDim.x >> 5); w++) {
+        const int64_t t = s_warp[w];
+        if (w < warp) base += t;
+        tot += t;
+    }
+    __syncthreads();
+    *total = tot;
+    return base + incl - v;
+}
+
+// k_scatter, k_short_cap and the scan of the capacities for products of few
+// rows, by one CTA: bound by the latencies of a launch and a host round trip
+// each, not by the work.  The totals go straight to pinned memory (host, the
+// 64 words of `small` with B's largest value in words 58 and 59), which the
+// host reads after the stream: no copy.
+// cap: slots of the single-pass temporary (min(products, columns) for rows of
+// the bins in short_mask, and of the rank bin unless a row of it will be split
+// over CTAs: rank_max > max(split_min, flops / (4 SMs))), scanned into trow.
+constexpr int kPlanThreads = 1024;
+constexpr int kPlanRows = 8 * kPlanThreads;
+
+__global__ void __launch_bounds__(kPlanThreads) k_plan_small(int64_t m, int64_t ncols, const uint8_t *bin_of,
+                                                             const int64_t *flops, const int32_t *small,
+                                                             const uint64_t *vmax, uint32_t short_mask,
+                                                             int64_t split_min, int sms, int32_t *lists, int64_t *cnt,
+                                                             int64_t *trow, int32_t *host) {
+    constexpr int K = 2 * kNumBins;   // per bin: heavy rows from the front, the others from the back
+    __shared__ int32_t off[kNumBins + 1], s_at[K];
+    __shared__ int64_t s_warp[32];
+    const int tid = threadIdx.x, lane = tid & 31;
+    if (tid == 0) {
+        int32_t s = 0;
+        for (int b = 0; b < kNumBins; b++) { off[b] = s; s += small[b]; }
+        off[kNumBins] = s;
+        trow[0] = 0;
+    }
+    if (tid < K) s_at[tid] = 0;
+    if (tid < 64) host[tid] = vmax && (tid == 58 || tid == 59) ? ((const int32_t *)vmax)[tid - 58] : small[tid];
+    const unsigned long long total = *(const unsigned long long *)(small + 32);
+    const unsigned long long dmax = *(const unsigned long long *)(small + 36), rmax = *(const unsigned long long *)(small + 54);
+    const int64_t part = max(split_min, (int64_t)(total / (4ull * sms)));
+    if ((int64_t)rmax <= part) short_mask |= 1u << kBinRank;
+    __syncthreads();
+    int64_t base = 0;
+    for (int64_t r0 = 0; r0 < m; r0 += kPlanThreads) {
+        const int64_t r = r0 + tid;
+        int b = kEmptyBin, key = K;
+        int64_t cap = 0;
+        if (r < m) {
+            b = bin_of[r] & kBinMask;
+            if (b == kEmptyBin) {
+                cnt[r] = 0;   // rows without products have no entries
+            } else {
+                const int64_t f = flops[r];
+                key = 2 * b + ((b == kBinDense && f > (int64_t)(dmax >> 3)) || (b == kBinRank && f > (int64_t)(rmax >> 3)) ? 0 : 1);
+                if ((short_mask >> b) & 1u) cap = f < ncols ? f : ncols;
+            }
+        }
+        const unsigned peers = __match_any_sync(kFull, key);
+        const int leader = __ffs(peers) - 1;
+        int32_t p = 0;
+        if (lane == leader && key != K) p = atomicAdd(&s_at[key], __popc(peers));
+        p = __shfl_sync(kFull, p, leader) + __popc(peers & ((1u << lane) - 1u));
+        if (key != K) lists[key & 1 ? off[b + 1] - 1 - p : off[b] + p] = (int32_t)r;
+        int64_t tot;
+        const int64_t excl = block_scan_i64(cap, s_warp, &tot);
+        if (r < m) trow[r + 1] = base + excl + cap;
+        base += tot;
+    }
+}
+
 // ------------------------------------------------------------------------
 // tiny bin: one warp per row, <= 32 products held one per lane
 // ------------------------------------------------------------------------
 
+// (first, nwarps: this warp's number among the warps that share the rows; the
+// same form for every short-row kernel, so that k_short can run several)
 template <typename V, bool NUMERIC>
-__global__ void __launch_bounds__(256) k_tiny(DevCsr A, DevCsr B, DevCsr C, const int32_t *rows, int32_t nrows,
-                                              int64_t *cnt, int *st) {
+__device__ __forceinline__ void tiny_rows(const DevCsr &A, const DevCsr &B, const DevCsr &C, const int32_t *rows,
+                                          int32_t nrows, int64_t *cnt, int *st, int64_t first, int64_t nwarps) {
     const int lane = threadIdx.x & 31;
     const unsigned lt_mask = (1u << lane) - 1u;
-    const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
     const V *Aval = (const V *)A.val;
     const V *Bval = (const V *)B.val;
     bool ovf = false;
-    for (int64_t w = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; w < nrows; w += nwarps) {
+    for (int64_t w = first; w < nrows; w += nwarps) {
         const int32_t r = rows[w];
         const int64_t a0 = A.rowptr[r], a1 = A.rowptr[r + 1];
         int32_t key = INT_MAX;
@@ -795,6 +879,13 @@ __global__ void __launch_bounds__(256) k_tiny(DevCsr A, DevCsr B, DevCsr C, cons
         }
     }
     if (__any_sync(kFull, ovf) && lane == 0) raise_status(st, kOverflow);
+}
+
+template <typename V, bool NUMERIC>
+__global__ void __launch_bounds__(256) k_tiny(DevCsr A, DevCsr B, DevCsr C, const int32_t *rows, int32_t nrows,
+                                              int64_t *cnt, int *st) {
+    tiny_rows<V, NUMERIC>(A, B, C, rows, nrows, cnt, st, ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5,
+                          ((int64_t)gridDim.x * blockDim.x) >> 5);
 }
 
 // Warp bin: rows whose output has at most kWarpCols columns and whose
@@ -963,19 +1054,18 @@ __global__ void __launch_bounds__(kWarpWarps * 32) k_warp(DevCsr A, DevCsr B, De
 // aligned group) and merges equal columns with segmented suffix sums, as
 // the warp-per-row bin does for up to 32 products.
 template <typename V, bool NUMERIC, int G>
-__global__ void __launch_bounds__(256) k_micro(DevCsr A, DevCsr B, DevCsr C, const int32_t *rows, int32_t nrows,
-                                               int64_t *cnt, int *st) {
+__device__ __forceinline__ void micro_rows(const DevCsr &A, const DevCsr &B, const DevCsr &C, const int32_t *rows,
+                                           int32_t nrows, int64_t *cnt, int *st, int64_t first, int64_t nwarps) {
     static_assert(G >= 1 && G <= 16 && (G & (G - 1)) == 0, "G must be a power of two up to 16");
     constexpr int RPW = 32 / G;                       // rows per warp
     const int lane = threadIdx.x & 31;
     const int g = lane & (G - 1);
     const int gbase = lane & ~(G - 1);
     const unsigned gmask = G == 32 ? kFull : (((1u << G) - 1u) << gbase);
-    const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
     const V *Aval = (const V *)A.val;
     const V *Bval = (const V *)B.val;
     bool ovf = false;
-    for (int64_t w0 = (((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5) * RPW; w0 < nrows; w0 += nwarps * RPW) {
+    for (int64_t w0 = first * RPW; w0 < nrows; w0 += nwarps * RPW) {
         const int64_t w = w0 + lane / G;
         const bool active = w < nrows;
         int32_t r = 0;
@@ -1050,6 +1140,13 @@ __global__ void __launch_bounds__(256) k_micro(DevCsr A, DevCsr B, DevCsr C, con
         }
     }
     if (__any_sync(kFull, ovf) && lane == 0) raise_status(st, kOverflow);
+}
+
+template <typename V, bool NUMERIC, int G>
+__global__ void __launch_bounds__(256) k_micro(DevCsr A, DevCsr B, DevCsr C, const int32_t *rows, int32_t nrows,
+                                               int64_t *cnt, int *st) {
+    micro_rows<V, NUMERIC, G>(A, B, C, rows, nrows, cnt, st, ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5,
+                              ((int64_t)gridDim.x * blockDim.x) >> 5);
 }
 
 // ------------------------------------------------------------------------
@@ -1569,6 +1666,45 @@ __global__ void __launch_bounds__(NT) k_hash(DevCsr A, DevCsr B, DevCsr C, const
 #include "row_kernels.cuh"
 #include "sort_rows.cuh"
 #include "bucket_rows.cuh"
+
+// The short-row bins of a small product in one launch: each bin's rows go to
+// CTAs of their own (the bins would otherwise follow one another, a launch's
+// latency each, on a device that they leave all but empty).
+struct ShortBin {
+    const int32_t *rows = nullptr;
+    int32_t n = 0;
+    int32_t ctas = 0;
+};
+
+template <typename V, bool PK>
+__global__ void __launch_bounds__(kWarpWarps * 32) k_short(DevCsr A, DevCsr B, const V *aval, RowB<V> rb, bool a_ones,
+                                                           bool b_ones, DevCsr C, ShortBin micro, ShortBin tiny,
+                                                           ShortBin warp, ShortBin sort, int32_t W, int64_t *cnt,
+                                                           const uint8_t *bin_of, int *st) {
+    static_assert(kSortWarps == kWarpWarps, "one CTA size");
+    const int w = threadIdx.x >> 5;
+    int b = blockIdx.x;
+    if (b < micro.ctas) {
+        micro_rows<V, true, 4>(A, B, C, micro.rows, micro.n, cnt, st, (int64_t)b * kWarpWarps + w,
+                               (int64_t)micro.ctas * kWarpWarps);
+        return;
+    }
+    b -= micro.ctas;
+    if (b < tiny.ctas) {
+        tiny_rows<V, true>(A, B, C, tiny.rows, tiny.n, cnt, st, (int64_t)b * kWarpWarps + w,
+                           (int64_t)tiny.ctas * kWarpWarps);
+        return;
+    }
+    b -= tiny.ctas;
+    if (b < warp.ctas) {
+        warp_window_rows<V, PK>(A, aval, rb, C, warp.rows, warp.n, W, cnt, bin_of, st, (int64_t)b * kWarpWarps + w,
+                                (int64_t)warp.ctas * kWarpWarps);
+        return;
+    }
+    b -= warp.ctas;
+    sort_rows<V, 8>(A, B, a_ones, b_ones, C, sort.rows, sort.n, cnt, st, bin_of, (int64_t)b * kWarpWarps + w,
+                    (int64_t)sort.ctas * kWarpWarps);
+}
 
 // ------------------------------------------------------------------------
 // dense bin: one CTA per row, windowed presence bytes + counters in shared memory
@@ -2637,31 +2773,10 @@ constexpr int kScanThreads = 256;
 constexpr int kScanItems = 8;
 constexpr int kScanTile = kScanThreads * kScanItems;
 
-__device__ __forceinline__ int64_t block_scan_i64(int64_t v, int64_t *s_warp, int64_t *total) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    int64_t incl = v;
-#pragma unroll
-    for (int d = 1; d < 32; d <<= 1) {
-        const int64_t o = __shfl_up_sync(kFull, incl, d);
-        if (lane >= d) incl += o;
-    }
-    if (lane == 31) s_warp[warp] = incl;
-    __syncthreads();
-    int64_t base = 0, tot = 0;
-    for (int w = 0; w < (int)(blockDim.x >> 5); w++) {
-        const int64_t t = s_warp[w];
-        if (w < warp) base += t;
-        tot += t;
-    }
-    __syncthreads();
-    *total = tot;
-    return base + incl - v;
-}
-
 // rowptr[i+1] = inclusive partial sums within a tile; tile sums to tile_sum.
 __global__ void __launch_bounds__(kScanThreads) k_scan_tiles(const int64_t *cnt, int64_t m, int64_t *rowptr,
                                                              int64_t *tile_sum, unsigned long long *row_max,
-                                                             int64_t expect, int *st) {
+                                                             int64_t expect, int *st, int64_t *host, int *host_st) {
     __shared__ int64_t s_warp[32];
     const int64_t t0 = (int64_t)blockIdx.x * kScanTile + (int64_t)threadIdx.x * kScanItems;
     int64_t v[kScanItems];
@@ -2688,6 +2803,16 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_tiles(const int64_t *cnt,
     }
     if (threadIdx.x == 0) tile_sum[blockIdx.x] = tot;
     if (gridDim.x == 1 && threadIdx.x == 0) rowptr[0] = 0;
+    if (host) {
+        // one tile: the total, the longest row and the status words straight to
+        // pinned memory (the host waits for this kernel, no copy follows)
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            host[0] = tot;
+            host[1] = (int64_t)*(volatile unsigned long long *)row_max;
+        }
+        if (threadIdx.x < kNumStatus) host_st[threadIdx.x] = ((volatile int *)st)[threadIdx.x];
+    }
 }
 
 // One block: exclusive scan of the tile sums in place.
@@ -2805,6 +2930,32 @@ int occupancy(rmcm_handle *h, F *kernel, int threads, int64_t bytes) {
     known[key] = n;
     return n;
 }
+
+// Device memory of a handle, given back at the end of a scope unless taken.
+struct DevHold {
+    rmcm_handle *h;
+    void *p = nullptr;
+    int64_t bytes = 0;
+    explicit DevHold(rmcm_handle *h) : h(h) {}
+    DevHold(const DevHold &) = delete;
+    DevHold &operator=(const DevHold &) = delete;
+    bool alloc(int64_t n) {
+        if (dev_alloc(h, &p, n) != RMCM_OK) {
+            h->last_error.clear();
+            return false;
+        }
+        bytes = n;
+        return true;
+    }
+    void *take() {
+        void *q = p;
+        p = nullptr;
+        return q;
+    }
+    ~DevHold() {
+        if (p) dev_free(h, p, bytes);
+    }
+};
 
 // Row-padded temporary of the single-pass dense rows, and the buffers of the
 // rows split over several CTAs.
@@ -2964,6 +3115,38 @@ int32_t launch_bins(rmcm_handle *h, const DevCsr &A, const DevCsr &B, const DevC
     int32_t off = 0;
     const int64_t ncols = B.cols;
     const int micro_g = h->tune.threads_per_row;
+    if (NUMERIC && lean && temp->no_risky && micro_g == 4) {
+        // two or more short-row bins that together leave the device room: one launch
+        ShortBin sb[4];
+        const int bins[4] = {kBinMicro, kBinTiny, kBinWarp, kBinHash512}, per[4] = {8, 1, 1, 1};
+        int kinds = 0;
+        int64_t ctas = 0;
+        uint32_t taken = 0;
+        for (int i = 0; i < 4; i++) {
+            const int b = bins[i];
+            if (counts[b] == 0 || !((bin_mask >> b) & 1u) || (b == kBinHash512 && !sort_takes(h, ncols, 8))) continue;
+            int32_t at = 0;
+            for (int x = 0; x < b; x++) at += counts[x];
+            sb[i].rows = lists + at;
+            sb[i].n = counts[b];
+            sb[i].ctas = (counts[b] + per[i] * kWarpWarps - 1) / (per[i] * kWarpWarps);
+            ctas += sb[i].ctas;
+            kinds++;
+            taken |= 1u << b;
+        }
+        if (kinds >= 2 && ctas <= (int64_t)h->sm_count * 3) {
+            const int32_t W = (int32_t)((ncols + 127) / 128 * 128);
+            int64_t sm = sb[2].n ? (int64_t)kWarpWarps * W * sizeof(V) : 0;
+            if (sb[3].n) sm = std::max<int64_t>(sm, kSortWarps * (int64_t)sizeof(SortStage<V, 8>));
+            auto kern = lean->B.words ? k_short<V, true> : k_short<V, false>;
+            RMCM_TRY(set_smem(h, kern, sm));
+            kern<<<(int)ctas, kWarpWarps * 32, sm, s>>>(A, B, lean->aval, lean->B, a_ones, b_ones, C, sb[0], sb[1],
+                                                        sb[2], sb[3], W, cnt, bin_of, st);
+            h->launches++;
+            RMCM_CUDA(h, cudaGetLastError());
+            bin_mask &= ~taken;
+        }
+    }
     for (int b = 0; b < kNumBins; b++) {
         const int32_t n = counts[b];
         const int32_t *list = lists + off;
@@ -3183,14 +3366,15 @@ int32_t launch_bins(rmcm_handle *h, const DevCsr &A, const DevCsr &B, const DevC
 // Exclusive scan of the row lengths into rowptr (rowptr[0] = 0); one tile
 // needs one launch.  expect >= 0 checks the total (replays).
 int32_t scan_rowptr(rmcm_handle *h, const int64_t *cnt, int64_t m, int64_t *rowptr, int64_t *tile_sum,
-                    unsigned long long *row_max, int64_t expect) {
+                    unsigned long long *row_max, int64_t expect, bool to_host = false) {
     cudaStream_t s = h->stream;
     const int64_t ntiles = std::max<int64_t>(1, (m + kScanTile - 1) / kScanTile);
     if (m == 0) {
         RMCM_CUDA(h, cudaMemsetAsync(rowptr, 0, sizeof(int64_t), s));
         return RMCM_OK;
     }
-    k_scan_tiles<<<(unsigned)ntiles, kScanThreads, 0, s>>>(cnt, m, rowptr, tile_sum, row_max, expect, h->d_status);
+    k_scan_tiles<<<(unsigned)ntiles, kScanThreads, 0, s>>>(cnt, m, rowptr, tile_sum, row_max, expect, h->d_status,
+                                                               to_host ? h->h_pinned : nullptr, h->h_status);
     h->launches++;
     if (ntiles > 1) {
         k_scan_sums<<<1, 1024, 0, s>>>(tile_sum, ntiles, rowptr);
@@ -3264,8 +3448,6 @@ int32_t spgemm_t(rmcm_handle *h, const rmcm_mat *Am, const rmcm_mat *Bm, rmcm_ma
     // B may be packed for the warp and dense bins (positive, one window)
     const bool pack_cand = positive && !Bm->ones && B.cols >= 2 &&
                            B.cols <= (sizeof(V) == 4 ? kDenseWinU32 : kDenseWinU64) && B.nnz > 0;
-    if (pack_cand && !replay)
-        RMCM_CUDA(h, cudaMemcpyAsync(small + 58, B.vmax, 8, cudaMemcpyDeviceToDevice, s));
 
     ProdRecord *rec = nullptr;
     size_t rec_idx = 0;
@@ -3276,6 +3458,14 @@ int32_t spgemm_t(rmcm_handle *h, const rmcm_mat *Am, const rmcm_mat *Bm, rmcm_ma
         for (auto &e : rec->ev) RMCM_CUDA(h, cudaEventCreate(&e));
         RMCM_CUDA(h, cudaEventRecord(rec->ev[0], s));
     }
+    h->status_read = false;
+    // products of few rows: one kernel for the row lists and the single-pass
+    // temporary's row pointers, whose totals need no copy
+    constexpr uint32_t kShortBins = (1u << kBinTiny) | (1u << kBinHash512) | (1u << kBinHash2k) |
+                                    (1u << kBinHash8k) | (1u << kBinMicro) | (1u << kBinWarp);
+    DevHold plan_rows(h);
+    const bool small_plan = !replay && m > 0 && m <= kPlanRows && h->tune.short_single_pass &&
+                            plan_rows.alloc(16 * (m + 1));
     void *long_mem = nullptr;
     int64_t long_bytes = 0;
     BinParams bp;
@@ -3338,7 +3528,11 @@ int32_t spgemm_t(rmcm_handle *h, const rmcm_mat *Am, const rmcm_mat *Bm, rmcm_ma
                                                                    lsat);
             h->launches += 2;
         }
-        k_scatter<<<grid_for(h, m, 256, 8), 256, 0, s>>>(
+        if (small_plan)
+            k_plan_small<<<1, kPlanThreads, 0, s>>>(m, B.cols, bin_of, flops, small, pack_cand ? B.vmax : nullptr,
+                                                    kShortBins, kSplitMinFlops, h->sm_count, lists, cnt,
+                                                    (int64_t *)plan_rows.p, (int32_t *)h->h_pinned);
+        else k_scatter<<<grid_for(h, m, 256, 8), 256, 0, s>>>(
             m, bin_of, flops, small, (const unsigned long long *)(small + 36), (const unsigned long long *)(small + 54),
             small + 8, small + 22, lists, cnt);
         h->launches += 1;
@@ -3360,20 +3554,29 @@ int32_t spgemm_t(rmcm_handle *h, const rmcm_mat *Am, const rmcm_mat *Bm, rmcm_ma
     int32_t dense_max_alen = 0;
     int64_t flops_total = 0;
     int64_t cap_short = 0, cap_rank = 0;
+    int64_t max_dense_f = 0, max_rank_f = 0;   // largest products of a dense and a rank row
     uint64_t bmax = 1;   // B's largest value (when it may be packed; ones otherwise)
     bool certain = false;
     if (replay) {
         memcpy(counts, plan->counts, sizeof(counts));
         dense_max_alen = plan->dense_max_alen;
         flops_total = plan->flops;
+        max_dense_f = plan->max_dense_flops;
+        max_rank_f = plan->max_rank_flops;
     } else {
-        RMCM_CUDA(h, cudaMemcpyAsync(h->h_pinned, small, 64 * sizeof(int32_t), cudaMemcpyDeviceToHost, s));
+        if (!small_plan) {
+            RMCM_CUDA(h, cudaMemcpyAsync(h->h_pinned, small, 64 * sizeof(int32_t), cudaMemcpyDeviceToHost, s));
+            if (pack_cand)
+                RMCM_CUDA(h, cudaMemcpyAsync((int32_t *)h->h_pinned + 58, B.vmax, 8, cudaMemcpyDeviceToHost, s));
+        }
         RMCM_CUDA(h, cudaStreamSynchronize(s));
         memcpy(counts, h->h_pinned, sizeof(counts));
         dense_max_alen = ((int32_t *)h->h_pinned)[16];
         memcpy(&flops_total, (int32_t *)h->h_pinned + 32, sizeof(int64_t));
         memcpy(&cap_short, (int32_t *)h->h_pinned + 18, sizeof(int64_t));
         memcpy(&cap_rank, (int32_t *)h->h_pinned + 20, sizeof(int64_t));
+        memcpy(&max_dense_f, (int32_t *)h->h_pinned + 36, sizeof(int64_t));
+        memcpy(&max_rank_f, (int32_t *)h->h_pinned + 54, sizeof(int64_t));
         if (pack_cand) memcpy(&bmax, (int32_t *)h->h_pinned + 58, sizeof(uint64_t));
         certain = ((int32_t *)h->h_pinned)[40] != 0;
         if (sizeof(V) == 4 && h->abort_on_certain_overflow && !certain) {
@@ -3390,6 +3593,8 @@ int32_t spgemm_t(rmcm_handle *h, const rmcm_mat *Am, const rmcm_mat *Bm, rmcm_ma
         memcpy(plan->counts, counts, sizeof(counts));
         plan->dense_max_alen = dense_max_alen;
         plan->flops = flops_total;
+        plan->max_dense_flops = max_dense_f;
+        plan->max_rank_flops = max_rank_f;
     }
     if (flops_out) *flops_out = flops_total;
     if (certain && h->abort_on_certain_overflow) {
@@ -3459,8 +3664,7 @@ int32_t spgemm_t(rmcm_handle *h, const rmcm_mat *Am, const rmcm_mat *Bm, rmcm_ma
         // single-pass dense bin, uint32, positive, no row able to overflow, a
         // large product whose rows need no split over CTAs (skewed rows keep
         // the split kernels); not inside a batch recording (plain runs only).
-        int64_t mdf = 0;
-        if (!replay) memcpy(&mdf, (int32_t *)h->h_pinned + 36, sizeof(int64_t));
+        const int64_t mdf = max_dense_f;
         const int64_t fpart0 = std::max<int64_t>(kSplitMinFlops, flops_total / ((int64_t)h->sm_count * 4));
         // (uint64 products, whose dense parts are whole-row GEMMs in the
         // retail and stress chains, take it even with skewed rows; uint32
@@ -3525,10 +3729,6 @@ int32_t spgemm_t(rmcm_handle *h, const rmcm_mat *Am, const rmcm_mat *Bm, rmcm_ma
     }
     // Dense rows with far more products than a fair share of the device are
     // split over several CTAs (k_dense_split).
-    int64_t max_dense_f = 0;
-    if (replay) max_dense_f = plan->max_dense_flops;
-    else memcpy(&max_dense_f, (int32_t *)h->h_pinned + 36, sizeof(int64_t));
-    if (record) plan->max_dense_flops = max_dense_f;
     if (dtemp.active && (!dtemp.dpart.S || dtemp.dpart.lflops)) {
         // (with a tensor-core part the rows' light products decide, in
         // smaller parts: the GEMM has taken the bulk of the work; without
@@ -3599,10 +3799,6 @@ int32_t spgemm_t(rmcm_handle *h, const rmcm_mat *Am, const rmcm_mat *Bm, rmcm_ma
     }
     // Rank-bin rows likewise (k_rank_split_*)
     RankSplit rsplit;
-    int64_t max_rank_f = 0;
-    if (replay) max_rank_f = plan->max_rank_flops;
-    else memcpy(&max_rank_f, (int32_t *)h->h_pinned + 54, sizeof(int64_t));
-    if (record) plan->max_rank_flops = max_rank_f;
     dtemp.max_rank_flops = max_rank_f;
     if (counts[kBinRank] > 0) {
         const int64_t fpart = std::max<int64_t>(kSplitMinFlops, flops_total / ((int64_t)h->sm_count * 4));
@@ -3684,8 +3880,6 @@ int32_t spgemm_t(rmcm_handle *h, const rmcm_mat *Am, const rmcm_mat *Bm, rmcm_ma
     // min(products, columns) slots in a temporary, their numeric kernels
     // write there and report each row's length (the symbolic pass is skipped
     // for them), and after the scan the rows are copied into C.
-    constexpr uint32_t kShortBins = (1u << kBinTiny) | (1u << kBinHash512) | (1u << kBinHash2k) |
-                                    (1u << kBinHash8k) | (1u << kBinMicro) | (1u << kBinWarp);
     uint32_t short_mask = kShortBins | (rsplit.active ? 0u : (1u << kBinRank));
     if (replay && plan->short_temp) short_mask = plan->short_mask;
     struct {
@@ -3713,16 +3907,25 @@ int32_t spgemm_t(rmcm_handle *h, const rmcm_mat *Am, const rmcm_mat *Bm, rmcm_ma
             // slots: a capacity per row (m of them, then scanned in place of
             // a copy) and the row pointers of the temporary
             stemp.rp_bytes = 16 * (m + 1);
-            if (dev_alloc(h, (void **)&stemp.rowptr, stemp.rp_bytes) == RMCM_OK) {
+            // (k_plan_small made the row pointers for this mask, unless the split
+            // rank rows' buffers could not be had)
+            const int64_t rank_part = std::max<int64_t>(kSplitMinFlops, flops_total / ((int64_t)h->sm_count * 4));
+            const bool planned =
+                small_plan && ((short_mask >> kBinRank) & 1u) == (max_rank_f <= rank_part ? 1u : 0u);
+            if (planned) stemp.rowptr = (int64_t *)plan_rows.take();
+            if (planned || dev_alloc(h, (void **)&stemp.rowptr, stemp.rp_bytes) == RMCM_OK) {
+                int32_t src = RMCM_OK;
                 int64_t *capr = stemp.rowptr + (m + 1);
-                k_short_cap<<<grid_for(h, m, 256, 8), 256, 0, s>>>(m, bin_of, flops, B.cols, short_mask, capr);
-                h->launches++;
-                int32_t src = cudaGetLastError() == cudaSuccess ? RMCM_OK : set_error(h, RMCM_ECUDA, "short capacity");
+                if (!planned) {
+                    k_short_cap<<<grid_for(h, m, 256, 8), 256, 0, s>>>(m, bin_of, flops, B.cols, short_mask, capr);
+                    h->launches++;
+                    if (cudaGetLastError() != cudaSuccess) src = set_error(h, RMCM_ECUDA, "short capacity");
+                }
                 // the total came with the analysis (no read-back here); the
                 // scan checks it on the device
                 stemp.total = replay ? plan->short_total
                                      : cap_short + (((short_mask >> kBinRank) & 1u) ? cap_rank : 0);
-                if (src == RMCM_OK)
+                if (src == RMCM_OK && !planned)
                     src = scan_rowptr(h, capr, m, stemp.rowptr, tiles, (unsigned long long *)(small + 44), stemp.total);
                 const int64_t room = h->budget - h->in_use;
                 stemp.c_bytes = 4 * std::max<int64_t>(stemp.total, 1);
@@ -3769,6 +3972,7 @@ int32_t spgemm_t(rmcm_handle *h, const rmcm_mat *Am, const rmcm_mat *Bm, rmcm_ma
     const LeanArgs<V> *lean = positive ? &lean_args : nullptr;
 
     // symbolic
+    const bool one_tile = !replay && m > 0 && m <= kScanTile;
     rmcm_mat *C = nullptr;
     int32_t rc = mat_alloc(h, m, B.cols, -1, Am->valtype, &C);
     if (rc != RMCM_OK) {
@@ -3796,15 +4000,27 @@ int32_t spgemm_t(rmcm_handle *h, const rmcm_mat *Am, const rmcm_mat *Bm, rmcm_ma
         rc = launch_bins<V, false>(h, A, B, C->d, lists, counts, dense_max_alen, cnt, cursors, cursor_cap, &dtemp,
                                    bin_of, positive, Bm->distinct, &rsplit, lean, Am->ones, Bm->ones, other_bins);
     if (rc == RMCM_OK)
-        rc = scan_rowptr(h, cnt, m, C->d.rowptr, tiles, (unsigned long long *)(small + 44), replay ? plan->nnz : -1);
+        rc = scan_rowptr(h, cnt, m, C->d.rowptr, tiles, (unsigned long long *)(small + 44), replay ? plan->nnz : -1,
+                         one_tile);
     if (rec) cudaEventRecord(h->prof[rec_idx].ev[3], s);
     // nnz to the host, then the output arrays
     int64_t *hp = h->h_pinned;
     if (rc == RMCM_OK && !replay) {
-        cudaError_t e = cudaMemcpyAsync(hp, C->d.rowptr + m, sizeof(int64_t), cudaMemcpyDeviceToHost, s);
-        if (e == cudaSuccess) e = cudaMemcpyAsync(hp + 1, small + 44, sizeof(int64_t), cudaMemcpyDeviceToHost, s);
+        cudaError_t e = cudaSuccess;
+        if (!one_tile) {
+            e = cudaMemcpyAsync(hp, C->d.rowptr + m, sizeof(int64_t), cudaMemcpyDeviceToHost, s);
+            if (e == cudaSuccess) e = cudaMemcpyAsync(hp + 1, small + 44, sizeof(int64_t), cudaMemcpyDeviceToHost, s);
+            if (e == cudaSuccess)
+                e = cudaMemcpyAsync(h->h_status, h->d_status, sizeof(int) * kNumStatus, cudaMemcpyDeviceToHost, s);
+        }
         if (e == cudaSuccess) e = cudaStreamSynchronize(s);
         if (e != cudaSuccess) rc = cuda_error(h, e, "spgemm nnz download");
+        // the status words are final when every row's counts are computed: the
+        // numeric pass below only copies
+        h->status_read = rc == RMCM_OK;
+        for (int b = 0; b < kNumBins; b++)
+            if (counts[b] > 0 && !(stemp.active && ((short_mask >> b) & 1u)) && !(b == kBinDense && dtemp.active))
+                h->status_read = false;
     }
     const int64_t nnz = replay ? plan->nnz : hp[0];
     const int64_t c_max_row = replay ? plan->c_max_row : hp[1];
@@ -3815,10 +4031,8 @@ int32_t spgemm_t(rmcm_handle *h, const rmcm_mat *Am, const rmcm_mat *Bm, rmcm_ma
     if (rc == RMCM_OK && h->abort_on_certain_overflow && !replay) {
         // single-pass dense rows already computed their counts: stop early if
         // any of them overflowed, so the caller can recompute in uint64
-        cudaError_t e = cudaMemcpyAsync(h->h_status, h->d_status, sizeof(int) * kNumStatus, cudaMemcpyDeviceToHost, s);
-        if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-        if (e != cudaSuccess) rc = cuda_error(h, e, "spgemm status download");
-        else if (h->h_status[kOverflow]) {
+        if (h->h_status[kOverflow]) {
+            h->status_read = false;
             cudaMemsetAsync(h->d_status + kOverflow, 0, sizeof(int), s);
             drop_short();
             drop_cursors();

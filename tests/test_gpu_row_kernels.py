@@ -345,3 +345,22 @@ def test_every_index_of_full_matrices_is_heavy(native, vt, k):
     check_product(native, eng, A, B, getattr(native, vt))
     assert eng.product_stats()[-1]["gemm_inner"] == k
     eng.close()
+
+
+@pytest.mark.parametrize("m", [1, 3, 1023, 1024, 1025, 2047, 2048, 2049, 8191, 8192, 8193])
+@pytest.mark.parametrize("n", [1500, 50000])
+def test_small_products_at_the_limits_of_their_plan(native, engine, m, n):
+    """Row counts around the one-kernel plan's tiles and its end and the
+    one-tile scan's; rows of every bin, many of one kind or a few of each, and
+    rows without products."""
+    rng = np.random.default_rng(m + n)
+    k = 600
+    B = random_csr(rng, k, n, rng.choice(np.array([0, 1, 2, 3, 7, 12, 40, 90]), k), hi=6)
+    for lens in (rng.integers(0, 3, m), rng.choice([0, 1, 2, 5, 9, 30, 110], m)):
+        if lens.sum() > 40000:
+            lens[rng.random(m) < 0.8] = 1
+        A = random_csr(rng, m, k, lens, hi=6)
+        for vt in (native.VAL_U32, native.VAL_U64):
+            check_product(native, engine, A, B, vt)
+    empty = sp.csr_matrix((m, k), dtype=np.uint64)
+    check_product(native, engine, empty, B, native.VAL_U32)
