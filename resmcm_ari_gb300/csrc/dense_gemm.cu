@@ -164,10 +164,21 @@ __global__ void __launch_bounds__(kGatherThreads) k_gather_a(DevCsr A, const int
                     if ((lm >> u) & 1u) lf += (unsigned long long)(browptr[c[u] + 1] - browptr[c[u]]);
             }
         }
-        if (sum) atomicAdd(&s_sum, sum);
-        if (mx) atomicMax(&s_max, mx);
-        if (lf) atomicAdd(&s_lf, lf);
-        if (nheavy) atomicAdd(&s_heavy, nheavy);
+        // one shared atomic per warp (64-bit ones are compare-and-swap loops)
+#pragma unroll
+        for (int d = 16; d > 0; d >>= 1) {
+            sum += __shfl_xor_sync(0xffffffffu, sum, d);
+            lf += __shfl_xor_sync(0xffffffffu, lf, d);
+            const unsigned long long o = __shfl_xor_sync(0xffffffffu, mx, d);
+            mx = o > mx ? o : mx;
+        }
+        nheavy = __reduce_add_sync(0xffffffffu, nheavy);
+        if (lane == 0) {
+            if (sum) atomicAdd(&s_sum, sum);
+            if (mx) atomicMax(&s_max, mx);
+            if (lf) atomicAdd(&s_lf, lf);
+            if (nheavy) atomicAdd(&s_heavy, nheavy);
+        }
         __syncthreads();
         uint4 *dst = (uint4 *)(Ad + r * (int64_t)ld);
         for (int i = threadIdx.x; i < ld / 8; i += kGatherThreads) dst[i] = ((const uint4 *)row)[i];
@@ -243,13 +254,23 @@ __global__ void __launch_bounds__(kGatherThreads) k_gather_bt(DevCsr B, const in
     __syncthreads();
     for (int hr = warp; hr < 64; hr += kGatherThreads / 32) {
         const int64_t e = s_end[hr];
-        for (int64_t k = s_beg[hr] + lane; k < e; k += 32) {
-            const int32_t c = B.col[k];
-            const V v = bv[k];
-            mx = (unsigned long long)v > mx ? (unsigned long long)v : mx;
-            for (int l = 0; l < limbs; l++)
-                tiles[(int64_t)l * (kBtCols * kBtPitch) + (c - c0) * kBtPitch + hr] =
-                    __uint2half_rn((uint32_t)((v >> (bits * l)) & mask));
+        for (int64_t k0 = s_beg[hr] + lane; k0 < e; k0 += 128) {
+            // four entries per lane in flight
+            int32_t c[4];
+            V v[4];
+#pragma unroll
+            for (int u = 0; u < 4; u++) {
+                c[u] = k0 + 32 * u < e ? __ldg(B.col + k0 + 32 * u) : -1;
+                v[u] = k0 + 32 * u < e ? __ldg(bv + k0 + 32 * u) : (V)0;
+            }
+#pragma unroll
+            for (int u = 0; u < 4; u++) {
+                if (c[u] < 0) continue;
+                mx = (unsigned long long)v[u] > mx ? (unsigned long long)v[u] : mx;
+                for (int l = 0; l < limbs; l++)
+                    tiles[(int64_t)l * (kBtCols * kBtPitch) + (c[u] - c0) * kBtPitch + hr] =
+                        __uint2half_rn((uint32_t)((v[u] >> (bits * l)) & mask));
+            }
         }
     }
     __syncthreads();
@@ -404,7 +425,9 @@ __global__ void __launch_bounds__(kGatherThreads) k_gather_al(DevCsr A, const in
             __syncthreads();
         }
         if (lcol) {
-            if (lf) atomicAdd(&s_lf, lf);
+#pragma unroll
+            for (int d = 16; d > 0; d >>= 1) lf += __shfl_xor_sync(0xffffffffu, lf, d);
+            if (lane == 0 && lf) atomicAdd(&s_lf, lf);
             __syncthreads();
             if (threadIdx.x == 0) {
                 lcnt[r] = s_light;

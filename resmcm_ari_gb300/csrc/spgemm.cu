@@ -570,38 +570,66 @@ inline int analyze_lanes(int64_t rows, int64_t nnz) {
     return g;
 }
 
-// Row records of a matrix (DevCsr::info and top; warp per row) and its largest
-// value (*vmax, zeroed by the caller).  The largest addition a row makes to one
-// column is its largest value, or its sum when columns may repeat in a row.
+// Row records of a matrix (DevCsr::info and top) and its largest value (*vmax,
+// zeroed by the caller), G lanes per row (analyze_lanes).  The largest addition
+// a row makes to one column is its largest value, or its sum when columns may
+// repeat in a row.  One million rows of nine: 235 us with a warp per row.
 template <typename V>
-__global__ void k_rowinfo(DevCsr M, bool distinct, V *info, V *top_out, unsigned long long *vmax) {
-    const int lane = threadIdx.x & 31;
-    const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
+__global__ void __launch_bounds__(256) k_rowinfo(DevCsr M, bool distinct, int G, V *info, V *top_out,
+                                                 unsigned long long *vmax) {
+    const int lane = threadIdx.x & 31, sub = lane & (G - 1), rows = 32 / G;
+    const int64_t step = ((int64_t)gridDim.x * blockDim.x >> 5) * rows;
     const V *v = (const V *)M.val;
+    const unsigned long long vm = sizeof(V) == 4 ? 0xffffffffull : ~0ull;
     unsigned long long all = 0;
-    for (int64_t r = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; r < M.rows; r += nwarps) {
-        const int64_t q0 = M.rowptr[r], q1 = M.rowptr[r + 1];
-        unsigned long long sum = 0, top = 0;
-        for (int64_t q = q0 + lane; q < q1; q += 32) {
-            const unsigned long long x = (unsigned long long)v[q];
-            sum = sat_add(sum, x);
-            top = x > top ? x : top;
+    for (int64_t r0 = (((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5) * rows; r0 < M.rows; r0 += step) {
+        const int64_t r = r0 + lane / G;
+        int64_t q0 = 0, q1 = 0;
+        if (r < M.rows) {
+            q0 = M.rowptr[r];
+            q1 = M.rowptr[r + 1];
         }
+        unsigned long long sum = 0, top = 0;
+        auto walk = [&](int64_t q, int64_t end, int by, unsigned long long &sum, unsigned long long &top) {
+            auto take = [&](unsigned long long x) {
+                sum = sat_add(sum, x);
+                top = x > top ? x : top;
+            };
+            for (; q + 3 * (int64_t)by < end; q += 4 * (int64_t)by) {
+                V x[4];
 #pragma unroll
-        for (int d = 16; d > 0; d >>= 1) {
-            sum = sat_add(sum, __shfl_xor_sync(kFull, sum, d));
-            const unsigned long long o = __shfl_xor_sync(kFull, top, d);
-            top = o > top ? o : top;
+                for (int u = 0; u < 4; u++) x[u] = __ldg(v + q + u * (int64_t)by);
+#pragma unroll
+                for (int u = 0; u < 4; u++) take((unsigned long long)x[u]);
+            }
+            for (; q < end; q += by) take((unsigned long long)__ldg(v + q));
+            for (int d = by >> 1; d > 0; d >>= 1) {
+                sum = sat_add(sum, __shfl_xor_sync(kFull, sum, d));
+                const unsigned long long o = __shfl_xor_sync(kFull, top, d);
+                top = o > top ? o : top;
+            }
+        };
+        // rows longer than 16 G by the whole warp, after their group
+        const bool wide = G < 32 && q1 - q0 > 16 * (int64_t)G;
+        walk(q0 + sub, wide ? q0 : q1, G, sum, top);
+        for (unsigned m = __ballot_sync(kFull, wide && sub == 0); m; m &= m - 1) {
+            const int src = __ffs(m) - 1;
+            unsigned long long s2 = 0, t2 = 0;
+            walk(__shfl_sync(kFull, q0, src) + lane, __shfl_sync(kFull, q1, src), 32, s2, t2);
+            if (lane == src) {
+                sum = s2;
+                top = t2;
+            }
         }
         all = top > all ? top : all;
         if (!distinct) top = sum;
-        const unsigned long long vm = sizeof(V) == 4 ? 0xffffffffull : ~0ull;
-        if (lane == 0) {
+        if (sub == 0 && r < M.rows) {
             info[2 * r] = (V)min((unsigned long long)(q1 - q0), vm);
             info[2 * r + 1] = (V)min(sum, vm);
             top_out[r] = (V)min(top, vm);
         }
     }
+    all = warp_max_u64(all);
     if (lane == 0 && all) atomicMax(vmax, all);
 }
 
@@ -2573,6 +2601,11 @@ __global__ void __launch_bounds__(512) k_rank_split_count(const int32_t *rows, c
 
 // One CTA per split row: per-word ranks (set bits before the word) into
 // gpre, the sorted columns into C, the row's values zeroed.
+// Part blockIdx.y of a row's bitmap: the bits before it (counted again, from
+// the L2), then its own words' ranks and sorted columns.  A row of 250,000
+// columns written by one CTA took 430 us.
+constexpr int kPrepParts = 8;
+
 template <typename V>
 __global__ void __launch_bounds__(kRankThreads) k_rank_split_prep(DevCsr C, const int32_t *rows,
                                                                   const int32_t *row_of_slot, const int32_t *nslots,
@@ -2580,41 +2613,39 @@ __global__ void __launch_bounds__(kRankThreads) k_rank_split_prep(DevCsr C, cons
                                                                   const uint32_t *gbits, uint32_t *gpre, int *st) {
     constexpr int NT = kRankThreads, NW = NT / 32;
     __shared__ int s_warp[NW];
-    __shared__ uint32_t s_bpre[kRankCols / 1024];
+    __shared__ uint32_t s_bpre[kRankCols / 1024 / kPrepParts + 1];
     const int ns = min(*nslots, max_slots);
     const int tid = threadIdx.x, lane = tid & 31;
     const int nblocks = nwords >> 5;                          // nwords is a multiple of 32
-    const int per = (nblocks + NT - 1) / NT;
-    const int b0 = min(tid * per, nblocks), b1 = min(b0 + per, nblocks);
+    const int part = blockIdx.y, p0 = nblocks * part / kPrepParts, p1 = nblocks * (part + 1) / kPrepParts;
     for (int slot = blockIdx.x; slot < ns; slot += gridDim.x) {
         const int32_t r = rows[row_of_slot[slot]];
         const uint32_t *g = gbits + (int64_t)slot * nwords;
         uint32_t *pre = gpre + (int64_t)slot * nwords;
+        int mine = 0;
+        for (int w = tid; w < p0 * 32; w += NT) mine += __popc(g[w]);
+        int excl;
+        const int before = block_excl_scan<NT>(mine, &excl, s_warp);
         // set bits per 32-word block (a warp per block, coalesced)
-        for (int b = tid >> 5; b < nblocks; b += NW) {
+        for (int b = p0 + (tid >> 5); b < p1; b += NW) {
             const int x = warp_incl_scan(__popc(g[b * 32 + lane]));
-            if (lane == 31) s_bpre[b] = (uint32_t)x;
+            if (lane == 31) s_bpre[b - p0] = (uint32_t)x;
         }
         __syncthreads();
-        int mine = 0;
-        for (int b = b0; b < b1; b++) mine += (int)s_bpre[b];
-        int excl;
-        const int total = block_excl_scan<NT>(mine, &excl, s_warp);
-        for (int b = b0; b < b1; b++) {
-            const uint32_t t = s_bpre[b];
-            s_bpre[b] = (uint32_t)excl;
-            excl += (int)t;
-        }
+        // (a part has fewer blocks than the CTA threads)
+        const int n = p0 + tid < p1 ? (int)s_bpre[tid] : 0;
+        const int total = block_excl_scan<NT>(n, &excl, s_warp);
+        if (p0 + tid < p1) s_bpre[tid] = (uint32_t)(before + excl);
         __syncthreads();
         const int64_t base = C.rowptr[r];
         const int64_t rlen = C.rowptr[r + 1] - base;
-        if (tid == 0 && total != rlen) raise_status(st, kInvariant);
+        if (tid == 0 && part == kPrepParts - 1 && before + total != rlen) raise_status(st, kInvariant);
         // per-word ranks and the sorted columns, a warp per block again
-        for (int b = tid >> 5; b < nblocks; b += NW) {
+        for (int b = p0 + (tid >> 5); b < p1; b += NW) {
             const int w = b * 32 + lane;
             uint32_t word = g[w];
             const int p = __popc(word);
-            int64_t pos = (int64_t)s_bpre[b] + warp_incl_scan(p) - p;
+            int64_t pos = (int64_t)s_bpre[b - p0] + warp_incl_scan(p) - p;
             pre[w] = (uint32_t)pos;
             while (word) {
                 const int bit = __ffs(word) - 1;
@@ -2630,7 +2661,6 @@ __global__ void __launch_bounds__(kRankThreads) k_rank_split_prep(DevCsr C, cons
     }
 }
 
-// One CTA per task: the part's products added at their ranks.
 template <typename V>
 __global__ void __launch_bounds__(kRankThreads) k_rank_split_val(DevCsr A, DevCsr B, DevCsr C, const int32_t *rows,
                                                                  const int32_t *row_of_slot, const int32_t *parts,
@@ -3011,6 +3041,7 @@ struct RankSplit {
 
 // Rows with fewer products than this are never split.
 constexpr int64_t kSplitMinFlops = 1 << 17;
+constexpr int64_t kSplitMinRank = BucketCap<512>::max_flops;   // rank rows that k_bucket does not take
 constexpr int64_t kSplitMinLight = 1 << 18;   // light products of rows beside a tensor-core part
 
 // A rows with more entries than this are analysed by the whole grid: twice the
@@ -3246,7 +3277,7 @@ int32_t launch_bins(rmcm_handle *h, const DevCsr &A, const DevCsr &B, const DevC
                         k_rank_split_count<<<rs->max_slots, 512, 0, h->aux>>>(
                             rs->perm, rs->row_of_slot, rs->nslots, rs->max_slots, (int32_t)snw, rs->gbits, cnt);
                     } else {
-                        k_rank_split_prep<V><<<rs->max_slots, kRankThreads, 0, h->aux>>>(
+                        k_rank_split_prep<V><<<dim3(rs->max_slots, kPrepParts), kRankThreads, 0, h->aux>>>(
                             C, rs->perm, rs->row_of_slot, rs->nslots, rs->max_slots, (int32_t)snw, rs->gbits,
                             rs->gpre, st);
                         k_rank_split_val<V><<<sgrid, kRankThreads, 0, h->aux>>>(
@@ -3398,8 +3429,9 @@ int32_t spgemm_t(rmcm_handle *h, const rmcm_mat *Am, const rmcm_mat *Bm, rmcm_ma
         RMCM_TRY(dev_alloc(h, (void **)&Bw->rowinfo, rowinfo_bytes(Bm)));
         unsigned long long *vm = (unsigned long long *)(Bw->rowinfo + rowinfo_records(Bm));
         RMCM_CUDA(h, cudaMemsetAsync(vm, 0, 8, s));
-        k_rowinfo<V><<<grid_for(h, Bm->d.rows * 32, 256, 8), 256, 0, s>>>(
-            Bm->d, Bm->distinct, (V *)Bw->rowinfo, (V *)(vm + 1), vm);
+        const int G = analyze_lanes(Bm->d.rows, Bm->d.nnz);
+        k_rowinfo<V><<<grid_for(h, Bm->d.rows * G, 256, 8), 256, 0, s>>>(Bm->d, Bm->distinct, G, (V *)Bw->rowinfo,
+                                                                        (V *)(vm + 1), vm);
         h->launches++;
         RMCM_CUDA(h, cudaGetLastError());
     }
@@ -3530,7 +3562,7 @@ int32_t spgemm_t(rmcm_handle *h, const rmcm_mat *Am, const rmcm_mat *Bm, rmcm_ma
         }
         if (small_plan)
             k_plan_small<<<1, kPlanThreads, 0, s>>>(m, B.cols, bin_of, flops, small, pack_cand ? B.vmax : nullptr,
-                                                    kShortBins, kSplitMinFlops, h->sm_count, lists, cnt,
+                                                    kShortBins, kSplitMinRank, h->sm_count, lists, cnt,
                                                     (int64_t *)plan_rows.p, (int32_t *)h->h_pinned);
         else k_scatter<<<grid_for(h, m, 256, 8), 256, 0, s>>>(
             m, bin_of, flops, small, (const unsigned long long *)(small + 36), (const unsigned long long *)(small + 54),
@@ -3801,7 +3833,7 @@ int32_t spgemm_t(rmcm_handle *h, const rmcm_mat *Am, const rmcm_mat *Bm, rmcm_ma
     RankSplit rsplit;
     dtemp.max_rank_flops = max_rank_f;
     if (counts[kBinRank] > 0) {
-        const int64_t fpart = std::max<int64_t>(kSplitMinFlops, flops_total / ((int64_t)h->sm_count * 4));
+        const int64_t fpart = std::max<int64_t>(kSplitMinRank, flops_total / ((int64_t)h->sm_count * 4));
         if (max_rank_f > fpart) {
             const int32_t nr = counts[kBinRank];
             const int32_t max_slots = (int32_t)std::min<int64_t>(std::min<int64_t>(1024, nr), flops_total / fpart + 1);
@@ -3909,7 +3941,7 @@ int32_t spgemm_t(rmcm_handle *h, const rmcm_mat *Am, const rmcm_mat *Bm, rmcm_ma
             stemp.rp_bytes = 16 * (m + 1);
             // (k_plan_small made the row pointers for this mask, unless the split
             // rank rows' buffers could not be had)
-            const int64_t rank_part = std::max<int64_t>(kSplitMinFlops, flops_total / ((int64_t)h->sm_count * 4));
+            const int64_t rank_part = std::max<int64_t>(kSplitMinRank, flops_total / ((int64_t)h->sm_count * 4));
             const bool planned =
                 small_plan && ((short_mask >> kBinRank) & 1u) == (max_rank_f <= rank_part ? 1u : 0u);
             if (planned) stemp.rowptr = (int64_t *)plan_rows.take();
