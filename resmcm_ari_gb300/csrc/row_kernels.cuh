@@ -31,6 +31,7 @@
 // array; the L1, not the instruction rate, bounds such rows.
 constexpr int kOwnLen = 4;
 constexpr int kMidLen = 64;
+constexpr int kGroup = 4;
 
 // Right operand of a row kernel: columns and values, or (PK) one 32-bit word
 // per entry: column in the low cbits, value - addend above them (a matrix of
@@ -143,17 +144,21 @@ __device__ __forceinline__ void add_own(const RowB<V> &B, const int64_t (&bs)[E]
     }
 }
 
-// Adds va * B[q0 .. q0 + n) from eight lanes (sub = 0..7).
+// Adds va * B[q0 .. q0 + n) from kGroup lanes (sub = 0 .. kGroup - 1), four
+// positions a lane in flight.
 template <bool NARROW, bool PK, typename V>
 __device__ __forceinline__ void add_group(const RowB<V> &B, int64_t q0, int32_t n, V va, const Window<V> &win,
                                           int sub) {
-    for (int32_t p = sub; p < n; p += 16) {
-        Entry<V, PK> e0, e1;
-        e0.load(B, q0 + p);
-        e1.clear();
-        if (p + 8 < n) e1.load(B, q0 + p + 8);
-        win.template add<NARROW>(e0.col(B), (V)(va * e0.value(B)));
-        if (p + 8 < n) win.template add<NARROW>(e1.col(B), (V)(va * e1.value(B)));
+    for (int32_t p = sub; p < n; p += 4 * kGroup) {
+        Entry<V, PK> e[4];
+#pragma unroll
+        for (int u = 0; u < 4; u++) {
+            e[u].clear();
+            if (p + u * kGroup < n) e[u].load(B, q0 + p + u * kGroup);
+        }
+#pragma unroll
+        for (int u = 0; u < 4; u++)
+            if (p + u * kGroup < n) win.template add<NARROW>(e[u].col(B), (V)(va * e[u].value(B)));
     }
 }
 
@@ -247,7 +252,8 @@ __device__ __forceinline__ void row_warp_products(const DevCsr &A, const V *aval
         }
         add_own<NARROW, PK, E>(B, bs, len, va, win);
         __syncwarp();
-        for (int i = lane >> 3; i < nm; i += 4) add_group<NARROW, PK>(B, sl.bs[i], sl.len[i], sl.va[i], win, lane & 7);
+        for (int i = lane / kGroup; i < nm; i += 32 / kGroup)
+            add_group<NARROW, PK>(B, sl.bs[i], sl.len[i], sl.va[i], win, lane % kGroup);
         __syncwarp();
         for (int j = 0; j < nl; j++) {
             const int i = 32 * E - 1 - j;
@@ -396,8 +402,8 @@ __device__ __forceinline__ void row_window_products(const DevCsr &A, const V *av
                 turn -= np;
             }
         }
-        for (int i = tid >> 3; i < nm; i += NT / 8)
-            add_group<NARROW, PK>(B, sl.bs[i], sl.len[i], sl.va[i], win, tid & 7);
+        for (int i = tid / kGroup; i < nm; i += NT / kGroup)
+            add_group<NARROW, PK>(B, sl.bs[i], sl.len[i], sl.va[i], win, tid % kGroup);
         cur ^= 1;
         __syncthreads();   // the list is free; after the last step, every product has landed
     }
