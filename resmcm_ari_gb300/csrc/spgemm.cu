@@ -667,7 +667,14 @@ __global__ void __launch_bounds__(256) k_pack(DevCsr B, int32_t cbits, uint32_t 
 __global__ void __launch_bounds__(256) k_scatter(int64_t m, const uint8_t *bin_of, const int64_t *flops,
                                                  const int32_t *bin_count, const unsigned long long *dense_max,
                                                  const unsigned long long *rank_max, int32_t *front, int32_t *back,
-                                                 int32_t *lists, int64_t *cnt) {
+                                                 int32_t *lists, int64_t *cnt, const int32_t *small,
+                                                 const uint64_t *vmax, int32_t *host) {
+    // what the host decides by, to pinned memory as in k_plan_small (none of
+    // the words that it reads changes here)
+    if (host && blockIdx.x == 0 && threadIdx.x < 64) {
+        const int t = threadIdx.x;
+        host[t] = vmax && (t == 58 || t == 59) ? ((const int32_t *)vmax)[t - 58] : small[t];
+    }
     // slots are handed out per tile of 256 rows: lanes of a warp with the
     // same bin take consecutive ranks (one shared add per warp and bin), the
     // tile one global add per bin, so a million rows do not queue on a few
@@ -730,7 +737,7 @@ __device__ __forceinline__ int64_t block_scan_i64(int64_t v, int64_t *s_warp, in
     return base + incl - v;
 }
 
-// k_scatter, k_short_cap and the scan of the capacities for products of few
+// k_scatter and the scan of the capacities for products of few
 // rows, by one CTA: bound by the latencies of a launch and a host round trip
 // each, not by the work.  The totals go straight to pinned memory (host, the
 // 64 words of `small` with B's largest value in words 58 and 59), which the
@@ -2717,16 +2724,6 @@ __global__ void __launch_bounds__(kRankThreads) k_rank_split_val(DevCsr A, DevCs
     if (__syncthreads_or(ovf) && threadIdx.x == 0) raise_status(st, kOverflow);
 }
 
-// Slots of the short-row temporary: min(products, columns) for a row of
-// the short-row bins, none for the others.
-__global__ void k_short_cap(int64_t m, const uint8_t *bin_of, const int64_t *flops, int64_t cols, uint32_t mask,
-                            int64_t *cap) {
-    for (int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r < m; r += (int64_t)gridDim.x * blockDim.x) {
-        const int b = bin_of[r] & kBinMask;
-        cap[r] = (b != kEmptyBin && ((mask >> b) & 1u)) ? (flops[r] < cols ? flops[r] : cols) : 0;
-    }
-}
-
 // The single-pass bins' rows from their slots in the temporary into C (a
 // warp per row, four entries per lane in flight; the row's length is C's,
 // from the scan of the reported lengths).
@@ -2803,17 +2800,55 @@ constexpr int kScanThreads = 256;
 constexpr int kScanItems = 8;
 constexpr int kScanTile = kScanThreads * kScanItems;
 
+// What a scan adds up: a row's entries (bin_of null), or its slots in the
+// short-row temporary (min(products, columns) for a row of the bins in mask,
+// none for the others), which are never stored.
+struct ScanIn {
+    const int64_t *cnt = nullptr;
+    const uint8_t *bin_of = nullptr;
+    const int64_t *flops = nullptr;
+    int64_t cols = 0;
+    uint32_t mask = 0;
+};
+
+// Where the host reads a scan's outcome: the total, the longest row and the
+// status words in pinned memory (the host waits for the kernel, no copy).
+struct ScanHost {
+    int64_t *size = nullptr;
+    int *status = nullptr;
+    const unsigned long long *row_max = nullptr;
+};
+
+__device__ __forceinline__ void scan_to_host(const ScanHost &h, int64_t total, int *st) {
+    if (threadIdx.x == 0) {
+        h.size[0] = total;
+        h.size[1] = (int64_t)*(volatile const unsigned long long *)h.row_max;
+    }
+    if (threadIdx.x < kNumStatus) h.status[threadIdx.x] = ((volatile int *)st)[threadIdx.x];
+}
+
 // rowptr[i+1] = inclusive partial sums within a tile; tile sums to tile_sum.
-__global__ void __launch_bounds__(kScanThreads) k_scan_tiles(const int64_t *cnt, int64_t m, int64_t *rowptr,
-                                                             int64_t *tile_sum, unsigned long long *row_max,
-                                                             int64_t expect, int *st, int64_t *host, int *host_st) {
+// One tile: the scan is complete here (expect >= 0: a replay checks its size).
+template <bool CAP>
+__global__ void __launch_bounds__(kScanThreads) k_scan_tiles(ScanIn in, int64_t m, int64_t *rowptr, int64_t *tile_sum,
+                                                             unsigned long long *row_max, int64_t expect, int *st,
+                                                             ScanHost host) {
     __shared__ int64_t s_warp[32];
     const int64_t t0 = (int64_t)blockIdx.x * kScanTile + (int64_t)threadIdx.x * kScanItems;
     int64_t v[kScanItems];
     int64_t s = 0, mx = 0;
 #pragma unroll
     for (int i = 0; i < kScanItems; i++) {
-        v[i] = (t0 + i < m) ? cnt[t0 + i] : 0;
+        v[i] = 0;
+        if (t0 + i < m) {
+            if (CAP) {
+                const int b = in.bin_of[t0 + i] & kBinMask;
+                const int64_t f = in.flops[t0 + i];
+                if (b != kEmptyBin && ((in.mask >> b) & 1u)) v[i] = f < in.cols ? f : in.cols;
+            } else {
+                v[i] = in.cnt[t0 + i];
+            }
+        }
         s += v[i];
         mx = max(mx, v[i]);
     }
@@ -2828,25 +2863,18 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_tiles(const int64_t *cnt,
     for (int i = 0; i < kScanItems; i++) {
         run += v[i];
         if (t0 + i < m) rowptr[t0 + i + 1] = run;
-        // one tile: the scan is complete here (a replay checks its size)
         if (gridDim.x == 1 && t0 + i == m - 1 && expect >= 0 && run != expect) raise_status(st, kInvariant);
     }
     if (threadIdx.x == 0) tile_sum[blockIdx.x] = tot;
-    if (gridDim.x == 1 && threadIdx.x == 0) rowptr[0] = 0;
-    if (host) {
-        // one tile: the total, the longest row and the status words straight to
-        // pinned memory (the host waits for this kernel, no copy follows)
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            host[0] = tot;
-            host[1] = (int64_t)*(volatile unsigned long long *)row_max;
-        }
-        if (threadIdx.x < kNumStatus) host_st[threadIdx.x] = ((volatile int *)st)[threadIdx.x];
+    if (blockIdx.x == 0 && threadIdx.x == 0) rowptr[0] = 0;
+    if (gridDim.x == 1 && host.size) {
+        __syncthreads();   // this tile's largest row is in row_max
+        scan_to_host(host, tot, st);
     }
 }
 
-// One block: exclusive scan of the tile sums in place.
-__global__ void __launch_bounds__(1024) k_scan_sums(int64_t *tile_sum, int64_t ntiles, int64_t *rowptr) {
+// Exclusive scan of the tile sums in place, for more than kScanDirect tiles.
+__global__ void __launch_bounds__(1024) k_scan_sums(int64_t *tile_sum, int64_t ntiles) {
     __shared__ int64_t s_warp[32];
     __shared__ int64_t s_carry;
     if (threadIdx.x == 0) s_carry = 0;
@@ -2862,23 +2890,41 @@ __global__ void __launch_bounds__(1024) k_scan_sums(int64_t *tile_sum, int64_t n
         if (threadIdx.x == 0) s_carry = carry + tot;
         __syncthreads();
     }
-    if (threadIdx.x == 0) rowptr[0] = 0;
 }
 
+// Adds what comes before each tile: tile_sum holds the exclusive sums
+// (scanned), or the tiles' own, which every CTA adds up to its tile itself.
+// That costs a tile's CTA one read of at most kScanDirect sums from the L2 and
+// saves the launch between.  The last tile writes the size, the longest row
+// and the status words for the host, in place of three copies.  With the
+// capacities made in the scan and the analysis' outcome written by k_scatter,
+// a product of more than kPlanRows rows has three launches and five copies
+// fewer: 418 -> 385 us for 100,003 rows of 6 entries, 8121 -> 7609 us for
+// the replayed batch of 64 chains.
+constexpr int64_t kScanDirect = 4096;
+
 __global__ void __launch_bounds__(kScanThreads) k_scan_add(int64_t m, int64_t *rowptr, const int64_t *tile_sum,
-                                                           int64_t expect, int *st) {
+                                                           bool scanned, int64_t expect, int *st, ScanHost host) {
+    __shared__ int64_t s_warp[32];
     const int64_t t0 = (int64_t)blockIdx.x * kScanTile;
-    const int64_t add = tile_sum[blockIdx.x];
-    if (add == 0 && (expect < 0 || t0 + kScanTile < m)) return;
-    for (int i = threadIdx.x; i < kScanTile; i += kScanThreads) {
-        const int64_t r = t0 + i;
-        if (r < m) {
-            const int64_t v = rowptr[r + 1] + add;
-            if (add) rowptr[r + 1] = v;
-            // the last row's end is the product's size (a replay checks it)
-            if (r == m - 1 && expect >= 0 && v != expect) raise_status(st, kInvariant);
-        }
+    const bool last = blockIdx.x == gridDim.x - 1;
+    int64_t add;
+    if (scanned) {
+        add = tile_sum[blockIdx.x];
+    } else {
+        int64_t part = 0;
+        for (int64_t i = threadIdx.x; i < (int64_t)blockIdx.x; i += kScanThreads) part += tile_sum[i];
+        block_scan_i64(part, s_warp, &add);
     }
+    int64_t end = 0;   // of the last row, before the add (the last tile's)
+    if (last) end = rowptr[m];
+    __syncthreads();
+    if (add)
+        for (int64_t r = t0 + threadIdx.x; r < min(t0 + kScanTile, m); r += kScanThreads) rowptr[r + 1] += add;
+    if (!last) return;
+    // the last row's end is the product's size (a replay checks it)
+    if (threadIdx.x == 0 && expect >= 0 && end + add != expect) raise_status(st, kInvariant);
+    if (host.size) scan_to_host(host, end + add, st);
 }
 
 // ------------------------------------------------------------------------
@@ -3396,7 +3442,7 @@ int32_t launch_bins(rmcm_handle *h, const DevCsr &A, const DevCsr &B, const DevC
 
 // Exclusive scan of the row lengths into rowptr (rowptr[0] = 0); one tile
 // needs one launch.  expect >= 0 checks the total (replays).
-int32_t scan_rowptr(rmcm_handle *h, const int64_t *cnt, int64_t m, int64_t *rowptr, int64_t *tile_sum,
+int32_t scan_rowptr(rmcm_handle *h, const ScanIn &in, int64_t m, int64_t *rowptr, int64_t *tile_sum,
                     unsigned long long *row_max, int64_t expect, bool to_host = false) {
     cudaStream_t s = h->stream;
     const int64_t ntiles = std::max<int64_t>(1, (m + kScanTile - 1) / kScanTile);
@@ -3404,18 +3450,23 @@ int32_t scan_rowptr(rmcm_handle *h, const int64_t *cnt, int64_t m, int64_t *rowp
         RMCM_CUDA(h, cudaMemsetAsync(rowptr, 0, sizeof(int64_t), s));
         return RMCM_OK;
     }
-    k_scan_tiles<<<(unsigned)ntiles, kScanThreads, 0, s>>>(cnt, m, rowptr, tile_sum, row_max, expect, h->d_status,
-                                                               to_host ? h->h_pinned : nullptr, h->h_status);
+    ScanHost host;
+    if (to_host) host = {h->h_pinned, h->h_status, row_max};
+    auto kern = in.bin_of ? k_scan_tiles<true> : k_scan_tiles<false>;
+    kern<<<(unsigned)ntiles, kScanThreads, 0, s>>>(in, m, rowptr, tile_sum, row_max, expect, h->d_status, host);
     h->launches++;
     if (ntiles > 1) {
-        k_scan_sums<<<1, 1024, 0, s>>>(tile_sum, ntiles, rowptr);
-        k_scan_add<<<(unsigned)ntiles, kScanThreads, 0, s>>>(m, rowptr, tile_sum, expect, h->d_status);
-        h->launches += 2;
+        const bool scanned = ntiles > kScanDirect;
+        if (scanned) {
+            k_scan_sums<<<1, 1024, 0, s>>>(tile_sum, ntiles);
+            h->launches++;
+        }
+        k_scan_add<<<(unsigned)ntiles, kScanThreads, 0, s>>>(m, rowptr, tile_sum, scanned, expect, h->d_status, host);
+        h->launches++;
     }
     RMCM_CUDA(h, cudaGetLastError());
     return RMCM_OK;
 }
-
 
 template <typename V>
 int32_t spgemm_t(rmcm_handle *h, const rmcm_mat *Am, const rmcm_mat *Bm, rmcm_mat **Cout, int64_t *flops_out,
@@ -3497,7 +3548,7 @@ int32_t spgemm_t(rmcm_handle *h, const rmcm_mat *Am, const rmcm_mat *Bm, rmcm_ma
                                     (1u << kBinHash8k) | (1u << kBinMicro) | (1u << kBinWarp);
     DevHold plan_rows(h);
     const bool small_plan = !replay && m > 0 && m <= kPlanRows && h->tune.short_single_pass &&
-                            plan_rows.alloc(16 * (m + 1));
+                            plan_rows.alloc(8 * (m + 1));
     void *long_mem = nullptr;
     int64_t long_bytes = 0;
     BinParams bp;
@@ -3566,7 +3617,8 @@ int32_t spgemm_t(rmcm_handle *h, const rmcm_mat *Am, const rmcm_mat *Bm, rmcm_ma
                                                     (int64_t *)plan_rows.p, (int32_t *)h->h_pinned);
         else k_scatter<<<grid_for(h, m, 256, 8), 256, 0, s>>>(
             m, bin_of, flops, small, (const unsigned long long *)(small + 36), (const unsigned long long *)(small + 54),
-            small + 8, small + 22, lists, cnt);
+            small + 8, small + 22, lists, cnt, small, pack_cand ? B.vmax : nullptr,
+            replay ? nullptr : (int32_t *)h->h_pinned);
         h->launches += 1;
         if (long_mem) {
             dev_free(h, long_mem, long_bytes);
@@ -3596,12 +3648,8 @@ int32_t spgemm_t(rmcm_handle *h, const rmcm_mat *Am, const rmcm_mat *Bm, rmcm_ma
         max_dense_f = plan->max_dense_flops;
         max_rank_f = plan->max_rank_flops;
     } else {
-        if (!small_plan) {
-            RMCM_CUDA(h, cudaMemcpyAsync(h->h_pinned, small, 64 * sizeof(int32_t), cudaMemcpyDeviceToHost, s));
-            if (pack_cand)
-                RMCM_CUDA(h, cudaMemcpyAsync((int32_t *)h->h_pinned + 58, B.vmax, 8, cudaMemcpyDeviceToHost, s));
-        }
         RMCM_CUDA(h, cudaStreamSynchronize(s));
+        if (m == 0) memset(h->h_pinned, 0, 64 * sizeof(int32_t));   // no row, no kernel
         memcpy(counts, h->h_pinned, sizeof(counts));
         dense_max_alen = ((int32_t *)h->h_pinned)[16];
         memcpy(&flops_total, (int32_t *)h->h_pinned + 32, sizeof(int64_t));
@@ -3936,9 +3984,8 @@ int32_t spgemm_t(rmcm_handle *h, const rmcm_mat *Am, const rmcm_mat *Bm, rmcm_ma
             if ((short_mask >> b) & 1u) n_short += counts[b];
         bool want = replay ? plan->short_temp : (n_short > 0 && h->tune.short_single_pass);
         if (want) {
-            // slots: a capacity per row (m of them, then scanned in place of
-            // a copy) and the row pointers of the temporary
-            stemp.rp_bytes = 16 * (m + 1);
+            // the row pointers of the temporary
+            stemp.rp_bytes = 8 * (m + 1);
             // (k_plan_small made the row pointers for this mask, unless the split
             // rank rows' buffers could not be had)
             const int64_t rank_part = std::max<int64_t>(kSplitMinRank, flops_total / ((int64_t)h->sm_count * 4));
@@ -3947,18 +3994,13 @@ int32_t spgemm_t(rmcm_handle *h, const rmcm_mat *Am, const rmcm_mat *Bm, rmcm_ma
             if (planned) stemp.rowptr = (int64_t *)plan_rows.take();
             if (planned || dev_alloc(h, (void **)&stemp.rowptr, stemp.rp_bytes) == RMCM_OK) {
                 int32_t src = RMCM_OK;
-                int64_t *capr = stemp.rowptr + (m + 1);
-                if (!planned) {
-                    k_short_cap<<<grid_for(h, m, 256, 8), 256, 0, s>>>(m, bin_of, flops, B.cols, short_mask, capr);
-                    h->launches++;
-                    if (cudaGetLastError() != cudaSuccess) src = set_error(h, RMCM_ECUDA, "short capacity");
-                }
                 // the total came with the analysis (no read-back here); the
                 // scan checks it on the device
                 stemp.total = replay ? plan->short_total
                                      : cap_short + (((short_mask >> kBinRank) & 1u) ? cap_rank : 0);
                 if (src == RMCM_OK && !planned)
-                    src = scan_rowptr(h, capr, m, stemp.rowptr, tiles, (unsigned long long *)(small + 44), stemp.total);
+                    src = scan_rowptr(h, {nullptr, bin_of, flops, B.cols, short_mask}, m, stemp.rowptr, tiles, nullptr,
+                                      stemp.total);
                 const int64_t room = h->budget - h->in_use;
                 stemp.c_bytes = 4 * std::max<int64_t>(stemp.total, 1);
                 stemp.v_bytes = (int64_t)sizeof(V) * std::max<int64_t>(stemp.total, 1);
@@ -4004,7 +4046,6 @@ int32_t spgemm_t(rmcm_handle *h, const rmcm_mat *Am, const rmcm_mat *Bm, rmcm_ma
     const LeanArgs<V> *lean = positive ? &lean_args : nullptr;
 
     // symbolic
-    const bool one_tile = !replay && m > 0 && m <= kScanTile;
     rmcm_mat *C = nullptr;
     int32_t rc = mat_alloc(h, m, B.cols, -1, Am->valtype, &C);
     if (rc != RMCM_OK) {
@@ -4032,14 +4073,14 @@ int32_t spgemm_t(rmcm_handle *h, const rmcm_mat *Am, const rmcm_mat *Bm, rmcm_ma
         rc = launch_bins<V, false>(h, A, B, C->d, lists, counts, dense_max_alen, cnt, cursors, cursor_cap, &dtemp,
                                    bin_of, positive, Bm->distinct, &rsplit, lean, Am->ones, Bm->ones, other_bins);
     if (rc == RMCM_OK)
-        rc = scan_rowptr(h, cnt, m, C->d.rowptr, tiles, (unsigned long long *)(small + 44), replay ? plan->nnz : -1,
-                         one_tile);
+        rc = scan_rowptr(h, {cnt}, m, C->d.rowptr, tiles, (unsigned long long *)(small + 44),
+                         replay ? plan->nnz : -1, !replay);
     if (rec) cudaEventRecord(h->prof[rec_idx].ev[3], s);
     // nnz to the host, then the output arrays
     int64_t *hp = h->h_pinned;
     if (rc == RMCM_OK && !replay) {
         cudaError_t e = cudaSuccess;
-        if (!one_tile) {
+        if (m == 0) {
             e = cudaMemcpyAsync(hp, C->d.rowptr + m, sizeof(int64_t), cudaMemcpyDeviceToHost, s);
             if (e == cudaSuccess) e = cudaMemcpyAsync(hp + 1, small + 44, sizeof(int64_t), cudaMemcpyDeviceToHost, s);
             if (e == cudaSuccess)

@@ -364,3 +364,20 @@ def test_small_products_at_the_limits_of_their_plan(native, engine, m, n):
             check_product(native, engine, A, B, vt)
     empty = sp.csr_matrix((m, k), dtype=np.uint64)
     check_product(native, engine, empty, B, native.VAL_U32)
+
+
+@pytest.mark.parametrize("m", [8194, 20480, 20481, 4096 * 2048, 4096 * 2048 + 1])
+def test_row_pointers_over_many_tiles(native, engine, m):
+    """The scan of the row lengths at whole tiles and their remainders, and at
+    the count of tiles where their sums get a launch of their own; long gaps of
+    empty rows, the last row empty or not."""
+    rng = np.random.default_rng(m)
+    k = 50
+    B = random_csr(rng, k, 300, rng.integers(0, 5, k), hi=6)
+    for last in (0, 1):
+        lens = (rng.random(m) < 0.3).astype(np.int64)
+        lens[m // 3: m // 2] = 0
+        lens[-1] = last
+        rp = np.concatenate([[0], np.cumsum(lens)])
+        A = sp.csr_matrix((rng.integers(1, 6, rp[-1], dtype=np.uint64), rng.integers(0, k, rp[-1]), rp), shape=(m, k))
+        check_product(native, engine, A, B, native.VAL_U32)
