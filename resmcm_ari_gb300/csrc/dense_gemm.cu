@@ -52,17 +52,23 @@ __global__ void k_col_sample(DevCsr A, uint32_t *cnt) {
     }
 }
 
-// heavy[u] = score threshold met; slot[u] = its index in the heavy list
-// (order of discovery: the list order never changes a result), list[slot] = u.
+// slot[u] of an inner index that meets the score threshold: its index in the
+// heavy list (order of discovery: the list order never changes a result),
+// list[slot] = u.  Of a light one: ~(its row length in B), so that counting a
+// row's light products needs no second gather (kLongLen: read the row pointers).
+constexpr int32_t kLongLen = INT32_MAX - 1;
+
 __global__ void k_heavy_select(int64_t nin, const uint32_t *cnt, const int64_t *browptr, double thr,
-                               uint8_t *heavy, int32_t *slot, int32_t *list, int32_t *nheavy, int32_t cap) {
+                               int32_t *slot, int32_t *list, int32_t *nheavy, int32_t cap) {
     const int lane = threadIdx.x & 31;
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
     for (int64_t u0 = (int64_t)blockIdx.x * blockDim.x; u0 < nin; u0 += stride) {
         const int64_t u = u0 + threadIdx.x;
         bool hv = false;
+        int64_t len = 0;
         if (u < nin) {
-            const double score = (double)cnt[u] * kSample * (double)(browptr[u + 1] - browptr[u]);
+            len = browptr[u + 1] - browptr[u];
+            const double score = (double)cnt[u] * kSample * (double)len;
             hv = score >= thr;
         }
         const unsigned b = __ballot_sync(0xffffffffu, hv);
@@ -76,31 +82,171 @@ __global__ void k_heavy_select(int64_t nin, const uint32_t *cnt, const int64_t *
                 if (s < cap) list[s] = (int32_t)u;
                 else s = -1;
             }
-            heavy[u] = s >= 0;
-            slot[u] = s;
+            slot[u] = s >= 0 ? s : ~(int32_t)min(len, (int64_t)kLongLen);
+        }
+    }
+}
+
+// A's panels over the heavy indices, a CTA per row: built in shared memory and
+// written whole.  A row of more than kGatherLong entries is zeroed and listed
+// in pieces of kGatherPiece, which k_gather_long scatters to global memory:
+// with Zipf rows one CTA worked on the longest row (some 700,000 entries) while
+// the others had long finished, SMs active 22% of k_gather_al's 424 us; in
+// pieces C-I-U-I-C takes 5190 us in place of 6103.  A piece is four steps of a
+// CTA, enough for its reductions not to show.
+constexpr int64_t kGatherPiece = 4 * kGatherPer * kGatherThreads;
+constexpr int64_t kGatherLong = 2 * kGatherPiece;
+
+// Listed rows: n[0] of them, n[1] pieces; per row its sums over the pieces.
+struct GatherLong {
+    int32_t *n = nullptr, *row = nullptr, *done = nullptr, *heavy = nullptr;
+    unsigned long long *sum = nullptr, *lf = nullptr;
+    int2 *task = nullptr;   // {listed row, piece}
+};
+
+// What a thread sees of a row: sum, largest and number of its heavy values,
+// and the products of its light ones.
+struct GatherSums {
+    unsigned long long sum = 0, mx = 0, lf = 0;
+    int32_t heavy = 0;
+    __device__ __forceinline__ void warp_reduce() {
+#pragma unroll
+        for (int d = 16; d > 0; d >>= 1) {
+            sum += __shfl_xor_sync(0xffffffffu, sum, d);
+            lf += __shfl_xor_sync(0xffffffffu, lf, d);
+            const unsigned long long o = __shfl_xor_sync(0xffffffffu, mx, d);
+            mx = o > mx ? o : mx;
+        }
+        heavy = __reduce_add_sync(0xffffffffu, heavy);
+    }
+};
+
+// Entries [k0, k1) of a row of A: heavy values to row[slot] as FP16 (LIMBS:
+// limb l0 + l, (v >> (bits (l0 + l))) & (2^bits - 1), to row[l * row_ld + slot]
+// for l < ng), the light entries (lcol not null), in any order, from lcol + a0
+// and lval + a0 at places taken from *light.  kGatherPer entries per thread per
+// step: their gathers overlap, and a warp reserves places once per step.
+template <typename TA, bool LIMBS>
+__device__ __forceinline__ void gather_entries(const DevCsr &A, const int32_t *slot, int64_t k0, int64_t k1,
+                                               int64_t a0, __half *row, int64_t row_ld, int l0, int ng, int bits,
+                                               int32_t *lcol, TA *lval, int32_t *light, const int64_t *browptr,
+                                               bool products, GatherSums &g) {
+    const int lane = threadIdx.x & 31;
+    const TA *av = (const TA *)A.val;
+    const uint64_t mask = (1ull << bits) - 1ull;
+    for (; k0 < k1; k0 += kGatherPer * kGatherThreads) {
+        int32_t c[kGatherPer], sl[kGatherPer];
+        TA v[kGatherPer];
+#pragma unroll
+        for (int u = 0; u < kGatherPer; u++) {
+            const int64_t k = k0 + u * kGatherThreads + threadIdx.x;
+            c[u] = k < k1 ? A.col[k] : -1;
+            v[u] = k < k1 ? av[k] : (TA)0;
+        }
+#pragma unroll
+        for (int u = 0; u < kGatherPer; u++) sl[u] = c[u] >= 0 ? slot[c[u]] : -1;
+        uint32_t lm = 0;
+#pragma unroll
+        for (int u = 0; u < kGatherPer; u++) {
+            if (sl[u] >= 0) {
+                if (LIMBS) {
+                    for (int l = 0; l < ng; l++)
+                        row[l * row_ld + sl[u]] =
+                            __uint2half_rn((uint32_t)(((uint64_t)v[u] >> (bits * (l0 + l))) & mask));
+                } else {
+                    row[sl[u]] = __uint2half_rn((uint32_t)v[u]);
+                    g.sum += v[u];
+                    g.mx = v[u] > g.mx ? v[u] : g.mx;
+                    g.heavy++;
+                }
+            } else if (c[u] >= 0) {
+                lm |= 1u << u;
+            }
+        }
+        if (!lcol) continue;
+        const int nl = __popc(lm);
+        int incl = nl;
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+            const int t = __shfl_up_sync(0xffffffffu, incl, d);
+            if (lane >= d) incl += t;
+        }
+        const int wtot = __shfl_sync(0xffffffffu, incl, 31);
+        int base = 0;
+        if (lane == 0 && wtot) base = atomicAdd(light, wtot);
+        base = __shfl_sync(0xffffffffu, base, 0);
+        int64_t o = a0 + base + incl - nl;
+#pragma unroll
+        for (int u = 0; u < kGatherPer; u++) {
+            if ((lm >> u) & 1u) {
+                lcol[o] = c[u];
+                lval[o] = v[u];
+                o++;
+                if (products) {
+                    const int32_t len = ~sl[u];
+                    g.lf += len < kLongLen ? (unsigned long long)len
+                                           : (unsigned long long)(browptr[c[u] + 1] - browptr[c[u]]);
+                }
+            }
+        }
+    }
+}
+
+// Lists row r of len entries for k_gather_long and zeroes its panel rows (the
+// whole CTA).
+__device__ __forceinline__ void gather_list(const GatherLong &gl, int64_t r, int64_t len, __half *Ad, int32_t ld,
+                                            int32_t limbs, int64_t limb_stride, int32_t *lcnt) {
+    __shared__ int32_t s_at[2];
+    const int32_t np = (int32_t)((len + kGatherPiece - 1) / kGatherPiece);
+    if (threadIdx.x == 0) {
+        s_at[0] = atomicAdd(gl.n, 1);
+        s_at[1] = atomicAdd(gl.n + 1, np);
+        gl.row[s_at[0]] = (int32_t)r;
+        if (lcnt) lcnt[r] = 0;
+    }
+    __syncthreads();
+    for (int32_t p = threadIdx.x; p < np; p += kGatherThreads) gl.task[s_at[1] + p] = make_int2(s_at[0], p);
+    for (int l = 0; l < limbs; l++) {
+        uint4 *dst = (uint4 *)(Ad + l * limb_stride + r * (int64_t)ld);
+        for (int i = threadIdx.x; i < ld / 8; i += kGatherThreads) dst[i] = make_uint4(0, 0, 0, 0);
+    }
+    __syncthreads();
+}
+
+// A row's totals into the product's: stats[0] = largest row sum of heavy
+// values, stats[7] = the most heavy entries in a row; with lflops the row's
+// light products, stats[5] = their largest row sum, stats[6] = their total.
+__device__ __forceinline__ void gather_row_stats(int64_t r, unsigned long long sum, int32_t heavy,
+                                                 unsigned long long lf, unsigned long long *stats, int64_t *lflops) {
+    if (sum) atomicMax(stats, sum);
+    if (heavy) atomicMax(stats + 7, (unsigned long long)heavy);
+    if (lflops) {
+        lflops[r] = (int64_t)lf;
+        if (lf) {
+            atomicMax(stats + 5, lf);
+            atomicAdd(stats + 6, lf);
         }
     }
 }
 
 // Row panel of A over the heavy indices: Ad[r][slot[u]] = A[r][u] as FP16
-// (ld columns, zero elsewhere), built in shared memory and written whole.
-// The row's other (light) entries go, in any order, to the front of its
-// segment of (lcol, lval); lcnt[r] = their number.  stats[0] = largest row
-// sum of heavy values, stats[1] = largest heavy value.  With lflops (B's row
-// pointers in browptr) also the row's light products: lflops[r] = the sum of
-// B's row lengths over its light entries, stats[5] = their largest row sum,
-// stats[6] = their total.  stats[7] = the most heavy entries in a row.
+// (ld columns, zero elsewhere).  The row's other (light) entries go, in any
+// order, to the front of its segment of (lcol, lval); lcnt[r] = their number.
+// stats[1] = largest heavy value; the others as gather_row_stats has them.
 __global__ void __launch_bounds__(kGatherThreads) k_gather_a(DevCsr A, const int32_t *slot, int32_t ld, __half *Ad,
                                                              int32_t *lcol, uint32_t *lval, int32_t *lcnt,
                                                              unsigned long long *stats, const int64_t *browptr,
-                                                             int64_t *lflops) {
+                                                             int64_t *lflops, GatherLong gl) {
     extern __shared__ __align__(16) unsigned char smem[];
     __half *row = (__half *)smem;
     __shared__ unsigned long long s_sum, s_max, s_lf;
     __shared__ int32_t s_light, s_heavy;
-    const int lane = threadIdx.x & 31;
-    const uint32_t *av = (const uint32_t *)A.val;
     for (int64_t r = blockIdx.x; r < A.rows; r += gridDim.x) {
+        const int64_t a0 = A.rowptr[r], a1 = A.rowptr[r + 1];
+        if (gl.n && a1 - a0 > kGatherLong) {
+            gather_list(gl, r, a1 - a0, Ad, ld, 1, 0, lcnt);
+            continue;
+        }
         for (int i = threadIdx.x; i < ld / 8; i += kGatherThreads) ((uint4 *)row)[i] = make_uint4(0, 0, 0, 0);
         if (threadIdx.x == 0) {
             s_sum = 0;
@@ -110,92 +256,67 @@ __global__ void __launch_bounds__(kGatherThreads) k_gather_a(DevCsr A, const int
             s_heavy = 0;
         }
         __syncthreads();
-        const int64_t a0 = A.rowptr[r], a1 = A.rowptr[r + 1];
-        unsigned long long sum = 0, mx = 0, lf = 0;
-        int32_t nheavy = 0;
-        // kGatherPer entries per thread per step: their gathers overlap; the
-        // light ones are placed with one shared reservation per warp and step
-        for (int64_t k0 = a0; k0 < a1; k0 += kGatherPer * kGatherThreads) {
-            int32_t c[kGatherPer], sl[kGatherPer];
-            uint32_t v[kGatherPer];
-#pragma unroll
-            for (int u = 0; u < kGatherPer; u++) {
-                const int64_t k = k0 + u * kGatherThreads + threadIdx.x;
-                c[u] = k < a1 ? A.col[k] : -1;
-                v[u] = k < a1 ? av[k] : 0u;
-            }
-#pragma unroll
-            for (int u = 0; u < kGatherPer; u++) sl[u] = c[u] >= 0 ? slot[c[u]] : -1;
-            uint32_t lm = 0;
-#pragma unroll
-            for (int u = 0; u < kGatherPer; u++) {
-                if (sl[u] >= 0) {
-                    row[sl[u]] = __uint2half_rn(v[u]);
-                    sum += v[u];
-                    mx = v[u] > mx ? v[u] : mx;
-                    nheavy++;
-                } else if (c[u] >= 0) {
-                    lm |= 1u << u;
-                }
-            }
-            const int nl = __popc(lm);
-            int incl = nl;
-#pragma unroll
-            for (int d = 1; d < 32; d <<= 1) {
-                const int t = __shfl_up_sync(0xffffffffu, incl, d);
-                if (lane >= d) incl += t;
-            }
-            const int wtot = __shfl_sync(0xffffffffu, incl, 31);
-            int base = 0;
-            if (lane == 0 && wtot) base = atomicAdd(&s_light, wtot);
-            base = __shfl_sync(0xffffffffu, base, 0);
-            int64_t o = a0 + base + incl - nl;
-#pragma unroll
-            for (int u = 0; u < kGatherPer; u++) {
-                if ((lm >> u) & 1u) {
-                    lcol[o] = c[u];
-                    lval[o] = v[u];
-                    o++;
-                }
-            }
-            if (lflops) {
-#pragma unroll
-                for (int u = 0; u < kGatherPer; u++)
-                    if ((lm >> u) & 1u) lf += (unsigned long long)(browptr[c[u] + 1] - browptr[c[u]]);
-            }
-        }
+        GatherSums g;
+        gather_entries<uint32_t, false>(A, slot, a0, a1, a0, row, 0, 0, 1, 0, lcol, lval, &s_light, browptr,
+                                        lflops != nullptr, g);
         // one shared atomic per warp (64-bit ones are compare-and-swap loops)
-#pragma unroll
-        for (int d = 16; d > 0; d >>= 1) {
-            sum += __shfl_xor_sync(0xffffffffu, sum, d);
-            lf += __shfl_xor_sync(0xffffffffu, lf, d);
-            const unsigned long long o = __shfl_xor_sync(0xffffffffu, mx, d);
-            mx = o > mx ? o : mx;
-        }
-        nheavy = __reduce_add_sync(0xffffffffu, nheavy);
-        if (lane == 0) {
-            if (sum) atomicAdd(&s_sum, sum);
-            if (mx) atomicMax(&s_max, mx);
-            if (lf) atomicAdd(&s_lf, lf);
-            if (nheavy) atomicAdd(&s_heavy, nheavy);
+        g.warp_reduce();
+        if ((threadIdx.x & 31) == 0) {
+            if (g.sum) atomicAdd(&s_sum, g.sum);
+            if (g.mx) atomicMax(&s_max, g.mx);
+            if (g.lf) atomicAdd(&s_lf, g.lf);
+            if (g.heavy) atomicAdd(&s_heavy, g.heavy);
         }
         __syncthreads();
         uint4 *dst = (uint4 *)(Ad + r * (int64_t)ld);
         for (int i = threadIdx.x; i < ld / 8; i += kGatherThreads) dst[i] = ((const uint4 *)row)[i];
         if (threadIdx.x == 0) {
             lcnt[r] = s_light;
-            if (s_sum) atomicMax(stats, s_sum);
             if (s_max) atomicMax(stats + 1, s_max);
-            if (s_heavy) atomicMax(stats + 7, (unsigned long long)s_heavy);
-            if (lflops) {
-                lflops[r] = (int64_t)s_lf;
-                if (s_lf) {
-                    atomicMax(stats + 5, s_lf);
-                    atomicAdd(stats + 6, s_lf);
-                }
-            }
+            gather_row_stats(r, s_sum, s_heavy, s_lf, stats, lflops);
         }
         __syncthreads();
+    }
+}
+
+// The listed rows' pieces, a CTA each: heavy values straight to the zeroed
+// panel rows, light places from lcnt[r], sums to the row's; the CTA that
+// finishes a row's last piece adds the row to stats.
+template <typename TA, bool LIMBS>
+__global__ void __launch_bounds__(kGatherThreads) k_gather_long(DevCsr A, const int32_t *slot, int32_t ld,
+                                                                int32_t limbs, int32_t bits, __half *Ad,
+                                                                int64_t limb_stride, int32_t *lcol, TA *lval,
+                                                                int32_t *lcnt, unsigned long long *stats,
+                                                                const int64_t *browptr, int64_t *lflops,
+                                                                GatherLong gl) {
+    const int32_t ntask = gl.n[1];
+    for (int32_t t = blockIdx.x; t < ntask; t += gridDim.x) {
+        const int2 q = gl.task[t];
+        const int32_t r = gl.row[q.x];
+        const int64_t a0 = A.rowptr[r], a1 = A.rowptr[r + 1];
+        const int64_t k0 = a0 + q.y * kGatherPiece, k1 = min(k0 + kGatherPiece, a1);
+        GatherSums g;
+        gather_entries<TA, LIMBS>(A, slot, k0, k1, a0, Ad + r * (int64_t)ld, limb_stride, 0, limbs, bits, lcol, lval,
+                                  lcnt + r, browptr, lflops != nullptr, g);
+        if (LIMBS && !lcol) continue;   // panels only: nothing to add up
+        g.warp_reduce();
+        if ((threadIdx.x & 31) == 0) {
+            if (g.sum) atomicAdd(gl.sum + q.x, g.sum);
+            if (g.mx) atomicMax(stats + 1, g.mx);
+            if (g.lf) atomicAdd(gl.lf + q.x, g.lf);
+            if (g.heavy) atomicAdd(gl.heavy + q.x, g.heavy);
+        }
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            __threadfence();
+            const int32_t np = (int32_t)((a1 - a0 + kGatherPiece - 1) / kGatherPiece);
+            if (atomicAdd(gl.done + q.x, 1) == np - 1) {
+                __threadfence();
+                gather_row_stats(r, *(volatile unsigned long long *)(gl.sum + q.x),
+                                 *(volatile int32_t *)(gl.heavy + q.x),
+                                 *(volatile unsigned long long *)(gl.lf + q.x), stats, lflops);
+            }
+        }
     }
 }
 
@@ -340,8 +461,7 @@ __global__ void __launch_bounds__(kGatherThreads) k_heavy_stats(DevCsr A, const 
 // Row panels of A in limbs (TA: A's value type): limb l of each heavy
 // value, (A[r][u] >> (bits l)) & (2^bits - 1) as FP16 at Ad[l][r][slot[u]].
 // A CTA per row holds `group` limb rows in shared memory and fills them in
-// one pass over the row's entries, kGatherPer entries per thread per step
-// (the column -> slot gathers overlap); a row with more limbs than fit takes
+// one pass over the row's entries; a row with more limbs than fit takes
 // one pass per group.  With lcol (first pass only) the light entries are
 // compacted per row and, with lflops, their products counted, as in
 // k_gather_a.
@@ -350,72 +470,29 @@ __global__ void __launch_bounds__(kGatherThreads) k_gather_al(DevCsr A, const in
                                                               int32_t limbs, int32_t group, int32_t bits,
                                                               __half *Ad, int64_t limb_stride, int32_t *lcol,
                                                               TA *lval, int32_t *lcnt, unsigned long long *stats,
-                                                              const int64_t *browptr, int64_t *lflops) {
+                                                              const int64_t *browptr, int64_t *lflops,
+                                                              GatherLong gl) {
     extern __shared__ __align__(16) unsigned char smem[];
     __half *rows = (__half *)smem;
     __shared__ int32_t s_light;
     __shared__ unsigned long long s_lf;
-    const int lane = threadIdx.x & 31;
-    const TA *av = (const TA *)A.val;
-    const uint64_t mask = (1ull << bits) - 1ull;
     for (int64_t r = blockIdx.x; r < A.rows; r += gridDim.x) {
         const int64_t a0 = A.rowptr[r], a1 = A.rowptr[r + 1];
+        if (gl.n && a1 - a0 > kGatherLong) {
+            gather_list(gl, r, a1 - a0, Ad, ld, limbs, limb_stride, lcol ? lcnt : nullptr);
+            continue;
+        }
         if (threadIdx.x == 0) {
             s_light = 0;
             s_lf = 0;
         }
-        unsigned long long lf = 0;
+        GatherSums g;
         for (int l0 = 0; l0 < limbs; l0 += group) {
             const int ng = min(group, limbs - l0);
-            const bool compact = lcol && l0 == 0;
             for (int i = threadIdx.x; i < ng * ld / 8; i += kGatherThreads) ((uint4 *)rows)[i] = make_uint4(0, 0, 0, 0);
             __syncthreads();
-            for (int64_t k0 = a0; k0 < a1; k0 += kGatherPer * kGatherThreads) {
-                int32_t c[kGatherPer], sl[kGatherPer];
-                uint64_t v[kGatherPer];
-#pragma unroll
-                for (int u = 0; u < kGatherPer; u++) {
-                    const int64_t k = k0 + u * kGatherThreads + threadIdx.x;
-                    c[u] = k < a1 ? A.col[k] : -1;
-                    v[u] = k < a1 ? (uint64_t)av[k] : 0ull;
-                }
-#pragma unroll
-                for (int u = 0; u < kGatherPer; u++) sl[u] = c[u] >= 0 ? slot[c[u]] : -1;
-                uint32_t lm = 0;
-#pragma unroll
-                for (int u = 0; u < kGatherPer; u++) {
-                    if (sl[u] >= 0) {
-                        for (int l = 0; l < ng; l++)
-                            rows[l * ld + sl[u]] = __uint2half_rn((uint32_t)((v[u] >> (bits * (l0 + l))) & mask));
-                    } else if (c[u] >= 0) {
-                        lm |= 1u << u;
-                    }
-                }
-                if (compact) {
-                    // one shared reservation per warp and step for its light entries
-                    const int nl = __popc(lm);
-                    int incl = nl;
-#pragma unroll
-                    for (int d = 1; d < 32; d <<= 1) {
-                        const int t = __shfl_up_sync(0xffffffffu, incl, d);
-                        if (lane >= d) incl += t;
-                    }
-                    const int wtot = __shfl_sync(0xffffffffu, incl, 31);
-                    int base = 0;
-                    if (lane == 0 && wtot) base = atomicAdd(&s_light, wtot);
-                    base = __shfl_sync(0xffffffffu, base, 0);
-                    int64_t o = a0 + base + incl - nl;
-#pragma unroll
-                    for (int u = 0; u < kGatherPer; u++) {
-                        if ((lm >> u) & 1u) {
-                            lcol[o] = c[u];
-                            lval[o] = (TA)v[u];
-                            o++;
-                            if (lflops) lf += (unsigned long long)(browptr[c[u] + 1] - browptr[c[u]]);
-                        }
-                    }
-                }
-            }
+            gather_entries<TA, true>(A, slot, a0, a1, a0, rows, ld, l0, ng, bits, l0 == 0 ? lcol : nullptr, lval,
+                                     &s_light, browptr, lflops != nullptr, g);
             __syncthreads();
             for (int l = 0; l < ng; l++) {
                 uint4 *dst = (uint4 *)(Ad + (l0 + l) * limb_stride + r * (int64_t)ld);
@@ -425,19 +502,12 @@ __global__ void __launch_bounds__(kGatherThreads) k_gather_al(DevCsr A, const in
             __syncthreads();
         }
         if (lcol) {
-#pragma unroll
-            for (int d = 16; d > 0; d >>= 1) lf += __shfl_xor_sync(0xffffffffu, lf, d);
-            if (lane == 0 && lf) atomicAdd(&s_lf, lf);
+            g.warp_reduce();
+            if ((threadIdx.x & 31) == 0 && g.lf) atomicAdd(&s_lf, g.lf);
             __syncthreads();
             if (threadIdx.x == 0) {
                 lcnt[r] = s_light;
-                if (lflops) {
-                    lflops[r] = (int64_t)s_lf;
-                    if (s_lf) {
-                        atomicMax(stats + 5, s_lf);
-                        atomicAdd(stats + 6, s_lf);
-                    }
-                }
+                gather_row_stats(r, 0, 0, s_lf, stats, lflops);
             }
             __syncthreads();
         }
@@ -466,25 +536,40 @@ bool gather_bt_smem(int32_t limbs) {
 struct HeavySet {
     char *sel = nullptr;
     int64_t sel_bytes = 0;
-    uint8_t *flag = nullptr;
     int32_t *slot = nullptr, *list = nullptr;
+    GatherLong gl;                         // A's rows beyond kGatherLong
+    int64_t gl_bytes = 0;                  // of its counters, from gl.n
+    bool long_rows = false;                // A may have such rows
     unsigned long long *stats = nullptr;   // device: [2] largest B value seen, [3..4] as above
     int64_t nh = 0;
     uint64_t hrow = 0, amax = 0;
 };
 
-int32_t select_heavy(rmcm_handle *h, const DevCsr &A, const DevCsr &B, bool stats64, HeavySet &hs) {
+int32_t select_heavy(rmcm_handle *h, const DevCsr &A, const DevCsr &B, int64_t a_max_row, bool stats64,
+                     HeavySet &hs) {
     hs = HeavySet{};
     cudaStream_t s = h->stream;
     const int64_t M = A.rows, N = B.cols, K = A.cols;
     const double thr = (double)M * (double)N / (double)h->tune.gemm_inv_density;
     auto al = [](int64_t x) { return (x + 255) & ~255LL; };
-    const int64_t o_cnt = 0, o_flag = o_cnt + al(4 * K), o_slot = o_flag + al(K), o_list = o_slot + al(4 * K);
+    const int64_t o_cnt = 0, o_slot = o_cnt + al(4 * K), o_list = o_slot + al(4 * K);
     const int64_t o_small = o_list + al(4 * kMaxHeavy);
-    hs.sel_bytes = o_small + 256;
+    hs.long_rows = A.nnz > kGatherLong && (a_max_row < 0 || a_max_row > kGatherLong);
+    const int64_t max_long = hs.long_rows ? A.nnz / kGatherLong + 1 : 0;
+    const int64_t o_gl = o_small + 256, o_task = o_gl + al(256 + 28 * max_long);
+    hs.sel_bytes = o_task + al(8 * (max_long ? A.nnz / kGatherPiece + max_long : 0));
     RMCM_TRY(dev_alloc(h, (void **)&hs.sel, hs.sel_bytes));
     uint32_t *cnt = (uint32_t *)(hs.sel + o_cnt);
-    hs.flag = (uint8_t *)(hs.sel + o_flag);
+    if (hs.long_rows) {
+        hs.gl_bytes = o_task - o_gl;
+        hs.gl.n = (int32_t *)(hs.sel + o_gl);
+        hs.gl.sum = (unsigned long long *)(hs.sel + o_gl + 256);
+        hs.gl.lf = hs.gl.sum + max_long;
+        hs.gl.row = (int32_t *)(hs.gl.lf + max_long);
+        hs.gl.done = hs.gl.row + max_long;
+        hs.gl.heavy = hs.gl.done + max_long;
+        hs.gl.task = (int2 *)(hs.sel + o_task);
+    }
     hs.slot = (int32_t *)(hs.sel + o_slot);
     hs.list = (int32_t *)(hs.sel + o_list);
     int32_t *nheavy = (int32_t *)(hs.sel + o_small);
@@ -492,7 +577,7 @@ int32_t select_heavy(rmcm_handle *h, const DevCsr &A, const DevCsr &B, bool stat
     RMCM_CUDA(h, cudaMemsetAsync(cnt, 0, 4 * K, s));
     RMCM_CUDA(h, cudaMemsetAsync(hs.sel + o_small, 0, 256, s));
     k_col_sample<<<h->sm_count * 8, 256, 0, s>>>(A, cnt);
-    k_heavy_select<<<h->sm_count * 8, 256, 0, s>>>(K, cnt, B.rowptr, thr, hs.flag, hs.slot, hs.list, nheavy,
+    k_heavy_select<<<h->sm_count * 8, 256, 0, s>>>(K, cnt, B.rowptr, thr, hs.slot, hs.list, nheavy,
                                                   (int32_t)kMaxHeavy);
     h->launches += 2;
     if (stats64) {
@@ -527,11 +612,11 @@ int32_t build_limbs(rmcm_handle *h, const DevCsr &A, const DevCsr &B, uint64_t b
                     cudaEvent_t ev_begin, cudaEvent_t ev_end, bool light_flops, const LightPart *pre);
 
 // Builds the tensor-core part of C = A B (uint32, single-window dense rows):
-// on success dp.S holds the uint32 seeds (rows x ld) and dp.skip
-// flags the heavy inner indices; otherwise dp stays empty (and the product
-// runs sparse).  bmax: an upper bound on B's values.
-int32_t dense_part_build(rmcm_handle *h, const DevCsr &A, const DevCsr &B, uint64_t bmax, DensePart &dp,
-                         cudaEvent_t ev_begin, cudaEvent_t ev_end, bool light_flops) {
+// on success dp.S holds the uint32 seeds (rows x ld); otherwise dp stays empty
+// (and the product runs sparse).  a_max_row: A's longest row (-1: unknown);
+// bmax: an upper bound on B's values.
+int32_t dense_part_build(rmcm_handle *h, const DevCsr &A, int64_t a_max_row, const DevCsr &B, uint64_t bmax,
+                         DensePart &dp, cudaEvent_t ev_begin, cudaEvent_t ev_end, bool light_flops) {
     dp = DensePart{};
     const int32_t inv_density = h->tune.gemm_inv_density;
     if (inv_density <= 0 || A.rows == 0 || B.cols == 0 || A.cols == 0) return RMCM_OK;
@@ -540,10 +625,9 @@ int32_t dense_part_build(rmcm_handle *h, const DevCsr &A, const DevCsr &B, uint6
     const int64_t ldn = (N + 7) / 8 * 8;
     auto al = [](int64_t x) { return (x + 255) & ~255LL; };
     HeavySet hs;
-    RMCM_TRY(select_heavy(h, A, B, false, hs));
+    RMCM_TRY(select_heavy(h, A, B, a_max_row, false, hs));
     char *sel = hs.sel;
     const int64_t sel_bytes = hs.sel_bytes;
-    uint8_t *flag = hs.flag;
     int32_t *slot = hs.slot, *list = hs.list;
     unsigned long long *stats = hs.stats;
     auto fail = [&](int32_t rc) {
@@ -589,9 +673,15 @@ int32_t dense_part_build(rmcm_handle *h, const DevCsr &A, const DevCsr &B, uint6
             return fail2(RMCM_OK);
         }
         const int grid = (int)std::min<int64_t>(M, (int64_t)h->sm_count * 8);
+        if (hs.long_rows) RMCM_CUDA(h, cudaMemsetAsync(hs.gl.n, 0, hs.gl_bytes, s));
         k_gather_a<<<grid, kGatherThreads, smem, s>>>(A, slot, (int32_t)ldk, Ad, lcol, lval, lcnt, stats, B.rowptr,
-                                                      lflops);
+                                                      lflops, hs.gl);
         h->launches++;
+        if (hs.long_rows) {
+            k_gather_long<uint32_t, false><<<h->sm_count * 8, kGatherThreads, 0, s>>>(
+                A, slot, (int32_t)ldk, 1, 0, Ad, 0, lcol, lval, lcnt, stats, B.rowptr, lflops, hs.gl);
+            h->launches++;
+        }
         RMCM_CUDA(h, cudaGetLastError());
     }
     RMCM_CUDA(h, cudaMemcpyAsync(h->h_pinned + 8, stats, 8 * sizeof(uint64_t), cudaMemcpyDeviceToHost, s));
@@ -676,7 +766,6 @@ int32_t dense_part_build(rmcm_handle *h, const DevCsr &A, const DevCsr &B, uint6
     dp.heavy = nh;
     dp.sel = sel;
     dp.sel_bytes = sel_bytes;
-    dp.skip = flag;
     return RMCM_OK;
 }
 
@@ -698,7 +787,6 @@ int32_t build_limbs(rmcm_handle *h, const DevCsr &A, const DevCsr &B, uint64_t b
     auto al = [](int64_t x) { return (x + 255) & ~255LL; };
     char *sel = hs.sel;
     const int64_t sel_bytes = hs.sel_bytes;
-    uint8_t *flag = hs.flag;
     int32_t *slot = hs.slot, *list = hs.list;
     unsigned long long *stats = hs.stats;
     auto fail = [&](int32_t rc) {
@@ -791,10 +879,17 @@ int32_t build_limbs(rmcm_handle *h, const DevCsr &A, const DevCsr &B, uint64_t b
             return fail3(RMCM_OK);
         }
         const int grid = (int)std::min<int64_t>(M, (int64_t)h->sm_count * 8);
+        if (hs.long_rows) RMCM_CUDA(h, cudaMemsetAsync(hs.gl.n, 0, hs.gl_bytes, s));
         // (with pre the light entries are already compacted: panels only)
         k_gather_al<V><<<grid, kGatherThreads, smem, s>>>(A, slot, (int32_t)ldk, la, (int32_t)group, bits, Ad,
                                                           a_limb, pre ? nullptr : lcol, lval, lcnt, stats, B.rowptr,
-                                                          pre ? nullptr : lflops);
+                                                          pre ? nullptr : lflops, hs.gl);
+        if (hs.long_rows) {
+            k_gather_long<V, true><<<h->sm_count * 8, kGatherThreads, 0, s>>>(
+                A, slot, (int32_t)ldk, la, bits, Ad, a_limb, pre ? nullptr : lcol, lval, lcnt, stats, B.rowptr,
+                pre ? nullptr : lflops, hs.gl);
+            h->launches++;
+        }
         dim3 bgrid((unsigned)(ldk / 64), (unsigned)((ldn + kBtCols - 1) / kBtCols));
         if (!gather_bt_smem<V>(lb)) return fail3(RMCM_OK);
         k_gather_bt<V><<<bgrid, kGatherThreads, lb * kBtTileBytes, s>>>(B, list, (int32_t)nh, (int32_t)ldk, (int32_t)ldn,
@@ -842,17 +937,16 @@ int32_t build_limbs(rmcm_handle *h, const DevCsr &A, const DevCsr &B, uint64_t b
     dp.heavy = nh;
     dp.sel = sel;
     dp.sel_bytes = sel_bytes;
-    dp.skip = flag;
     return RMCM_OK;
 }
 
-int32_t dense_part_build64(rmcm_handle *h, const DevCsr &A, const DevCsr &B, DensePart &dp, cudaEvent_t ev_begin,
-                           cudaEvent_t ev_end) {
+int32_t dense_part_build64(rmcm_handle *h, const DevCsr &A, int64_t a_max_row, const DevCsr &B, DensePart &dp,
+                           cudaEvent_t ev_begin, cudaEvent_t ev_end) {
     dp = DensePart{};
     const int32_t inv_density = h->tune.gemm_inv_density;
     if (inv_density <= 0 || A.rows == 0 || B.cols == 0 || A.cols == 0) return RMCM_OK;
     HeavySet hs;
-    RMCM_TRY(select_heavy(h, A, B, true, hs));
+    RMCM_TRY(select_heavy(h, A, B, a_max_row, true, hs));
     // B's largest value (row sums' last slot; 1 for a matrix of ones)
     uint64_t bmax = 1;
     if (B.vmax) {

@@ -239,8 +239,8 @@ int32_t convert_values(rmcm_handle *h, const rmcm_mat *src, int32_t valtype, rmc
 // dense_gemm.cu: tensor-core part of a dense-bin product.  S holds the
 // dense part's exact counts in the product's value type (A.rows x ld): the
 // sum over the limb GEMMs of G << (bits (i + j)), formed by the GEMM's
-// epilogue (tc_gemm.cu).  skip[u] flags the inner indices it covers; the
-// entries of A on the others are listed per row (lcol, lval, lcnt).
+// epilogue (tc_gemm.cu).  The entries of A on the inner indices that it does
+// not cover are listed per row (lcol, lval, lcnt).
 struct DensePart {
     const void *S = nullptr;
     int64_t ld = 0;
@@ -248,7 +248,6 @@ struct DensePart {
     int32_t alimbs = 1, abits = 0;    // A's limbs (limb form; 1 and 0 for the one-limb uint32 form)
     int32_t chunks = 1;               // chunks of the heavy indices (uint64 products)
     int64_t heavy = 0;
-    const uint8_t *skip = nullptr;
     // A's light entries: row r's are lcol/lval[rowptr[r] .. + lcnt[r])
     const int32_t *lcol = nullptr;
     const uint32_t *lval = nullptr;
@@ -262,10 +261,11 @@ struct DensePart {
 };
 // ev_begin / ev_end (may be null) are recorded around the GEMMs; light_flops
 // also counts each row's light products (dp.lflops, dp.lmax, dp.ltotal).
-int32_t dense_part_build(rmcm_handle *h, const DevCsr &A, const DevCsr &B, uint64_t bmax, DensePart &dp,
-                         cudaEvent_t ev_begin = nullptr, cudaEvent_t ev_end = nullptr, bool light_flops = false);
+int32_t dense_part_build(rmcm_handle *h, const DevCsr &A, int64_t a_max_row, const DevCsr &B, uint64_t bmax,
+                         DensePart &dp, cudaEvent_t ev_begin = nullptr, cudaEvent_t ev_end = nullptr,
+                         bool light_flops = false);
 // uint64 products: A split into limbs too and the heavy indices into chunks.
-int32_t dense_part_build64(rmcm_handle *h, const DevCsr &A, const DevCsr &B, DensePart &dp,
+int32_t dense_part_build64(rmcm_handle *h, const DevCsr &A, int64_t a_max_row, const DevCsr &B, DensePart &dp,
                            cudaEvent_t ev_begin = nullptr, cudaEvent_t ev_end = nullptr);
 void dense_part_release(rmcm_handle *h, DensePart &dp);
 // tc_gemm.cu: S (M x ldn of uint32 or uint64, vbytes) = sum over limbs and

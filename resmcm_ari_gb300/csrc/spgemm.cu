@@ -3761,9 +3761,9 @@ int32_t spgemm_t(rmcm_handle *h, const rmcm_mat *Am, const rmcm_mat *Bm, rmcm_ma
             cudaEvent_t e0 = rec ? h->prof[rec_idx].ev[6] : nullptr, e1 = rec ? h->prof[rec_idx].ev[7] : nullptr;
             int32_t drc = RMCM_OK;
             if (sizeof(V) == 4) {
-                drc = dense_part_build(h, A, B, bmax, dtemp.dpart, e0, e1, skewed);
+                drc = dense_part_build(h, A, Am->max_row, B, bmax, dtemp.dpart, e0, e1, skewed);
             } else {
-                drc = dense_part_build64(h, A, B, dtemp.dpart, e0, e1);
+                drc = dense_part_build64(h, A, Am->max_row, B, dtemp.dpart, e0, e1);
             }
             if (drc != RMCM_OK) {
                 dense_part_release(h, dtemp.dpart);

@@ -381,3 +381,25 @@ def test_row_pointers_over_many_tiles(native, engine, m):
         rp = np.concatenate([[0], np.cumsum(lens)])
         A = sp.csr_matrix((rng.integers(1, 6, rp[-1], dtype=np.uint64), rng.integers(0, k, rp[-1]), rp), shape=(m, k))
         check_product(native, engine, A, B, native.VAL_U32)
+
+
+@pytest.mark.parametrize("vt,hi", [("VAL_U32", 4), ("VAL_U32", 5000), ("VAL_U64", 4), ("VAL_U64", 2 ** 20)])
+def test_long_rows_of_the_tensor_part(native, vt, hi):
+    """Panels of rows about the length where they are filled in by pieces, at a
+    piece's edges and beyond, with heavy inner indices and light ones of every
+    length, one limb of values and several."""
+    eng = native.Engine(device=0)
+    eng.set_tuning(gemm_min_mflops=1)
+    rng = np.random.default_rng(hi)
+    k, n = 60000, 1000
+    rows = [0, 5000, 16384, 16385, 24576, 24577, 32768, 60000] + [16385] * 40 + [900] * 40
+    A = random_csr(rng, len(rows), k, rows, lo=1, hi=hi)
+    lens = rng.integers(0, 4, k)
+    lens[rng.permutation(k)[:400]] = n
+    B = random_csr(rng, k, n, lens, lo=1, hi=min(hi, 6))
+    eng.set_profiling(1)
+    check_product(native, eng, A, B, getattr(native, vt))
+    # an index in the sample of A's columns is heavy: 7 of 8 with 16 entries each
+    st = eng.product_stats()[-1]
+    assert st["gemm_inner"] >= 300, st
+    eng.close()
