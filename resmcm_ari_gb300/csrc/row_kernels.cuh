@@ -26,7 +26,7 @@
 
 // How the products of one entry of A are spread, by the length of its B row:
 // up to kOwnLen positions by the thread that read the entry, up to kMidLen by
-// eight lanes (32 bytes of a row per load), longer ones by whole warps.  A
+// kGroup lanes, each with four positions in flight, longer ones by whole warps.  A
 // lane reading a row of ten by itself touches a sector per position and
 // array; the L1, not the instruction rate, bounds such rows.
 constexpr int kOwnLen = 4;
@@ -314,7 +314,7 @@ __global__ void __launch_bounds__(kWarpWarps * 32, 8) k_row_warp(DevCsr A, const
 // row-padded temporary T (stride tstride), its length to cnt.  The CTA takes
 // up to four entries of A per thread and step: entries with short B rows are
 // added by their thread, the others listed in shared memory, mid entries
-// (eight lanes each) from the front and long ones from the back.  With at
+// (kGroup lanes each) from the front and long ones from the back.  With at
 // least two long entries per warp, warps take them one at a time; with fewer,
 // every entry is dealt to the warps in pieces of 128 positions, so a row of a
 // few long B rows (a 30,000-vertex type joined through 50) keeps every warp

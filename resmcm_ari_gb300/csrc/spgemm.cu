@@ -8,25 +8,34 @@
 // ascending columns; its column SET is the reference's row.
 //
 // Pipeline of one product C = A * B (m = A.rows, n = B.cols):
-//   1. k_analyze    warp per row: flops(u) = sum |B[a]|, bin of the row.
-//   2. k_scatter    row ids into per-bin lists (device-computed offsets).
-//   3. symbolic     exact |C[u]| per bin kernel (same kernels, NUMERIC=false).
+//   1. k_analyze    lanes of a warp per row: flops(u) = sum |B[a]|, bin of the row.
+//   2. k_scatter    row ids into per-bin lists (k_plan_small: products of few
+//                   rows, with the temporary's row pointers of step 3).
+//   3. the bins     rows of the short, rank and one-window dense bins once, into
+//                   bounded temporaries; the others count |C[u]| (NUMERIC=false).
 //   4. scan         device exclusive scan of |C[u]| into C.rowptr (int64).
-//   5. numeric      columns + counts per bin kernel (NUMERIC=true).
+//   5. copies       of the temporaries' rows into C; numeric pass of the others.
 // Bins (see classify; the thresholds are the handle's tunables):
 //   micro   flops <= G      G lanes per row (G = 1..16), one product per lane,
 //                           G-wide bitonic sort (only when G is tuned below 32).
 //   tiny    flops <= 32     one warp per row; products in registers, bitonic
 //                           sort across the warp, segmented sum, ballot compaction.
-//   hash*   flops <= 4096   one CTA per row; linear-probing hash table in shared
-//                           memory of at least min(flops, n) / load slots
-//                           (512/2048/8192; load 0.5 by default, at most 0.75),
-//                           then in-place compaction and a bitonic sort.
-//   dense   otherwise       one CTA per row; bitmap + counters over a window of
-//                           W columns in shared memory; rows wider than W are
-//                           processed window by window with per-entry cursors
-//                           (B rows are sorted).  Output is emitted word by word
-//                           with ballot compaction, so stores are coalesced.
+//   warp    n <= 2048       a warp per row, a window of its own (row_kernels.cuh).
+//   hash*   flops <= 4096   the 512- and 2048-slot tables' rows, of up to 256 and
+//                           1024 products: a warp per row, sorted and merged in
+//                           registers (sort_rows.cuh).  Where that cannot be (see
+//                           sort_takes) and for 8192 slots: one CTA per row,
+//                           linear-probing hash table in shared memory of at least
+//                           min(flops, n) / load slots, compaction, bitonic sort.
+//   dense   otherwise       a CTA per row over a window of W columns in shared
+//                           memory: k_row_window where no count can overflow
+//                           (row_kernels.cuh), else k_dense, bitmap + counters;
+//                           rows wider than W are processed window by window with
+//                           per-entry cursors (B rows are sorted).  Output is
+//                           emitted with ballot compaction, stores are coalesced.
+//   rank    wider rows      products partitioned by column into buckets that
+//                           warps sort (bucket_rows.cuh); the largest by a bitmap
+//                           of the whole row (k_rank), or split over CTAs.
 // Overflow: products and sums are checked against the value type; an
 // overflow raises the kOverflow status word (the structure stays exact).
 #include <cuda_runtime.h>
