@@ -3094,7 +3094,10 @@ struct RankSplit {
     int64_t bytes = 0;
 };
 
-// Rows with fewer products than this are never split.
+// Rows with fewer products than this are never split: the split costs four
+// launches and a host wait.  With 2^15 C-I-U-I-C at a twentieth took 940 us in
+// place of 1,012, T-I-C-I-T at a twentieth 515 in place of 479, the larger
+// chains the same.
 constexpr int64_t kSplitMinFlops = 1 << 17;
 constexpr int64_t kSplitMinRank = BucketCap<512>::max_flops;   // rank rows that k_bucket does not take
 constexpr int64_t kSplitMinLight = 1 << 18;   // light products of rows beside a tensor-core part
@@ -3346,10 +3349,14 @@ int32_t launch_bins(rmcm_handle *h, const DevCsr &A, const DevCsr &B, const DevC
                 if (NUMERIC && rn > 0) {
                     // k_rank takes the rows these leave: too many products, or too
                     // many on one range of columns
-                    RMCM_TRY((launch_bucket<V, 128>(h, A, B, a_ones, b_ones, C, rl, rn, temp, 0, cnt, bin_of, 0)));
-                    if (temp->max_rank_flops > BucketCap<128>::max_flops)
+                    // no more rows than the device holds CTAs of 512 threads at once (two an
+                    // SM): a row's time is the product's, so all of them take 512 threads
+                    const bool few = rn <= 2 * h->sm_count;
+                    if (!few)
+                        RMCM_TRY((launch_bucket<V, 128>(h, A, B, a_ones, b_ones, C, rl, rn, temp, 0, cnt, bin_of, 0)));
+                    if (few || temp->max_rank_flops > BucketCap<128>::max_flops)
                         RMCM_TRY((launch_bucket<V, 512>(h, A, B, a_ones, b_ones, C, rl, rn, temp,
-                                                        BucketCap<128>::max_flops, cnt, bin_of, 1)));
+                                                        few ? 0 : BucketCap<128>::max_flops, cnt, bin_of, 1)));
                 }
                 if (rn > 0)
                     kern<<<std::max(1, std::min(grid, rn)), kRankThreads, sm, s>>>(A, B, C, rl, rn, cnt, st, bin_of);

@@ -403,3 +403,15 @@ def test_long_rows_of_the_tensor_part(native, vt, hi):
     st = eng.product_stats()[-1]
     assert st["gemm_inner"] >= 300, st
     eng.close()
+
+
+@pytest.mark.parametrize("vt", ["VAL_U32", "VAL_U64"])
+@pytest.mark.parametrize("rows", [3, 304, 305, 700])
+def test_bucketed_rows_few_and_many(native, engine, rows, vt):
+    """Rank-bin rows about the count (two an SM) up to which every row takes the
+    larger CTAs; products from the fewest to beyond a smaller CTA's."""
+    rng = np.random.default_rng(rows)
+    n, k = 500_003, 400
+    B = random_csr(rng, k, n, rng.choice([3, 20, 40, 130], k), hi=30)
+    A = random_csr(rng, rows, k, rng.choice([30, 60, 190, 280], rows), hi=30)
+    check_product(native, engine, A, B, getattr(native, vt))
