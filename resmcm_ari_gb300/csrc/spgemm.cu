@@ -2122,50 +2122,50 @@ __global__ void __launch_bounds__(1024) k_split_tasks(const int32_t *parts, cons
     if (ns == 0 && tid == 0) task_start[0] = 0;
 }
 
+// Task -> slot (last slot whose first task is <= task).
+__device__ __forceinline__ int split_slot_of(const int32_t *task_start, int ns, int task) {
+    int lo = 0, hi = ns - 1;
+    while (lo < hi) {
+        const int mid = (lo + hi + 1) >> 1;
+        if (task_start[mid] <= task) lo = mid;
+        else hi = mid - 1;
+    }
+    return lo;
+}
+
 // One CTA per task (slot, part): the part's A-entry range into the shared
 // window, then its nonzero counters into the slot's global accumulator.
-template <typename V, bool PRES = true>
+template <typename V>
 __global__ void __launch_bounds__(kSplitThreads) k_dense_split(DevCsr A, DevCsr B, const int32_t *rows,
                                                                const int32_t *row_of_slot, const int32_t *parts,
                                                                const int32_t *task_start, const int32_t *nslots,
                                                                int32_t max_slots, int32_t W,
                                                                unsigned long long *G, uint32_t *Gbits,
                                                                const uint8_t *bin_of, int *st, int32_t wc,
-                                                               bool pull_ok, const uint32_t *pk, int32_t cbits,
-                                                               const int32_t *lcnt) {
+                                                               bool pull_ok) {
     constexpr int NT = kSplitThreads;
     constexpr int kPull = 4;   // register accumulators per thread: rows of up to 4 * NT columns
     static_assert(kChunk == NT, "one staged A entry per thread");
     const V *Aval = (const V *)A.val;
     const V *Bval = (const V *)B.val;
     extern __shared__ __align__(16) unsigned char smem[];
-    // PRES = false (every value >= 1, no row can overflow): counters alone
-    // mark presence and the window holds only them
     uint8_t *present = smem;
-    V *acc = (V *)(PRES ? smem + (((size_t)W + 15) & ~(size_t)15) : smem);
+    V *acc = (V *)(smem + (((size_t)W + 15) & ~(size_t)15));
     __shared__ ChunkStage<V> sg;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const unsigned lt_mask = (1u << lane) - 1u;
     const int ns = min(*nslots, max_slots);
     const int ntasks = task_start[ns];
-    if (PRES)
-        for (int i = tid; i < W / 16; i += NT) ((uint4 *)present)[i] = make_uint4(0, 0, 0, 0);
+    for (int i = tid; i < W / 16; i += NT) ((uint4 *)present)[i] = make_uint4(0, 0, 0, 0);
     for (int i = tid; i < W; i += NT) acc[i] = 0;
     bool ovf = false;
     __syncthreads();
     for (int task = blockIdx.x; task < ntasks; task += gridDim.x) {
-        int lo = 0, hi = ns - 1;   // last slot with task_start <= task
-        while (lo < hi) {
-            const int mid = (lo + hi + 1) >> 1;
-            if (task_start[mid] <= task) lo = mid;
-            else hi = mid - 1;
-        }
-        const int slot = lo;
+        const int slot = split_slot_of(task_start, ns, task);
         const int part = task - task_start[slot];
         const int np = parts[slot];
         const int32_t r = rows[row_of_slot[slot]];
-        // (lcnt: A holds the row's light entries only, lcnt[r] of them)
-        const int64_t a0 = A.rowptr[r], alen = lcnt ? (int64_t)lcnt[r] : A.rowptr[r + 1] - a0;
+        const int64_t a0 = A.rowptr[r], alen = A.rowptr[r + 1] - a0;
         const int64_t ka = a0 + alen * part / np, kb = a0 + alen * (part + 1) / np;
         const bool checked = (bin_of[r] & kRiskyBit) != 0;
         // B rows covering all wc columns ("full", as in the dense bin) are
@@ -2219,26 +2219,17 @@ __global__ void __launch_bounds__(kSplitThreads) k_dense_split(DevCsr A, DevCsr 
             // entries are added by the thread that staged them
             if (checked) {
                 auto vis = [&](int32_t c, V p) {
-                    if (PRES) present[c] = 1;
+                    present[c] = 1;
                     add_shared_chk(acc + c, p, ovf);
                 };
                 if (tl) stream_long_fast<V, true, true>(sg, tl, B, ovf, vis);
                 for (int64_t q = own_lo; q < own_hi; q++) vis(__ldg(B.col + q), mul_chk(own_a, __ldg(Bval + q), ovf));
             } else {
                 auto vis = [&](int32_t c, V p) {
-                    if (PRES) present[c] = 1;
+                    present[c] = 1;
                     add_shared(acc + c, p);
                 };
-                if (tl) {
-                    bool done = false;
-                    if constexpr (sizeof(V) == 4 && !PRES) {
-                        if (pk) {
-                            stream_long_packed(sg, tl, pk, cbits, vis);
-                            done = true;
-                        }
-                    }
-                    if (!done) stream_long_fast<V, true, false>(sg, tl, B, ovf, vis);
-                }
+                if (tl) stream_long_fast<V, true, false>(sg, tl, B, ovf, vis);
                 int64_t q = own_lo;
                 for (; q + 3 < own_hi; q += 4) {
                     int32_t c[4];
@@ -2288,7 +2279,7 @@ __global__ void __launch_bounds__(kSplitThreads) k_dense_split(DevCsr A, DevCsr 
                 if (c < wc) {
                     if (checked) ovf |= acc[c] > (V)~(V)0 - preg[j];
                     acc[c] += preg[j];
-                    if (PRES) present[c] = 1;
+                    present[c] = 1;
                 }
             }
             __syncthreads();
@@ -2297,7 +2288,7 @@ __global__ void __launch_bounds__(kSplitThreads) k_dense_split(DevCsr A, DevCsr 
         unsigned long long *g = G + (int64_t)slot * W;
         uint32_t *gb = Gbits + (int64_t)slot * (W / 32);
         for (int c = tid; c < W; c += NT) {
-            const bool here = PRES ? present[c] != 0 : acc[c] != 0;
+            const bool here = present[c] != 0;
             const unsigned bits = __ballot_sync(kFull, here);
             if (here) {
                 const unsigned long long v = (unsigned long long)acc[c];
@@ -2305,8 +2296,65 @@ __global__ void __launch_bounds__(kSplitThreads) k_dense_split(DevCsr A, DevCsr 
                     const unsigned long long old = atomicAdd(g + c, v);
                     ovf |= old > ~0ull - v;
                 }
-                if (PRES) present[c] = 0;
+                present[c] = 0;
                 acc[c] = 0;
+            }
+            if (lane == 0 && bits) atomicOr(gb + (c >> 5), bits);
+        }
+        __syncthreads();
+    }
+    if (__syncthreads_or(ovf) && tid == 0) raise_status(st, kOverflow);
+}
+
+// The same for products whose counts cannot overflow and whose values are all
+// >= 1, by the row kernels' products: no presence bytes, packed B.  With lcnt,
+// A holds a row's light entries only, lcnt[r] of them, beside its tensor-core
+// part.  Bound as k_row_window is, by the L1 and the shared adds: a thread per
+// staged entry of k_dense_split's, with barriers around lists of 512, was
+// bound by its gathers' latency (C-I-T-I-U-I-C at 0.06 of its size 1,290 -> 1,204
+// us, at a tenth 1,701 -> 1,566, at a quarter 3,158 -> 2,923).
+template <typename V, bool PK>
+__global__ void __launch_bounds__(kSplitThreads, 2) k_row_split(DevCsr A, const V *aval, RowB<V> B,
+                                                                const int32_t *rows, const int32_t *row_of_slot,
+                                                                const int32_t *parts, const int32_t *task_start,
+                                                                const int32_t *nslots, int32_t max_slots, int32_t W,
+                                                                unsigned long long *G, uint32_t *Gbits,
+                                                                const uint8_t *bin_of, int *st,
+                                                                const int32_t *lcnt) {
+    constexpr int NT = kSplitThreads;
+    extern __shared__ __align__(16) unsigned char smem[];
+    const Window<V> win(smem, W);
+    __shared__ RowLists<NT, V> sl;
+    const int tid = threadIdx.x, lane = tid & 31;
+    const int ns = min(*nslots, max_slots);
+    const int ntasks = task_start[ns];
+    for (int i = tid; i < W; i += NT) win.set(i, 0);
+    if (tid < 2) {
+        sl.nmid[tid] = 0;
+        sl.nlong[tid] = 0;
+        sl.ctr[tid] = 0;
+    }
+    __syncthreads();
+    bool ovf = false;
+    int cur = 0;
+    for (int task = blockIdx.x; task < ntasks; task += gridDim.x) {
+        const int slot = split_slot_of(task_start, ns, task);
+        const int part = task - task_start[slot], np = parts[slot];
+        const int32_t r = rows[row_of_slot[slot]];
+        const int64_t a0 = A.rowptr[r], alen = lcnt ? (int64_t)lcnt[r] : A.rowptr[r + 1] - a0;
+        const int64_t ka = a0 + alen * part / np, kb = a0 + alen * (part + 1) / np;
+        if (sizeof(V) == 4 || (bin_of[r] & kNarrowBit)) row_window_products<true, PK>(A, aval, B, ka, kb, win, sl, cur);
+        else row_window_products<false, PK>(A, aval, B, ka, kb, win, sl, cur);
+        // merge: one global atomic per present column, then clear the window
+        unsigned long long *g = G + (int64_t)slot * W;
+        uint32_t *gb = Gbits + (int64_t)slot * (W / 32);
+        for (int c = tid; c < W; c += NT) {
+            const unsigned long long v = (unsigned long long)win.get(c);
+            const unsigned bits = __ballot_sync(kFull, v != 0);
+            if (v) {
+                const unsigned long long old = atomicAdd(g + c, v);
+                ovf |= old > ~0ull - v;
+                win.set(c, 0);
             }
             if (lane == 0 && bits) atomicOr(gb + (c >> 5), bits);
         }
@@ -2550,16 +2598,6 @@ __global__ void __launch_bounds__(kRankThreads) k_rank(DevCsr A, DevCsr B, DevCs
 // per-word ranks, writes the sorted columns and zeroes the values; then a CTA
 // per part adds its products at their ranks with global atomics.
 
-// Task -> slot (last slot whose first task is <= task).
-__device__ __forceinline__ int split_slot_of(const int32_t *task_start, int ns, int task) {
-    int lo = 0, hi = ns - 1;
-    while (lo < hi) {
-        const int mid = (lo + hi + 1) >> 1;
-        if (task_start[mid] <= task) lo = mid;
-        else hi = mid - 1;
-    }
-    return lo;
-}
 
 template <typename V>
 __global__ void __launch_bounds__(kRankThreads) k_rank_split_sym(DevCsr A, DevCsr B, const int32_t *rows,
@@ -3387,18 +3425,27 @@ int32_t launch_bins(rmcm_handle *h, const DevCsr &A, const DevCsr &B, const DevC
                         }
                         if (temp->split) {
                             // the split rows run on the second stream, beside the dense bin
-                            const bool slite = positive && temp->no_risky;
-                            const int64_t ssm = slite ? sm_lite : sm;
-                            auto ks = slite ? k_dense_split<V, false> : k_dense_split<V, true>;
-                            RMCM_TRY(set_smem(h, ks, ssm));
                             RMCM_CUDA(h, cudaEventRecord(h->ev_fork, s));
                             RMCM_CUDA(h, cudaStreamWaitEvent(h->aux, h->ev_fork, 0));
-                            const int sper = (int)std::max<int64_t>(1, std::min<int64_t>(4, (200 * 1024) / std::max<int64_t>(ssm, 1)));
-                            ks<<<(int)((int64_t)h->sm_count * sper), kSplitThreads, ssm, h->aux>>>(
-                                Al, B, temp->perm, temp->row_of_slot, temp->parts, temp->task_start, temp->nslots,
-                                temp->max_slots, (int32_t)W, temp->G, temp->Gbits, bin_of, st, (int32_t)ncols,
-                                b_distinct && ncols <= 4 * kSplitThreads, temp->pk, temp->cbits,
-                                temp->dpart.S ? temp->dpart.lcnt : nullptr);
+                            auto split_grid = [&](int64_t bytes) {
+                                const int64_t per_sm = (200 * 1024) / std::max<int64_t>(bytes, 1);
+                                return h->sm_count * (int)std::max<int64_t>(1, std::min<int64_t>(4, per_sm));
+                            };
+                            if (lean && temp->no_risky) {
+                                auto ks = lean->B.words ? k_row_split<V, true> : k_row_split<V, false>;
+                                RMCM_TRY(set_smem(h, ks, sm_lite));
+                                ks<<<split_grid(sm_lite), kSplitThreads, sm_lite, h->aux>>>(
+                                    Al, temp->dpart.S ? (const V *)Al.val : lean->aval, lean->B, temp->perm,
+                                    temp->row_of_slot, temp->parts, temp->task_start, temp->nslots, temp->max_slots,
+                                    (int32_t)W, temp->G, temp->Gbits, bin_of, st,
+                                    temp->dpart.S ? temp->dpart.lcnt : nullptr);
+                            } else {
+                                RMCM_TRY(set_smem(h, k_dense_split<V>, sm));
+                                k_dense_split<V><<<split_grid(sm), kSplitThreads, sm, h->aux>>>(
+                                    A, B, temp->perm, temp->row_of_slot, temp->parts, temp->task_start, temp->nslots,
+                                    temp->max_slots, (int32_t)W, temp->G, temp->Gbits, bin_of, st, (int32_t)ncols,
+                                    b_distinct && ncols <= 4 * kSplitThreads);
+                            }
                             k_split_finish<V><<<temp->max_slots, kSplitThreads, 0, h->aux>>>(
                                 T, temp->perm, temp->row_of_slot, temp->nslots, temp->max_slots, ncols, (int32_t)W,
                                 temp->G, temp->Gbits, temp->stride, cnt, st, (const V *)temp->dpart.S,

@@ -415,3 +415,26 @@ def test_bucketed_rows_few_and_many(native, engine, rows, vt):
     B = random_csr(rng, k, n, rng.choice([3, 20, 40, 130], k), hi=30)
     A = random_csr(rng, rows, k, rng.choice([30, 60, 190, 280], rows), hi=30)
     check_product(native, engine, A, B, getattr(native, vt))
+
+
+@pytest.mark.parametrize("vt,hi,bhi", [("VAL_U32", 4, 4), ("VAL_U32", 4, 2 ** 20), ("VAL_U64", 4, 4),
+                                       ("VAL_U64", 2 ** 20, 2 ** 24)])
+@pytest.mark.parametrize("n", [97, 128, 2049, 22528])
+def test_split_rows(native, engine, n, vt, hi, bhi):
+    """Rows split over CTAs: windows of one block and at their limits, B packed
+    and not, counts within 32 bits and beyond, B rows of every length class."""
+    rng = np.random.default_rng(n)
+    k = 30000
+    lens = np.minimum(rng.choice([0, 1, 4, 5, 9, 40, 64, 65, 200], k), n)
+    hub = rng.integers(0, n, 40)
+    rows = np.repeat(np.arange(k), lens)
+    cols = np.concatenate([rng.permutation(n)[:x] for x in lens])
+    cols[rng.random(cols.size) < 0.02] = hub[0]
+    B = sp.csr_matrix((rng.integers(1, bhi, cols.size, dtype=np.uint64), (rows, cols)), shape=(k, n))
+    B.sum_duplicates()
+    A = random_csr(rng, 40, k, [29000, 12000, 30000] + [30] * 37, hi=hi)
+    if vt == "VAL_U32" and bhi > 4:
+        A.data[:] = 1
+        B.data[:] = 1 + B.data % 2
+        B.data[::50000] = bhi      # too wide to pack beside the widest columns, sums within 32 bits
+    check_product(native, engine, A, B, getattr(native, vt))
