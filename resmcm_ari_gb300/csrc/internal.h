@@ -101,6 +101,7 @@ struct ProductPlan {
     int32_t n_front = 0;
     int64_t max_rank_flops = 0;
     int32_t risky_rows = 0;
+    bool c_positive = false;         // the result's positive flag
     bool rank_split = false;
     int32_t rank_n_front = 0;
     int64_t scratch_bytes = 0;
@@ -214,6 +215,8 @@ void mat_release(rmcm_handle *h, rmcm_mat *m);
 // Copies up to three device ranges into pinned host buffers with a small
 // kernel on stream s (chain_dp.cu); false if a buffer is not device-mapped.
 bool copy_out_launch(const void *const *src, void *const *dst_host, const int64_t *bytes, cudaStream_t s);
+// Queues the copy of the device status words to h_status.
+int32_t status_fetch(rmcm_handle *h);
 // Read and clear the device status words; maps them to a status code.
 int32_t check_status(rmcm_handle *h);
 // The same for words already read back (rmcm_handle::status_read), else check_status.

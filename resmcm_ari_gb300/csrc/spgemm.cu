@@ -4209,6 +4209,23 @@ int32_t spgemm_t(rmcm_handle *h, const rmcm_mat *Am, const rmcm_mat *Bm, rmcm_ma
     drop_cursors();
     drop_temp();
     drop_rank();
+    // A count that wrapped may be 0, and the kernels of the next product take
+    // a counter > 0 for the mark of a column: with rows that may overflow, the
+    // result is positive only when none did (the words gather over a chain's
+    // products).
+    bool c_positive = positive;
+    if (replay) {
+        c_positive = plan->c_positive;
+    } else if (positive && !dtemp.no_risky && rc == RMCM_OK) {
+        if (!h->status_read) {   // a bin's counts come with the numeric pass
+            rc = status_fetch(h);
+            const cudaError_t e = cudaStreamSynchronize(s);
+            if (rc == RMCM_OK && e != cudaSuccess) rc = cuda_error(h, e, "spgemm status download");
+            h->status_read = rc == RMCM_OK;
+        }
+        c_positive = rc == RMCM_OK && h->h_status[kOverflow] == 0;
+    }
+    if (record) plan->c_positive = c_positive;
     if (rc != RMCM_OK) {
         mat_release(h, C);
         return rc;
@@ -4261,7 +4278,7 @@ int32_t spgemm_t(rmcm_handle *h, const rmcm_mat *Am, const rmcm_mat *Bm, rmcm_ma
             st.bytes_c = (m + 1) * 8 + nnz * (4 + iv);
         }
     }
-    C->positive = positive;
+    C->positive = c_positive;
     C->distinct = true;
     C->max_row = c_max_row;
     *Cout = C;
