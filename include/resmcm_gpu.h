@@ -213,7 +213,8 @@ RMCM_API int32_t rmcm_order(rmcm_handle *h, const double *c, int32_t len, int32_
 /* ---- stage (c): Gustavson SpGEMM ------------------------------------------
  * Replaces SpGEMM / row_wise_SpGEMM_based_on_bitmap (efficient/resmcm.cpp:586-647).
  * C = A*B with exact integer path counts in A's value type; C's rows are
- * sorted.  Returns RMCM_EOVERFLOW (C kept) if a count overflowed. */
+ * sorted.  Returns RMCM_EOVERFLOW (C kept) if a count overflowed.  C is
+ * written when the call returns (it waits for the handle's stream). */
 RMCM_API int32_t rmcm_spgemm(rmcm_handle *h, const rmcm_mat *A, const rmcm_mat *B, rmcm_mat **C);
 
 /* ---- (a)+(b)+(c): one chain -----------------------------------------------

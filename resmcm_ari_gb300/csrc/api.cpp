@@ -1589,6 +1589,9 @@ RMCM_API int32_t rmcm_spgemm(rmcm_handle *h, const rmcm_mat *A, const rmcm_mat *
     int32_t rc = spgemm(h, A, B, C, nullptr);
     if (rc != RMCM_OK) return rc;
     rc = product_status(h);
+    // the copies of the single-pass rows into C are queued behind the status
+    const cudaError_t e = cudaStreamSynchronize(h->stream);
+    if (e != cudaSuccess) rc = cuda_error(h, e, "spgemm");
     if (rc == RMCM_EOVERFLOW) (*C)->positive = false;   // wrapped counts may be 0
     if (rc != RMCM_OK && rc != RMCM_EOVERFLOW) {
         mat_release(h, *C);

@@ -1,4 +1,4 @@
-"""What a product leaves behind when counts overflow."""
+"""What a product leaves behind when counts overflow, and when its call is done."""
 import numpy as np
 import pytest
 import scipy.sparse as sp
@@ -47,4 +47,26 @@ def test_a_count_that_wraps_to_zero_keeps_its_column(native, vt, n, rows):
     assert np.array_equal(rp, np.arange(rows + 1) * cols.size)
     assert np.array_equal(col.reshape(rows, -1), np.tile(cols, (rows, 1)))
     assert np.array_equal(val.reshape(rows, -1)[[0, -1]].astype(np.uint64), np.array([[want[c] for c in cols]] * 2, np.uint64))
+    eng.close()
+
+
+def test_spgemm_returns_with_its_result_written(native):
+    """Rows of a single-pass product are copied into the result last: the call
+    waits for that, nothing of it is left on the stream."""
+    import torch
+
+    eng = native.Engine(device=0)
+    st = torch.cuda.Stream()
+    eng.set_stream(st.cuda_stream)
+    rng = np.random.default_rng(2)
+    m, k, n = 20000, 60, 3000
+    A = _rows([([r % k, (r * 7 + 1) % k] if (r * 7 + 1) % k != r % k else [r % k], [1] * (2 if (r * 7 + 1) % k != r % k else 1))
+               for r in range(m)], k)
+    B = _rows([(np.sort(rng.choice(n, 2000, replace=False)), rng.integers(1, 9, 2000)) for _ in range(k)], n)
+    a, b = _upload(eng, A, native.VAL_U32), _upload(eng, B, native.VAL_U32)
+    for _ in range(5):
+        C = eng.spgemm(a, b)      # some 50M entries to copy
+        assert st.query()
+        C.free()
+    a.free(), b.free()
     eng.close()
