@@ -514,15 +514,13 @@ __global__ void __launch_bounds__(kGatherThreads) k_gather_al(DevCsr A, const in
     }
 }
 
-// Opts k_gather_bt<V> in to the shared memory of `limbs` tiles; false when
-// the device refuses (the caller keeps the product sparse).
-template <typename V>
-bool gather_bt_smem(int32_t limbs) {
-    const int64_t bytes = limbs * kBtTileBytes;
-    if (bytes <= 48 * 1024) return true;
-    if (cudaFuncSetAttribute(k_gather_bt<V>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) == cudaSuccess)
-        return true;
+// Opts a gather kernel in to its shared memory; false when the device refuses
+// (the caller keeps the product sparse).
+template <typename F>
+bool gather_smem(rmcm_handle *h, F *kernel, int64_t bytes) {
+    if (set_smem(h, kernel, bytes) == RMCM_OK) return true;
     cudaGetLastError();
+    h->last_error.clear();
     return false;
 }
 
@@ -667,11 +665,7 @@ int32_t dense_part_build(rmcm_handle *h, const DevCsr &A, int64_t a_max_row, con
     };
     {
         const int64_t smem = ldk * 2;
-        if (smem > 48 * 1024 &&
-            cudaFuncSetAttribute(k_gather_a, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) {
-            cudaGetLastError();
-            return fail2(RMCM_OK);
-        }
+        if (!gather_smem(h, k_gather_a, smem)) return fail2(RMCM_OK);
         const int grid = (int)std::min<int64_t>(M, (int64_t)h->sm_count * 8);
         if (hs.long_rows) RMCM_CUDA(h, cudaMemsetAsync(hs.gl.n, 0, hs.gl_bytes, s));
         k_gather_a<<<grid, kGatherThreads, smem, s>>>(A, slot, (int32_t)ldk, Ad, lcol, lval, lcnt, stats, B.rowptr,
@@ -682,7 +676,8 @@ int32_t dense_part_build(rmcm_handle *h, const DevCsr &A, int64_t a_max_row, con
                 A, slot, (int32_t)ldk, 1, 0, Ad, 0, lcol, lval, lcnt, stats, B.rowptr, lflops, hs.gl);
             h->launches++;
         }
-        RMCM_CUDA(h, cudaGetLastError());
+        const cudaError_t e = cudaGetLastError();
+        if (e != cudaSuccess) return fail2(cuda_error(h, e, "tensor part: panel of A"));
     }
     RMCM_CUDA(h, cudaMemcpyAsync(h->h_pinned + 8, stats, 8 * sizeof(uint64_t), cudaMemcpyDeviceToHost, s));
     RMCM_CUDA(h, cudaStreamSynchronize(s));
@@ -729,12 +724,13 @@ int32_t dense_part_build(rmcm_handle *h, const DevCsr &A, int64_t a_max_row, con
     };
     {
         dim3 grid((unsigned)(ldk / 64), (unsigned)((ldn + kBtCols - 1) / kBtCols));
-        if (!gather_bt_smem<uint32_t>(limbs)) return fail3(RMCM_OK);
+        if (!gather_smem(h, k_gather_bt<uint32_t>, limbs * kBtTileBytes)) return fail3(RMCM_OK);
         k_gather_bt<uint32_t><<<grid, kGatherThreads, limbs * kBtTileBytes, s>>>(B, list, (int32_t)nh, (int32_t)ldk,
                                                                                   (int32_t)ldn,
                                                              limbs, bits, BdT, b_limb, stats);
         h->launches++;
-        RMCM_CUDA(h, cudaGetLastError());
+        const cudaError_t e = cudaGetLastError();
+        if (e != cudaSuccess) return fail3(cuda_error(h, e, "tensor part: panel of B"));
     }
     if (ev_begin) cudaEventRecord(ev_begin, s);
     {
@@ -872,12 +868,8 @@ int32_t build_limbs(rmcm_handle *h, const DevCsr &A, const DevCsr &B, uint64_t b
     V *S = (V *)(mem + bd_bytes);
     {
         const int64_t smem = group * ldk * 2;
-        if (smem > 48 * 1024 &&
-            cudaFuncSetAttribute(k_gather_al<V>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
-                cudaSuccess) {
-            cudaGetLastError();
+        if (!gather_smem(h, k_gather_al<V>, smem) || !gather_smem(h, k_gather_bt<V>, lb * kBtTileBytes))
             return fail3(RMCM_OK);
-        }
         const int grid = (int)std::min<int64_t>(M, (int64_t)h->sm_count * 8);
         if (hs.long_rows) RMCM_CUDA(h, cudaMemsetAsync(hs.gl.n, 0, hs.gl_bytes, s));
         // (with pre the light entries are already compacted: panels only)
@@ -891,12 +883,12 @@ int32_t build_limbs(rmcm_handle *h, const DevCsr &A, const DevCsr &B, uint64_t b
             h->launches++;
         }
         dim3 bgrid((unsigned)(ldk / 64), (unsigned)((ldn + kBtCols - 1) / kBtCols));
-        if (!gather_bt_smem<V>(lb)) return fail3(RMCM_OK);
         k_gather_bt<V><<<bgrid, kGatherThreads, lb * kBtTileBytes, s>>>(B, list, (int32_t)nh, (int32_t)ldk, (int32_t)ldn,
                                                                         lb, bits,
                                                        BdT, b_limb, stats);
         h->launches += 2;
-        RMCM_CUDA(h, cudaGetLastError());
+        const cudaError_t e = cudaGetLastError();
+        if (e != cudaSuccess) return fail3(cuda_error(h, e, "tensor part: panels"));
     }
     // every limb pair and chunk of the heavy indices in one kernel, summed
     // with its shift into one seed per output

@@ -6,6 +6,7 @@
 #include <cstdint>
 #include <functional>
 #include <map>
+#include <mutex>
 #include <set>
 #include <string>
 #include <tuple>
@@ -221,6 +222,23 @@ int32_t status_fetch(rmcm_handle *h);
 int32_t check_status(rmcm_handle *h);
 // The same for words already read back (rmcm_handle::status_read), else check_status.
 int32_t product_status(rmcm_handle *h);
+
+// Opt a kernel in to `bytes` of dynamic shared memory (static shared memory
+// counts against the same 48 KB default, so the attribute is set whenever the
+// request is non-zero and above what this kernel was last given; it only
+// grows, so that handles of other threads keep what they asked for).
+template <typename F>
+int32_t set_smem(rmcm_handle *h, F *kernel, int64_t bytes) {
+    static std::mutex mu;
+    static std::map<std::pair<int, const void *>, int64_t> given;
+    std::lock_guard<std::mutex> lock(mu);
+    auto key = std::make_pair(h->device, (const void *)kernel);
+    auto it = given.find(key);
+    if (it != given.end() && it->second >= bytes) return RMCM_OK;
+    RMCM_CUDA(h, cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+    given[key] = bytes;
+    return RMCM_OK;
+}
 
 inline int64_t val_bytes(int32_t valtype) { return valtype == RMCM_VAL_U64 ? 8 : 4; }
 // Row records of a matrix, its largest value and its rows' (rmcm_mat::rowinfo).

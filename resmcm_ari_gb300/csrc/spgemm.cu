@@ -3018,22 +3018,6 @@ int grid_for(rmcm_handle *h, int64_t work, int threads, int per_sm) {
     return (int)g;
 }
 
-// Opt a kernel in to `bytes` of dynamic shared memory (static shared memory
-// counts against the same 48 KB default, so the attribute is set whenever the
-// request is non-zero and above what this kernel was last given).
-template <typename F>
-int32_t set_smem(rmcm_handle *h, F *kernel, int64_t bytes) {
-    static std::mutex mu;
-    static std::map<std::pair<int, const void *>, int64_t> given;
-    std::lock_guard<std::mutex> lock(mu);
-    auto key = std::make_pair(h->device, (const void *)kernel);
-    auto it = given.find(key);
-    if (it != given.end() && it->second >= bytes) return RMCM_OK;
-    RMCM_CUDA(h, cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
-    given[key] = bytes;
-    return RMCM_OK;
-}
-
 // Resident CTAs per SM of `kernel` at `threads` threads and `bytes` of dynamic
 // shared memory (cached per device, kernel and size; the kernel's shared
 // memory limit must already be set).

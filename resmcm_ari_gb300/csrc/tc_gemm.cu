@@ -478,9 +478,7 @@ int32_t launch_tc(rmcm_handle *h, const CUtensorMap &ma, const CUtensorMap &mb, 
                                      (M - r0) * (int64_t)p.ldn * (int64_t)sizeof(V), s));
     }
     const int64_t grid = full + (tiles - full) * splits;
-    if (cudaFuncSetAttribute(k_tc_seed<V, BN, MSUB>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) !=
-        cudaSuccess)
-        return set_error(h, RMCM_ECUDA, "tc_seed_gemm: shared memory opt-in");
+    RMCM_TRY(set_smem(h, k_tc_seed<V, BN, MSUB>, smem));
     k_tc_seed<V, BN, MSUB><<<(unsigned)grid, kTcThreads, smem, s>>>(ma, mb, p);
     h->launches++;
     RMCM_CUDA(h, cudaGetLastError());
