@@ -48,8 +48,10 @@ __global__ void __launch_bounds__(32) k_chain_dp(const double *c_all, const int3
         const int i = lane;
         if (i < len - l) {
             const int j = i + l;
+            // (a cost that is not below DBL_MAX, a NaN's included, leaves the first
+            // split: the walk below needs one inside the interval)
             double best = DBL_MAX;
-            int bk = 0;
+            int bk = i;
             for (int k = i; k < j; k++) {
                 const double tmp = __dadd_rn(__dadd_rn(sc[i * kMaxLen + k], sc[(k + 1) * kMaxLen + j]), sc[i * kMaxLen + j]);
                 const double cost = __dadd_rn(__dadd_rn(sm[i * kMaxLen + k], sm[(k + 1) * kMaxLen + j]), tmp);
