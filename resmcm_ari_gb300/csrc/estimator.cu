@@ -59,11 +59,14 @@ __device__ __forceinline__ double factor_product(const DevCsr &M, const double *
     double p[U];
     int32_t v[U];
 #pragma unroll
+    for (int u = 0; u < U; u++) v[u] = k0 + u * (int64_t)G < k1 ? __ldg(M.col + k0 + u * (int64_t)G) : -1;
+#pragma unroll
     for (int u = 0; u < U; u++) {
-        p[u] = 1.0;
-        v[u] = k0 + u * (int64_t)G < k1 ? __ldg(M.col + k0 + u * (int64_t)G) : -1;
+        p[u] = v[u] >= 0 ? __ldg(q_next + (int64_t)v[u] * stride) : 1.0;
+        const int64_t kn = k0 + (U + u) * (int64_t)G;
+        v[u] = kn < k1 ? __ldg(M.col + kn) : -1;
     }
-    for (int64_t k = k0; k < k1; k += U * (int64_t)G) {
+    for (int64_t k = k0 + U * (int64_t)G; k < k1; k += U * (int64_t)G) {
         double q[U];
 #pragma unroll
         for (int u = 0; u < U; u++) q[u] = v[u] >= 0 ? __ldg(q_next + (int64_t)v[u] * stride) : 1.0;
@@ -97,14 +100,20 @@ inline int32_t level_tile(int64_t rows, int64_t blocks_cap) {
 // groups of jp lanes, enough for four entries a lane (32 / jp groups at most),
 // and are laid out group after group, the largest first: every step multiplies
 // 32 / jp groups' entries, three multiplies and one per halving of the largest
-// row in it.  A row of more than kWideLane entries a lane would hold up the
-// warp; the CTA's warps multiply a slice of each such row together afterwards.
-// Against a row per warp step (one to three of 32 lanes busy on most rows of a
-// Zipf leaf) and 4,096 entries as one warp's share: a six-matrix chain over the
-// 1,000,000 x 300,000 leaf with 20M entries 1,626 -> 777 us in all (its two
-// 20M-entry levels 355 -> 200 and 353 -> 220 us, the 2,000-row level 377 -> 43,
-// the last matrix, a row per thread now, 54 -> 9, the nine rows of up to
-// 53,000 entries 183 -> 37).
+// row in it.  Against a row per warp step (one to three of 32 lanes busy on
+// most rows of a Zipf leaf) and 4,096 entries as one warp's share: a six-matrix
+// chain over the 1,000,000 x 300,000 leaf with 20M entries 1,626 -> 715 us in
+// all.
+//
+// A chunk's rows lie nch apart, so that neighbours of like length (rows sorted
+// by degree, hubs numbered together) come to different CTAs: with 32
+// consecutive rows a warp, one CTA held most of the long ones (100,000 rows of
+// 60,000 / (rank + 10) entries, six matrices: 3,468 us so, 287 now).
+// Rows of more than kWideLane entries a lane hold up their warp.  The CTA's
+// warps multiply a slice of each together where one warp has more than twice
+// the average of them; that costs a slice's combining multiplies and two
+// barriers a row, so evenly long rows stay with their warps (3,000 rows of 900,
+// five matrices: 199 us shared, 139 not) unless a slice is long itself.
 constexpr int kWideLane = 64;
 
 __device__ __forceinline__ void res_level_body(const DevCsr &M, const double *q_next, double *q_cur,
@@ -122,6 +131,8 @@ __device__ __forceinline__ void res_level_body(const DevCsr &M, const double *q_
     __shared__ double s_tp[NW][32 * kMaxLen];   // tile products: [t * jp + jo]
     __shared__ double s_wide[NW][kMaxLen];      // slices of a wide row
     __shared__ uint8_t s_ord[NW][32];           // the warp's rows, most groups first
+    __shared__ uint2 s_mask[NW];                // each warp's wide rows, the huge ones, and the former's entries
+    __shared__ int32_t s_load[NW];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const unsigned lt_mask = (1u << lane) - 1u;
     const int T = la.tile;                      // rows per warp and chunk (1 .. 32)
@@ -129,18 +140,19 @@ __device__ __forceinline__ void res_level_body(const DevCsr &M, const double *q_
     const int ng = 32 / jp;                     // groups per step
     const int emax = 31 - __clz(ng);
     const int64_t wide_min = kWideLane * (int64_t)ng;
+    const int64_t nch = (M.rows + NW * T - 1) / (NW * T);   // chunks
     const int jo = lane & (jp - 1);             // target i + 1 + jo
     const bool active_j = jo < la.nj;
     const double dimj = active_j ? la.dims[la.i + 1 + jo] : 0.0;
     double term_sum = 0.0;                      // this lane's rows of target jo
     double *tp = s_tp[warp];
-    for (int64_t c0 = bid * (NW * T); c0 < M.rows; c0 += nblk * (NW * T)) {
-        const int64_t t0 = c0 + (int64_t)warp * T;
-        const int nrow = t0 >= M.rows ? 0 : M.rows - t0 < (int64_t)T ? (int)(M.rows - t0) : T;
+    for (int64_t c = bid; c < nch; c += nblk) {
+        auto row_at = [&](int p) { return p * nch + c; };   // row of place p of the chunk
+        const int nrow = __popc(__ballot_sync(kFull, lane < T && row_at(warp * T + lane) < M.rows));
         // r_ii of the tile's rows, a lane each (one division for T rows)
         int64_t my_a0 = 0, my_len = 0;
         if (lane < nrow) {
-            const int64_t ul = t0 + lane;
+            const int64_t ul = row_at(warp * T + lane);
             my_a0 = M.rowptr[ul];
             my_len = M.rowptr[ul + 1] - my_a0;
             double r = __ddiv_rn((double)my_len, la.dim_leaf);
@@ -149,7 +161,26 @@ __device__ __forceinline__ void res_level_body(const DevCsr &M, const double *q_
         }
         const bool is_long = skip_long && my_len > kEstLongRow;   // a cluster of k_res_long takes it
         const uint32_t skipped = __ballot_sync(kFull, is_long);
-        const uint32_t wide = __ballot_sync(kFull, !is_long && my_len > wide_min);
+        // wide rows that the CTA's warps multiply together
+        uint32_t wide = __ballot_sync(kFull, !is_long && my_len > wide_min);
+        const bool any_wide = __syncthreads_or(wide != 0);
+        bool uneven = false;
+        if (any_wide) {
+            const uint32_t huge = __ballot_sync(kFull, !is_long && my_len > 16 * wide_min);
+            const int load = __reduce_add_sync(kFull, (wide >> lane) & 1u ? (int)min(my_len, (int64_t)(INT_MAX >> 9)) : 0);
+            if (lane == 0) {
+                s_mask[warp] = make_uint2(wide, huge);
+                s_load[warp] = load;
+            }
+            __syncthreads();
+            int64_t most = 0, all = 0;
+            for (int w = 0; w < NW; w++) {
+                most = s_load[w] > most ? s_load[w] : most;
+                all += s_load[w];
+            }
+            uneven = most * NW > 2 * all;
+            if (!uneven) wide = huge;
+        }
         // the row's groups: 2^e of them, -1 for none (its product is 1, or
         // another part of the kernel's)
         int e = -1;
@@ -213,16 +244,13 @@ __device__ __forceinline__ void res_level_body(const DevCsr &M, const double *q_
             }
             if (live && g == 0 && active_j) tp[t * jp + jo] = prod;
         }
-        // wide rows of the CTA's tiles, in row order: every warp a slice
-        if (__syncthreads_or(wide != 0)) {
-            __shared__ uint32_t s_mask[NW];
-            if (lane == 0) s_mask[warp] = wide;
-            __syncthreads();
+        // their products, warp by warp: every warp a slice
+        if (any_wide) {
             const int G = 32 / jp, wg = lane / jp;
             for (int w = 0; w < NW; w++) {
-                for (uint32_t m = s_mask[w]; m; m &= m - 1) {
+                for (uint32_t m = uneven ? s_mask[w].x : s_mask[w].y; m; m &= m - 1) {
                     const int t = __ffs(m) - 1;
-                    const int64_t u = c0 + (int64_t)w * T + t;
+                    const int64_t u = row_at(w * T + t);
                     const int64_t a0 = M.rowptr[u], len = M.rowptr[u + 1] - a0;
                     const int64_t k0 = a0 + len * warp / NW, k1 = a0 + len * (warp + 1) / NW;
                     double prod = 1.0;
@@ -246,7 +274,7 @@ __device__ __forceinline__ void res_level_body(const DevCsr &M, const double *q_
             for (int t = lane / jp; t < nrow; t += 32 / jp) {
                 if ((skipped >> t) & 1u) continue;
                 const double r = __dsub_rn(1.0, tp[t * jp + jo]);
-                q_cur[(t0 + t) * qs + 1 + jo] = __dsub_rn(1.0, r);
+                q_cur[row_at(warp * T + t) * qs + 1 + jo] = __dsub_rn(1.0, r);
                 term_sum = __dadd_rn(term_sum, __dmul_rn(r, dimj));
             }
         }
@@ -270,34 +298,29 @@ __global__ void __launch_bounds__(kEstThreads, 5) k_res_level(DevCsr M, const do
     res_level_body(M, q_next, q_cur, la, partial, skip_long, blockIdx.x, gridDim.x);
 }
 
-// A cluster of CTAs per long row (rows listed ascending): each of the
-// cluster's warps multiplies the factors of one of as many equal slices of the
-// row, the CTA's warp products are combined in warp order and the CTAs' (read
-// through distributed shared memory) in rank order.  One SM's FP64 pipe takes
-// 110 us for a row of 53,000 entries and five targets; eight take it in turn.
-// The row's terms s * dim_j go to the partial of its place in the list, after
-// the partials of k_res_level, so the reduction still adds them in a fixed
-// order.
+// Long rows (listed ascending): a CTA each, its warps multiplying the factors
+// of one of as many equal slices of the row, combined in warp order; rows of
+// more than kEstSpreadRow entries a cluster of CTAs, whose products (read
+// through distributed shared memory) are combined in rank order.  The row's
+// terms s * dim_j go to the partial of its place in the list, after the
+// partials of k_res_level, so the reduction still adds them in a fixed order.
 constexpr int kEstLongThreads = 256;
 constexpr int kEstLongCluster = 8;
+constexpr int64_t kEstSpreadRow = 8192;
 
-__device__ __forceinline__ void res_long_body(const DevCsr &M, const double *q_next, double *q_cur,
-                                              const LevelArgs &la, const int32_t *long_rows, double *partial,
-                                              int64_t place) {
-    constexpr int NW = kEstLongThreads / 32, NS = NW * kEstLongCluster;
+__device__ __forceinline__ void res_long_row(const DevCsr &M, const double *q_next, double *q_cur, const LevelArgs &la,
+                                             int64_t u, double *partial, int rank, int ranks) {
+    constexpr int NW = kEstLongThreads / 32;
     __shared__ double s_prod[NW][kMaxLen];
     __shared__ double s_cta[kMaxLen];
-    cooperative_groups::cluster_group cluster = cooperative_groups::this_cluster();
-    const int rank = (int)cluster.block_rank();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int G = 32 / la.jp;
     const int g = lane / la.jp;
     const int jo = lane % la.jp;
     const bool active_j = jo < la.nj;
-    const int64_t u = long_rows[place];
     const int64_t a0 = M.rowptr[u], len = M.rowptr[u + 1] - a0;
-    const int slice = rank * NW + warp;
-    const int64_t k0 = a0 + len * slice / NS, k1 = a0 + len * (slice + 1) / NS;
+    const int slice = rank * NW + warp, slices = ranks * NW;
+    const int64_t k0 = a0 + len * slice / slices, k1 = a0 + len * (slice + 1) / slices;
     double prod = 1.0;
     if (active_j) prod = factor_product(M, q_next + jo, la.nj, k0 + g, k1, G);
     for (int d = la.jp; d < 32; d <<= 1) {
@@ -306,25 +329,51 @@ __device__ __forceinline__ void res_long_body(const DevCsr &M, const double *q_n
     }
     if (g == 0 && active_j) s_prod[warp][jo] = prod;
     __syncthreads();
+    double p = 1.0;
     if ((int)threadIdx.x < la.nj) {
-        double p = 1.0;
         for (int w = 0; w < NW; w++) p = __dmul_rn(p, s_prod[w][threadIdx.x]);
         s_cta[threadIdx.x] = p;
     }
-    cluster.sync();
+    if (ranks > 1) {
+        cooperative_groups::cluster_group cluster = cooperative_groups::this_cluster();
+        cluster.sync();
+        if (rank == 0 && (int)threadIdx.x < la.nj)
+            for (int c = 1; c < ranks; c++) p = __dmul_rn(p, cluster.map_shared_rank(s_cta, c)[threadIdx.x]);
+        cluster.sync();   // the products are read: the CTAs may go on
+    }
     if (rank == 0 && (int)threadIdx.x < la.nj) {
-        double p = s_cta[threadIdx.x];
-        for (int c = 1; c < kEstLongCluster; c++) p = __dmul_rn(p, cluster.map_shared_rank(s_cta, c)[threadIdx.x]);
         const double sv = __dsub_rn(1.0, p);
         q_cur[u * (la.nj + 1) + 1 + threadIdx.x] = __dsub_rn(1.0, sv);   // q = 1 - r for the next level
-        partial[place * kMaxLen + threadIdx.x] = __dmul_rn(sv, la.dims[la.i + 1 + threadIdx.x]);
+        partial[threadIdx.x] = __dmul_rn(sv, la.dims[la.i + 1 + threadIdx.x]);
     }
-    cluster.sync();   // the products are read: the CTAs may go
+    __syncthreads();   // s_prod is free
 }
 
+// The rows of places p0 .. p1 - 1 by one cluster: those a CTA takes alone dealt
+// to its CTAs, then those that the cluster takes together.  row(place, ranks,
+// rank) works on one of them; length(place) is its entries.
+template <typename Length, typename Row>
+__device__ __forceinline__ void res_long_rows(int64_t p0, int64_t p1, Length length, Row row) {
+    const int rank = (int)cooperative_groups::this_cluster().block_rank();
+    for (int64_t p = p0 + rank; p < p1; p += kEstLongCluster)
+        if (length(p) <= kEstSpreadRow) row(p, 0, 1);
+    for (int64_t p = p0; p < p1; p++)
+        if (length(p) > kEstSpreadRow) row(p, rank, kEstLongCluster);
+}
+
+// Places a cluster takes: one while the device has room for a cluster each.
+inline int32_t long_places(int64_t nlong, int sm_count) { return nlong <= 2 * sm_count ? 1 : kEstLongCluster; }
+
 __global__ void __cluster_dims__(kEstLongCluster, 1, 1) __launch_bounds__(kEstLongThreads)
-    k_res_long(DevCsr M, const double *q_next, double *q_cur, LevelArgs la, const int32_t *long_rows, double *partial) {
-    res_long_body(M, q_next, q_cur, la, long_rows, partial, blockIdx.x / kEstLongCluster);
+    k_res_long(DevCsr M, const double *q_next, double *q_cur, LevelArgs la, const int32_t *long_rows, int32_t nlong,
+               int32_t places, double *partial) {
+    const int64_t p0 = (int64_t)(blockIdx.x / kEstLongCluster) * places;
+    res_long_rows(
+        p0, min(p0 + places, (int64_t)nlong),
+        [&](int64_t p) { return M.rowptr[long_rows[p] + 1] - M.rowptr[long_rows[p]]; },
+        [&](int64_t p, int rank, int ranks) {
+            res_long_row(M, q_next, q_cur, la, long_rows[p], partial + p * kMaxLen, rank, ranks);
+        });
 }
 
 // One block, target jo: c[i*len + j] = sum over blocks (fixed pairwise order).
@@ -371,10 +420,10 @@ struct LevelJob {
     double *q_cur;
     double *partial;
     double *c;                  // the chain's len x len estimates
-    const int32_t *long_rows;   // rows with a CTA of their own (nlong of them)
+    const int32_t *long_rows;   // rows that k_res_long takes (nlong of them)
     LevelArgs la;
     int64_t first, blocks;      // CTAs of the level launch
-    int64_t lfirst;             // CTAs of the long-row launch: lfirst .. lfirst + nlong - 1
+    int64_t lfirst;             // its places among the long rows of the launch: lfirst .. lfirst + nlong - 1
     int32_t nlong;
 };
 
@@ -395,10 +444,20 @@ __global__ void __launch_bounds__(kEstThreads, 5) k_res_level_multi(const LevelJ
 }
 
 __global__ void __cluster_dims__(kEstLongCluster, 1, 1) __launch_bounds__(kEstLongThreads)
-    k_res_long_multi(const LevelJob *jobs, int32_t njobs) {
-    const int64_t place = blockIdx.x / kEstLongCluster;
-    const LevelJob &jb = jobs[find_job(jobs, njobs, place, true)];
-    res_long_body(jb.M, jb.q_next, jb.q_cur, jb.la, jb.long_rows, jb.partial + jb.blocks * kMaxLen, place - jb.lfirst);
+    k_res_long_multi(const LevelJob *jobs, int32_t njobs, int64_t nlong, int32_t places) {
+    const int64_t p0 = (int64_t)(blockIdx.x / kEstLongCluster) * places;
+    res_long_rows(
+        p0, min(p0 + places, nlong),
+        [&](int64_t p) {
+            const LevelJob &jb = jobs[find_job(jobs, njobs, p, true)];
+            const int64_t u = jb.long_rows[p - jb.lfirst];
+            return jb.M.rowptr[u + 1] - jb.M.rowptr[u];
+        },
+        [&](int64_t p, int rank, int ranks) {
+            const LevelJob &jb = jobs[find_job(jobs, njobs, p, true)];
+            res_long_row(jb.M, jb.q_next, jb.q_cur, jb.la, jb.long_rows[p - jb.lfirst],
+                         jb.partial + (jb.blocks + p - jb.lfirst) * kMaxLen, rank, ranks);
+        });
 }
 
 __global__ void __launch_bounds__(256) k_res_reduce_multi(const LevelJob *jobs) {
@@ -463,8 +522,9 @@ int32_t estimate(rmcm_handle *h, rmcm_mat *const *chain, int32_t len, double *c_
         k_res_level<<<(unsigned)blocks, kEstThreads, 0, s>>>(M, r_next, r_cur, la, lp, nlong > 0);
         h->launches++;
         if (nlong > 0) {
-            k_res_long<<<(unsigned)(nlong * kEstLongCluster), kEstLongThreads, 0, s>>>(M, r_next, r_cur, la, chain[i]->est_long,
-                                                                   lp + (int64_t)blocks * kMaxLen);
+            const int32_t places = long_places(nlong, h->sm_count);
+            k_res_long<<<(unsigned)((nlong + places - 1) / places * kEstLongCluster), kEstLongThreads, 0, s>>>(
+                M, r_next, r_cur, la, chain[i]->est_long, nlong, places, lp + (int64_t)blocks * kMaxLen);
             h->launches++;
         }
         e = cudaGetLastError();
@@ -560,7 +620,9 @@ int32_t estimate_multi(rmcm_handle *h, const EstChain *chains, int32_t n, TableA
         k_res_level_multi<<<(unsigned)nb, kEstThreads, 0, s>>>((const LevelJob *)dp, (int32_t)jobs.size());
         h->launches++;
         if (nl > 0) {
-            k_res_long_multi<<<(unsigned)(nl * kEstLongCluster), kEstLongThreads, 0, s>>>((const LevelJob *)dp, (int32_t)jobs.size());
+            const int32_t places = long_places(nl, h->sm_count);
+            k_res_long_multi<<<(unsigned)((nl + places - 1) / places * kEstLongCluster), kEstLongThreads, 0, s>>>(
+                (const LevelJob *)dp, (int32_t)jobs.size(), nl, places);
             h->launches++;
         }
         if (st > 0) {   // (the first step is every chain's last level: no targets)
