@@ -409,8 +409,18 @@ __device__ __forceinline__ void row_window_products(const DevCsr &A, const V *av
     }
 }
 
+// CTAs an SM should hold: warps cover the gathers' latency, so uint32 rows of a
+// packed B run with 40 to 51 registers (40 to 48 warps; 1.4G multiply-adds
+// through 500 B rows of 1,700 took 778 us at 64 registers and 32 warps, 520 in
+// k_dense at 40).  The other forms would spill.
 template <typename V, int NT, bool PK>
-__global__ void __launch_bounds__(NT, NT == 128 ? 8 : NT == 256 ? 4 : NT == 512 ? 2 : 1)
+constexpr int row_window_ctas() {
+    return sizeof(V) == 4 && PK ? (NT == 128 ? 10 : NT == 256 ? 6 : NT == 512 ? 3 : 1)
+                                : (NT == 128 ? 8 : NT == 256 ? 4 : NT == 512 ? 2 : 1);
+}
+
+template <typename V, int NT, bool PK>
+__global__ void __launch_bounds__(NT, row_window_ctas<V, NT, PK>())
     k_row_window(DevCsr A, const V *aval, RowB<V> B, DevCsr T, const int32_t *rows, int32_t nrows, int64_t tstride,
                  int32_t W, int32_t ncols, int64_t *cnt, const uint8_t *bin_of, const V *S, int64_t gld,
                  const int32_t *lcnt, int32_t *next_row, bool by_row) {
