@@ -3447,19 +3447,31 @@ int32_t launch_bins(rmcm_handle *h, const DevCsr &A, const DevCsr &B, const DevC
                         // kernel takes its front
                         const int32_t *dl = temp->split ? temp->perm : list;
                         const int32_t dn = temp->split ? temp->n_front : n;
+                        // the rows that may overflow run on the second stream (unless split
+                        // rows do), started first: few of them take as long as their
+                        // largest, which then passes beside the others (one such row of
+                        // 467,000 products among 3,000: 862 us after them, 677 so)
+                        const bool risky = dn > 0 && (!lean || !temp->no_risky);
+                        const bool beside = risky && lean && !temp->split;
+                        auto launch_dense = [&](cudaStream_t on) {
+                            kern<<<std::max(1, std::min(grid, dn)), kDenseThreads, sm, on>>>(
+                                Al, B, T, dl, dn, cnt, nullptr, 0, (int32_t)W, st, temp->stride, bin_of, positive,
+                                b_distinct, h->abort_on_certain_overflow, lean != nullptr, temp->by_row,
+                                dense_extra(temp, true));
+                            if (lean) h->launches++;
+                        };
+                        if (beside) {
+                            RMCM_CUDA(h, cudaEventRecord(h->ev_fork, s));
+                            RMCM_CUDA(h, cudaStreamWaitEvent(h->aux, h->ev_fork, 0));
+                            launch_dense(h->aux);
+                        }
                         if (dn > 0 && lean)
                             RMCM_TRY(launch_row_window<V>(h, Al, temp->dpart.S ? (const V *)Al.val : lean->aval,
                                                           lean->B, T, dl, dn, temp->stride, ncols, cnt, bin_of,
                                                           dense_extra(temp, true), temp->next_row, temp->by_row,
                                                           temp->mean_flops));
-                        if (dn > 0 && (!lean || !temp->no_risky)) {
-                            kern<<<std::max(1, std::min(grid, dn)), kDenseThreads, sm, s>>>(
-                                Al, B, T, dl, dn, cnt, nullptr, 0, (int32_t)W, st, temp->stride, bin_of, positive,
-                                b_distinct, h->abort_on_certain_overflow, lean != nullptr, temp->by_row,
-                                dense_extra(temp, true));
-                            if (lean) h->launches++;
-                        }
-                        if (temp->split) {
+                        if (risky && !beside) launch_dense(s);
+                        if (temp->split || beside) {
                             RMCM_CUDA(h, cudaEventRecord(h->ev_join, h->aux));
                             RMCM_CUDA(h, cudaStreamWaitEvent(s, h->ev_join, 0));
                         }
