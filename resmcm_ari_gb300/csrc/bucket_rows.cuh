@@ -1,20 +1,57 @@
 // Rank-bin rows (outputs wider than a dense window, many products) without a
 // bitmap of the whole output: the row's products are partitioned by column
-// range into buckets of about a hundred in shared memory, and a warp sorts and
-// merges each bucket in registers (sort_rows.cuh).  Included by spgemm.cu.
+// range into buckets of about two hundred (up to 330 in the largest rows) in
+// shared memory, and a warp sorts and merges each bucket in registers
+// (sort_rows.cuh).  Included by spgemm.cu.
 #pragma once
 
 constexpr int kBucketBits = 9;        // products a bucket may hold: 512
 constexpr int kBucketMean = 200;      // products a bucket is meant for: a sort of 256 with room for their spread
-constexpr int kBucketPasses = 3;      // fullest passes over the products of the largest row taken
 
 // A CTA of NT threads holds 22 NT products at a time (the SM then takes 1024
 // threads with uint32 counts) and partitions a row into at most NT buckets.
 template <int NT>
 struct BucketCap {
     static constexpr int value = 22 * NT;
-    static constexpr int64_t max_flops = (int64_t)value * kBucketPasses;   // rows of more products are left alone
 };
+
+// The rows a launch of k_bucket takes: more than `over` products, at most
+// `upto`, [1] for rows whose B rows average kWideBucket positions or more, [0]
+// for the others.  Each fill of the buckets is another pass over the row's
+// entries, and the count is one before them.
+struct BucketRange {
+    int64_t over[2], upto[2];
+};
+constexpr int kWideBucket = 32;
+
+// Fills a row may take in a CTA of 128 and of 512 threads, by launch (few:
+// 512 threads only).  Rows beyond are k_rank's, whose cost grows with the
+// output's width instead (its bitmap, one CTA an SM beyond some 500,000
+// columns).  2,000 rows, us, uint32: 8,000 products through B rows of 5, 300,000
+// columns: k_rank 541, one fill of 512 threads 519, three of 128 789; through 40,
+// 200,000 columns: 429, 351, 412.  8,000 rows of 4,000 through 40: k_rank 765,
+// one fill of 512 703, two of 128 592.  16,000 products, two fills of 512: through
+// 5 1,141 (k_rank 959), through 40 641 (688).  uint64 (half the CTAs an SM), 6,000
+// through 20, 300,000 columns: k_rank 344, 512 threads 415, 128 404; a million
+// columns: 546, 422, 410.
+inline BucketRange bucket_range(int nt, bool u64, int64_t cols, bool few) {
+    constexpr int64_t c128 = BucketCap<128>::value, c512 = BucketCap<512>::value;
+    const bool wide_output = !u64 || cols > (1 << 19);
+    BucketRange small{{0, 0}, {c128, c128}};
+    if (wide_output) {
+        small.upto[1] = 2 * c128;
+        if (u64) small.upto[0] = 2 * c128;
+    }
+    if (nt == 128) return small;
+    BucketRange r{{0, 0}, {0, 0}};
+    if (!few) {
+        r.over[0] = small.upto[0];
+        r.over[1] = small.upto[1];
+    }
+    if (wide_output || few) r.upto[0] = r.upto[1] = c512;
+    if (wide_output) r.upto[1] = 3 * c512;
+    return r;
+}
 
 template <typename V, int NT>
 struct BucketShared {
@@ -116,7 +153,7 @@ __device__ __forceinline__ void bucket_stream(const DevCsr &A, const DevCsr &B, 
 template <typename V, int NT>
 __global__ void __launch_bounds__(NT, 1024 / NT) k_bucket(DevCsr A, DevCsr B, bool a_ones, bool b_ones, DevCsr C,
                                                            const int32_t *rows, int32_t nrows, const int64_t *flops,
-                                                           int64_t min_flops, int64_t *cnt, int *st,
+                                                           BucketRange take, int64_t *cnt, int *st,
                                                            uint8_t *bin_of, int32_t *next_row) {
     constexpr int NW = NT / 32, CAP = BucketCap<NT>::value;
     extern __shared__ __align__(16) unsigned char smem[];
@@ -135,12 +172,13 @@ __global__ void __launch_bounds__(NT, 1024 / NT) k_bucket(DevCsr A, DevCsr B, bo
         const uint8_t flags = bin_of[r];
         __syncthreads();   // the row before is done with the shared words
         if (tid == 0) sh.row = (int32_t)gridDim.x + atomicAdd(next_row, 1);
-        if (f <= min_flops || f > BucketCap<NT>::max_flops) {
+        const int64_t a0 = A.rowptr[r], a1 = A.rowptr[r + 1];
+        const bool wide = f >= kWideBucket * (a1 - a0);
+        if (f <= (wide ? take.over[1] : take.over[0]) || f > (wide ? take.upto[1] : take.upto[0])) {
             __syncthreads();
             ri = sh.row;
             continue;
         }
-        const int64_t a0 = A.rowptr[r], a1 = A.rowptr[r + 1];
         // bucket of column c: c * nb / columns, in 32-bit fixed point
         const int nb = (int)min((int64_t)NT, (f + kBucketMean - 1) / kBucketMean);
         const uint64_t scale = ((uint64_t)nb << 32) / (uint64_t)B.cols;

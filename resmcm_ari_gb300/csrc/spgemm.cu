@@ -3122,7 +3122,11 @@ struct RankSplit {
 // place of 1,012, T-I-C-I-T at a twentieth 515 in place of 479, the larger
 // chains the same.
 constexpr int64_t kSplitMinFlops = 1 << 17;
-constexpr int64_t kSplitMinRank = BucketCap<512>::max_flops;   // rank rows that k_bucket does not take
+// Rank rows: three fills of the largest bucket CTA.  A split also costs the
+// other rank rows their single pass; with one row of 36,000 to 150,000 products
+// beside 2,000 of 8,000 it still gains: 519 to 1,356 us without, 417 to 788 with
+// it.
+constexpr int64_t kSplitMinRank = 3 * BucketCap<512>::value;
 constexpr int64_t kSplitMinLight = 1 << 18;   // light products of rows beside a tensor-core part
 
 // A rows with more entries than this are analysed by the whole grid: twice the
@@ -3165,17 +3169,17 @@ int32_t launch_sort(rmcm_handle *h, const DevCsr &A, const DevCsr &B, bool a_one
     return RMCM_OK;
 }
 
-// Rank-bin rows of min_flops + 1 .. BucketCap<NT>::max_flops products.
+// The rank-bin rows that bucket_range gives to CTAs of NT threads.
 template <typename V, int NT>
 int32_t launch_bucket(rmcm_handle *h, const DevCsr &A, const DevCsr &B, bool a_ones, bool b_ones, const DevCsr &C,
-                      const int32_t *rows, int32_t n, const DenseTemp *temp, int64_t min_flops, int64_t *cnt,
+                      const int32_t *rows, int32_t n, const DenseTemp *temp, const BucketRange &take, int64_t *cnt,
                       const uint8_t *bin_of, int which) {
     auto kern = k_bucket<V, NT>;
     const int64_t sm = (int64_t)sizeof(BucketShared<V, NT>);
     RMCM_TRY(set_smem(h, kern, sm));
     const int per_sm = std::max(1, occupancy(h, kern, NT, sm));
     kern<<<std::min(n, h->sm_count * per_sm), NT, sm, h->stream>>>(A, B, a_ones, b_ones, C, rows, n, temp->row_flops,
-                                                                   min_flops, cnt, h->d_status,
+                                                                   take, cnt, h->d_status,
                                                                    const_cast<uint8_t *>(bin_of),
                                                                    temp->bucket_rows + which);
     h->launches++;
@@ -3381,11 +3385,12 @@ int32_t launch_bins(rmcm_handle *h, const DevCsr &A, const DevCsr &B, const DevC
                     // no more rows than the device holds CTAs of 512 threads at once (two an
                     // SM): a row's time is the product's, so all of them take 512 threads
                     const bool few = rn <= 2 * h->sm_count;
+                    const BucketRange r128 = bucket_range(128, sizeof(V) == 8, ncols, few);
+                    const BucketRange r512 = bucket_range(512, sizeof(V) == 8, ncols, few);
                     if (!few)
-                        RMCM_TRY((launch_bucket<V, 128>(h, A, B, a_ones, b_ones, C, rl, rn, temp, 0, cnt, bin_of, 0)));
-                    if (few || temp->max_rank_flops > BucketCap<128>::max_flops)
-                        RMCM_TRY((launch_bucket<V, 512>(h, A, B, a_ones, b_ones, C, rl, rn, temp,
-                                                        few ? 0 : BucketCap<128>::max_flops, cnt, bin_of, 1)));
+                        RMCM_TRY((launch_bucket<V, 128>(h, A, B, a_ones, b_ones, C, rl, rn, temp, r128, cnt, bin_of, 0)));
+                    if (r512.upto[1] > 0 && temp->max_rank_flops > r512.over[0])
+                        RMCM_TRY((launch_bucket<V, 512>(h, A, B, a_ones, b_ones, C, rl, rn, temp, r512, cnt, bin_of, 1)));
                 }
                 if (rn > 0)
                     kern<<<std::max(1, std::min(grid, rn)), kRankThreads, sm, s>>>(A, B, C, rl, rn, cnt, st, bin_of);
