@@ -21,6 +21,7 @@ struct BucketCap {
 // entries, and the count is one before them.
 struct BucketRange {
     int64_t over[2], upto[2];
+    int32_t least2;   // only rows whose B rows average least2 / 2 positions or more
 };
 constexpr int kWideBucket = 32;
 
@@ -33,17 +34,19 @@ constexpr int kWideBucket = 32;
 // one fill of 512 703, two of 128 592.  16,000 products, two fills of 512: through
 // 5 1,141 (k_rank 959), through 40 641 (688).  uint64 (half the CTAs an SM), 6,000
 // through 20, 300,000 columns: k_rank 344, 512 threads 415, 128 404; a million
-// columns: 546, 422, 410.
+// columns: 546, 422, 410.  Through B rows of one position the entries cost more than
+// the products: 3,000 rows of 2,500 on 60,000 columns 641 against 556, uint64 811
+// against 592 (and through two 508 against 467), on a million 652 against 975.
 inline BucketRange bucket_range(int nt, bool u64, int64_t cols, bool few) {
     constexpr int64_t c128 = BucketCap<128>::value, c512 = BucketCap<512>::value;
     const bool wide_output = !u64 || cols > (1 << 19);
-    BucketRange small{{0, 0}, {c128, c128}};
+    BucketRange small{{0, 0}, {c128, c128}, cols > (1 << 19) ? 0 : u64 && cols <= (1 << 17) ? 6 : 3};
     if (wide_output) {
         small.upto[1] = 2 * c128;
         if (u64) small.upto[0] = 2 * c128;
     }
     if (nt == 128) return small;
-    BucketRange r{{0, 0}, {0, 0}};
+    BucketRange r{{0, 0}, {0, 0}, small.least2};
     if (!few) {
         r.over[0] = small.upto[0];
         r.over[1] = small.upto[1];
@@ -174,7 +177,8 @@ __global__ void __launch_bounds__(NT, 1024 / NT) k_bucket(DevCsr A, DevCsr B, bo
         if (tid == 0) sh.row = (int32_t)gridDim.x + atomicAdd(next_row, 1);
         const int64_t a0 = A.rowptr[r], a1 = A.rowptr[r + 1];
         const bool wide = f >= kWideBucket * (a1 - a0);
-        if (f <= (wide ? take.over[1] : take.over[0]) || f > (wide ? take.upto[1] : take.upto[0])) {
+        if (f <= (wide ? take.over[1] : take.over[0]) || f > (wide ? take.upto[1] : take.upto[0]) ||
+            2 * f < take.least2 * (a1 - a0)) {
             __syncthreads();
             ri = sh.row;
             continue;

@@ -59,3 +59,22 @@ def test_rows_up_to_two_an_sm(native, engine, more, vt):
         assert engine.product_stats()[-1]["bin_rows"][RANK] == rows
     finally:
         engine.set_profiling(0)
+
+
+@pytest.mark.parametrize("vt", ["VAL_U32", "VAL_U64"])
+@pytest.mark.parametrize("n", [70_001, 2 ** 17, 2 ** 17 + 1, 2 ** 19, 2 ** 19 + 1])
+@pytest.mark.parametrize("rows", [90, 400])
+def test_rows_through_short_rows_of_b(native, engine, rows, n, vt):
+    """B rows of 1, 1.5, 2 and 3 positions on average, some rows taken and some
+    left in one product."""
+    rng = np.random.default_rng(n)
+    per = np.repeat([1, 2, 3], 1300)
+    rp = np.concatenate([[0], np.cumsum(per)])
+    third = n // 3                               # one column of each third
+    col = np.concatenate([np.arange(x) for x in per]) * third + rng.integers(0, third, rp[-1])
+    B = sp.csr_matrix((rng.integers(1, 30, col.size, dtype=np.uint64), col, rp), shape=(per.size, n))
+    first = [0, 650, 1300, 2600]                 # 1,300 rows of B from here: 1, 1.5, 2 and 3 positions
+    picks = [first[r % 4] + np.sort(rng.permutation(1300)[: 1100 + r // 2]) for r in range(rows)]
+    ap = np.concatenate([[0], np.cumsum([p.size for p in picks])])
+    A = sp.csr_matrix((rng.integers(1, 30, ap[-1], dtype=np.uint64), np.concatenate(picks), ap), shape=(rows, per.size))
+    check_product(native, engine, A, B, getattr(native, vt))
