@@ -529,7 +529,7 @@ bool gather_smem(rmcm_handle *h, F *kernel, int64_t bytes) {
 // Heavy inner indices of C = A B: sampled column counts of A and the density
 // rule give each heavy index a slot (k_heavy_select).  With stats64 also the
 // largest number of heavy entries in a row of A and the largest heavy value
-// (k_heavy_stats64).  On success hs.sel holds the buffers (the caller frees
+// (k_heavy_stats).  On success hs.sel holds the buffers (the caller frees
 // it); nh < 64 means the caller gives up.
 struct HeavySet {
     char *sel = nullptr;
@@ -902,7 +902,7 @@ int32_t build_limbs(rmcm_handle *h, const DevCsr &A, const DevCsr &B, uint64_t b
     if (ev_end) cudaEventRecord(ev_end, s);
     if (light_flops || sizeof(V) == 4) {
         // light products (stats[5], stats[6]) and, for uint32, the largest
-        // B value the gather saw (stats[2]: bmax came from the row scan)
+        // B value the gather saw (stats[2]: bmax came from the row records)
         RMCM_CUDA(h, cudaMemcpyAsync(h->h_pinned + 8, stats, 7 * sizeof(uint64_t), cudaMemcpyDeviceToHost, s));
         RMCM_CUDA(h, cudaStreamSynchronize(s));
         const uint64_t *st = (const uint64_t *)(h->h_pinned + 8);
@@ -939,7 +939,7 @@ int32_t dense_part_build64(rmcm_handle *h, const DevCsr &A, int64_t a_max_row, c
     if (inv_density <= 0 || A.rows == 0 || B.cols == 0 || A.cols == 0) return RMCM_OK;
     HeavySet hs;
     RMCM_TRY(select_heavy(h, A, B, a_max_row, true, hs));
-    // B's largest value (row sums' last slot; 1 for a matrix of ones)
+    // B's largest value (after its row records; 1 for a matrix of ones)
     uint64_t bmax = 1;
     if (B.vmax) {
         RMCM_CUDA(h, cudaMemcpyAsync(h->h_pinned + 24, B.vmax, 8, cudaMemcpyDeviceToHost, h->stream));

@@ -116,7 +116,7 @@ __device__ __forceinline__ int sort_merge(uint32_t *key, V *val, int n, int lane
 // where their columns come out.  Against a CTA with a hash table, whose barriers and shared-memory
 // sort these rows took before: 52,860 rows of 68 products on 131,071 columns
 // 355 -> 71 us, 25,195 uint64 rows of 120 258 -> 57 us; up to 1,024 products
-// 581 -> 440 us (a wave of 64 chains).
+// 581 -> 330 us (a wave of 64 chains).
 template <typename V, int BITS>
 __device__ __forceinline__ void sort_rows(const DevCsr &A, const DevCsr &B, bool a_ones, bool b_ones, const DevCsr &C,
                                           const int32_t *rows, int32_t nrows, int64_t *cnt, int *st,
